@@ -36,7 +36,7 @@ def build(quiet: bool = True) -> None:
     out = subprocess.DEVNULL if quiet else None
     subprocess.run(["make", "-s", "-C", HERE], check=True, stdout=out)
     ref_tree = os.environ.get("REFERENCE", "/root/reference")
-    if os.path.isdir(ref_tree):
+    if os.path.isdir(ref_tree) and os.listdir(ref_tree):  # an empty folder is no tree
         subprocess.run(["make", "-s", "-C", HERE, "ref", f"REFERENCE={ref_tree}"], check=True, stdout=out)
 
 
