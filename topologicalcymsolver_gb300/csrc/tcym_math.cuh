@@ -156,13 +156,58 @@ TCYM_HD void half_angle(double d2, double &f, double &co) {
     Real<double>::sincos_(0.5 * d, &s, &co);
     f = s / d;
 }
-TCYM_HD void half_angle(f2 d2, f2 &f, f2 &co) {  // no packed sine: lane by lane
-    half_angle(d2.v.x, f.v.x, co.v.x);
-    half_angle(d2.v.y, f.v.y, co.v.y);
+// f as half_angle and cm1 = cos(d/2) - 1 = -sin^2(d/2) / (1 + cos(d/2)), without cancellation
+template <class T> TCYM_HD void half_angle_general(T d2, T &f, T &cm1) {
+    T co;
+    half_angle(d2, f, co);
+    cm1 = -(f * f * d2) / (T(1) + co);
 }
-TCYM_HD float quot(float a, float b) { return a / b; }
-TCYM_HD double quot(double a, double b) { return a / b; }
-TCYM_HD f2 quot(f2 a, f2 b) { return f2(a.v.x / b.v.x, a.v.y / b.v.y); }
+// The same from the Taylor series in y = (d/2)^2 of sin(sqrt y)/sqrt y and
+// cos(sqrt y) - 1, without a root, a sine or a division: y <= 1/16 (a link update's
+// exponent is dt |E|, a few hundredths), the first omitted terms below half an ulp
+// (FP32: y^4/9! = 4e-11 of f, y^5/10! = 3e-13 beside y/2; FP64: y^8/17! and y^9/18!
+// below 1e-24).  Larger exponents take the general form.
+TCYM_HD void half_angle_m1(double d2, double &f, double &cm1) {
+    const double y = 0.25 * d2;
+    if (!(y <= 0.0625)) { half_angle_general(d2, f, cm1); return; }
+    double s = -1.0 / 1307674368000.0;
+    s = fma(s, y, 1.0 / 6227020800.0);
+    s = fma(s, y, -1.0 / 39916800.0);
+    s = fma(s, y, 1.0 / 362880.0);
+    s = fma(s, y, -1.0 / 5040.0);
+    s = fma(s, y, 1.0 / 120.0);
+    s = fma(s, y, -1.0 / 6.0);
+    f = fma(0.5 * s, y, 0.5);
+    double c = 1.0 / 20922789888000.0;
+    c = fma(c, y, -1.0 / 87178291200.0);
+    c = fma(c, y, 1.0 / 479001600.0);
+    c = fma(c, y, -1.0 / 3628800.0);
+    c = fma(c, y, 1.0 / 40320.0);
+    c = fma(c, y, -1.0 / 720.0);
+    c = fma(c, y, 1.0 / 24.0);
+    cm1 = y * fma(c, y, -0.5);
+}
+template <class T> TCYM_HD void half_angle_m1_series(T d2, T &f, T &cm1) {
+    const T y = T(0.25) * d2;
+    T s = fma(T(-1.0 / 5040.0), y, T(1.0 / 120.0));
+    s = fma(s, y, T(-1.0 / 6.0));
+    f = fma(T(0.5) * s, y, T(0.5));
+    T c = fma(T(1.0 / 40320.0), y, T(-1.0 / 720.0));
+    c = fma(c, y, T(1.0 / 24.0));
+    cm1 = y * fma(c, y, T(-0.5));
+}
+TCYM_HD void half_angle_m1(float d2, float &f, float &cm1) {
+    if (d2 <= 0.25f) half_angle_m1_series(d2, f, cm1);
+    else half_angle_general(d2, f, cm1);
+}
+TCYM_HD void half_angle_m1(f2 d2, f2 &f, f2 &cm1) {
+    if (d2.v.x <= 0.25f && d2.v.y <= 0.25f) {
+        half_angle_m1_series(d2, f, cm1);
+    } else {  // no packed sine: lane by lane, each by its own size
+        half_angle_m1(d2.v.x, f.v.x, cm1.v.x);
+        half_angle_m1(d2.v.y, f.v.y, cm1.v.y);
+    }
+}
 
 template <class T> struct cx {
     T re, im;
@@ -228,9 +273,8 @@ template <class T> struct SU2 {
     static TCYM_HD Mat iexp_mul(T c, const T *e, const Mat &u) {
         const T x0 = c * e[0], x1 = c * e[1], x2 = c * e[2];
         const T d2 = fma(x0, x0, fma(x1, x1, x2 * x2));
-        T f, co;
-        half_angle(d2, f, co);
-        const T cm1 = -quot(f * f * d2, T(1) + co);
+        T f, cm1;
+        half_angle_m1(d2, f, cm1);
         const Mat w = mul(Mat{{f * x0, f * x1, f * x2, cm1}}, u);
         return Mat{{u.q[0] + w.q[0], u.q[1] + w.q[1], u.q[2] + w.q[2], u.q[3] + w.q[3]}};
     }
@@ -533,54 +577,58 @@ template <class T> struct SU3 {
     // norm the same way and carry a long FP32 gradient flow off the group.
     // Otherwise the scaled-and-squared exponential is used.
     static TCYM_HD Mat iexp_mul(T c, const T *e, const Mat &u) {
-        const Mat q = algebra_matrix(c, e);
+        // Q = c e^a t^a, Hermitian and traceless, by its real diagonal and the entries
+        // above it; every product with a real or a repeated entry is formed once
+        const T is3 = T(0.57735026918962576450914878050196);
+        const T h = T(0.5) * c;
+        const T e7 = is3 * e[7];
+        const T d0 = h * (e7 + e[2]), d1 = h * (e7 - e[2]), d2 = -(c * e7);
+        const cx<T> q01{h * e[0], -(h * e[1])}, q02{h * e[3], -(h * e[4])}, q12{h * e[5], -(h * e[6])};
         // c1 = tr(Q^2)/2 = sum_ij |Q_ij|^2 / 2
-        const T d0 = q.m[0][0].re, d1 = q.m[1][1].re, d2 = q.m[2][2].re;
-        const T o01 = q.m[0][1].re * q.m[0][1].re + q.m[0][1].im * q.m[0][1].im;
-        const T o02 = q.m[0][2].re * q.m[0][2].re + q.m[0][2].im * q.m[0][2].im;
-        const T o12 = q.m[1][2].re * q.m[1][2].re + q.m[1][2].im * q.m[1][2].im;
-        const T c1 = T(0.5) * (d0 * d0 + d1 * d1 + d2 * d2) + (o01 + o02 + o12);
+        const T o01 = fma(q01.re, q01.re, q01.im * q01.im);
+        const T o02 = fma(q02.re, q02.re, q02.im * q02.im);
+        const T o12 = fma(q12.re, q12.re, q12.im * q12.im);
+        const T c1 = fma(T(0.5), fma(d0, d0, fma(d1, d1, d2 * d2)), o01 + o02 + o12);
         if (any_gt(c1 * T(4.0 / 3.0), T(0.25))) {
             if constexpr (Packed<T>::value) return iexp_mul_lanes(c, e, u);
-            else return mulu<false, false>(iexp_hermitian(q), u);
+            else return mulu<false, false>(iexp_hermitian(algebra_matrix(c, e)), u);
         }
-        // rows 0 and 1 of Q^2 (Hermitian Q)
-        cx<T> q2[2][3];
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = i; j < 3; ++j) {
-                cx<T> acc{T(0), T(0)};
-#pragma unroll
-                for (int k = 0; k < 3; ++k) acc = cfma(q.m[i][k], q.m[k][j], acc);
-                q2[i][j] = acc;
-            }
-        q2[1][0] = conj(q2[0][1]);
-        // c0 = det Q (real for Hermitian Q)
-        const T c0 = d0 * (d1 * d2 - o12) - d1 * o02 - d2 * o01 +
-                     T(2) * (q.m[0][1].re * (q.m[1][2].re * q.m[2][0].re - q.m[1][2].im * q.m[2][0].im) -
-                             q.m[0][1].im * (q.m[1][2].re * q.m[2][0].im + q.m[1][2].im * q.m[2][0].re));
+        // Q^2, with q_ii + q_jj = -q_kk
+        const T s00 = fma(d0, d0, o01 + o02), s11 = fma(d1, d1, o01 + o12);
+        const cx<T> s01 = cfma_nc(q02, q12, cx<T>{-(d2 * q01.re), -(d2 * q01.im)});
+        const cx<T> s02 = cfma(q01, q12, cx<T>{-(d1 * q02.re), -(d1 * q02.im)});
+        const cx<T> s12 = cfma_cn(q01, q02, cx<T>{-(d0 * q12.re), -(d0 * q12.im)});
+        // c0 = det Q = d0 d1 d2 - d0 |q12|^2 - d1 |q02|^2 - d2 |q01|^2 + 2 Re(q01 q12 conj(q02))
+        const T tr = fma(q01.re, fma(q12.re, q02.re, q12.im * q02.im), q01.im * fma(q12.re, q02.im, -(q12.im * q02.re)));
+        const T c0 = fma(d0, fma(d1, d2, -o12), fma(-d1, o02, fma(-d2, o01, T(2) * tr)));
         T f0r, f0i, f1r, f1i, f2r, f2i;
         if constexpr (kSingle) {
-            // terms of the series by the spectral radius r (r^2 <= 4 c1 / 3): the first
-            // omitted term r^(N+1)/(N+1)! stays below half an FP32 ulp, 3e-8, with 5
-            // terms for r^2 <= 0.02 (the common case: |dt E| is small) and 8 up to r = 1/2
-            if (any_gt(c1 * T(4.0 / 3.0), T(0.02))) series_coeffs<8, true>(c0, c1, f0r, f0i, f1r, f1i, f2r, f2i);
-            else series_coeffs<5, true>(c0, c1, f0r, f0i, f1r, f1i, f2r, f2i);
+            // eight terms for r <= 1/2 (the first omitted one, r^9/9!, is 5e-9), Q^n reduced by
+            // hand: Q^3 = c1 Q + c0, ..., Q^8 = (c1^3 + c0^2) Q^2 + 3 c0 c1^2 Q + 2 c0^2 c1
+            const T k = c0 * c0;
+            f0r = k * fma(c1, T(1.0 / 20160), T(-1.0 / 720));
+            f0i = c0 * fma(c1, fma(c1, T(-1.0 / 5040), T(1.0 / 120)), T(-1.0 / 6));
+            f1r = c0 * fma(c1, fma(c1, T(1.0 / 13440), T(-1.0 / 360)), T(1.0 / 24));
+            f1i = fma(c1, fma(c1, fma(c1, T(-1.0 / 5040), T(1.0 / 120)), T(-1.0 / 6)), fma(k, T(-1.0 / 5040), T(1)));
+            f2r = fma(c1, fma(c1, fma(c1, T(1.0 / 40320), T(-1.0 / 720)), T(1.0 / 24)), fma(k, T(1.0 / 40320), T(-0.5)));
+            f2i = c0 * fma(c1, T(-1.0 / 2520), T(1.0 / 120));
         } else {
-            series_coeffs<16, true>(c0, c1, f0r, f0i, f1r, f1i, f2r, f2i);
+            // r^2 <= 0.02 (a link update's |dt E|): 10 terms, the first omitted one 1e-17
+            if (any_gt(c1 * T(4.0 / 3.0), T(0.02))) series_coeffs<16, true>(c0, c1, f0r, f0i, f1r, f1i, f2r, f2i);
+            else series_coeffs<10, true>(c0, c1, f0r, f0i, f1r, f1i, f2r, f2i);
         }
-        Mat w;  // rows 0 and 1 of exp(iQ) - 1
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const cx<T> x = q.m[i][j], y = q2[i][j];
-                T re = fma(f1r, x.re, fma(-f1i, x.im, fma(f2r, y.re, -f2i * y.im)));
-                T im = fma(f1r, x.im, fma(f1i, x.re, fma(f2r, y.im, f2i * y.re)));
-                if (i == j) { re += f0r; im += f0i; }
-                w.m[i][j] = cx<T>{re, im};
-            }
+        // rows 0 and 1 of exp(iQ) - 1 = (f0 - 1) + f1 Q + f2 Q^2
+        auto mix = [&](cx<T> x, cx<T> y) {
+            return cx<T>{fma(f1r, x.re, fma(-f1i, x.im, fma(f2r, y.re, -(f2i * y.im)))),
+                         fma(f1r, x.im, fma(f1i, x.re, fma(f2r, y.im, f2i * y.re)))};
+        };
+        Mat w;
+        w.m[0][0] = cx<T>{fma(f1r, d0, fma(f2r, s00, f0r)), fma(f1i, d0, fma(f2i, s00, f0i))};
+        w.m[1][1] = cx<T>{fma(f1r, d1, fma(f2r, s11, f0r)), fma(f1i, d1, fma(f2i, s11, f0i))};
+        w.m[0][1] = mix(q01, s01);
+        w.m[1][0] = mix(conj(q01), conj(s01));
+        w.m[0][2] = mix(q02, s02);
+        w.m[1][2] = mix(q12, s12);
         return mulu_inc(w, u);  // reads rows 0 and 1 of w only
     }
     // rows 0 and 1 of u + w u (each accumulator starts at u's entry), row 2 rebuilt
