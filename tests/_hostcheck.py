@@ -34,6 +34,7 @@ def load():
         L.hc_edotb_pair.argtypes = [ctypes.c_int, ip, _vp, _vp, _vp]
         L.hc_gauss_restore.argtypes = [ctypes.c_int, ip, _vp, _vp, ctypes.c_double, ctypes.c_int]
         L.hc_reunitarize.argtypes = [ctypes.c_int, ip, _vp]
+        L.hc_reunitarize_fp64.argtypes = [ctypes.c_int, ip, _vp]
         L.hc_block.argtypes = [ctypes.c_int, ip, _vp, _vp]
         L.hc_from_aos_range.argtypes = [ctypes.c_int, ip, _vp, _vp, _vp, _vp, ctypes.c_int64, ctypes.c_int64]
         L.hc_step_range.argtypes = [ctypes.c_int, ip, _vp, _vp, _vp, ctypes.c_double, ctypes.c_int64, ctypes.c_int64]
@@ -121,6 +122,10 @@ class HostLattice:
 
     def reunitarize(self):
         self.L.hc_reunitarize(self.fmt, self.n, _p(self.U[self.cur]))
+
+    def reunitarize_fp64(self):
+        """The projection in FP64 arithmetic, whatever the storage."""
+        self.L.hc_reunitarize_fp64(self.fmt, self.n, _p(self.U[self.cur]))
 
     def poison(self):
         """Every stored value NaN (so that reading anything not written since shows)."""

@@ -189,6 +189,18 @@ template <int FMT> struct H {
     static void geodesic(const Geom &g, const void *Uold, const void *Unew, double c, void *Umid, void *Emid) {
         for (int64_t s = 0; s < g.V; ++s) site_geodesic<F>(g, Uold, Unew, c, Umid, Emid, s);
     }
+    static void reunitarize(const Geom &g, void *U) {
+        if constexpr (F::PAIRED) {
+            for (int64_t p = 0; p < pair_sites(g.V); ++p)
+                for (int mu = 0; mu < 3; ++mu) pair_reunitarize<F>(U, g.V, mu, p);
+        } else {
+            for (int64_t s = 0; s < g.V; ++s) site_reunitarize<F>(g, U, s);
+        }
+    }
+    // the FP64 projection whatever the storage
+    static void reunitarize_fp64(const Geom &g, void *U) {
+        for (int64_t s = 0; s < g.V; ++s) site_reunitarize<F>(g, U, s);
+    }
     static int gauss_restore(const Geom &g, const void *U, void *E, double tol, int maxit) {
         std::vector<double> G((size_t)F::NA * g.V);
         const double gam[3] = {7.0 / 24.0, 7.0 / 48.0, 7.0 / 72.0};
@@ -286,7 +298,12 @@ int hc_gauss_restore(int fmt, const int *n, const void *U, void *E, double tol, 
 }
 int hc_reunitarize(int fmt, const int *n, void *U) {
     Geom g = geom(n);
-    HC_DISPATCH(fmt, for (int64_t s = 0; s < g.V; ++s) site_reunitarize<HH::F>(g, U, s));
+    HC_DISPATCH(fmt, HH::reunitarize(g, U));
+    return 0;
+}
+int hc_reunitarize_fp64(int fmt, const int *n, void *U) {
+    Geom g = geom(n);
+    HC_DISPATCH(fmt, HH::reunitarize_fp64(g, U));
     return 0;
 }
 // Block of the links of extents n into Ub (extents n / 2, the same format)

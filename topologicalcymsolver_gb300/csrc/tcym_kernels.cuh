@@ -430,6 +430,11 @@ template <int FMT> __global__ void k_reunitarize(Geom g, void *U) {
     int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s < g.V) site_reunitarize<Fmt<FMT>>(g, U, s);
 }
+// FP32 storage: one thread per pair and direction (blockIdx.y)
+template <int FMT> __global__ void __launch_bounds__(128) k_reunitarize_pair(Geom g, void *U) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < pair_sites(g.V)) pair_reunitarize<Fmt<FMT>>(U, g.V, blockIdx.y, p);
+}
 template <int FMT>
 __global__ void k_geodesic(Geom g, const void *Uold, const void *Unew, double c, void *Umid, void *Emid) {
     int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -607,7 +612,10 @@ template <int FMT> struct Launch {
         return cudaGetLastError();
     }
     static cudaError_t reunitarize(const Geom &g, void *U, cudaStream_t st) {
-        k_reunitarize<FMT><<<grid_for(g.V, 128), 128, 0, st>>>(g, U);
+        if constexpr (F::PAIRED)
+            k_reunitarize_pair<FMT><<<dim3((unsigned)grid_for(pair_sites(g.V), 128), 3), 128, 0, st>>>(g, U);
+        else
+            k_reunitarize<FMT><<<grid_for(g.V, 128), 128, 0, st>>>(g, U);
         return cudaGetLastError();
     }
     // sites [s0, s0 + n) (n < 0: all)
