@@ -499,15 +499,12 @@ extern "C" int tcym_random_links(tcym_lattice lat, double sigma, uint64_t seed) 
     return TCYM_OK;
 }
 
-// Runs the observables reduction with `mask` and the finaliser; result on device.
+// Runs the observables reduction with `mask`; result on device.
 int tcym_reduce(tcym_lattice lat, int mask, double ncs_dt) {
     tcym_ctx ctx = lat->ctx;
-    int blocks = 0;
-    DISPATCH(lat->fmt, {
-        blocks = L::reduce_grid(lat->g, lat->max_blocks);
-        CK(L::observables(lat->g, lat->U[lat->cur], lat->E, mask, lat->partial, blocks, lat->stream));
-    });
-    CK(finalize_obs(lat->partial, blocks, lat->nc == 2 ? 3 : 8, lat->g.V, ncs_dt, lat->result, lat->stream));
+    const Finish fin = make_finish(lat->result, lat->nc == 2 ? 3 : 8, lat->g.V, ncs_dt);
+    DISPATCH(lat->fmt, CK(L::observables(lat->g, lat->U[lat->cur], lat->E, mask, lat->partial, lat->max_blocks, fin,
+                                         lat->stream)));
     return TCYM_OK;
 }
 
@@ -521,7 +518,7 @@ static int fetch_result(tcym_lattice lat) {
 // GaussLawRestoration::Restore (GAUSSLAWFIXING/GaussRestore.cpp:131-167).  Each
 // iteration is three (deviation, update) sub-steps; the reference stops once the
 // signed maximum of the third deviation is <= tol (GaussRestore.cpp:150).  The
-// iterations are queued in growing batches between host checks: the finaliser of
+// iterations are queued in growing batches between host checks: the last block of
 // the deciding deviation writes the stopping iteration into the device control
 // block, and the kernels of later iterations return at once, so the result, the
 // iteration count and the final maximum are those of the reference's loop, with
@@ -537,15 +534,13 @@ extern "C" int tcym_gauss_restore(tcym_lattice lat, double tol, int maxit, int *
     if (!lat->gauss) CK(tcym_lattice_alloc(lat, (void **)&lat->gauss, sizeof(double) * gauss_scratch_doubles(lat)));
     double *ctl = lat->gauss + (size_t)na * (size_t)lat->g.V;
     const double gam[3] = {7.0 / 24.0, 7.0 / 48.0, 7.0 / 72.0};
-    int blocks = 0;
-    DISPATCH(lat->fmt, blocks = L::reduce_grid(lat->g, lat->max_blocks));
     CK(cudaMemsetAsync(lat->result + R_NONFINITE, 0, sizeof(double), lat->stream));
     const double init[4] = {(double)maxit, 0.0, 0.0, 0.0};
     CK(cudaMemcpyAsync(ctl, init, sizeof(init), cudaMemcpyHostToDevice, lat->stream));
     auto deviation = [&](int it, bool check) -> int {
-        DISPATCH(lat->fmt, CK(L::gauss_compute_it(lat->g, lat->U[lat->cur], lat->E, lat->gauss, lat->partial, blocks,
-                                                  ctl, it, lat->stream)));
-        CK(finalize_restore(lat->partial, blocks, na, lat->g.V, lat->result, ctl, tol, it, check, lat->stream));
+        const Finish fin = make_finish(lat->result, na, lat->g.V, 0.0, ctl, tol, it, check);
+        DISPATCH(lat->fmt, CK(L::gauss_compute_it(lat->g, lat->U[lat->cur], lat->E, lat->gauss, lat->partial,
+                                                  lat->max_blocks, fin, lat->stream)));
         return TCYM_OK;
     };
     // initial deviation (GaussRestore.cpp:143)

@@ -128,7 +128,7 @@ template <int FMT> static void fill_group(tcym_ensemble ens, FmtGroup &G, int sm
         G.classes.back().m1 = (int)i + 1;
         G.classes.back().item1 = blk;
         m.red_begin = red;
-        m.red_blocks = grid_for(L->g.V, kRedThreads);
+        m.red_blocks = member_records(m.paired, L->g.V);
         red += m.red_blocks;
         m.ncs_dt = 0.0;
     }
@@ -499,12 +499,12 @@ extern "C" int tcym_ensemble_step(tcym_ensemble ens, int nsteps) {
     return TCYM_OK;
 }
 
-template <int FMT> static cudaError_t launch_group_obs(tcym_ensemble ens, int f, int mask) {
+template <int FMT> static cudaError_t launch_group_sample(tcym_ensemble ens, int f) {
     using T = typename Fmt<FMT>::T;
     const FmtGroup &G = ens->groups[f];
     if (G.idx.empty()) return cudaSuccess;
-    return LaunchBatch<FMT>::observables(static_cast<const Member<T> *>(G.d_members), (int)G.idx.size(), G.red_total,
-                                         mask, ens->partial + (size_t)G.red_offset * P_WIDTH, G.red_grid, ens->st[0]);
+    return LaunchBatch<FMT>::sample(static_cast<const Member<T> *>(G.d_members), (int)G.idx.size(), G.red_total,
+                                    ens->partial + (size_t)G.red_offset * P_WIDTH, G.red_grid, ens->st[0]);
 }
 
 extern "C" int tcym_ensemble_measure(tcym_ensemble ens, int ncs_stride, double *edotb, double *ncs) {
@@ -514,10 +514,10 @@ extern "C" int tcym_ensemble_measure(tcym_ensemble ens, int ncs_stride, double *
     cudaSetDevice(ens->ctx->device);
     int r = upload_tables(ens);
     if (r) return r;
-    cudaError_t e = launch_group_obs<FMT_SU2_F32>(ens, FMT_SU2_F32, OBS_EDOTB);
-    if (e == cudaSuccess) e = launch_group_obs<FMT_SU2_F64>(ens, FMT_SU2_F64, OBS_EDOTB);
-    if (e == cudaSuccess) e = launch_group_obs<FMT_SU3_F32>(ens, FMT_SU3_F32, OBS_EDOTB);
-    if (e == cudaSuccess) e = launch_group_obs<FMT_SU3_F64>(ens, FMT_SU3_F64, OBS_EDOTB);
+    cudaError_t e = launch_group_sample<FMT_SU2_F32>(ens, FMT_SU2_F32);
+    if (e == cudaSuccess) e = launch_group_sample<FMT_SU2_F64>(ens, FMT_SU2_F64);
+    if (e == cudaSuccess) e = launch_group_sample<FMT_SU3_F32>(ens, FMT_SU3_F32);
+    if (e == cudaSuccess) e = launch_group_sample<FMT_SU3_F64>(ens, FMT_SU3_F64);
     if (e != cudaSuccess) return fail(ens->ctx, e, "ensemble observables");
     // per-member finalisers, in ensemble order
     std::vector<MemberReduce> items(n);
@@ -526,7 +526,7 @@ extern "C" int tcym_ensemble_measure(tcym_ensemble ens, int ncs_stride, double *
         int red = 0;
         for (size_t i = 0; i < G.idx.size(); ++i) {
             const EnsMember &m = ens->members[G.idx[i]];
-            const int rb = grid_for(m.lat->g.V, kRedThreads);
+            const int rb = member_records((f == FMT_SU2_F32 || f == FMT_SU3_F32) && m.lat->g.nz % 2 == 0, m.lat->g.V);
             items[G.idx[i]] = MemberReduce{ens->partial + (size_t)G.red_offset * P_WIDTH, red, rb,
                                            m.lat->nc == 2 ? 3 : 8, m.lat->g.V,
                                            ncs_stride > 0 ? m.dt * ncs_stride : 0.0, m.lat->result};

@@ -20,7 +20,9 @@ enum : int {
 // device result block (doubles), written by finalize_obs
 enum : int {
     R_ESQ0 = 0, R_BSQ0 = 3, R_GMAX = 6, R_GRMS = 7, R_GABS = 8, R_UMAX = 9, R_URMS = 10, R_EDB = 11,
-    R_NCS = 12, R_NCS_COMP = 13, R_NONFINITE = 14, R_WIDTH = 16
+    R_NCS = 12, R_NCS_COMP = 13, R_NONFINITE = 14,
+    R_TICKET = 15,  // an integer: blocks of the running reduction that are done (0 between reductions)
+    R_WIDTH = 16
 };
 
 #ifndef TCYM_SU2_THREADS
@@ -199,27 +201,155 @@ __device__ __forceinline__ double warp_max(double v) {
     return v;
 }
 
-// Reduce vals[0..P_WIDTH) over the block into partial[blockIdx.x * P_WIDTH ..].
-__device__ __forceinline__ void block_partial(double *vals, double *partial) {
-    __shared__ double sh[32][P_WIDTH];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+// Reductions.  On GB300 a warp's FP64 add takes 16 cycles of its SM's one FP64 unit, so
+// a block's record (up to 12 values) is summed with as few as the tree allows: every
+// thread's values go to shared memory, a warp takes a value, adds its 256/32 columns and
+// finishes by shuffles, 12 warp-adds a value where a shuffle tree in every warp took 48.
+// Only the slots a kernel fills (USED) are reduced.  The last block to finish sums the
+// blocks' records in block order and writes the result, so a reduction is one launch
+// (a second one cost 5 to 10 us); the order of every sum depends on the launch's shape
+// alone.
+constexpr unsigned kUsedSample = (1u << P_ESQ0) * 7u | (1u << P_BSQ0) * 7u | 1u << P_EDB;
+constexpr unsigned kUsedGauss = 1u << P_GSQ | 1u << P_GMAX | 1u << P_GABS;
+constexpr unsigned kUsedAll = (1u << P_WIDTH) - 1u;
+constexpr int used_count(unsigned used) { return used == 0 ? 0 : (int)(used & 1u) + used_count(used >> 1); }
+// the slot of the q-th used value
+__device__ __forceinline__ int used_slot(unsigned used, int q) {
+    for (; q > 0; --q) used &= used - 1;
+    return __ffs((int)used) - 1;
+}
+__device__ __forceinline__ double slot_op(int k, double a, double b) { return k < P_GMAX ? a + b : fmax(a, b); }
+__device__ __forceinline__ double warp_op(int k, double v) {
 #pragma unroll
-    for (int k = 0; k < P_WIDTH; ++k) vals[k] = k < P_GMAX ? warp_sum(vals[k]) : warp_max(vals[k]);
-    if (lane == 0)
+    for (int o = 16; o > 0; o >>= 1) v = slot_op(k, v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// The block's record from its threads' values; sh: used_count(USED) * NT doubles.
+template <unsigned USED, int NT>
+__device__ __forceinline__ void block_record(const double *v, double *sh, double *record) {
+    constexpr int NQ = used_count(USED);
+    const int lane = threadIdx.x & 31;
+    int q = 0;
 #pragma unroll
-        for (int k = 0; k < P_WIDTH; ++k) sh[w][k] = vals[k];
+    for (int k = 0; k < P_WIDTH; ++k)
+        if (USED >> k & 1) sh[(q++) * NT + threadIdx.x] = v[k];
     __syncthreads();
-    if (threadIdx.x < P_WIDTH) {
-        const int k = threadIdx.x;
-        double r = sh[0][k];
-        for (int i = 1; i < nw; ++i) r = k < P_GMAX ? r + sh[i][k] : fmax(r, sh[i][k]);
-        partial[(int64_t)blockIdx.x * P_WIDTH + k] = r;
+    for (q = threadIdx.x >> 5; q < NQ; q += NT / 32) {
+        const int k = used_slot(USED, q);
+        double r = sh[q * NT + lane];
+#pragma unroll
+        for (int i = 1; i < NT / 32; ++i) r = slot_op(k, r, sh[q * NT + lane + 32 * i]);
+        r = warp_op(k, r);
+        if (lane == 0) record[k] = r;
     }
 }
 
-template <int FMT>
+// What the summed records become.
+struct Finish {
+    double *result;              // the result block
+    double *ctl;                 // a restore's control block (finish_record), else nullptr
+    double inv_v, na_v, three_v; // 1 / V, na V, 3 V
+    double ncs_dt;               // N_CS advances by ncs_dt E.B / (8 pi^2) (0: it stays)
+    double tol;                  // restore: the stopping rule of iteration `it`
+    int it, check;
+};
+inline Finish make_finish(double *result, int na, int64_t V, double ncs_dt, double *ctl = nullptr, double tol = 0.0,
+                          int it = 0, bool check = false) {
+    return Finish{result, ctl, 1.0 / (double)V, (double)na * (double)V, 3.0 * (double)V, ncs_dt, tol, it, check ? 1 : 0};
+}
+
+// The totals t[0..P_WIDTH) into the result block, by the block's first warps: the
+// divisions and roots (hundreds of cycles each) side by side.  A restore (f.ctl): a
+// non-finite reduction sets ctl[1] and stops it after this iteration; with `check` (the
+// deviation the reference tests, GaussRestore.cpp:150), a signed maximum <= tol stops it.
+__device__ __forceinline__ void finish_record(const double *t, const Finish &f, double *edb = nullptr,
+                                              double *ncs = nullptr) {
+    double *res = f.result;
+    const int i = threadIdx.x;
+    if (i < 6) res[R_ESQ0 + i] = t[P_ESQ0 + i] * f.inv_v;  // E^2 and B^2: the same order in both
+    else if (i == 6) res[R_GMAX] = t[P_GMAX];
+    else if (i == 7) res[R_GABS] = t[P_GABS];
+    else if (i == 8) res[R_UMAX] = t[P_UMAX];
+    else if (i == 32) res[R_GRMS] = sqrt(t[P_GSQ] / f.na_v);
+    else if (i == 64) res[R_URMS] = sqrt(t[P_USQ] / f.three_v);
+    else if (i == 96) {
+        bool bad = false;
+        for (int k = 0; k < P_WIDTH; ++k) bad |= !isfinite(t[k]);
+        res[R_EDB] = t[P_EDB];
+        bad |= res[R_NONFINITE] != 0.0;
+        res[R_NONFINITE] = bad ? 1.0 : 0.0;
+        double sum = res[R_NCS];
+        if (f.ncs_dt != 0.0) {
+            // Kahan: sum += ncs_dt * E.B / (8 pi^2) with running compensation
+            const double inv8pi2 = 0.125 / (3.14159265358979323846 * 3.14159265358979323846);
+            const double y = f.ncs_dt * t[P_EDB] * inv8pi2 - res[R_NCS_COMP];
+            const double s = sum + y;
+            res[R_NCS_COMP] = (s - sum) - y;
+            res[R_NCS] = sum = s;
+        }
+        if (edb) *edb = t[P_EDB];
+        if (ncs) *ncs = sum;
+        if (f.ctl) {
+            const double gmax = t[P_GMAX];
+            bad |= !(gmax == gmax);
+            if (bad) f.ctl[1] = 1.0;
+            if (bad || (f.check && gmax <= f.tol)) f.ctl[0] = fmin(f.ctl[0], (double)(f.it + 1));
+        }
+    }
+}
+
+// The totals of `blocks` records (in block order, a warp a value) into t.
+template <unsigned USED, int NT>
+__device__ __forceinline__ void sum_records(const double *partial, int blocks, double *t) {
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < P_WIDTH) t[threadIdx.x] = 0.0;
+    __syncthreads();
+    for (int q = threadIdx.x >> 5; q < used_count(USED); q += NT / 32) {
+        const int k = used_slot(USED, q);
+        double r = 0.0;  // every slot's sum or maximum starts at 0
+        for (int b = lane; b < blocks; b += 32) r = slot_op(k, r, __ldcg(&partial[(int64_t)b * P_WIDTH + k]));
+        r = warp_op(k, r);
+        if (lane == 0) t[k] = r;
+    }
+    __syncthreads();
+}
+
+// The end of a reduction kernel of NT >= 128 threads a block: this block's record, and
+// in the last block the result.
+template <unsigned USED, int NT>
+__device__ __forceinline__ void reduce_and_finish(const double *v, double *partial, const Finish &f) {
+    static_assert(NT >= 128, "finish_record spreads over four warps");
+    __shared__ double sh[used_count(USED) * NT];
+    __shared__ int last;
+    block_record<USED, NT>(v, sh, partial + (int64_t)blockIdx.x * P_WIDTH);
+    __threadfence();  // the record before the ticket
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned *ticket = reinterpret_cast<unsigned *>(f.result + R_TICKET);
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        if (last) *ticket = 0;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    sum_records<USED, NT>(partial, gridDim.x, sh);
+    finish_record(sh, f);
+}
+
+// the record alone (callers that sum the records in a launch of their own)
+__device__ __forceinline__ void block_partial(const double *vals, double *partial) {
+    __shared__ double sh[used_count(kUsedGauss) * kRedThreads];
+    double *record = partial + (int64_t)blockIdx.x * P_WIDTH;
+    if (threadIdx.x < P_WIDTH) record[threadIdx.x] = 0.0;
+    __syncthreads();
+    block_record<kUsedGauss, kRedThreads>(vals, sh, record);
+}
+
+// FULL: the Gauss and unitarity slots are filled too
+template <int FMT, bool FULL>
 __global__ void __launch_bounds__(kRedThreads) k_observables(Geom g, const void *U, const void *E, int mask,
-                                                             double *partial) {
+                                                             double *partial, Finish fin) {
     using F = Fmt<FMT>;
     double v[P_WIDTH];
 #pragma unroll
@@ -237,19 +367,24 @@ __global__ void __launch_bounds__(kRedThreads) k_observables(Geom g, const void 
         for (int m = 0; m < 3; ++m) { v[P_USQ] += o.un[m] * o.un[m]; v[P_UMAX] = fmax(v[P_UMAX], o.un[m]); }
         v[P_EDB] += o.edotb;
     }
-    block_partial(v, partial);
+    reduce_and_finish<FULL ? kUsedAll : kUsedSample, kRedThreads>(v, partial, fin);
 }
 
-// The N_CS sample (mask OBS_EDOTB) of FP32 pair storage with even nz: one thread
-// per site pair, the same block partials as k_observables with that mask (the
-// Gauss and unitarity slots stay 0).
-template <int FMT>
-__global__ void __launch_bounds__(kRedThreads) k_edotb_obs_pair(Geom g, const void *U, const void *E,
-                                                                double *partial) {
+// The observables of FP32 pair storage with even nz, one thread per site pair in packed
+// FP32: the N_CS sample (mask OBS_EDOTB: E^2, plaquette B^2, clover E.B), and FULL
+// (OBS_ALL) the Gauss and unitarity violations too.  A pair's sums run in packed FP32
+// (the Gauss violation's, which cancel, exactly), everything across pairs in FP64.  Per
+// site, with FP64 sums and one lane of every pair vector used, all observables took
+// 2794 us for SU(3) and 638 us for SU(2) at 128^3 on GB300.
+constexpr int kThreadsObs = 128;
+template <int FMT, bool FULL>
+__global__ void __launch_bounds__(kThreadsObs, Fmt<FMT>::NA == 8 ? 2 : 4)
+    k_obs_pair(Geom g, const void *U, const void *E, double *partial, Finish fin) {
     using F = Fmt<FMT>;
     double v[P_WIDTH];
 #pragma unroll
     for (int k = 0; k < P_WIDTH; ++k) v[k] = 0.0;
+    float gmax = 0.f, gabs = 0.f, umax = 0.f;
     const int64_t Vh = g.V >> 1, plane = (int64_t)g.nx * g.ny;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < Vh; p += (int64_t)gridDim.x * blockDim.x) {
         const bool seam = p < plane || p >= Vh - plane;
@@ -265,16 +400,37 @@ __global__ void __launch_bounds__(kRedThreads) k_edotb_obs_pair(Geom g, const vo
             else { v[P_ESQ0 + 2] += es; v[P_BSQ0 + 2] += bs; }
             v[P_EDB] += (double)edb.v.x + (double)edb.v.y;
         }
+        if constexpr (FULL) {
+            f2 gv[F::NA], gsq(0.0), usq(0.0);
+            pair_gauss<F, true>(g, U, E, p, gv);
+#pragma unroll
+            for (int a = 0; a < F::NA; ++a) {
+                const float x = gv[a].v.x, y = gv[a].v.y;
+                gsq = fma(gv[a], gv[a], gsq);
+                gmax = fmaxf(gmax, fmaxf(x, y));
+                gabs = fmaxf(gabs, fmaxf(fabsf(x), fabsf(y)));
+            }
+#pragma unroll 1
+            for (int mu = 0; mu < 3; ++mu) {
+                const f2 n = F::G2::unitarity_square(F::load2(U, Vh, mu, p, false));
+                usq = usq + n;
+                umax = fmaxf(umax, fmaxf(n.v.x, n.v.y));
+            }
+            v[P_GSQ] += (double)gsq.v.x + (double)gsq.v.y;
+            v[P_USQ] += (double)usq.v.x + (double)usq.v.y;
+        }
     }
-    block_partial(v, partial);
+    v[P_GMAX] = gmax;
+    v[P_GABS] = gabs;
+    v[P_UMAX] = sqrtf(umax);
+    reduce_and_finish<FULL ? kUsedAll : kUsedSample, kThreadsObs>(v, partial, fin);
 }
 
 // Gauss violation into the FP64 scratch G[a*V + s]; partial maxima as for observables.
 template <int FMT>
 __device__ __forceinline__ void gauss_compute_block(const Geom &g, const void *U, const void *E, double *G,
-                                                    double *partial) {
+                                                    double *v) {
     using F = Fmt<FMT>;
-    double v[P_WIDTH];
 #pragma unroll
     for (int k = 0; k < P_WIDTH; ++k) v[k] = 0.0;
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < g.V; s += (int64_t)gridDim.x * blockDim.x) {
@@ -287,12 +443,13 @@ __device__ __forceinline__ void gauss_compute_block(const Geom &g, const void *U
             v[P_GABS] = fmax(v[P_GABS], fabs(gv[a]));
         }
     }
-    block_partial(v, partial);
 }
 template <int FMT>
 __global__ void __launch_bounds__(kRedThreads) k_gauss_compute(Geom g, const void *U, const void *E, double *G,
                                                                double *partial) {
-    gauss_compute_block<FMT>(g, U, E, G, partial);
+    double v[P_WIDTH];
+    gauss_compute_block<FMT>(g, U, E, G, v);
+    block_partial(v, partial);
 }
 
 template <int FMT>
@@ -304,14 +461,16 @@ __global__ void __launch_bounds__(threads_for<FMT>()) k_gauss_update(Geom g, con
 }
 
 // The same two kernels for iteration `it` of a restore whose control block
-// holds, in ctl[0], the first iteration that is not to run (the finaliser of the
-// deciding reduction lowers it): a kernel of a later iteration returns at once,
+// holds, in ctl[0], the first iteration that is not to run (the last block of the
+// deciding reduction lowers it, when every block has read it): a kernel of a later iteration returns at once,
 // so the host can queue many iterations between its checks.
 template <int FMT>
 __global__ void __launch_bounds__(kRedThreads) k_gauss_compute_it(Geom g, const void *U, const void *E, double *G,
-                                                                  double *partial, const double *ctl, int it) {
-    if ((double)it >= ctl[0]) return;  // the same value for every thread of the grid
-    gauss_compute_block<FMT>(g, U, E, G, partial);
+                                                                  double *partial, Finish fin) {
+    if ((double)fin.it >= fin.ctl[0]) return;  // the same value for every thread of the grid
+    double v[P_WIDTH];
+    gauss_compute_block<FMT>(g, U, E, G, v);
+    reduce_and_finish<kUsedGauss, kRedThreads>(v, partial, fin);
 }
 template <int FMT>
 __global__ void __launch_bounds__(threads_for<FMT>()) k_gauss_update_it(Geom g, const void *U, void *E, const double *G,
@@ -334,8 +493,8 @@ __global__ void __launch_bounds__(threads_for<FMT>()) k_gauss_update_it(Geom g, 
 
 template <int FMT>
 __global__ void __launch_bounds__(kRedThreads) k_gauss_compute_pair_it(Geom g, const void *U, const void *E, f2 *G2,
-                                                                       double *partial, const double *ctl, int it) {
-    if ((double)it >= ctl[0]) return;
+                                                                       double *partial, Finish fin) {
+    if ((double)fin.it >= fin.ctl[0]) return;
     using F = Fmt<FMT>;
     using GG = typename F::G2;
     constexpr int NA = F::NA;
@@ -376,7 +535,7 @@ __global__ void __launch_bounds__(kRedThreads) k_gauss_compute_pair_it(Geom g, c
     v[P_GSQ] = gsq;
     v[P_GMAX] = gmax;
     v[P_GABS] = gabs;
-    block_partial(v, partial);
+    reduce_and_finish<kUsedGauss, kRedThreads>(v, partial, fin);
 }
 
 // E_mu(x) -= gam (G(x) - U_mu(x) G(x+mu) U_mu^dag(x)) for both sites of a pair, in FP32
@@ -541,39 +700,37 @@ template <int FMT> struct Launch {
         int b = grid_for(g.V, kRedThreads);
         return b < max_blocks ? b : max_blocks;
     }
-    static cudaError_t observables(const Geom &g, const void *U, const void *E, int mask, double *partial, int blocks,
-                                   cudaStream_t st) {
+    // the observables `mask` into fin's result block; max_blocks: records in `partial`
+    static cudaError_t observables(const Geom &g, const void *U, const void *E, int mask, double *partial,
+                                   int max_blocks, const Finish &fin, cudaStream_t st) {
         if constexpr (Fmt<FMT>::PAIRED) {
-            if (mask == OBS_EDOTB && g.nz % 2 == 0) {  // the N_CS sample: paired FP32
-                k_edotb_obs_pair<FMT><<<blocks, kRedThreads, 0, st>>>(g, U, E, partial);
+            if ((mask == OBS_EDOTB || mask == OBS_ALL) && g.nz % 2 == 0) {
+                const int need = grid_for(g.V >> 1, kThreadsObs), blocks = need < max_blocks ? need : max_blocks;
+                if (mask == OBS_ALL) k_obs_pair<FMT, true><<<blocks, kThreadsObs, 0, st>>>(g, U, E, partial, fin);
+                else k_obs_pair<FMT, false><<<blocks, kThreadsObs, 0, st>>>(g, U, E, partial, fin);
                 return cudaGetLastError();
             }
         }
-        k_observables<FMT><<<blocks, kRedThreads, 0, st>>>(g, U, E, mask, partial);
-        return cudaGetLastError();
-    }
-    static cudaError_t gauss_compute(const Geom &g, const void *U, const void *E, double *G, double *partial,
-                                     int blocks, cudaStream_t st) {
-        k_gauss_compute<FMT><<<blocks, kRedThreads, 0, st>>>(g, U, E, G, partial);
-        return cudaGetLastError();
-    }
-    static cudaError_t gauss_update(const Geom &g, const void *U, void *E, const double *G, double gam,
-                                    cudaStream_t st) {
-        k_gauss_update<FMT><<<grid_for(g.V, TPB), TPB, 0, st>>>(g, U, E, G, gam);
+        const int blocks = reduce_grid(g, max_blocks);
+        if (mask & (OBS_GAUSS | OBS_UNIT))
+            k_observables<FMT, true><<<blocks, kRedThreads, 0, st>>>(g, U, E, mask, partial, fin);
+        else
+            k_observables<FMT, false><<<blocks, kRedThreads, 0, st>>>(g, U, E, mask, partial, fin);
         return cudaGetLastError();
     }
     // the restore iteration: paired FP32 kernels where the storage is paired
     static constexpr bool restore_paired(const Geom &g) { return TCYM_RESTORE_PAIRED && Fmt<FMT>::PAIRED && g.nz % 2 == 0; }
     static cudaError_t gauss_compute_it(const Geom &g, const void *U, const void *E, double *G, double *partial,
-                                        int blocks, const double *ctl, int it, cudaStream_t st) {
+                                        int max_blocks, const Finish &fin, cudaStream_t st) {
         if constexpr (Fmt<FMT>::PAIRED) {
             if (restore_paired(g)) {
+                const int need = grid_for(g.V >> 1, kRedThreads), blocks = need < max_blocks ? need : max_blocks;
                 k_gauss_compute_pair_it<FMT><<<blocks, kRedThreads, 0, st>>>(g, U, E, reinterpret_cast<f2 *>(G),
-                                                                             partial, ctl, it);
+                                                                             partial, fin);
                 return cudaGetLastError();
             }
         }
-        k_gauss_compute_it<FMT><<<blocks, kRedThreads, 0, st>>>(g, U, E, G, partial, ctl, it);
+        k_gauss_compute_it<FMT><<<reduce_grid(g, max_blocks), kRedThreads, 0, st>>>(g, U, E, G, partial, fin);
         return cudaGetLastError();
     }
     static cudaError_t gauss_update_it(const Geom &g, const void *U, void *E, const double *G, double gam,
@@ -639,11 +796,4 @@ cudaError_t finalize_obs(const double *partial, int blocks, int na, int64_t V, d
                          cudaStream_t st);
 // loads k_finalize's code now (with lazy module loading it would load at its first launch)
 cudaError_t preload_finalize();
-// The finaliser of a Gauss restore's reduction in iteration `it` (-1: the initial
-// deviation), skipped when it >= ctl[0].  A non-finite reduction sets ctl[1] and
-// stops the restore after this iteration; with `check` (the deviation the
-// reference tests, GaussRestore.cpp:150), a signed maximum <= tol stops it too.
-cudaError_t finalize_restore(const double *partial, int blocks, int na, int64_t V, double *result, double *ctl,
-                             double tol, int it, bool check, cudaStream_t st);
-
 }  // namespace tcym

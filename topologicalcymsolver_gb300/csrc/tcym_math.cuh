@@ -289,6 +289,17 @@ template <class T> struct SU2 {
         const Mat w = mulx<false, true>(a, b);
         proj(w, out);
     }
+    // components of V^dagger (e^a t^a) V for a group element V: the rotation
+    // e + 2 (v3 q x e + q x (q x e)) of its vector part q
+    static TCYM_HD void transport(const Mat &v, const T *e, T *out) {
+        const T *q = v.q;
+        const T c0 = T(2) * fma(q[1], e[2], -(q[2] * e[1]));
+        const T c1 = T(2) * fma(q[2], e[0], -(q[0] * e[2]));
+        const T c2 = T(2) * fma(q[0], e[1], -(q[1] * e[0]));
+        out[0] = fma(q[1], c2, fma(-q[2], c1, fma(q[3], c0, e[0])));
+        out[1] = fma(q[2], c0, fma(-q[0], c2, fma(q[3], c1, e[1])));
+        out[2] = fma(q[0], c1, fma(-q[1], c0, fma(q[3], c2, e[2])));
+    }
     static TCYM_HD T retr_one_minus(const Mat &v) { return T(2) * (T(1) - v.q[3]); }
     // exp(i c t^k e^k) = cos(d/2) + i sin(d/2) (c e / d).sigma, d = |c e|
     static TCYM_HD Mat iexp(T c, const T *e) {
@@ -310,10 +321,11 @@ template <class T> struct SU2 {
         out[0] = w.q[0]; out[1] = w.q[1]; out[2] = w.q[2];
     }
     // ||V V^dagger - 1|| over the four components (SU2/GroupOperations.cpp:172-184)
-    static TCYM_HD T unitarity_norm(const Mat &v) {
+    static TCYM_HD T unitarity_square(const Mat &v) {
         Mat c = mulx<false, true>(v, v);
-        return Real<T>::sqrt_(c.q[0] * c.q[0] + c.q[1] * c.q[1] + c.q[2] * c.q[2] + (c.q[3] - T(1)) * (c.q[3] - T(1)));
+        return c.q[0] * c.q[0] + c.q[1] * c.q[1] + c.q[2] * c.q[2] + (c.q[3] - T(1)) * (c.q[3] - T(1));
     }
+    static TCYM_HD T unitarity_norm(const Mat &v) { return Real<T>::sqrt_(unitarity_square(v)); }
     static TCYM_HD Mat reunitarize(const Mat &v) {
         T n = Real<T>::rsqrt_(v.q[0] * v.q[0] + v.q[1] * v.q[1] + v.q[2] * v.q[2] + v.q[3] * v.q[3]);
         return scale(n, v);
@@ -472,6 +484,44 @@ template <class T> struct SU3 {
                 }
             }
         proj(w, p);
+    }
+    // components of V^dagger (e^a t^a) V for a group element V.  With H = 2 e^a t^a,
+    // only columns 0 and 1 of H V are formed: the entries below the diagonal and the
+    // first two diagonal ones of V^dagger (H V) need no more, and the third follows
+    // from the trace (108 operations; inverse_adjoint's two full products take 216).
+    static TCYM_HD void transport(const Mat &v, const T *e, T *out) {
+        const T is3 = T(0.57735026918962576450914878050196);
+        const T a7 = is3 * e[7];
+        const T a0 = a7 + e[2], a1 = a7 - e[2], a2 = T(-2) * a7;
+        const cx<T> h10{e[0], e[1]}, h20{e[3], e[4]}, h21{e[5], e[6]};
+        cx<T> w[3][2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const cx<T> x = v.m[0][j], y = v.m[1][j], z = v.m[2][j];
+            w[0][j] = cfma_cn(h10, y, cfma_cn(h20, z, cx<T>{a0 * x.re, a0 * x.im}));
+            w[1][j] = cfma(h10, x, cfma_cn(h21, z, cx<T>{a1 * y.re, a1 * y.im}));
+            w[2][j] = cfma(h20, x, cfma(h21, y, cx<T>{a2 * z.re, a2 * z.im}));
+        }
+        auto column = [&](int i, int j) {  // (V^dagger W)_ij
+            const cx<T> x = v.m[0][i], y = w[0][j];
+            cx<T> acc{x.re * y.re, x.re * y.im};
+            acc.re = fma(x.im, y.im, acc.re);
+            acc.im = fma(-x.im, y.re, acc.im);
+            return cfma_cn(v.m[2][i], w[2][j], cfma_cn(v.m[1][i], w[1][j], acc));
+        };
+        auto diagonal = [&](int i) {
+            T r = v.m[0][i].re * w[0][i].re;
+            r = fma(v.m[0][i].im, w[0][i].im, r);
+            r = fma(v.m[1][i].re, w[1][i].re, fma(v.m[1][i].im, w[1][i].im, r));
+            return fma(v.m[2][i].re, w[2][i].re, fma(v.m[2][i].im, w[2][i].im, r));
+        };
+        const cx<T> m10 = column(1, 0), m20 = column(2, 0), m21 = column(2, 1);
+        const T m00 = diagonal(0), m11 = diagonal(1);
+        out[0] = m10.re; out[1] = m10.im;
+        out[2] = T(0.5) * (m00 - m11);
+        out[3] = m20.re; out[4] = m20.im;
+        out[5] = m21.re; out[6] = m21.im;
+        out[7] = T(0.86602540378443864676) * (m00 + m11);
     }
     static TCYM_HD T retr_one_minus(const Mat &v) { return T(3) - (v.m[0][0].re + v.m[1][1].re + v.m[2][2].re); }
 
@@ -710,7 +760,7 @@ template <class T> struct SU3 {
         algebra_components(w, out);
     }
     // ||V V^dagger - 1||_F (SU3/GroupOperations.cpp:351-363)
-    static TCYM_HD T unitarity_norm(const Mat &v) {
+    static TCYM_HD T unitarity_square(const Mat &v) {
         Mat c = mulx<false, true>(v, v);
         T n = T(0);
         for (int i = 0; i < 3; ++i)
@@ -718,8 +768,9 @@ template <class T> struct SU3 {
                 T re = c.m[i][j].re - (i == j ? T(1) : T(0)), im = c.m[i][j].im;
                 n = fma(re, re, fma(im, im, n));
             }
-        return Real<T>::sqrt_(n);
+        return n;
     }
+    static TCYM_HD T unitarity_norm(const Mat &v) { return Real<T>::sqrt_(unitarity_square(v)); }
     // third row of an SU(3) matrix from the first two: r2 = conj(r0 x r1)
     static TCYM_HD void complete_row2(Mat &u) {
         const cx<T> *a = u.m[0], *b = u.m[1];

@@ -618,6 +618,39 @@ template <class T> struct ExactSum {
     }
     TCYM_HD T value() const { return s + e; }
 };
+// The Gauss violation G(x) = sum_mu E_mu(x) - U_mu^dag(x-mu) E_mu(x-mu) U_mu(x-mu) of both
+// sites of pair p of FP32 pair storage (even nz).  G of a restored field is a sum that
+// cancels, so its six terms are summed with their rounding errors (ExactSum).
+template <class F, bool SEAM> TCYM_HD void pair_gauss(const Geom &g, const void *U, const void *E, int64_t p, f2 *gv) {
+    using G2 = typename F::G2;
+    constexpr int NA = F::NA;
+    const int64_t Vh = g.V >> 1;
+    const PairNbhd nb(g, p);
+    ExactSum<f2> s[NA];
+#pragma unroll
+    for (int a = 0; a < NA; ++a) s[a] = ExactSum<f2>(f2(0.0));
+#pragma unroll 1
+    for (int mu = 0; mu < 3; ++mu) {
+        const int64_t pm = nb.at(mu, -1);
+        const bool sw = SEAM && nb.swapped(mu, -1);
+        f2 e[NA], t[NA];
+        F::load_e2(E, Vh, mu, pm, e);
+        if (sw) {
+#pragma unroll
+            for (int a = 0; a < NA; ++a) e[a] = swap_f2(e[a]);
+        }
+        G2::transport(F::load2(U, Vh, mu, pm, sw), e, t);
+        F::load_e2(E, Vh, mu, p, e);
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            s[a].add(e[a]);
+            s[a].add(-t[a]);
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < NA; ++a) gv[a] = s[a].value();
+}
+
 // Gauss violation G(x) in working precision T, for the restore iteration.
 template <class F>
 TCYM_HD void site_gauss(const Geom &g, const void *U, const void *E, int64_t s, double *gv) {
