@@ -626,7 +626,16 @@ template <class T> struct SU3 {
     // itself rounds next to 1 in FP32, which would move every updated link's
     // norm the same way and carry a long FP32 gradient flow off the group.
     // Otherwise the scaled-and-squared exponential is used.
+    // FP32 takes iexp_mul_single, FP64 a second form, with Q^2 and det Q from real and
+    // repeated entries and the series by hand (SU(3) 48^3: 676 -> 625 us a step).  In FP32
+    // the second form gains 2% of a 64^3 step, which waits for L2, but rounds links
+    // differently, and a cooled field's force is made of such roundings: after 240 sweeps
+    // at 64^3 both forms' forces are 2.8e-5 off exact arithmetic, each in its own way.
     static TCYM_HD Mat iexp_mul(T c, const T *e, const Mat &u) {
+        if constexpr (kSingle) return iexp_mul_single(c, e, u);
+        else return iexp_mul_double(c, e, u);
+    }
+    template <class P = T> static TCYM_HD Mat iexp_mul_double(P c, const P *e, const Mat &u) {
         // Q = c e^a t^a, Hermitian and traceless, by its real diagonal and the entries
         // above it; every product with a real or a repeated entry is formed once
         const T is3 = T(0.57735026918962576450914878050196);
@@ -639,10 +648,7 @@ template <class T> struct SU3 {
         const T o02 = fma(q02.re, q02.re, q02.im * q02.im);
         const T o12 = fma(q12.re, q12.re, q12.im * q12.im);
         const T c1 = fma(T(0.5), fma(d0, d0, fma(d1, d1, d2 * d2)), o01 + o02 + o12);
-        if (any_gt(c1 * T(4.0 / 3.0), T(0.25))) {
-            if constexpr (Packed<T>::value) return iexp_mul_lanes(c, e, u);
-            else return mulu<false, false>(iexp_hermitian(algebra_matrix(c, e)), u);
-        }
+        if (any_gt(c1 * T(4.0 / 3.0), T(0.25))) return mulu<false, false>(iexp_hermitian(algebra_matrix(c, e)), u);
         // Q^2, with q_ii + q_jj = -q_kk
         const T s00 = fma(d0, d0, o01 + o02), s11 = fma(d1, d1, o01 + o12);
         const cx<T> s01 = cfma_nc(q02, q12, cx<T>{-(d2 * q01.re), -(d2 * q01.im)});
@@ -652,20 +658,22 @@ template <class T> struct SU3 {
         const T tr = fma(q01.re, fma(q12.re, q02.re, q12.im * q02.im), q01.im * fma(q12.re, q02.im, -(q12.im * q02.re)));
         const T c0 = fma(d0, fma(d1, d2, -o12), fma(-d1, o02, fma(-d2, o01, T(2) * tr)));
         T f0r, f0i, f1r, f1i, f2r, f2i;
-        if constexpr (kSingle) {
-            // eight terms for r <= 1/2 (the first omitted one, r^9/9!, is 5e-9), Q^n reduced by
-            // hand: Q^3 = c1 Q + c0, ..., Q^8 = (c1^3 + c0^2) Q^2 + 3 c0 c1^2 Q + 2 c0^2 c1
-            const T k = c0 * c0;
-            f0r = k * fma(c1, T(1.0 / 20160), T(-1.0 / 720));
-            f0i = c0 * fma(c1, fma(c1, T(-1.0 / 5040), T(1.0 / 120)), T(-1.0 / 6));
-            f1r = c0 * fma(c1, fma(c1, T(1.0 / 13440), T(-1.0 / 360)), T(1.0 / 24));
-            f1i = fma(c1, fma(c1, fma(c1, T(-1.0 / 5040), T(1.0 / 120)), T(-1.0 / 6)), fma(k, T(-1.0 / 5040), T(1)));
-            f2r = fma(c1, fma(c1, fma(c1, T(1.0 / 40320), T(-1.0 / 720)), T(1.0 / 24)), fma(k, T(1.0 / 40320), T(-0.5)));
-            f2i = c0 * fma(c1, T(-1.0 / 2520), T(1.0 / 120));
+        // r^2 <= 0.02 (a link update's |dt E|): 10 terms by hand, the first omitted one 1e-17;
+        // Q^n = c0 d_{n-1} + d_{n+1} Q + d_n Q^2 with d_n = c1 d_{n-2} + c0 d_{n-3}
+        if (any_gt(c1 * T(4.0 / 3.0), T(0.02))) {
+            series_coeffs<16, true>(c0, c1, f0r, f0i, f1r, f1i, f2r, f2i);
         } else {
-            // r^2 <= 0.02 (a link update's |dt E|): 10 terms, the first omitted one 1e-17
-            if (any_gt(c1 * T(4.0 / 3.0), T(0.02))) series_coeffs<16, true>(c0, c1, f0r, f0i, f1r, f1i, f2r, f2i);
-            else series_coeffs<10, true>(c0, c1, f0r, f0i, f1r, f1i, f2r, f2i);
+            const T k = c0 * c0;
+            f0r = k * fma(c1, fma(c1, T(-1.0 / 1209600), T(1.0 / 20160)), T(-1.0 / 720));
+            f0i = c0 * fma(c1, fma(c1, fma(c1, T(1.0 / 362880), T(-1.0 / 5040)), T(1.0 / 120)),
+                           fma(k, T(1.0 / 362880), T(-1.0 / 6)));
+            f1r = c0 * fma(c1, fma(c1, fma(c1, T(-1.0 / 907200), T(1.0 / 13440)), T(-1.0 / 360)),
+                           fma(k, T(-1.0 / 3628800), T(1.0 / 24)));
+            f1i = fma(c1, fma(c1, fma(c1, fma(c1, T(1.0 / 362880), T(-1.0 / 5040)), T(1.0 / 120)), T(-1.0 / 6)),
+                      fma(k, fma(c1, T(1.0 / 120960), T(-1.0 / 5040)), T(1)));
+            f2r = fma(c1, fma(c1, fma(c1, fma(c1, T(-1.0 / 3628800), T(1.0 / 40320)), T(-1.0 / 720)), T(1.0 / 24)),
+                      fma(k, fma(c1, T(-1.0 / 1209600), T(1.0 / 40320)), T(-0.5)));
+            f2i = c0 * fma(c1, fma(c1, T(1.0 / 120960), T(-1.0 / 2520)), T(1.0 / 120));
         }
         // rows 0 and 1 of exp(iQ) - 1 = (f0 - 1) + f1 Q + f2 Q^2
         auto mix = [&](cx<T> x, cx<T> y) {
@@ -679,6 +687,53 @@ template <class T> struct SU3 {
         w.m[1][0] = mix(conj(q01), conj(s01));
         w.m[0][2] = mix(q02, s02);
         w.m[1][2] = mix(q12, s12);
+        return mulu_inc(w, u);  // reads rows 0 and 1 of w only
+    }
+    template <class P = T> static TCYM_HD Mat iexp_mul_single(P c, const P *e, const Mat &u) {
+        const Mat q = algebra_matrix(c, e);
+        // c1 = tr(Q^2)/2 = sum_ij |Q_ij|^2 / 2
+        const T d0 = q.m[0][0].re, d1 = q.m[1][1].re, d2 = q.m[2][2].re;
+        const T o01 = q.m[0][1].re * q.m[0][1].re + q.m[0][1].im * q.m[0][1].im;
+        const T o02 = q.m[0][2].re * q.m[0][2].re + q.m[0][2].im * q.m[0][2].im;
+        const T o12 = q.m[1][2].re * q.m[1][2].re + q.m[1][2].im * q.m[1][2].im;
+        const T c1 = T(0.5) * (d0 * d0 + d1 * d1 + d2 * d2) + (o01 + o02 + o12);
+        if (any_gt(c1 * T(4.0 / 3.0), T(0.25))) {
+            if constexpr (Packed<T>::value) return iexp_mul_lanes(c, e, u);
+            else return mulu<false, false>(iexp_hermitian(q), u);
+        }
+        // rows 0 and 1 of Q^2 (Hermitian Q)
+        cx<T> q2[2][3];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = i; j < 3; ++j) {
+                cx<T> acc{T(0), T(0)};
+#pragma unroll
+                for (int k = 0; k < 3; ++k) acc = cfma(q.m[i][k], q.m[k][j], acc);
+                q2[i][j] = acc;
+            }
+        q2[1][0] = conj(q2[0][1]);
+        // c0 = det Q (real for Hermitian Q)
+        const T c0 = d0 * (d1 * d2 - o12) - d1 * o02 - d2 * o01 +
+                     T(2) * (q.m[0][1].re * (q.m[1][2].re * q.m[2][0].re - q.m[1][2].im * q.m[2][0].im) -
+                             q.m[0][1].im * (q.m[1][2].re * q.m[2][0].im + q.m[1][2].im * q.m[2][0].re));
+        T f0r, f0i, f1r, f1i, f2r, f2i;
+        // terms of the series by the spectral radius r (r^2 <= 4 c1 / 3): the first
+        // omitted term r^(N+1)/(N+1)! stays below half an FP32 ulp, 3e-8, with 5
+        // terms for r^2 <= 0.02 (the common case: |dt E| is small) and 8 up to r = 1/2
+        if (any_gt(c1 * T(4.0 / 3.0), T(0.02))) series_coeffs<8, true>(c0, c1, f0r, f0i, f1r, f1i, f2r, f2i);
+        else series_coeffs<5, true>(c0, c1, f0r, f0i, f1r, f1i, f2r, f2i);
+        Mat w;  // rows 0 and 1 of exp(iQ) - 1
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const cx<T> x = q.m[i][j], y = q2[i][j];
+                T re = fma(f1r, x.re, fma(-f1i, x.im, fma(f2r, y.re, -f2i * y.im)));
+                T im = fma(f1r, x.im, fma(f1i, x.re, fma(f2r, y.im, f2i * y.re)));
+                if (i == j) { re += f0r; im += f0i; }
+                w.m[i][j] = cx<T>{re, im};
+            }
         return mulu_inc(w, u);  // reads rows 0 and 1 of w only
     }
     // rows 0 and 1 of u + w u (each accumulator starts at u's entry), row 2 rebuilt
