@@ -29,6 +29,7 @@ def load():
         L.hc_step.argtypes = [ctypes.c_int, ip, _vp, _vp, _vp, ctypes.c_int, ctypes.c_double, ctypes.c_double,
                               ctypes.c_double, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int, ctypes.c_int,
                               ctypes.c_int]
+        L.hc_march.argtypes = [ctypes.c_int, ip, _vp, _vp, _vp, ctypes.c_double] + [ctypes.c_int] * 4
         L.hc_flow_cb.argtypes = [ctypes.c_int, ip, _vp, ctypes.c_double, ctypes.c_int]
         L.hc_observables.argtypes = [ctypes.c_int, ip, _vp, _vp, ctypes.c_int, _vp]
         L.hc_edotb_pair.argtypes = [ctypes.c_int, ip, _vp, _vp, _vp]
@@ -94,6 +95,13 @@ class HostLattice:
     def leapfrog(self, dt, nsteps):
         for _ in range(nsteps):
             self.step(0, dt)
+
+    def march(self, dt, tx, ty=0, zl=0, threads=152):
+        """One leapfrog step in blocks that share their plaquettes, with the tiling tx x ty, zl planes a block (tx 0: the library's
+        rule for `threads` multiprocessors, 0: among an ensemble's members)."""
+        self.L.hc_march(self.fmt, self.n, _p(self.U[self.cur]), _p(self.U[1 - self.cur]), _p(self.E), dt, tx, ty, zl,
+                        threads)
+        self.cur ^= 1
 
     def langevin(self, dt, gamma, T, seed, step0, nsteps):
         for i in range(nsteps):

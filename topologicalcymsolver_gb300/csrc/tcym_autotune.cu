@@ -55,7 +55,7 @@ std::vector<Tile> candidates(const Geom &g) {
 
 template <int FMT> cudaError_t step_with(tcym_lattice p, const Tile &t) {
     const StepCoef<double> c = tcym_coef(p->a, MODE_LEAPFROG, 0.05, 0, 0, 0, 0);
-    return Launch<FMT>::step(p->g, p->U[0], p->U[1], p->E, c, true, true, p->stream, t);
+    return Launch<FMT>::step(p->g, p->U[0], p->U[1], p->E, c, t, MarchTile{}, p->stream);  // paired lattices only
 }
 
 // milliseconds for `reps` steps of the proxy with tiling t (negative: failed)
@@ -128,6 +128,12 @@ const Tile &tcym_lattice_tile_of(tcym_lattice lat) {
     if (it == lat->ctx->tiles.end()) it = lat->ctx->tiles.emplace(key, tune(lat)).first;
     lat->tile = it->second;
     return lat->tile;
+}
+
+const MarchTile &tcym_lattice_march_of(tcym_lattice lat, bool batched) {
+    MarchTile &t = lat->march[batched];
+    if (t.tx == 0) t = march_tile(lat->g, batched ? 0 : lat->ctx->sm_count);
+    return t;
 }
 
 extern "C" int tcym_lattice_tile(tcym_lattice lat, int *tx, int *ty) {

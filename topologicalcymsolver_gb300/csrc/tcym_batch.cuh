@@ -24,14 +24,10 @@ template <class T> struct Member {
     int red_blocks;      // reduction work items of this member
     int paired;          // step work items cover site pairs (FP32 format, even nz)
     Tile tile;           // their block tiling
+    MarchTile march;     // the tiling of the FP64 step
     double ncs_dt;       // Kahan increment factor for measurements (0: no N_CS update)
 };
 
-// 1: the batched kernels walk their work items with a grid of the resident
-// blocks; 0: one block per work item
-#ifndef TCYM_BATCH_PERSISTENT
-#define TCYM_BATCH_PERSISTENT 0
-#endif
 // the batched step reading its coefficients from the member table holds more
 // than the single-lattice step: SU(2) at 7 blocks per SM (72 registers) spills
 // there, so it keeps its own target (the uniform-coefficient kernel takes the
@@ -44,9 +40,7 @@ template <class T> struct Member {
 #define TCYM_SU3_BATCH_MINBLOCKS 3
 #endif
 template <int FMT> constexpr int batch_min_blocks_for() {
-    if constexpr (Fmt<FMT>::PAIRED && Fmt<FMT>::NA == 3) return TCYM_SU2_BATCH_MINBLOCKS;
-    if constexpr (Fmt<FMT>::PAIRED && Fmt<FMT>::NA == 8) return TCYM_SU3_BATCH_MINBLOCKS;
-    return Fmt<FMT>::PAIRED ? pair_min_blocks_for<FMT>() : min_blocks_for<FMT>();
+    return Fmt<FMT>::NA == 3 ? TCYM_SU2_BATCH_MINBLOCKS : TCYM_SU3_BATCH_MINBLOCKS;
 }
 
 // index of the member owning work item `item` (begins sorted ascending)
@@ -61,62 +55,51 @@ __device__ __forceinline__ int find_member(const Member<T> *m, int n, int item, 
     return lo;
 }
 
-// Step k of a chunk for every member: reads U[cur ^ (k&1)], writes U[cur ^ (k&1) ^ 1].
-// GENERAL = false is the lean kernel for the common case of a paired format whose
-// members all take pairs with the linear mapping; true handles every member kind.
-template <int FMT, bool GENERAL>
+// Step k of a chunk for every paired member: reads U[cur ^ (k&1)], writes
+// U[cur ^ (k&1) ^ 1]; one work item per block.
+template <int FMT>
+__global__ void __launch_bounds__(kThreadsPair, batch_min_blocks_for<FMT>())
+    k_step_batch(const Member<float> *__restrict__ members, int nmembers, int k) {
+    static_assert(Fmt<FMT>::PAIRED, "paired formats only");
+    // each thread's plaquette slots (its own only: no thread reads another's)
+    __shared__ f2 sm[plaq_slots<FMT>() * kThreadsPair];
+    const int item = blockIdx.x;
+    // the table is read-only and never aliases the fields (__restrict__), so the
+    // coefficients are read where used, block-uniform, from L1, rather than held in
+    // registers for the whole step
+    const Member<float> &m = members[find_member(members, nmembers, item, false)];
+    const Geom g = m.g;
+    int64_t p;
+    bool seam;
+    if (!tile_pair(g, m.tile, item - m.block_begin, threadIdx.x, p, seam)) return;
+    const int in = m.cur ^ (k & 1);
+    if (seam)
+        site_step_pair<Fmt<FMT>, true>(g, m.U[in], m.U[in ^ 1], m.E, m.c, p, (uint64_t)k, sm + threadIdx.x, kThreadsPair);
+    else
+        site_step_pair<Fmt<FMT>, false>(g, m.U[in], m.U[in ^ 1], m.E, m.c, p, (uint64_t)k, sm + threadIdx.x, kThreadsPair);
+}
+// The same for the members stepped per site, whose work items follow from item0 on: FP32
+// with odd nz, and FP64.
+template <int FMT>
 __global__ void __launch_bounds__(threads_for<FMT>(), batch_min_blocks_for<FMT>())
-    k_step_batch(const Member<typename Fmt<FMT>::T> *__restrict__ members, int nmembers, int total_blocks, int k) {
-    static_assert(!Fmt<FMT>::PAIRED || threads_for<FMT>() == kThreadsPair, "one block shape for both paths");
-    using T = typename Fmt<FMT>::T;
-    // each thread's plaquette slots (its own only: no thread reads another's); the
-    // per-site path of an FP32 member uses the same array as floats
-    using S = typename std::conditional<Fmt<FMT>::PAIRED, f2, T>::type;
-    __shared__ S sm_pair[plaq_slots<FMT>() * threads_for<FMT>()];
-    T *const sm_site = reinterpret_cast<T *>(sm_pair);
-    for (int item = blockIdx.x; item < total_blocks; item += gridDim.x) {
-        const int mi = find_member(members, nmembers, item, false);
-        // the table is read-only and never aliases the fields (__restrict__), so
-        // the coefficients are read where used, block-uniform, from L1, rather
-        // than held in registers for the whole step
-        const Member<typename Fmt<FMT>::T> &m = members[mi];
-        const Geom g = m.g;
-        if constexpr (Fmt<FMT>::PAIRED && !GENERAL) {
-            const int64_t p0 = (int64_t)(item - m.block_begin) * kThreadsPair, p = p0 + threadIdx.x;
-            if (p < (g.V >> 1)) {
-                const int in = m.cur ^ (k & 1);
-                if (pairs_touch_seam(g, p0, kThreadsPair))
-                    site_step_pair<Fmt<FMT>, true>(g, m.U[in], m.U[in ^ 1], m.E, m.c, p, (uint64_t)k,
-                                                   sm_pair + threadIdx.x, kThreadsPair);
-                else
-                    site_step_pair<Fmt<FMT>, false>(g, m.U[in], m.U[in ^ 1], m.E, m.c, p, (uint64_t)k,
-                                                    sm_pair + threadIdx.x, kThreadsPair);
-            }
-            continue;
-        }
-        if constexpr (Fmt<FMT>::PAIRED) {
-            if (m.paired) {  // block-uniform
-                int64_t p;
-                bool seam;
-                if (tile_pair(g, m.tile, item - m.block_begin, threadIdx.x, p, seam)) {
-                    const int in = m.cur ^ (k & 1);
-                    if (seam)
-                        site_step_pair<Fmt<FMT>, true>(g, m.U[in], m.U[in ^ 1], m.E, m.c, p, (uint64_t)k,
-                                                       sm_pair + threadIdx.x, kThreadsPair);
-                    else
-                        site_step_pair<Fmt<FMT>, false>(g, m.U[in], m.U[in ^ 1], m.E, m.c, p, (uint64_t)k,
-                                                        sm_pair + threadIdx.x, kThreadsPair);
-                }
-                continue;
-            }
-        }
-        const int64_t s = (int64_t)(item - m.block_begin) * blockDim.x + threadIdx.x;
-        if (s < g.V) {
-            const int in = m.cur ^ (k & 1);
-            site_step<Fmt<FMT>, true, true>(g, m.U[in], m.U[in ^ 1], m.E, m.c, s, (uint64_t)k,
-                                            sm_site + threadIdx.x, (int)blockDim.x);
-        }
-    }
+    k_sites_batch(const Member<float> *__restrict__ members, int nmembers, int item0, int k) {
+    __shared__ float sm[plaq_slots<FMT>() * threads_for<FMT>()];
+    const int item = item0 + blockIdx.x;
+    const Member<float> &m = members[find_member(members, nmembers, item, false)];
+    const Geom g = m.g;
+    const int64_t s = (int64_t)(item - m.block_begin) * blockDim.x + threadIdx.x;
+    if (s >= g.V) return;
+    const int in = m.cur ^ (k & 1);
+    site_step<Fmt<FMT>, true>(g, m.U[in], m.U[in ^ 1], m.E, m.c, s, (uint64_t)k, sm + threadIdx.x, (int)blockDim.x);
+}
+template <int FMT>
+__global__ void __launch_bounds__(kMarchThreads, march_min_blocks<FMT>())
+    k_march_batch(const Member<typename Fmt<FMT>::T> *__restrict__ members, int nmembers, int item0, int k) {
+    const int item = item0 + blockIdx.x;
+    const Member<typename Fmt<FMT>::T> &m = members[find_member(members, nmembers, item, false)];
+    const int in = m.cur ^ (k & 1);
+    march_block<Fmt<FMT>, true>(m.g, m.U[in], m.U[in ^ 1], m.E, m.c, m.march, SiteRange{0, m.g.nz, 0, m.g.V},
+                                item - m.block_begin, (uint64_t)k);
 }
 
 // The lean path when every member takes the same step coefficients (the same
@@ -133,27 +116,21 @@ __global__ void __launch_bounds__(kThreadsPair, pair_min_blocks_for<FMT>())
                          StepCoef<float> c) {
     static_assert(Fmt<FMT>::PAIRED, "paired formats only");
     __shared__ f2 sm[plaq_slots<FMT>() * kThreadsPair];
-#if TCYM_BATCH_PERSISTENT
-    for (int item = item0 + blockIdx.x; item < total_blocks; item += gridDim.x) {
-#else
-    {  // one work item per block
-        const int item = item0 + blockIdx.x;
-        if (item >= total_blocks) return;
-#endif
-        const int mi = find_member(members, nmembers, item, false);
-        const Member<float> &m = members[mi];
-        const Geom g = m.g;
-        const int64_t p0 = (int64_t)(item - m.block_begin) * kThreadsPair, p = p0 + threadIdx.x;
-        if (p < (g.V >> 1)) {
-            const int in = m.cur ^ (k & 1);
-            if (pairs_touch_seam(g, p0, kThreadsPair))
-                site_step_pair<Fmt<FMT>, true>(g, m.U[in], m.U[in ^ 1], m.E, c, m.c, p, (uint64_t)k,
-                                               sm + threadIdx.x, kThreadsPair);
-            else
-                site_step_pair<Fmt<FMT>, false>(g, m.U[in], m.U[in ^ 1], m.E, c, m.c, p, (uint64_t)k,
-                                                sm + threadIdx.x, kThreadsPair);
-        }
-    }
+    // one work item per block
+    const int item = item0 + blockIdx.x;
+    if (item >= total_blocks) return;
+    const int mi = find_member(members, nmembers, item, false);
+    const Member<float> &m = members[mi];
+    const Geom g = m.g;
+    const int64_t p0 = (int64_t)(item - m.block_begin) * kThreadsPair, p = p0 + threadIdx.x;
+    if (p >= (g.V >> 1)) return;
+    const int in = m.cur ^ (k & 1);
+    if (pairs_touch_seam(g, p0, kThreadsPair))
+        site_step_pair<Fmt<FMT>, true>(g, m.U[in], m.U[in ^ 1], m.E, c, m.c, p, (uint64_t)k, sm + threadIdx.x,
+                                       kThreadsPair);
+    else
+        site_step_pair<Fmt<FMT>, false>(g, m.U[in], m.U[in ^ 1], m.E, c, m.c, p, (uint64_t)k, sm + threadIdx.x,
+                                        kThreadsPair);
 }
 
 // ---------------------------------------------------------------- persistent
@@ -306,17 +283,25 @@ __global__ void __launch_bounds__(kThreadsObs, Fmt<FMT>::NA == 8 ? 2 : 4)
 // Launchers for one format.
 template <int FMT> struct LaunchBatch {
     using T = typename Fmt<FMT>::T;
-    static constexpr int TPB = threads_for<FMT>();
-    static int resident_blocks() {
-        int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_step_batch<FMT, true>, TPB, 0);
-        return b > 0 ? b : 1;
+    // every paired member (some of them tiled: coefficients from the table)
+    static cudaError_t step(const Member<T> *members, int n, int blocks, int k, cudaStream_t st) {
+        if constexpr (Fmt<FMT>::PAIRED) {
+            k_step_batch<FMT><<<blocks, kThreadsPair, 0, st>>>(members, n, k);
+            return cudaGetLastError();
+        }
+        return cudaErrorInvalidValue;
     }
-    // general: some member is unpaired or tiled (see k_step_batch)
-    static cudaError_t step(const Member<T> *members, int n, int total_blocks, int k, int grid, bool general,
-                            cudaStream_t st) {
-        if (general || !Fmt<FMT>::PAIRED) k_step_batch<FMT, true><<<grid, TPB, 0, st>>>(members, n, total_blocks, k);
-        else k_step_batch<FMT, false><<<grid, TPB, 0, st>>>(members, n, total_blocks, k);
+    // work items of a member stepped per site
+    static int site_items(const Geom &g, const MarchTile &m) {
+        return Fmt<FMT>::PAIRED ? grid_for(g.V, threads_for<FMT>()) : (int)march_blocks(m, g.nz);
+    }
+    // the members [m0, m0 + n) stepped per site, work items [item0, item1)
+    static cudaError_t sites(const Member<T> *members, int m0, int n, int item0, int item1, int k, size_t smem,
+                             cudaStream_t st) {
+        if constexpr (Fmt<FMT>::PAIRED)
+            k_sites_batch<FMT><<<item1 - item0, threads_for<FMT>(), 0, st>>>(members + m0, n, item0, k);
+        else
+            k_march_batch<FMT><<<item1 - item0, kMarchThreads, smem, st>>>(members + m0, n, item0, k);
         return cudaGetLastError();
     }
     // the members [m0, m0 + n) of one coefficient class, work items [item0, item1),
@@ -324,7 +309,7 @@ template <int FMT> struct LaunchBatch {
     static cudaError_t step_uniform(const Member<T> *members, int m0, int n, int item0, int item1, int k,
                                     const StepCoef<double> &cu, cudaStream_t st) {
         if constexpr (Fmt<FMT>::PAIRED) {
-            k_step_batch_uniform<FMT><<<item1 - item0, TPB, 0, st>>>(members + m0, n, item0, item1, k,
+            k_step_batch_uniform<FMT><<<item1 - item0, kThreadsPair, 0, st>>>(members + m0, n, item0, item1, k,
                                                                     coef_cast<float>(cu));
             return cudaGetLastError();
         }

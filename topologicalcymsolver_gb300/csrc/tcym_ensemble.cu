@@ -3,8 +3,8 @@
 // independent MPI ranks that only share a seed (SU2Solver.cpp:161-164); here
 // they share launches on one GPU.
 //
-// Per step and per storage format present, one persistent batched kernel
-// (k_step_batch) covers every member of that format; the formats run as
+// Per step and per storage format present, batched kernels (one for the members in
+// site pairs, one for those stepped per site) cover every member; the formats run as
 // independent chains on their own streams.  A chunk of K steps is captured
 // once as a CUDA graph and replayed; the member table (ping-pong parity and
 // noise counters) is refreshed in device memory before each replay, so the
@@ -20,11 +20,6 @@
 #include "../../include/tcym.h"
 #include "tcym_batch.cuh"
 #include "tcym_internal.h"
-
-// TCYM_BATCH_PERSISTENT (tcym_batch.cuh) 0, the default: one block per work
-// item, scheduled by the hardware, so the formats' launches interleave on the
-// SMs and tails fill; 1: one wave of resident blocks walking the work items
-// (measured 6% slower on a 256-member mixed ensemble).
 
 using namespace tcym;
 
@@ -42,8 +37,12 @@ struct FmtGroup {
     void *d_members = nullptr;   // device Member<T> table
     size_t d_bytes = 0;
     std::vector<char> h_members; // host copy of the table
-    int total_blocks = 0, red_total = 0, grid = 0, red_grid = 0, red_offset = 0;
-    bool general = false;        // some member is unpaired or tiled: the general batch kernel
+    // step work items: those of the paired members first (idx is ordered so), then from
+    // pair_blocks on those of the members stepped per site, the first of them npaired
+    int total_blocks = 0, pair_blocks = 0, npaired = 0;
+    size_t march_smem = 0;       // shared memory of the FP64 step's blocks (the largest)
+    int red_total = 0, red_grid = 0, red_offset = 0;
+    bool tiled = false;          // some paired member is tiled: the kernel that reads every member's tiling
     // runs of members (idx is ordered by coefficients) that share the mode, force, staple
     // and link factors: each steps in one launch with them as kernel parameters
     struct Class {
@@ -97,10 +96,11 @@ struct tcym_ensemble_s {
 
 template <int FMT> static void fill_group(tcym_ensemble ens, FmtGroup &G, int sm_count) {
     using T = typename Fmt<FMT>::T;
-    constexpr int TPB = threads_for<FMT>();
     std::vector<Member<T>> tab(G.idx.size());
     int blk = 0, red = 0;
-    G.general = false;
+    G.tiled = false;
+    G.pair_blocks = G.npaired = 0;
+    G.march_smem = 0;
     G.classes.clear();
     G.member_block.assign(G.idx.size(), 0);
     for (size_t i = 0; i < G.idx.size(); ++i) {
@@ -114,19 +114,31 @@ template <int FMT> static void fill_group(tcym_ensemble ens, FmtGroup &G, int sm
         m.result = L->result;
         const StepCoef<double> cd = tcym_coef(L->a, em.mode, em.dt, em.gamma, em.T, em.seed, em.next_step);
         m.c = coef_cast<T>(cd);
-        const FmtGroup::Class *last = G.classes.empty() ? nullptr : &G.classes.back();
-        if (!last || cd.mode != last->coef.mode || std::memcmp(cd.fc, last->coef.fc, sizeof cd.fc) ||
-            std::memcmp(cd.cnu, last->coef.cnu, sizeof cd.cnu) || std::memcmp(cd.uc, last->coef.uc, sizeof cd.uc))
-            G.classes.push_back(FmtGroup::Class{cd, (int)i, (int)i, blk, blk});
         m.cur = L->cur;
         m.block_begin = blk;
         G.member_block[i] = blk;
-        m.paired = Fmt<FMT>::PAIRED && L->g.nz % 2 == 0;
-        m.tile = m.paired ? tcym_lattice_tile_of(L) : Tile{0, 0, 0, 0, 0, 0};
-        if (!m.paired || m.tile.tx != 0) G.general = true;
-        blk += m.paired ? (int)tile_blocks(L->g, m.tile) : grid_for(L->g.V, TPB);
-        G.classes.back().m1 = (int)i + 1;
-        G.classes.back().item1 = blk;
+        m.paired = Launch<FMT>::paired_step(L->g);
+        m.tile = Tile{0, 0, 0, 0, 0, 0};
+        m.march = MarchTile{};
+        if (m.paired) {
+            const FmtGroup::Class *last = G.classes.empty() ? nullptr : &G.classes.back();
+            if (!last || cd.mode != last->coef.mode || std::memcmp(cd.fc, last->coef.fc, sizeof cd.fc) ||
+                std::memcmp(cd.cnu, last->coef.cnu, sizeof cd.cnu) || std::memcmp(cd.uc, last->coef.uc, sizeof cd.uc))
+                G.classes.push_back(FmtGroup::Class{cd, (int)i, (int)i, blk, blk});
+            m.tile = tcym_lattice_tile_of(L);
+            if (m.tile.tx != 0) G.tiled = true;
+            blk += (int)tile_blocks(L->g, m.tile);
+            G.classes.back().m1 = (int)i + 1;
+            G.classes.back().item1 = blk;
+            G.npaired = (int)i + 1;
+            G.pair_blocks = blk;
+        } else {
+            if (!Fmt<FMT>::PAIRED) {
+                m.march = tcym_lattice_march_of(L, true);
+                G.march_smem = std::max(G.march_smem, march_smem<Fmt<FMT>>(m.march));
+            }
+            blk += LaunchBatch<FMT>::site_items(L->g, m.march);
+        }
         m.red_begin = red;
         m.red_blocks = member_records(m.paired, L->g.V);
         red += m.red_blocks;
@@ -134,11 +146,6 @@ template <int FMT> static void fill_group(tcym_ensemble ens, FmtGroup &G, int sm
     }
     G.total_blocks = blk;
     G.red_total = red;
-#if TCYM_BATCH_PERSISTENT
-    G.grid = std::max(1, std::min(blk, sm_count * LaunchBatch<FMT>::resident_blocks()));
-#else
-    G.grid = std::max(1, blk);
-#endif
     G.red_grid = std::max(1, std::min(red, sm_count * 8));
     G.h_members.resize(sizeof(Member<T>) * tab.size());
     if (!tab.empty()) std::memcpy(G.h_members.data(), tab.data(), G.h_members.size());
@@ -147,12 +154,13 @@ template <int FMT> static void fill_group(tcym_ensemble ens, FmtGroup &G, int sm
 static void fill_all(tcym_ensemble ens) {
     for (int f = 0; f < 4; ++f) ens->groups[f].idx.clear();
     for (size_t i = 0; i < ens->members.size(); ++i) ens->groups[ens->members[i].lat->fmt].idx.push_back((int)i);
-    // members with the same step coefficients next to each other (mode, dt, spacings decide them)
+    // paired members first, and members with the same step coefficients next to each other
+    // (mode, dt, spacings decide them)
     for (auto &G : ens->groups)
         std::stable_sort(G.idx.begin(), G.idx.end(), [&](int x, int y) {
             const EnsMember &a = ens->members[x], &b = ens->members[y];
-            return std::make_tuple(a.mode, a.dt, a.lat->a[0], a.lat->a[1], a.lat->a[2]) <
-                   std::make_tuple(b.mode, b.dt, b.lat->a[0], b.lat->a[1], b.lat->a[2]);
+            return std::make_tuple(a.lat->g.nz % 2, a.mode, a.dt, a.lat->a[0], a.lat->a[1], a.lat->a[2]) <
+                   std::make_tuple(b.lat->g.nz % 2, b.mode, b.dt, b.lat->a[0], b.lat->a[1], b.lat->a[2]);
         });
     const int sm = ens->ctx->sm_count;
     fill_group<FMT_SU2_F32>(ens, ens->groups[FMT_SU2_F32], sm);
@@ -238,23 +246,27 @@ template <int FMT> static cudaError_t launch_group_step(tcym_ensemble ens, int f
     using T = typename Fmt<FMT>::T;
     const FmtGroup &G = ens->groups[f];
     const Member<T> *table = static_cast<const Member<T> *>(G.d_members);
+    cudaError_t e = cudaSuccess;
     if constexpr (Fmt<FMT>::PAIRED) {
-        if (!G.general) {
-            for (const FmtGroup::Class &c : G.classes) {
-                const cudaError_t e =
-                    LaunchBatch<FMT>::step_uniform(table, c.m0, c.m1 - c.m0, c.item0, c.item1, k, c.coef, s);
-                if (e != cudaSuccess) return e;
-            }
-            return cudaSuccess;
+        if (G.tiled) {
+            e = LaunchBatch<FMT>::step(table, G.npaired, G.pair_blocks, k, s);
+        } else {
+            for (const FmtGroup::Class &c : G.classes)
+                if (e == cudaSuccess)
+                    e = LaunchBatch<FMT>::step_uniform(table, c.m0, c.m1 - c.m0, c.item0, c.item1, k, c.coef, s);
         }
     }
-    return LaunchBatch<FMT>::step(table, (int)G.idx.size(), G.total_blocks, k, G.grid, G.general, s);
+    const int n = (int)G.idx.size();
+    if (e == cudaSuccess && n > G.npaired)
+        e = LaunchBatch<FMT>::sites(table, G.npaired, n - G.npaired, G.pair_blocks, G.total_blocks, k, G.march_smem, s);
+    return e;
 }
 
 // Does format f step by persistent K-step launches?
 static bool persistent_format(tcym_ensemble ens, int f) {
     const FmtGroup &G = ens->groups[f];
-    return ens->persistent && (f == FMT_SU2_F32 || f == FMT_SU3_F32) && !G.general && !G.idx.empty();
+    return ens->persistent && (f == FMT_SU2_F32 || f == FMT_SU3_F32) && !G.tiled && !G.idx.empty() &&
+           G.npaired == (int)G.idx.size();
 }
 
 // Schedules and control words of the persistent launches for chunks of nsteps

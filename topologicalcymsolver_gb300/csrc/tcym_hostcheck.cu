@@ -10,7 +10,7 @@
 #include <vector>
 
 #include "tcym_pipeline.h"
-#include "tcym_site.cuh"
+#include "tcym_march.cuh"
 
 using namespace tcym;
 
@@ -68,11 +68,39 @@ template <int FMT> struct H {
                 return;
             }
         }
-        for (int64_t s = 0; s < g.V; ++s) {
+        if (!doE) {
+            for (int64_t s = 0; s < g.V; ++s) site_update_u<F>(g, Uout, E, c, s);
+            return;
+        }
+        sites(g, Uin, Uout, E, c, doU, SiteRange{0, g.nz, 0, g.V});
+    }
+    // the per-site step as Launch::step_sites runs it
+    static void sites(const Geom &g, const void *Uin, void *Uout, void *E, const StepCoef<T> &c, bool doU,
+                      const SiteRange &r) {
+        if constexpr (F::PAIRED) {
             T sm[3 * F::NA];
-            if (doE && doU) site_step<F, true, true>(g, Uin, Uout, E, c, s, 0, sm, 1);
-            else if (doE) site_step<F, true, false>(g, Uin, Uout, E, c, s, 0, sm, 1);
-            else site_step<F, false, true>(g, Uin, Uout, E, c, s, 0, sm, 1);
+            for (int64_t s = r.s0; s < r.s1; ++s) {
+                if (doU) site_step<F, true>(g, Uin, Uout, E, c, s, 0, sm, 1);
+                else site_step<F, false>(g, Uin, Uout, E, c, s, 0, sm, 1);
+            }
+        } else {
+            march(g, Uin, Uout, E, c, doU, r, march_tile(g, 152));
+        }
+    }
+    // the device's FP64 step, block by block, phase by phase and thread by thread
+    static void march(const Geom &g, const void *Uin, void *Uout, void *E, const StepCoef<T> &c, bool doU,
+                      const SiteRange &r, const MarchTile &t) {
+        std::vector<unsigned char> sm(march_smem<F>(t));
+        for (int64_t b = 0; b < march_blocks(t, r.z1 - r.z0); ++b) {
+            const March<F> m(g, Uin, t, r, b, sm.data());
+            for (int i = 0; i < t.threads; ++i) m.setup(i, t.threads);
+            for (int z = m.z0; z < m.z1; ++z) {
+                for (int i = 0; i < t.threads; ++i) m.projections(z, i, t.threads);
+                for (int i = 0; i < t.threads; ++i) {
+                    if (doU) m.template links<true>(z, i, t.threads, Uout, E, c, r, 0);
+                    else m.template links<false>(z, i, t.threads, Uout, E, c, r, 0);
+                }
+            }
         }
     }
     // one fused step of the storage indices [i0, i1) as Launch::step_range runs it: the
@@ -95,10 +123,8 @@ template <int FMT> struct H {
                 return;
             }
         }
-        for (int64_t s = i0; s < i1; ++s) {
-            T sm[3 * F::NA];
-            site_step<F, true, true>(g, Uin, Uout, E, c, s, 0, sm, 1);
-        }
+        const int64_t plane = (int64_t)g.nx * g.ny;
+        sites(g, Uin, Uout, E, c, true, SiteRange{(int)(i0 / plane), (int)((i1 + plane - 1) / plane), i0, i1});
     }
     static void flow_cb(const Geom &g, void *U, double dtau, int nsweeps) {
         const T fc[3] = {T(-2), T(-2), T(-2)}, cn[3] = {T(1), T(1), T(1)}, uc[3] = {T(-dtau), T(-dtau), T(-dtau)};
@@ -272,6 +298,16 @@ int hc_step(int fmt, const int *n, const void *Uin, void *Uout, void *E, int mod
     Geom g = geom(n);
     StepCoef<double> c = coef(mode, dt, gamma, T, seed, step);
     HC_DISPATCH(fmt, HH::step(g, Uin, Uout, E, c, doE, doU, pairs));
+    return 0;
+}
+// one leapfrog step in blocks that share their plaquettes, with the tiling tx x ty, zl planes a block, `threads` threads
+// (tx 0: the rule for a device of `threads` multiprocessors, 0: among others)
+int hc_march(int fmt, const int *n, const void *Uin, void *Uout, void *E, double dt, int tx, int ty, int zl,
+             int threads) {
+    Geom g = geom(n);
+    StepCoef<double> c = coef(MODE_LEAPFROG, dt, 0, 0, 0, 0);
+    const MarchTile t = tx ? MarchTile{tx, ty, (g.nx + tx - 1) / tx, (g.ny + ty - 1) / ty, zl, threads} : march_tile(g, threads);
+    HC_DISPATCH(fmt, HH::march(g, Uin, Uout, E, cast<HH::T>(c), true, SiteRange{0, g.nz, 0, g.V}, t));
     return 0;
 }
 int hc_flow_cb(int fmt, const int *n, void *U, double dtau, int nsweeps) {

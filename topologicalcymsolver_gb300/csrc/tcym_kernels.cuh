@@ -9,6 +9,7 @@
 
 #include <cuda_runtime.h>
 
+#include "tcym_march.cuh"
 #include "tcym_site.cuh"
 
 namespace tcym {
@@ -31,15 +32,10 @@ enum : int {
 constexpr int kThreadsSU2 = TCYM_SU2_THREADS;
 constexpr int kThreadsSU3 = 128;
 constexpr int kRedThreads = 256;
-// Resident blocks per SM requested for the step kernels (register cap = 65536 / (blocks * threads)).
-#ifndef TCYM_SU3_STEP_MINBLOCKS
-#define TCYM_SU3_STEP_MINBLOCKS 4
-#endif
-#ifndef TCYM_SU2_STEP_MINBLOCKS
-#define TCYM_SU2_STEP_MINBLOCKS 8
-#endif
+// Resident blocks per SM requested for the per-site FP32 step and the checkerboard flow
+// (register cap = 65536 / (blocks * threads)).
 template <int FMT> constexpr int min_blocks_for() {
-    return Fmt<FMT>::NA == 8 ? TCYM_SU3_STEP_MINBLOCKS : (FMT == FMT_SU2_F32 ? TCYM_SU2_STEP_MINBLOCKS : 1);
+    return Fmt<FMT>::NA == 8 ? 4 : (FMT == FMT_SU2_F32 ? 8 : 1);
 }
 
 template <int FMT> constexpr int threads_for() { return Fmt<FMT>::NA == 3 ? kThreadsSU2 : kThreadsSU3; }
@@ -127,18 +123,50 @@ template <class T> StepCoef<T> coef_cast(const StepCoef<double> &c) {
 }
 
 // ------------------------------------------------------------------ kernels
-// sites [s0, s1)
 // shared-memory slots of the plaquette projections (site_step, site_step_pair)
 template <int FMT> constexpr int plaq_slots() { return 3 * Fmt<FMT>::NA; }
 
-template <int FMT, bool DO_E, bool DO_U>
+// the per-site FP32 step (odd nz; DO_U false: the E update alone), sites [s0, s1)
+template <int FMT, bool DO_U>
 __global__ void __launch_bounds__(threads_for<FMT>(), min_blocks_for<FMT>()) k_step(Geom g, const void *Uin, void *Uout, void *E,
-                                                             StepCoef<typename Fmt<FMT>::T> c, int64_t s0, int64_t s1) {
-    using T = typename Fmt<FMT>::T;
-    __shared__ T sm[DO_E ? plaq_slots<FMT>() * threads_for<FMT>() : 1];
+                                                             StepCoef<float> c, int64_t s0, int64_t s1) {
+    static_assert(Fmt<FMT>::PAIRED, "the FP64 formats step through k_march");
+    __shared__ float sm[plaq_slots<FMT>() * threads_for<FMT>()];
     const int64_t s = s0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= s1) return;
-    site_step<Fmt<FMT>, DO_E, DO_U>(g, Uin, Uout, E, c, s, 0, sm + threadIdx.x, threads_for<FMT>());
+    site_step<Fmt<FMT>, DO_U>(g, Uin, Uout, E, c, s, 0, sm + threadIdx.x, threads_for<FMT>());
+}
+
+// One block of the FP64 step (tcym_march.cuh): phases 1 and 2 of each of its planes.
+template <class F, bool DO_U>
+__device__ __forceinline__ void march_block(const Geom &g, const void *Uin, void *Uout, void *E,
+                                            const StepCoef<typename F::T> &c, const MarchTile &t, const SiteRange &r,
+                                            int64_t block, uint64_t step_add) {
+    extern __shared__ __align__(16) unsigned char march_sh[];
+    const March<F> m(g, Uin, t, r, block, march_sh);
+    const int tid = threadIdx.x, nt = blockDim.x;
+    m.setup(tid, nt);
+    __syncthreads();
+    for (int z = m.z0; z < m.z1; ++z) {
+        m.projections(z, tid, nt);
+        __syncthreads();
+        m.template links<DO_U>(z, tid, nt, Uout, E, c, r, step_add);
+        __syncthreads();
+    }
+}
+// Resident blocks of kMarchThreads per SM: two at 128 registers for SU(3) (FP64 keeps 72
+// bytes of spills; at one block, 255 registers, the FP64 unit is not kept busy), three for SU(2).
+template <int FMT> constexpr int march_min_blocks() { return Fmt<FMT>::NA == 8 ? 2 : 3; }
+// DO_U: the whole step, the new links into Uout; else the E update alone
+template <int FMT, bool DO_U>
+__global__ void __launch_bounds__(kMarchThreads, march_min_blocks<FMT>())
+    k_march(Geom g, const void *Uin, void *Uout, void *E, StepCoef<typename Fmt<FMT>::T> c, MarchTile t, SiteRange r) {
+    march_block<Fmt<FMT>, DO_U>(g, Uin, Uout, E, c, t, r, blockIdx.x, 0);
+}
+template <int FMT> __global__ void __launch_bounds__(128) k_update_u(Geom g, void *U, const void *E,
+                                                                     StepCoef<typename Fmt<FMT>::T> c) {
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < g.V) site_update_u<Fmt<FMT>>(g, U, E, c, s);
 }
 
 // one thread per site pair (FP32 formats, even nz); blocks touching the seam
@@ -651,22 +679,41 @@ template <int FMT> struct Launch {
     static constexpr int FMT_ID = FMT;
     static constexpr int TPB = threads_for<FMT>();
 
-    // t: the block tiling of the paired step (FP32 formats with even nz)
-    static cudaError_t step(const Geom &g, const void *Uin, void *Uout, void *E, const StepCoef<double> &cd, bool doE,
-                            bool doU, cudaStream_t st, const Tile &t = Tile{0, 0, 0, 0, 0, 0}) {
-        StepCoef<T> c = coef_cast<T>(cd);
+    // One fused step (E and links).  t: the block tiling of the paired step (FP32
+    // formats with even nz), m: of the FP64 step.
+    static cudaError_t step(const Geom &g, const void *Uin, void *Uout, void *E, const StepCoef<double> &cd, const Tile &t,
+                            const MarchTile &m, cudaStream_t st) {
         if constexpr (F::PAIRED) {
-            if (doE && doU && g.nz % 2 == 0) {
+            if (paired_step(g)) {
+                const StepCoef<T> c = coef_cast<T>(cd);
                 const unsigned blocks = (unsigned)tile_blocks(g, t);
                 if (t.tx) k_step_pair<FMT, true><<<blocks, kThreadsPair, 0, st>>>(g, Uin, Uout, E, c, t);
                 else k_step_pair<FMT, false><<<blocks, kThreadsPair, 0, st>>>(g, Uin, Uout, E, c, t);
                 return cudaGetLastError();
             }
         }
-        int grid = grid_for(g.V, TPB);
-        if (doE && doU) k_step<FMT, true, true><<<grid, TPB, 0, st>>>(g, Uin, Uout, E, c, 0, g.V);
-        else if (doE) k_step<FMT, true, false><<<grid, TPB, 0, st>>>(g, Uin, Uout, E, c, 0, g.V);
-        else k_step<FMT, false, true><<<grid, TPB, 0, st>>>(g, Uin, Uout, E, c, 0, g.V);
+        return step_sites<true>(g, Uin, Uout, E, cd, m, SiteRange{0, g.nz, 0, g.V}, st);
+    }
+    // the E update alone, per site
+    static cudaError_t update_e(const Geom &g, const void *U, void *E, const StepCoef<double> &cd, const MarchTile &m,
+                                cudaStream_t st) {
+        return step_sites<false>(g, U, nullptr, E, cd, m, SiteRange{0, g.nz, 0, g.V}, st);
+    }
+    static cudaError_t update_u(const Geom &g, void *U, const void *E, const StepCoef<double> &cd, cudaStream_t st) {
+        k_update_u<FMT><<<grid_for(g.V, 128), 128, 0, st>>>(g, U, E, coef_cast<T>(cd));
+        return cudaGetLastError();
+    }
+    // the sites of r (r.z0, r.z1: its planes), per site
+    template <bool DO_U>
+    static cudaError_t step_sites(const Geom &g, const void *Uin, void *Uout, void *E, const StepCoef<double> &cd,
+                                  const MarchTile &m, const SiteRange &r, cudaStream_t st) {
+        const StepCoef<T> c = coef_cast<T>(cd);
+        if constexpr (F::PAIRED) {
+            k_step<FMT, DO_U><<<grid_for(r.s1 - r.s0, TPB), TPB, 0, st>>>(g, Uin, Uout, E, c, r.s0, r.s1);
+        } else {
+            const unsigned blocks = (unsigned)march_blocks(m, r.z1 - r.z0);
+            k_march<FMT, DO_U><<<blocks, m.threads, march_smem<F>(m), st>>>(g, Uin, Uout, E, c, m, r);
+        }
         return cudaGetLastError();
     }
     // Does step() take the paired kernel (one thread per site pair)?
@@ -675,19 +722,19 @@ template <int FMT> struct Launch {
     // pairs when paired_step(g), else sites; i0 a multiple of 128 for pairs.
     // The linear block mapping.
     static cudaError_t step_range(const Geom &g, const void *Uin, void *Uout, void *E, const StepCoef<double> &cd,
-                                  int64_t i0, int64_t i1, cudaStream_t st) {
-        StepCoef<T> c = coef_cast<T>(cd);
+                                  int64_t i0, int64_t i1, const MarchTile &m, cudaStream_t st) {
         if (i1 <= i0) return cudaSuccess;
         if constexpr (F::PAIRED) {
             if (paired_step(g)) {
                 Tile t{0, 0, 0, 0, 0, (int)(i0 / kThreadsPair)};
                 const unsigned blocks = (unsigned)((i1 - i0 + kThreadsPair - 1) / kThreadsPair);
-                k_step_pair<FMT, false><<<blocks, kThreadsPair, 0, st>>>(g, Uin, Uout, E, c, t);
+                k_step_pair<FMT, false><<<blocks, kThreadsPair, 0, st>>>(g, Uin, Uout, E, coef_cast<T>(cd), t);
                 return cudaGetLastError();
             }
         }
-        k_step<FMT, true, true><<<grid_for(i1 - i0, TPB), TPB, 0, st>>>(g, Uin, Uout, E, c, i0, i1);
-        return cudaGetLastError();
+        const int64_t plane = (int64_t)g.nx * g.ny;
+        return step_sites<true>(g, Uin, Uout, E, cd, m,
+                           SiteRange{(int)(i0 / plane), (int)((i1 + plane - 1) / plane), i0, i1}, st);
     }
     static cudaError_t flow_cb(const Geom &g, void *U, int parity, int mu, const double *fc, const double *cn,
                                const double *uc, cudaStream_t st) {

@@ -289,6 +289,13 @@ template <class T> struct SU2 {
         const Mat w = mulx<false, true>(a, b);
         proj(w, out);
     }
+    // p = proj(a b^dag) / kLoopScale for group elements a, b (a plaquette's two halves):
+    // the vector part of the product, its sign left to the scale
+    static constexpr double kLoopScale = -1.0;
+    static TCYM_HD void loop_proj(const Mat &a, const Mat &b, T *p) {
+        const Mat w = mulx<false, true>(a, b);
+        p[0] = w.q[0]; p[1] = w.q[1]; p[2] = w.q[2];
+    }
     // components of V^dagger (e^a t^a) V for a group element V: the rotation
     // e + 2 (v3 q x e + q x (q x e)) of its vector part q
     static TCYM_HD void transport(const Mat &v, const T *e, T *out) {
@@ -484,6 +491,35 @@ template <class T> struct SU3 {
                 }
             }
         proj(w, p);
+    }
+    // p = proj(a b^dag) / kLoopScale for group elements a (rows 0 and 1 are read) and b:
+    // rows 0 and 1 of the product are formed, and of its row 2 = conj(row0 x row1) the
+    // parts that proj reads
+    static constexpr double kLoopScale = -0.5;
+    static TCYM_HD void loop_proj(const Mat &a, const Mat &b, T *p) {
+        cx<T> w[2][3];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                cx<T> acc{a.m[i][0].re * b.m[j][0].re, a.m[i][0].im * b.m[j][0].re};
+                acc.re = fma(a.m[i][0].im, b.m[j][0].im, acc.re);
+                acc.im = fma(-a.m[i][0].re, b.m[j][0].im, acc.im);
+                acc = cfma_nc(a.m[i][1], b.m[j][1], acc);
+                w[i][j] = cfma_nc(a.m[i][2], b.m[j][2], acc);
+            }
+        const cx<T> w20 = conj_cross(w[0][1], w[1][2], w[0][2], w[1][1]);
+        const cx<T> w21 = conj_cross(w[0][2], w[1][0], w[0][0], w[1][2]);
+        const T w22 = conj_cross(w[0][0], w[1][1], w[0][1], w[1][0]).im;
+        const T is3 = T(0.57735026918962576450914878050196);
+        p[0] = w[0][1].im + w[1][0].im;
+        p[1] = w[0][1].re - w[1][0].re;
+        p[2] = w[0][0].im - w[1][1].im;
+        p[3] = w[0][2].im + w20.im;
+        p[4] = w[0][2].re - w20.re;
+        p[5] = w[1][2].im + w21.im;
+        p[6] = w[1][2].re - w21.re;
+        p[7] = is3 * fma(T(-2), w22, w[0][0].im + w[1][1].im);
     }
     // components of V^dagger (e^a t^a) V for a group element V.  With H = 2 e^a t^a,
     // only columns 0 and 1 of H V are formed: the entries below the diagonal and the

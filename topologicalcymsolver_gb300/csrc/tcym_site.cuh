@@ -119,11 +119,9 @@ TCYM_HD void add_plaquette_force(const T *sm, int stride, int mu, const C (&cnu)
     for (int a = 0; a < NA; ++a) f[a] = fma(cp, sm[(mu * NA + a) * stride], fma(-cm, sm[(n2 * NA + a) * stride], f[a]));
 }
 
-// One site of a step.  DO_E: compute the force and update E; DO_U: move the
-// links by exp(i uc E) and write them to Uout (Uout may alias Uin only when
-// DO_E is false, i.e. for the pointwise link update).  sm: 3 * NA slots of T
-// for this site, stride apart (used when DO_E).
-template <class F, bool DO_E, bool DO_U>
+// One site of the FP32 formats' per-site step (odd nz; DO_U false: the E update alone,
+// Uout unused).  sm: 3 * NA slots of T for this site, stride apart.
+template <class F, bool DO_U>
 TCYM_HD void site_step(const Geom &g, const void *Uin, void *Uout, void *E, const StepCoef<typename F::T> &c,
                        int64_t s, uint64_t step_add, typename F::T *sm, int stride) {
     using G = typename F::G;
@@ -132,44 +130,44 @@ TCYM_HD void site_step(const Geom &g, const void *Uin, void *Uout, void *E, cons
     constexpr int NA = F::NA;
     const int64_t V = g.V;
     Nbhd nb(g, s);
-    if (DO_E) {
-        // link along d at x (a = 0) or at x + e_dir (a = 1)
-        auto load = [&](int d, int a, int dir) { return F::load(Uin, V, d, a ? nb.at(dir, 1) : s); };
-        plaquette_projections<F, M>(load, sm, stride);
-    }
+    // link along d at x (a = 0) or at x + e_dir (a = 1)
+    auto load = [&](int d, int a, int dir) { return F::load(Uin, V, d, a ? nb.at(dir, 1) : s); };
+    plaquette_projections<F, M>(load, sm, stride);
 #pragma unroll 1
     for (int mu = 0; mu < 3; ++mu) {
         T e[NA];
-        M u;
-        if (DO_E) {
-            const M A = lower_staple_sum<F>(Uin, V, nb, mu, c.cnu);
-            u = F::load(Uin, V, mu, s);
-            F::load_e(E, V, mu, s, e);
-            T f[NA];
-            G::proj_mul(u, A, f);
-            add_plaquette_force<NA>(sm, stride, mu, c.cnu, f);
-            const T fc = sel3(c.fc, mu);
-            if (c.mode == MODE_LANGEVIN) {
-                T xi[NA];
-                normals<T, NA>(c.seed, STREAM_NOISE, c.step + step_add, (uint32_t)s, (uint32_t)mu, xi);
-                const T damp = sel3(c.damp, mu), kick = sel3(c.kick, mu);
+        const M A = lower_staple_sum<F>(Uin, V, nb, mu, c.cnu);
+        const M u = F::load(Uin, V, mu, s);
+        F::load_e(E, V, mu, s, e);
+        T f[NA];
+        G::proj_mul(u, A, f);
+        add_plaquette_force<NA>(sm, stride, mu, c.cnu, f);
+        const T fc = sel3(c.fc, mu);
+        if (c.mode == MODE_LANGEVIN) {
+            T xi[NA];
+            normals<T, NA>(c.seed, STREAM_NOISE, c.step + step_add, (uint32_t)s, (uint32_t)mu, xi);
+            const T damp = sel3(c.damp, mu), kick = sel3(c.kick, mu);
 #pragma unroll
-                for (int a = 0; a < NA; ++a) e[a] = e[a] + (fc * f[a] - damp * e[a] + kick * xi[a]);
-            } else if (c.mode == MODE_FLOW) {
+            for (int a = 0; a < NA; ++a) e[a] = e[a] + (fc * f[a] - damp * e[a] + kick * xi[a]);
+        } else if (c.mode == MODE_FLOW) {
 #pragma unroll
-                for (int a = 0; a < NA; ++a) e[a] = fc * f[a];
-            } else {
-#pragma unroll
-                for (int a = 0; a < NA; ++a) e[a] = e[a] + fc * f[a];
-            }
-            F::store_e(E, V, mu, s, e);
+            for (int a = 0; a < NA; ++a) e[a] = fc * f[a];
         } else {
-            u = F::load(Uin, V, mu, s);
-            F::load_e(E, V, mu, s, e);
+#pragma unroll
+            for (int a = 0; a < NA; ++a) e[a] = e[a] + fc * f[a];
         }
-        if (DO_U) {
-            F::store(Uout, V, mu, s, G::iexp_mul(sel3(c.uc, mu), e, u));
-        }
+        F::store_e(E, V, mu, s, e);
+        if (DO_U) F::store(Uout, V, mu, s, G::iexp_mul(sel3(c.uc, mu), e, u));
+    }
+}
+
+// The link update alone: U_mu(s) <- exp(i uc E_mu(s)) U_mu(s), in place.
+template <class F> TCYM_HD void site_update_u(const Geom &g, void *U, const void *E, const StepCoef<typename F::T> &c, int64_t s) {
+#pragma unroll 1
+    for (int mu = 0; mu < 3; ++mu) {
+        typename F::T e[F::NA];
+        F::load_e(E, g.V, mu, s, e);
+        F::store(U, g.V, mu, s, F::G::iexp_mul(sel3(c.uc, mu), e, F::load(U, g.V, mu, s)));
     }
 }
 
@@ -186,9 +184,9 @@ TCYM_COLD void langevin_kick_pair(const StepCoef<float> &c, int mu, int64_t p, i
     for (int a = 0; a < NA; ++a) e[a] = e[a] + fma(kick, f2(x0[a], x1[a]), fma(-damp, e[a], fc * f[a]));
 }
 
-// site_step for both sites of pair p of an FP32 lattice with even nz, (x,y,z)
-// and (x,y,z+nz/2), in packed FP32 (f2): the same plaquettes, staples,
-// projections, E update and exponential per lane, at half the instructions.
+// A step of both sites of pair p of an FP32 lattice with even nz, (x,y,z) and
+// (x,y,z+nz/2), in packed FP32 (f2): the plaquettes, staples, projections, E update
+// and exponential of both at half the instructions.
 // SEAM: the pair may touch the seam z = nz/2, across which neighbour pairs
 // arrive with their lanes swapped; pairs away from it skip the swap tests.
 // cn: the Langevin noise's coefficients (seed, step, damping, kick), which may
