@@ -128,6 +128,19 @@ template <int FMT> struct H {
     }
     static void flow_cb(const Geom &g, void *U, double dtau, int nsweeps) {
         const T fc[3] = {T(-2), T(-2), T(-2)}, cn[3] = {T(1), T(1), T(1)}, uc[3] = {T(-dtau), T(-dtau), T(-dtau)};
+        if constexpr (F::PAIRED) {
+            if (g.nz % 4 == 0) {  // pairs of one parity, as the device takes them
+                const int64_t plane = (int64_t)g.nx * g.ny, Vh = g.V >> 1;
+                for (int k = 0; k < 6 * nsweeps; ++k)
+                    for (int64_t p = 0; p < Vh; ++p) {
+                        Nbhd nb(g, p);
+                        if (nb.parity() != k / 3 % 2) continue;
+                        if (p < plane || p >= Vh - plane) pair_link_flow<F, true>(g, U, k % 3, fc, cn, uc, p);
+                        else pair_link_flow<F, false>(g, U, k % 3, fc, cn, uc, p);
+                    }
+                return;
+            }
+        }
         for (int sw = 0; sw < nsweeps; ++sw)
             for (int p = 0; p < 2; ++p)
                 for (int mu = 0; mu < 3; ++mu)

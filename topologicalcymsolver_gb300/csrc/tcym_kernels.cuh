@@ -196,15 +196,14 @@ __global__ void __launch_bounds__(kThreadsPair, pair_min_blocks_for<FMT>())
 #endif
 }
 
-// sites of parity p, for even extents: t -> (x, row) with x of the right parity
+// Checkerboard sub-sweep of (parity, mu): the sites of the parity, for even extents,
+// t -> (x, row) with x of the right parity
+template <class T> struct FlowCoefT {
+    T fc[3], cn[3], uc[3];
+};
 template <int FMT>
 __global__ void __launch_bounds__(threads_for<FMT>(), min_blocks_for<FMT>()) k_flow_cb(Geom g, void *U, int parity, int mu,
-                                                                typename Fmt<FMT>::T fc0, typename Fmt<FMT>::T fc1,
-                                                                typename Fmt<FMT>::T fc2, typename Fmt<FMT>::T cn0,
-                                                                typename Fmt<FMT>::T cn1, typename Fmt<FMT>::T cn2,
-                                                                typename Fmt<FMT>::T uc0, typename Fmt<FMT>::T uc1,
-                                                                typename Fmt<FMT>::T uc2) {
-    using T = typename Fmt<FMT>::T;
+                                                                FlowCoefT<typename Fmt<FMT>::T> c) {
     int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= g.V / 2) return;
     const int hx = g.nx / 2;
@@ -213,8 +212,27 @@ __global__ void __launch_bounds__(threads_for<FMT>(), min_blocks_for<FMT>()) k_f
     int y = (int)(row % g.ny), z = (int)(row / g.ny);
     int x = 2 * xh + ((y + z + parity) & 1);
     int64_t s = x + (int64_t)g.nx * row;
-    const T fc[3] = {fc0, fc1, fc2}, cn[3] = {cn0, cn1, cn2}, uc[3] = {uc0, uc1, uc2};
-    link_flow<Fmt<FMT>>(g, U, mu, fc, cn, uc, s);
+    link_flow<Fmt<FMT>>(g, U, mu, c.fc, c.cn, c.uc, s);
+}
+// FP32 pair storage with nz / 2 even (a pair's sites have one parity): a thread per pair,
+// a block a tile of 8 pairs of the parity x 4 rows x 4 planes.  It waits for links from
+// L2 (13 of them a thread), of which the tile finds its neighbours' in L1.  A sweep (six
+// sub-sweeps) on GB300: SU(2) 96^3 149 us per site (one lane of every pair vector, twice the
+// sectors), 92 us by pairs in index order, 76 us by tiles; SU(3) 96^3 522 / 258 / 256 us.
+// (16 x 4 x 2: 75 and 250 us, but half idle at nx = 16.)
+constexpr int kCbX = 8, kCbY = 4, kCbZ = 4;
+static_assert(kCbX * kCbY * kCbZ == kThreadsPair, "a block is a tile");
+template <int FMT>
+__global__ void __launch_bounds__(kThreadsPair, Fmt<FMT>::NA == 8 ? 4 : 8)
+    k_flow_cb_pair(Geom g, void *U, int parity, int mu, FlowCoefT<float> c) {
+    const int i = threadIdx.x, nzh = g.nz >> 1;
+    const int xh = blockIdx.x * kCbX + i % kCbX, y = blockIdx.y * kCbY + i / kCbX % kCbY;
+    const int z0 = blockIdx.z * kCbZ, z = z0 + i / (kCbX * kCbY);
+    if (2 * xh >= g.nx || y >= g.ny || z >= nzh) return;
+    const int64_t p = 2 * xh + ((y + z + parity) & 1) + (int64_t)g.nx * (y + (int64_t)g.ny * z);
+    // block-uniform: does the block hold a plane next to the seam?
+    if (z0 == 0 || z0 + kCbZ >= nzh) pair_link_flow<Fmt<FMT>, true>(g, U, mu, c.fc, c.cn, c.uc, p);
+    else pair_link_flow<Fmt<FMT>, false>(g, U, mu, c.fc, c.cn, c.uc, p);
 }
 
 // block reduction helpers (FP64)
@@ -738,9 +756,17 @@ template <int FMT> struct Launch {
     }
     static cudaError_t flow_cb(const Geom &g, void *U, int parity, int mu, const double *fc, const double *cn,
                                const double *uc, cudaStream_t st) {
-        int grid = grid_for(g.V / 2, TPB);
-        k_flow_cb<FMT><<<grid, TPB, 0, st>>>(g, U, parity, mu, (T)fc[0], (T)fc[1], (T)fc[2], (T)cn[0], (T)cn[1],
-                                             (T)cn[2], (T)uc[0], (T)uc[1], (T)uc[2]);
+        FlowCoefT<T> c;
+        for (int i = 0; i < 3; ++i) { c.fc[i] = (T)fc[i]; c.cn[i] = (T)cn[i]; c.uc[i] = (T)uc[i]; }
+        if constexpr (F::PAIRED) {
+            if (g.nz % 4 == 0) {
+                const dim3 grid((unsigned)grid_for(g.nx / 2, kCbX), (unsigned)grid_for(g.ny, kCbY),
+                                (unsigned)grid_for(g.nz / 2, kCbZ));
+                k_flow_cb_pair<FMT><<<grid, kThreadsPair, 0, st>>>(g, U, parity, mu, c);
+                return cudaGetLastError();
+            }
+        }
+        k_flow_cb<FMT><<<grid_for(g.V / 2, TPB), TPB, 0, st>>>(g, U, parity, mu, c);
         return cudaGetLastError();
     }
     static int reduce_grid(const Geom &g, int max_blocks) {

@@ -330,6 +330,43 @@ TCYM_HD void link_flow(const Geom &g, void *U, int mu, const typename F::T (&fc)
     F::store(U, g.V, mu, s, G::iexp_mul(sel3(uc, mu), f, u));
 }
 
+// The same for both sites of pair p of FP32 pair storage with nz / 2 even, where the
+// partner (x, y, z + nz/2) has the parity of (x, y, z), in packed FP32.
+template <class F, bool SEAM>
+TCYM_HD void pair_link_flow(const Geom &g, void *U, int mu, const float (&fc)[3], const float (&cnu)[3],
+                            const float (&uc)[3], int64_t p) {
+    using G2 = typename F::G2;
+    using M2 = typename F::Mat2;
+    const int64_t Vh = g.V >> 1;
+    const PairNbhd nb(g, p);
+    M2 A = G2::zero();
+#pragma unroll 1
+    for (int k = 1; k <= 2; ++k) {
+        const int nu = mu + k >= 3 ? mu + k - 3 : mu + k;
+        const f2 c(sel3(cnu, nu));
+        {   // upper staple U_nu(x+mu) U_mu^dag(x+nu) U_nu^dag(x)
+            const M2 a1 = F::load2(U, Vh, nu, nb.at(mu, 1), SEAM && nb.swapped(mu, 1));
+            const M2 a2 = F::load2(U, Vh, mu, nb.at(nu, 1), SEAM && nb.swapped(nu, 1));
+            const M2 t = G2::template mulu<false, true>(a1, a2);
+            A = G2::add(A, G2::scale(c, G2::template mulu<false, true>(t, F::load2(U, Vh, nu, p, false))));
+        }
+        {   // lower staple U_nu^dag(x+mu-nu) U_mu^dag(x-nu) U_nu(x-nu)
+            const M2 b1 = F::load2(U, Vh, nu, nb.at(mu, 1, nu, -1), SEAM && nb.swapped(mu, 1, nu, -1));
+            const int64_t sb = nb.at(nu, -1);
+            const bool wb = SEAM && nb.swapped(nu, -1);
+            const M2 t = G2::template mulu<true, true>(b1, F::load2(U, Vh, mu, sb, wb));
+            A = G2::add(A, G2::scale(c, G2::template mulu<false, false>(t, F::load2(U, Vh, nu, sb, wb))));
+        }
+    }
+    const M2 u = F::load2(U, Vh, mu, p, false);
+    f2 f[F::NA];
+    G2::proj_mul(u, A, f);
+    const f2 fm(sel3(fc, mu));
+#pragma unroll
+    for (int a = 0; a < F::NA; ++a) f[a] = f[a] * fm;
+    F::store2(U, Vh, mu, p, G2::iexp_mul(f2(sel3(uc, mu)), f, u));
+}
+
 // ----------------------------------------------------------------- observables
 // Plaquette P_{mu nu}(x) in the four quadrants around x, each a loop from x
 // (Plaquettes.cpp:28-31):
