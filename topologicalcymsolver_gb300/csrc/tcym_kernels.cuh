@@ -196,6 +196,29 @@ __global__ void __launch_bounds__(kThreadsPair, pair_min_blocks_for<FMT>())
 #endif
 }
 
+// The paired step of a small lattice: a pair's three plaquettes, then its three links, by
+// three threads (warps 0, 1, 2 of a block of 32 pairs), the same arithmetic a third as
+// long.  Below about a wave of such blocks a step is the latency of one thread's work:
+// SU(3) at 24^3 13.4 us by k_step_pair on GB300.  split_step(): the lattices that take it.
+constexpr int kSplitPairs = 32;
+template <int FMT>
+__global__ void __launch_bounds__(3 * kSplitPairs, Fmt<FMT>::NA == 8 ? 5 : 8)
+    k_step_split(Geom g, const void *Uin, void *Uout, void *E, StepCoef<float> c) {
+    using F = Fmt<FMT>;
+    __shared__ f2 sm[plaq_slots<FMT>() * kSplitPairs];
+    const int mu = threadIdx.x / kSplitPairs, i = threadIdx.x - mu * kSplitPairs;
+    const int64_t p0 = (int64_t)blockIdx.x * kSplitPairs, Vh = g.V >> 1;
+    const int64_t p = p0 + i < Vh ? p0 + i : Vh - 1;  // a thread past the end repeats the last pair's plaquette
+    const PairNbhd nb(g, p);
+    const bool seam = pairs_touch_seam(g, p0, kSplitPairs);
+    if (seam) pair_plaquette<F, true>(g, nb, Uin, mu, p, sm + i, kSplitPairs);
+    else pair_plaquette<F, false>(g, nb, Uin, mu, p, sm + i, kSplitPairs);
+    __syncthreads();
+    if (p0 + i >= Vh) return;
+    if (seam) pair_link<F, true>(g, nb, Uin, Uout, E, c, c, mu, p, 0, sm + i, kSplitPairs);
+    else pair_link<F, false>(g, nb, Uin, Uout, E, c, c, mu, p, 0, sm + i, kSplitPairs);
+}
+
 // Checkerboard sub-sweep of (parity, mu): the sites of the parity, for even extents,
 // t -> (x, row) with x of the right parity
 template <class T> struct FlowCoefT {
@@ -705,7 +728,9 @@ template <int FMT> struct Launch {
             if (paired_step(g)) {
                 const StepCoef<T> c = coef_cast<T>(cd);
                 const unsigned blocks = (unsigned)tile_blocks(g, t);
-                if (t.tx) k_step_pair<FMT, true><<<blocks, kThreadsPair, 0, st>>>(g, Uin, Uout, E, c, t);
+                if (!t.tx && split_step(g))
+                    k_step_split<FMT><<<grid_for(g.V >> 1, kSplitPairs), 3 * kSplitPairs, 0, st>>>(g, Uin, Uout, E, c);
+                else if (t.tx) k_step_pair<FMT, true><<<blocks, kThreadsPair, 0, st>>>(g, Uin, Uout, E, c, t);
                 else k_step_pair<FMT, false><<<blocks, kThreadsPair, 0, st>>>(g, Uin, Uout, E, c, t);
                 return cudaGetLastError();
             }
@@ -734,6 +759,11 @@ template <int FMT> struct Launch {
         }
         return cudaGetLastError();
     }
+    // Lattices whose paired step spreads a pair over three threads (k_step_split): up to
+    // about a wave of its blocks.  Per step by k_step_pair / k_step_split on GB300: SU(3)
+    // 16^3 13.4 / 8.2 us, 24^3 13.4 / 8.3, 32^3 14.4 / 12.3, 48^3 23.7 / 26.6; SU(2) 16^3 to
+    // 32^3 8.2 / 6.2 us, 48^3 10.3 / 10.3.
+    static bool split_step(const Geom &g) { return (g.V >> 1) <= (F::NA == 8 ? 25000 : 33000); }
     // Does step() take the paired kernel (one thread per site pair)?
     static bool paired_step(const Geom &g) { return F::PAIRED && g.nz % 2 == 0; }
     // One fused step (E and links) of the storage indices [i0, i1) only: site

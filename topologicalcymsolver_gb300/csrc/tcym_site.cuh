@@ -96,19 +96,21 @@ template <class F, class T> struct GroupOf<F, T, true> { using type = typename F
 // sm[(k * NA + a) * stride], the caller's slots for this site (shared memory
 // on the device), where the per-direction phase reads them back.
 template <class F, class M, class T, class LOAD>
-TCYM_HD void plaquette_projections(LOAD load, T *sm, int stride) {
+TCYM_HD void plaquette_projection(LOAD load, int mu, T *sm, int stride) {
     using G = typename GroupOf<F, T>::type;
-#pragma unroll 1
-    for (int mu = 0; mu < 3; ++mu) {
-        const int nu = mu == 2 ? 0 : mu + 1;
-        // P_{mu nu}(x) = [U_mu(x) U_nu(x+mu)] [U_nu(x) U_mu(x+nu)]^dag
-        const M t1 = G::template mulu<false, false>(load(mu, 0, mu), load(nu, 1, mu));
-        const M t2 = G::template mulu<false, false>(load(nu, 0, mu), load(mu, 1, nu));
-        T pr[F::NA];
-        G::proj_mul_dag(t1, t2, pr);
+    const int nu = mu == 2 ? 0 : mu + 1;
+    // P_{mu nu}(x) = [U_mu(x) U_nu(x+mu)] [U_nu(x) U_mu(x+nu)]^dag
+    const M t1 = G::template mulu<false, false>(load(mu, 0, mu), load(nu, 1, mu));
+    const M t2 = G::template mulu<false, false>(load(nu, 0, mu), load(mu, 1, nu));
+    T pr[F::NA];
+    G::proj_mul_dag(t1, t2, pr);
 #pragma unroll
-        for (int a = 0; a < F::NA; ++a) sm[(mu * F::NA + a) * stride] = pr[a];
-    }
+    for (int a = 0; a < F::NA; ++a) sm[(mu * F::NA + a) * stride] = pr[a];
+}
+template <class F, class M, class T, class LOAD>
+TCYM_HD void plaquette_projections(LOAD load, T *sm, int stride) {
+#pragma unroll 1
+    for (int mu = 0; mu < 3; ++mu) plaquette_projection<F, M>(load, mu, sm, stride);
 }
 // f[a] += c_{mu+1} p_{mu,mu+1} - c_{mu+2} p_{mu+2,mu}
 template <int NA, class T, class C>
@@ -202,59 +204,71 @@ TCYM_COLD void langevin_kick_pair(const StepCoef<float> &c, int mu, int64_t p, i
 #ifndef TCYM_PAIR_STAPLE_ROLLED
 #define TCYM_PAIR_STAPLE_ROLLED 0
 #endif
+// Its two parts, so that a small lattice can spread a pair over three threads:
+// pair_plaquette forms p_{mu,mu+1} of the pair into sm, pair_link moves direction mu.
+template <class F, bool SEAM> TCYM_HD auto pair_load(const PairNbhd &nb, const void *U, int64_t Vh, int64_t p) {
+    return [=, &nb](int d, int a, int dir) {
+        return a ? F::load2(U, Vh, d, nb.at(dir, 1), SEAM && nb.swapped(dir, 1)) : F::load2(U, Vh, d, p, false);
+    };
+}
+template <class F, bool SEAM>
+TCYM_HD void pair_plaquette(const Geom &g, const PairNbhd &nb, const void *Uin, int mu, int64_t p, f2 *sm, int stride) {
+    plaquette_projection<F, typename F::Mat2>(pair_load<F, SEAM>(nb, Uin, g.V >> 1, p), mu, sm, stride);
+}
 template <class F, bool SEAM, int MODE = -1>
-TCYM_HD void site_step_pair(const Geom &g, const void *Uin, void *Uout, void *E, const StepCoef<float> &c,
-                            const StepCoef<float> &cn, int64_t p, uint64_t step_add, f2 *sm, int stride) {
+TCYM_HD void pair_link(const Geom &g, const PairNbhd &nb, const void *Uin, void *Uout, void *E,
+                       const StepCoef<float> &c, const StepCoef<float> &cn, int mu, int64_t p, uint64_t step_add,
+                       const f2 *sm, int stride) {
     using G2 = typename F::G2;
     using M2 = typename F::Mat2;
     constexpr int NA = F::NA;
     const int64_t Vh = g.V >> 1;
-    const PairNbhd nb(g, p);
-    auto load = [&](int d, int a, int dir) {
-        return a ? F::load2(Uin, Vh, d, nb.at(dir, 1), SEAM && nb.swapped(dir, 1)) : F::load2(Uin, Vh, d, p, false);
-    };
-    plaquette_projections<F, M2>(load, sm, stride);
-#pragma unroll 1
-    for (int mu = 0; mu < 3; ++mu) {
-        // lower staples S- = U_nu^dag(x+mu-nu) U_mu^dag(x-nu) U_nu(x-nu)
-        M2 A = G2::zero();
+    // lower staples S- = U_nu^dag(x+mu-nu) U_mu^dag(x-nu) U_nu(x-nu)
+    M2 A = G2::zero();
 #if TCYM_PAIR_STAPLE_ROLLED
 #pragma unroll 1
 #else
 #pragma unroll
 #endif
-        for (int k = 1; k <= 2; ++k) {
-            const int nu = mu + k >= 3 ? mu + k - 3 : mu + k;
-            const M2 b1 = F::load2(Uin, Vh, nu, nb.at(mu, 1, nu, -1), SEAM && nb.swapped(mu, 1, nu, -1));
-            const int64_t sb = nb.at(nu, -1);
-            const bool wb = SEAM && nb.swapped(nu, -1);
-            const M2 b2 = F::load2(Uin, Vh, mu, sb, wb);
-            const M2 b3 = F::load2(Uin, Vh, nu, sb, wb);
-            const M2 lo = G2::template mulu<false, false>(G2::template mulu<true, true>(b1, b2), b3);
-            A = G2::add(A, G2::scale(f2(sel3(c.cnu, nu)), lo));
-        }
-        // the link and its field are read after the staple sum, so that they are
-        // not live while it runs
-        const M2 u = F::load2(Uin, Vh, mu, p, false);
-        f2 e[NA];
-        F::load_e2(E, Vh, mu, p, e);
-        f2 f[NA];
-        G2::proj_mul(u, A, f);
-        add_plaquette_force<NA>(sm, stride, mu, c.cnu, f);
-        const f2 fc(sel3(c.fc, mu));
-        const int mode = MODE >= 0 ? MODE : c.mode;
-        if (mode == MODE_LANGEVIN) {
-            langevin_kick_pair<NA>(cn, mu, p, Vh, step_add, fc, f, e);
-        } else if (mode == MODE_FLOW) {
-#pragma unroll
-            for (int a = 0; a < NA; ++a) e[a] = fc * f[a];
-        } else {
-#pragma unroll
-            for (int a = 0; a < NA; ++a) e[a] = fma(fc, f[a], e[a]);
-        }
-        F::store_e2(E, Vh, mu, p, e);
-        F::store2(Uout, Vh, mu, p, G2::iexp_mul(f2(sel3(c.uc, mu)), e, u));
+    for (int k = 1; k <= 2; ++k) {
+        const int nu = mu + k >= 3 ? mu + k - 3 : mu + k;
+        const M2 b1 = F::load2(Uin, Vh, nu, nb.at(mu, 1, nu, -1), SEAM && nb.swapped(mu, 1, nu, -1));
+        const int64_t sb = nb.at(nu, -1);
+        const bool wb = SEAM && nb.swapped(nu, -1);
+        const M2 b2 = F::load2(Uin, Vh, mu, sb, wb);
+        const M2 b3 = F::load2(Uin, Vh, nu, sb, wb);
+        const M2 lo = G2::template mulu<false, false>(G2::template mulu<true, true>(b1, b2), b3);
+        A = G2::add(A, G2::scale(f2(sel3(c.cnu, nu)), lo));
     }
+    // the link and its field are read after the staple sum, so that they are
+    // not live while it runs
+    const M2 u = F::load2(Uin, Vh, mu, p, false);
+    f2 e[NA];
+    F::load_e2(E, Vh, mu, p, e);
+    f2 f[NA];
+    G2::proj_mul(u, A, f);
+    add_plaquette_force<NA>(sm, stride, mu, c.cnu, f);
+    const f2 fc(sel3(c.fc, mu));
+    const int mode = MODE >= 0 ? MODE : c.mode;
+    if (mode == MODE_LANGEVIN) {
+        langevin_kick_pair<NA>(cn, mu, p, Vh, step_add, fc, f, e);
+    } else if (mode == MODE_FLOW) {
+#pragma unroll
+        for (int a = 0; a < NA; ++a) e[a] = fc * f[a];
+    } else {
+#pragma unroll
+        for (int a = 0; a < NA; ++a) e[a] = fma(fc, f[a], e[a]);
+    }
+    F::store_e2(E, Vh, mu, p, e);
+    F::store2(Uout, Vh, mu, p, G2::iexp_mul(f2(sel3(c.uc, mu)), e, u));
+}
+template <class F, bool SEAM, int MODE = -1>
+TCYM_HD void site_step_pair(const Geom &g, const void *Uin, void *Uout, void *E, const StepCoef<float> &c,
+                            const StepCoef<float> &cn, int64_t p, uint64_t step_add, f2 *sm, int stride) {
+    const PairNbhd nb(g, p);
+    plaquette_projections<F, typename F::Mat2>(pair_load<F, SEAM>(nb, Uin, g.V >> 1, p), sm, stride);
+#pragma unroll 1
+    for (int mu = 0; mu < 3; ++mu) pair_link<F, SEAM, MODE>(g, nb, Uin, Uout, E, c, cn, mu, p, step_add, sm, stride);
 }
 
 template <class F, bool SEAM, int MODE = -1>
