@@ -1,21 +1,19 @@
-"""The FP32 formats' reunitarisation (increments from exactly summed deviations)
-against the FP64 projection rounded once, on the host build of the device code."""
+"""The FP32 formats' reunitarisation (increments as sums of a value and its error) against
+the FP64 projection rounded once, bit for bit, on the host build of the device code."""
 import numpy as np
 import pytest
 
 from tests import _hostcheck as hc
 
 # deviations of the stored rows: rounding, a long run, the edge of the increment form, beyond it
-DRIFTS = [0.0, 3e-6, 2e-4, 4e-3]
+DRIFTS = [0.0, 3e-6, 1.5e-5, 2e-4, 4e-3]
 
 
 @pytest.mark.parametrize("nc", [2, 3])
-@pytest.mark.parametrize("shape", [(4, 4, 4), (3, 3, 3), (8, 5, 2)])  # odd volume: a padded pair
+@pytest.mark.parametrize("shape", [(16, 16, 12), (3, 3, 3), (8, 5, 2)])  # odd volume: a padded pair
 @pytest.mark.parametrize("drift", DRIFTS)
 def test_projection_is_the_fp64_one_rounded_once(oracle_port, nc, shape, drift):
-    """Both forms round each entry once from values good to about 2e-10, so an entry
-    differs by one FP32 ulp at most (6e-8 below 1) and only where the exact value lies
-    within 2e-10 of the middle of two FP32 numbers: about 2e-10 / 3e-8 of the entries."""
+    """Each entry is the FP64 projection's, rounded once: equal to the last bit."""
     P = oracle_port[nc]
     V = int(np.prod(shape))
     U = np.zeros((V, 3, hc.NM[nc]))
@@ -26,13 +24,8 @@ def test_projection_is_the_fp64_one_rounded_once(oracle_port, nc, shape, drift):
         H.upload(U, None)
     A.reunitarize()
     B.reunitarize_fp64()
-    Ua, Ub = A.download()[0], B.download()[0]
-    if nc == 3:  # the stored rows (row 2 is rebuilt on load): entries (i, j) at i + 3 j
-        stored = [2 * (i + 3 * j) + c for i in (0, 1) for j in range(3) for c in (0, 1)]
-        Ua, Ub = Ua[:, :, stored], Ub[:, :, stored]
-    d = np.abs(Ua - Ub)
-    assert d.max() <= 2.0 ** -24
-    assert np.mean(d > 0) <= 0.02
+    # an odd volume's pad lane holds no site: compare the sites
+    assert np.array_equal(A.download()[0], B.download()[0])
 
 
 @pytest.mark.parametrize("nc", [2, 3])
@@ -52,5 +45,5 @@ def test_projection_of_a_broken_link_is_the_fp64_one(oracle_port, nc):
         out.append(H.download()[0])
     keep = np.ones((64, 3), bool)
     keep[3, 1] = keep[10, 0] = keep[40, 2] = False
-    assert np.abs(out[0][keep] - out[1][keep]).max() <= 2.0 ** -23  # the partner's row 2 is rebuilt in FP32
+    assert np.array_equal(out[0][keep], out[1][keep])
     assert not np.isfinite(out[1][3, 1]).all()

@@ -156,20 +156,28 @@ TCYM_HD void half_angle(double d2, double &f, double &co) {
     Real<double>::sincos_(0.5 * d, &s, &co);
     f = s / d;
 }
+TCYM_HD void half_angle(f2 d2, f2 &f, f2 &co) {  // no packed sine: lane by lane
+    half_angle(d2.v.x, f.v.x, co.v.x);
+    half_angle(d2.v.y, f.v.y, co.v.y);
+}
+TCYM_HD float quot(float a, float b) { return a / b; }
+TCYM_HD double quot(double a, double b) { return a / b; }
+TCYM_HD f2 quot(f2 a, f2 b) { return f2(a.v.x / b.v.x, a.v.y / b.v.y); }
 // f as half_angle and cm1 = cos(d/2) - 1 = -sin^2(d/2) / (1 + cos(d/2)), without cancellation
-template <class T> TCYM_HD void half_angle_general(T d2, T &f, T &cm1) {
+template <class T> TCYM_HD void half_angle_m1(T d2, T &f, T &cm1) {
     T co;
     half_angle(d2, f, co);
-    cm1 = -(f * f * d2) / (T(1) + co);
+    cm1 = -quot(f * f * d2, T(1) + co);
 }
-// The same from the Taylor series in y = (d/2)^2 of sin(sqrt y)/sqrt y and
-// cos(sqrt y) - 1, without a root, a sine or a division: y <= 1/16 (a link update's
-// exponent is dt |E|, a few hundredths), the first omitted terms below half an ulp
-// (FP32: y^4/9! = 4e-11 of f, y^5/10! = 3e-13 beside y/2; FP64: y^8/17! and y^9/18!
-// below 1e-24).  Larger exponents take the general form.
+// FP64: the same from the Taylor series in y = (d/2)^2 of sin(sqrt y)/sqrt y and
+// cos(sqrt y) - 1, without a root, a sine or a division (100 FP64 operations of a link's):
+// y <= 1/16 (a link update's exponent is dt |E|, a few hundredths), the first omitted
+// terms y^8/17! and y^9/18! below 1e-24.  Larger exponents take the general form.  (In FP32
+// the series gained 8% of a 128^3 step, and its other roundings moved a trajectory's E.B
+// as far as the form above is off exact arithmetic.)
 TCYM_HD void half_angle_m1(double d2, double &f, double &cm1) {
     const double y = 0.25 * d2;
-    if (!(y <= 0.0625)) { half_angle_general(d2, f, cm1); return; }
+    if (!(y <= 0.0625)) { half_angle_m1<double>(d2, f, cm1); return; }
     double s = -1.0 / 1307674368000.0;
     s = fma(s, y, 1.0 / 6227020800.0);
     s = fma(s, y, -1.0 / 39916800.0);
@@ -186,27 +194,6 @@ TCYM_HD void half_angle_m1(double d2, double &f, double &cm1) {
     c = fma(c, y, -1.0 / 720.0);
     c = fma(c, y, 1.0 / 24.0);
     cm1 = y * fma(c, y, -0.5);
-}
-template <class T> TCYM_HD void half_angle_m1_series(T d2, T &f, T &cm1) {
-    const T y = T(0.25) * d2;
-    T s = fma(T(-1.0 / 5040.0), y, T(1.0 / 120.0));
-    s = fma(s, y, T(-1.0 / 6.0));
-    f = fma(T(0.5) * s, y, T(0.5));
-    T c = fma(T(1.0 / 40320.0), y, T(-1.0 / 720.0));
-    c = fma(c, y, T(1.0 / 24.0));
-    cm1 = y * fma(c, y, T(-0.5));
-}
-TCYM_HD void half_angle_m1(float d2, float &f, float &cm1) {
-    if (d2 <= 0.25f) half_angle_m1_series(d2, f, cm1);
-    else half_angle_general(d2, f, cm1);
-}
-TCYM_HD void half_angle_m1(f2 d2, f2 &f, f2 &cm1) {
-    if (d2.v.x <= 0.25f && d2.v.y <= 0.25f) {
-        half_angle_m1_series(d2, f, cm1);
-    } else {  // no packed sine: lane by lane, each by its own size
-        half_angle_m1(d2.v.x, f.v.x, cm1.v.x);
-        half_angle_m1(d2.v.y, f.v.y, cm1.v.y);
-    }
 }
 
 template <class T> struct cx {

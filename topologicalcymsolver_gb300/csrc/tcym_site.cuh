@@ -811,21 +811,49 @@ template <class F> TCYM_HD void site_reunitarize(const Geom &g, void *U, int64_t
         F::store(U, g.V, mu, s, recast<T>(Group64<F>::reunitarize(recast<double>(F::load(U, g.V, mu, s)))));
 }
 
-// (1 + d)^(-1/2) - 1 for |d| <= 1e-3: the first omitted term is 3e-13
-template <class T> TCYM_HD T inv_root_m1(T d) { return d * fma(d, fma(d, T(-0.3125), T(0.375)), T(-0.5)); }
-
-// The same projection of the links of pair p in direction mu of FP32 storage.  A stored
-// link is within a few 1e-6 of the group, so its projection moves it by increments of
-// that size: what must be accurate beyond FP32 is only how far it is off (the norms'
-// differences from 1 and the rows' product, sums that cancel), formed as ExactSums; the
-// increments then fit FP32, and each entry is rounded once, as the FP64 projection's
-// result is.  SU(3): with d0 = |r0|^2 - 1 and D = <r0, r1>,
+// The same projection of the links of pair p in direction mu of FP32 storage, bit for
+// bit, in FP32 pairs of numbers.  A stored link is within a few 1e-6 of the group, so its
+// projection moves it by increments of that size: with d0 = |r0|^2 - 1 and D = <r0, r1>,
 //   r0' = r0 (1 + d0)^(-1/2),  r1' = (r1 - D r0 / (1 + d0)) (1 + d1)^(-1/2),
-//   d1 = |r1|^2 - 1 - |D|^2 / (1 + d0).
-// Links further off than 1e-3 (or not finite) take the FP64 projection.  The FP64 one
-// took 1184 us for SU(3) and 336 us for SU(2) at 128^3 on GB300 (FP64 rate); this one is
-// bound by memory (SU(3) 604 MB, 89 us at the measured copy rate).
+//   d1 = |r1|^2 - 1 - |D|^2 / (1 + d0)
+// (SU(2): the first line).  The deviations and the increments are formed as sums of a
+// value and its error (ExactSum), good to 3e-14 for deviations up to 3e-5, and added to
+// the entry with one rounding.  A pair with an entry whose sum lies within 1e-13 of the
+// middle of two FP32 numbers (about one warp in 200), or further off the group, or not
+// finite, takes the FP64 projection.  That one ran at the FP64 rate, 1184 us for SU(3) and
+// 336 us for SU(2) at 128^3 on GB300; this one is bound by memory and FP32 arithmetic.
+constexpr float kProjDeviation = 3e-5f, kProjTie = 1e-13f;
 TCYM_HD bool beyond(f2 d, float t) { return !(fabsf(d.v.x) <= t && fabsf(d.v.y) <= t); }
+// a value and its error
+struct F2E {
+    f2 s, e;
+};
+// a sum as its nearest FP32 number and the rest (two-sum: the carried errors may outweigh
+// what is left of a sum that cancels)
+TCYM_HD F2E split(const ExactSum<f2> &x) {
+    const f2 t = x.s + x.e, b = t - x.s;
+    return F2E{t, (x.s - (t - b)) + (x.e - b)};
+}
+// (1 + d)^(-1/2) - 1: -d/2 exactly, 3/8 d^2 - 5/16 d^3 in the error's place (d^4 is 1e-18)
+TCYM_HD F2E inv_root_m1(F2E d) {
+    return F2E{f2(-0.5) * d.s, fma(d.s * d.s, fma(f2(-0.3125), d.s, f2(0.375)), f2(-0.5) * d.e)};
+}
+// x + (i.s + i.e) rounded once; tie: the exact sum lies within kProjTie of a rounding
+// boundary of some lane (half the distance from the result to its neighbour on that side)
+TCYM_HD f2 add_once(f2 x, F2E i, bool &tie) {
+    const f2 t = x + i.s, b = t - x;
+    const f2 err = ((x - (t - b)) + (i.s - b)) + i.e;  // the exact sum is t + err
+    const f2 r = t + err;
+    const f2 left = err - (r - t);  // the exact sum is r + left
+    auto near_tie = [](float r, float left) {
+        if (left == 0.0f) return false;
+        // the neighbour of r on the side of the remainder, and half the way there
+        const float n = nextafterf(r, left > 0.0f ? INFINITY : -INFINITY);
+        return !(fabsf(fabsf(0.5f * (n - r)) - fabsf(left)) > kProjTie);
+    };
+    tie |= near_tie(r.v.x, left.v.x) || near_tie(r.v.y, left.v.y);
+    return r;
+}
 template <class F> TCYM_HD void pair_reunitarize_fp64(void *U, int64_t V, int mu, int64_t p) {
     using G64 = Group64<F>;
     const int64_t Vh = pair_sites(V);
@@ -836,15 +864,26 @@ template <class F> TCYM_HD void pair_reunitarize_fp64(void *U, int64_t V, int mu
 template <class F> TCYM_HD void pair_reunitarize(void *U, int64_t V, int mu, int64_t p) {
     const int64_t Vh = pair_sites(V);
     auto u = F::load2(U, Vh, mu, p, false);
+    // h x, plus what the caller adds
+    auto scaled = [](const F2E &h, f2 x) {
+        ExactSum<f2> s(f2(0.0));
+        s.mul(h.s, x);
+        s.e = fma(h.e, x, s.e);
+        return s;
+    };
+    bool slow = false;
     if constexpr (F::NA == 3) {
         ExactSum<f2> n(f2(-1.0));
 #pragma unroll
         for (int k = 0; k < 4; ++k) n.mul(u.q[k], u.q[k]);
-        const f2 d = n.value();
-        if (beyond(d, 1e-3f)) { pair_reunitarize_fp64<F>(U, V, mu, p); return; }
-        const f2 h = inv_root_m1(d);
+        const F2E d = split(n);
+        slow = beyond(d.s, kProjDeviation);
+        const F2E h = inv_root_m1(d);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) u.q[k] = fma(u.q[k], h, u.q[k]);
+        for (int k = 0; k < 4; ++k) {
+            const ExactSum<f2> i = scaled(h, u.q[k]);
+            u.q[k] = add_once(u.q[k], F2E{i.s, i.e}, slow);
+        }
     } else {
         ExactSum<f2> n0(f2(-1.0)), n1(f2(-1.0)), dr(f2(0.0)), di(f2(0.0));
 #pragma unroll
@@ -855,27 +894,30 @@ template <class F> TCYM_HD void pair_reunitarize(void *U, int64_t V, int mu, int
             dr.mul(a.re, b.re); dr.mul(a.im, b.im);
             di.mul(a.re, b.im); di.mul(-a.im, b.re);
         }
-        const f2 d0 = n0.value(), Dr = dr.value(), Di = di.value();
-        const f2 g = fma(d0, d0, f2(1.0) - d0);  // 1 / (1 + d0), beside factors of 1e-6
-        n1.add(-(g * fma(Dr, Dr, Di * Di)));
-        const f2 d1 = n1.value();
-        if (beyond(d0, 1e-3f) || beyond(d1, 1e-3f) || beyond(Dr, 1e-3f) || beyond(Di, 1e-3f)) {
-            pair_reunitarize_fp64<F>(U, V, mu, p);
-            return;
-        }
-        const f2 h0 = inv_root_m1(d0), h1 = inv_root_m1(d1);
-        const f2 w = fma(g, h1, g);
-        const cx<f2> c{w * Dr, w * Di};
+        const F2E d0 = split(n0), Dr = split(dr), Di = split(di);
+        n1.add(-fma(Dr.s, Dr.s, Di.s * Di.s));  // |D|^2, at most 2e-9, to 2e-16
+        const F2E d1 = split(n1);
+        slow = beyond(d0.s, kProjDeviation) || beyond(d1.s, kProjDeviation) || beyond(Dr.s, kProjDeviation) ||
+               beyond(Di.s, kProjDeviation);
+        const F2E h0 = inv_root_m1(d0), h1 = inv_root_m1(d1);
+        // c = D (1 + h1) / (1 + d0)
+        const f2 w = h1.s - d0.s;
+        const F2E cr{Dr.s, fma(w, Dr.s, Dr.e)}, ci{Di.s, fma(w, Di.s, Di.e)};
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const cx<f2> a = u.m[0][k], b = u.m[1][k];
-            const f2 ir = fma(h1, b.re, fma(-c.re, a.re, c.im * a.im));
-            const f2 ii = fma(h1, b.im, fma(-c.re, a.im, -(c.im * a.re)));
-            u.m[1][k] = cx<f2>{b.re + ir, b.im + ii};
-            u.m[0][k] = cx<f2>{fma(a.re, h0, a.re), fma(a.im, h0, a.im)};
+            ExactSum<f2> ir = scaled(h1, b.re), ii = scaled(h1, b.im);
+            ir.mul(-cr.s, a.re); ir.mul(ci.s, a.im);
+            ii.mul(-cr.s, a.im); ii.mul(-ci.s, a.re);
+            ir.e = fma(-cr.e, a.re, fma(ci.e, a.im, ir.e));
+            ii.e = fma(-cr.e, a.im, fma(-ci.e, a.re, ii.e));
+            u.m[1][k] = cx<f2>{add_once(b.re, F2E{ir.s, ir.e}, slow), add_once(b.im, F2E{ii.s, ii.e}, slow)};
+            const ExactSum<f2> jr = scaled(h0, a.re), ji = scaled(h0, a.im);
+            u.m[0][k] = cx<f2>{add_once(a.re, F2E{jr.s, jr.e}, slow), add_once(a.im, F2E{ji.s, ji.e}, slow)};
         }
     }
-    F::store2(U, Vh, mu, p, u);
+    if (slow) pair_reunitarize_fp64<F>(U, V, mu, p);
+    else F::store2(U, Vh, mu, p, u);
 }
 
 // GeodesicInterpolation (SUNc/AdvancedOperations.cpp:432-442) on the links of
