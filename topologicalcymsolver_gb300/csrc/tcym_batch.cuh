@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kThreadsObs, Fmt<FMT>::NA == 8 ? 2 : 4)
             for (int q = 0; q < 3; ++q) { v[P_ESQ0 + q] = o.esq[q]; v[P_BSQ0 + q] = o.bsq[q]; }
             v[P_EDB] = o.edotb;
         }
-        block_record<kUsedSample, kThreadsObs>(v, sh, partial + (int64_t)item * P_WIDTH);
+        block_record<kUsedSample, kThreadsObs, false>(v, sh, partial + (int64_t)item * P_WIDTH);
         __syncthreads();
     }
 }

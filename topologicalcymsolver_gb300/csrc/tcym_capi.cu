@@ -537,11 +537,39 @@ extern "C" int tcym_gauss_restore(tcym_lattice lat, double tol, int maxit, int *
     CK(cudaMemsetAsync(lat->result + R_NONFINITE, 0, sizeof(double), lat->stream));
     const double init[4] = {(double)maxit, 0.0, 0.0, 0.0};
     CK(cudaMemcpyAsync(ctl, init, sizeof(init), cudaMemcpyHostToDevice, lat->stream));
+    auto finish = [&](int it, bool check) { return make_finish(lat->result, na, lat->g.V, 0.0, ctl, tol, it, check); };
+    // the fused restore keeps the fields and G in two buffers each: the second E in the link
+    // buffer that the next step overwrites, the second G behind it (FP64) or in the second
+    // half of the violation array, which holds doubles (FP32 pairs)
+    bool fused = false;
+    size_t gbytes = 0;
+    DISPATCH(lat->fmt, { fused = L::restore_fused(lat->g); gbytes = L::restore_g_bytes(lat->g); });
+    const size_t ebytes = 3 * tcym_field_bytes(lat->fmt) * tcym_stored_sites(lat->fmt, lat->g.V);
+    char *const spare = static_cast<char *>(lat->U[1 - lat->cur]);
+    void *const Ebuf[2] = {lat->E, spare};
+    void *const Gbuf[2] = {lat->gauss, lat->precision == TCYM_FP64 ? spare + ebytes : reinterpret_cast<char *>(lat->gauss) + gbytes};
+    const void *U = lat->U[lat->cur];
     auto deviation = [&](int it, bool check) -> int {
-        const Finish fin = make_finish(lat->result, na, lat->g.V, 0.0, ctl, tol, it, check);
-        DISPATCH(lat->fmt, CK(L::gauss_compute_it(lat->g, lat->U[lat->cur], lat->E, lat->gauss, lat->partial,
-                                                  lat->max_blocks, fin, lat->stream)));
+        const Finish fin = finish(it, check);
+        DISPATCH(lat->fmt, CK(fused ? L::restore_deviation(lat->g, U, lat->E, Gbuf[0], lat->partial, lat->max_blocks, fin,
+                                                           lat->stream)
+                                    : L::gauss_compute_it(lat->g, U, lat->E, lat->gauss, lat->partial, lat->max_blocks,
+                                                          fin, lat->stream)));
         return TCYM_OK;
+    };
+    // sub-step k of iteration it
+    auto substep = [&](int it, int k) -> int {
+        int r = TCYM_OK;
+        if (fused) {  // its update, and the deviation of the next one (the first is the initial one)
+            const int n = (3 * it + k) & 1;
+            const Finish fin = k < 2 ? finish(it, k == 1) : finish(it + 1, false);
+            DISPATCH(lat->fmt, CK(L::restore_step(lat->g, U, Ebuf[n], Ebuf[1 - n], Gbuf[n], Gbuf[1 - n], gam[k], it,
+                                                  lat->partial, lat->max_blocks, fin, lat->stream)));
+        } else {
+            if ((r = deviation(it, k == 2))) return r;
+            DISPATCH(lat->fmt, CK(L::gauss_update_it(lat->g, U, lat->E, lat->gauss, gam[k], ctl, it, lat->stream)));
+        }
+        return r;
     };
     // initial deviation (GaussRestore.cpp:143)
     int r = deviation(-1, true);
@@ -552,20 +580,20 @@ extern "C" int tcym_gauss_restore(tcym_lattice lat, double tol, int maxit, int *
         CK(cudaMemcpyAsync(h, ctl, sizeof(h), cudaMemcpyDeviceToHost, lat->stream));
         if ((r = fetch_result(lat))) return r;  // synchronises the stream
         stop = (int)h[0];
-        if (h[1] != 0.0) {
-            tcym_set_error(ctx, "tcym_gauss_restore: non-finite violation at iteration %d", stop - 1);
-            return TCYM_ERR_NONFINITE;
-        }
-        if (stop <= queued || queued >= maxit) break;
+        if (h[1] != 0.0 || stop <= queued || queued >= maxit) break;
         const int n = std::min(batch, maxit - queued);
         for (int it = queued; it < queued + n; ++it)
-            for (int k = 0; k < 3; ++k) {
-                if ((r = deviation(it, k == 2))) return r;
-                DISPATCH(lat->fmt, CK(L::gauss_update_it(lat->g, lat->U[lat->cur], lat->E, lat->gauss, gam[k], ctl, it,
-                                                         lat->stream)));
-            }
+            for (int k = 0; k < 3; ++k)
+                if ((r = substep(it, k))) return r;
         queued += n;
         batch = std::min(2 * batch, 64);
+    }
+    // an odd number of fused sub-steps left the fields in the spare buffer
+    if (fused && std::min(stop, queued) % 2 != 0)
+        CK(cudaMemcpyAsync(lat->E, spare, ebytes, cudaMemcpyDeviceToDevice, lat->stream));
+    if (h[1] != 0.0) {
+        tcym_set_error(ctx, "tcym_gauss_restore: non-finite violation at iteration %d", stop - 1);
+        return TCYM_ERR_NONFINITE;
     }
     if (iters) *iters = std::min(stop, maxit);
     if (final_max) *final_max = lat->host_result[R_GMAX];

@@ -294,8 +294,9 @@ __device__ __forceinline__ double warp_op(int k, double v) {
     return v;
 }
 
-// The block's record from its threads' values; sh: used_count(USED) * NT doubles.
-template <unsigned USED, int NT>
+// The block's record from its threads' values, the used slots only, one after the other
+// (COMPACT) or each in its place; sh: used_count(USED) * NT doubles.
+template <unsigned USED, int NT, bool COMPACT>
 __device__ __forceinline__ void block_record(const double *v, double *sh, double *record) {
     constexpr int NQ = used_count(USED);
     const int lane = threadIdx.x & 31;
@@ -310,7 +311,7 @@ __device__ __forceinline__ void block_record(const double *v, double *sh, double
 #pragma unroll
         for (int i = 1; i < NT / 32; ++i) r = slot_op(k, r, sh[q * NT + lane + 32 * i]);
         r = warp_op(k, r);
-        if (lane == 0) record[k] = r;
+        if (lane == 0) record[COMPACT ? q : k] = r;
     }
 }
 
@@ -368,19 +369,28 @@ __device__ __forceinline__ void finish_record(const double *t, const Finish &f, 
     }
 }
 
-// The totals of `blocks` records (in block order, a warp a value) into t.
-template <unsigned USED, int NT>
-__device__ __forceinline__ void sum_records(const double *partial, int blocks, double *t) {
-    const int lane = threadIdx.x & 31;
-    if (threadIdx.x < P_WIDTH) t[threadIdx.x] = 0.0;
-    __syncthreads();
-    for (int q = threadIdx.x >> 5; q < used_count(USED); q += NT / 32) {
-        const int k = used_slot(USED, q);
-        double r = 0.0;  // every slot's sum or maximum starts at 0
-        for (int b = lane; b < blocks; b += 32) r = slot_op(k, r, __ldcg(&partial[(int64_t)b * P_WIDTH + k]));
-        r = warp_op(k, r);
-        if (lane == 0) t[k] = r;
+// The totals of `blocks` records into t[0..P_WIDTH): thread i takes the records i, i + NT,
+// ..., all slots' loads in flight together (a warp a slot, one load after the other, waited
+// 10 us for the 1024 records of a 64^3 lattice), then the block's columns are summed as any
+// block's.  sh: used_count(USED) * NT doubles.
+template <unsigned USED, int NT, bool COMPACT>
+__device__ __forceinline__ void sum_records(const double *partial, int blocks, double *sh, double *t) {
+    constexpr int NQ = used_count(USED);
+    double v[P_WIDTH];
+#pragma unroll
+    for (int k = 0; k < P_WIDTH; ++k) v[k] = 0.0;  // every slot's sum or maximum starts at 0
+#pragma unroll 4
+    for (int b = threadIdx.x; b < blocks; b += NT) {
+        int q = 0;
+#pragma unroll
+        for (int k = 0; k < P_WIDTH; ++k)
+            if (USED >> k & 1) {
+                v[k] = slot_op(k, v[k], __ldcg(&partial[COMPACT ? (int64_t)b * NQ + q : (int64_t)b * P_WIDTH + k]));
+                ++q;
+            }
     }
+    if (threadIdx.x < P_WIDTH) t[threadIdx.x] = 0.0;
+    block_record<USED, NT, false>(v, sh, t);
     __syncthreads();
 }
 
@@ -389,9 +399,9 @@ __device__ __forceinline__ void sum_records(const double *partial, int blocks, d
 template <unsigned USED, int NT>
 __device__ __forceinline__ void reduce_and_finish(const double *v, double *partial, const Finish &f) {
     static_assert(NT >= 128, "finish_record spreads over four warps");
-    __shared__ double sh[used_count(USED) * NT];
+    __shared__ double sh[used_count(USED) * NT], total[P_WIDTH];
     __shared__ int last;
-    block_record<USED, NT>(v, sh, partial + (int64_t)blockIdx.x * P_WIDTH);
+    block_record<USED, NT, true>(v, sh, partial + (int64_t)blockIdx.x * used_count(USED));
     __threadfence();  // the record before the ticket
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -402,17 +412,17 @@ __device__ __forceinline__ void reduce_and_finish(const double *v, double *parti
     __syncthreads();
     if (!last) return;
     __threadfence();
-    sum_records<USED, NT>(partial, gridDim.x, sh);
-    finish_record(sh, f);
+    if (f.ctl && (double)f.it >= f.ctl[0]) return;  // a deviation past the restore's stop: the result stays
+    sum_records<USED, NT, true>(partial, gridDim.x, sh, total);
+    finish_record(total, f);
 }
-
 // the record alone (callers that sum the records in a launch of their own)
 __device__ __forceinline__ void block_partial(const double *vals, double *partial) {
     __shared__ double sh[used_count(kUsedGauss) * kRedThreads];
     double *record = partial + (int64_t)blockIdx.x * P_WIDTH;
     if (threadIdx.x < P_WIDTH) record[threadIdx.x] = 0.0;
     __syncthreads();
-    block_record<kUsedGauss, kRedThreads>(vals, sh, record);
+    block_record<kUsedGauss, kRedThreads, false>(vals, sh, record);
 }
 
 // FULL: the Gauss and unitarity slots are filled too
@@ -550,52 +560,44 @@ __global__ void __launch_bounds__(threads_for<FMT>()) k_gauss_update_it(Geom g, 
     site_gauss_update<Fmt<FMT>>(g, U, E, G, gam, s);
 }
 
-// The restore iteration for the FP32 formats with even nz: one thread per site
-// pair in packed FP32, G(x) kept as FP32 pair planes G2[a * Vh + p] (the
-// storage's precision; the scratch holds na * V doubles, twice what they need).
-// The per-site sums run in FP32 per thread and the block partials in FP64,
-// with the same signed maximum (fmax drops NaN; the sums keep it).
-// 0: the FP32 formats restore through the per-site kernels too
-#ifndef TCYM_RESTORE_PAIRED
-#define TCYM_RESTORE_PAIRED 1
-#endif
-
-template <int FMT>
-__global__ void __launch_bounds__(kRedThreads) k_gauss_compute_pair_it(Geom g, const void *U, const void *E, f2 *G2,
-                                                                       double *partial, Finish fin) {
-    if ((double)fin.it >= fin.ctl[0]) return;
+// The fused restore (FP32 with even nz in site pairs, FP64): a thread per unit does a
+// sub-step's update and the next deviation (unit_restore), from the fields Ein and G Gin
+// into Eout and Gout, so a sub-step reads the links once and is one launch.  Bound by
+// memory (SU(3) FP32 128^3: 838 MB, 123 us at the measured copy rate); an iteration of
+// three (deviation, update) pairs of launches took 785 us there and 128 us at 64^3.
+// UPDATE: the update belongs to iteration `it`, the deviation to fin.it; a launch of an
+// iteration past the stop returns at once, and a deviation past it leaves the result of
+// the last one.
+constexpr int kThreadsRestore = 128;
+template <int FMT> constexpr bool restore_pairs() { return Fmt<FMT>::PAIRED; }
+template <int FMT, bool UPDATE>
+__global__ void __launch_bounds__(kThreadsRestore, 4)
+    k_restore(Geom g, const void *U, const void *Ein, void *Eout,
+              const typename RestoreUnit<Fmt<FMT>, restore_pairs<FMT>()>::T *Gin,
+              typename RestoreUnit<Fmt<FMT>, restore_pairs<FMT>()>::T *Gout, double gam, int it, double *partial,
+              Finish fin) {
     using F = Fmt<FMT>;
-    using GG = typename F::G2;
-    constexpr int NA = F::NA;
-    const int64_t Vh = g.V >> 1;
-    float gsq = 0.f, gmax = 0.f, gabs = 0.f;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < Vh; p += (int64_t)gridDim.x * blockDim.x) {
-        const PairNbhd nb(g, p);
-        f2 gv[NA];
+    constexpr bool PAIR = restore_pairs<FMT>();
+    using RU = RestoreUnit<F, PAIR>;
+    if (UPDATE && (double)it >= fin.ctl[0]) return;  // the same value for every thread of the grid
+    const int64_t n = RU::count(g);
+    typename RU::C gsq = 0, gmax = 0, gabs = 0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        typename RU::T gv[F::NA];
+        unit_restore<F, PAIR, UPDATE>(g, U, Ein, Eout, Gin, (typename RU::C)gam, i, gv);
 #pragma unroll
-        for (int a = 0; a < NA; ++a) gv[a] = f2(0.0);
-#pragma unroll 1
-        for (int mu = 0; mu < 3; ++mu) {
-            const int64_t pm = nb.at(mu, -1);
-            const bool sw = nb.swapped(mu, -1);
-            f2 e[NA], em[NA], t[NA];
-            F::load_e2(E, Vh, mu, pm, em);
-            if (sw) {
-#pragma unroll
-                for (int a = 0; a < NA; ++a) em[a] = swap_f2(em[a]);
+        for (int a = 0; a < F::NA; ++a) {
+            Gout[a * n + i] = gv[a];
+            if constexpr (PAIR) {
+                const float x = gv[a].v.x, y = gv[a].v.y;
+                gsq = fmaf(x, x, fmaf(y, y, gsq));
+                gmax = fmaxf(gmax, fmaxf(x, y));
+                gabs = fmaxf(gabs, fmaxf(fabsf(x), fabsf(y)));
+            } else {
+                gsq = fma(gv[a], gv[a], gsq);
+                gmax = fmax(gmax, gv[a]);
+                gabs = fmax(gabs, fabs(gv[a]));
             }
-            GG::inverse_adjoint(F::load2(U, Vh, mu, pm, sw), em, t);
-            F::load_e2(E, Vh, mu, p, e);
-#pragma unroll
-            for (int a = 0; a < NA; ++a) gv[a] += e[a] - t[a];
-        }
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-            G2[a * Vh + p] = gv[a];
-            const float x = gv[a].v.x, y = gv[a].v.y;
-            gsq = fmaf(x, x, fmaf(y, y, gsq));
-            gmax = fmaxf(gmax, fmaxf(x, y));
-            gabs = fmaxf(gabs, fmaxf(fabsf(x), fabsf(y)));
         }
     }
     double v[P_WIDTH];
@@ -604,38 +606,7 @@ __global__ void __launch_bounds__(kRedThreads) k_gauss_compute_pair_it(Geom g, c
     v[P_GSQ] = gsq;
     v[P_GMAX] = gmax;
     v[P_GABS] = gabs;
-    reduce_and_finish<kUsedGauss, kRedThreads>(v, partial, fin);
-}
-
-// E_mu(x) -= gam (G(x) - U_mu(x) G(x+mu) U_mu^dag(x)) for both sites of a pair, in FP32
-template <int FMT>
-__global__ void __launch_bounds__(kThreadsPair) k_gauss_update_pair_it(Geom g, const void *U, void *E, const f2 *G2,
-                                                                      float gam, const double *ctl, int it) {
-    if ((double)it >= ctl[0]) return;
-    using F = Fmt<FMT>;
-    using GG = typename F::G2;
-    constexpr int NA = F::NA;
-    const int64_t Vh = g.V >> 1;
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= Vh) return;
-    const PairNbhd nb(g, p);
-    const f2 mg(-(double)gam);
-    f2 gx[NA];
-#pragma unroll
-    for (int a = 0; a < NA; ++a) gx[a] = G2[a * Vh + p];
-#pragma unroll 1
-    for (int mu = 0; mu < 3; ++mu) {
-        const int64_t pp = nb.at(mu, 1);
-        const bool sw = nb.swapped(mu, 1);
-        f2 gp[NA], t[NA], e[NA];
-#pragma unroll
-        for (int a = 0; a < NA; ++a) gp[a] = sw ? swap_f2(G2[a * Vh + pp]) : G2[a * Vh + pp];
-        GG::adjoint(F::load2(U, Vh, mu, p, false), gp, t);
-        F::load_e2(E, Vh, mu, p, e);
-#pragma unroll
-        for (int a = 0; a < NA; ++a) e[a] = fma(mg, gx[a] - t[a], e[a]);
-        F::store_e2(E, Vh, mu, p, e);
-    }
+    reduce_and_finish<kUsedGauss, kThreadsRestore>(v, partial, fin);
 }
 
 template <int FMT> __global__ void k_set_zero(Geom g, void *U, void *E) {
@@ -821,32 +792,50 @@ template <int FMT> struct Launch {
             k_observables<FMT, false><<<blocks, kRedThreads, 0, st>>>(g, U, E, mask, partial, fin);
         return cudaGetLastError();
     }
-    // the restore iteration: paired FP32 kernels where the storage is paired
-    static constexpr bool restore_paired(const Geom &g) { return TCYM_RESTORE_PAIRED && Fmt<FMT>::PAIRED && g.nz % 2 == 0; }
+    // The fused restore's launches: E and G alternate between two buffers each.
+    static bool restore_fused(const Geom &g) { return !F::PAIRED || g.nz % 2 == 0; }
+    using GT = typename RestoreUnit<F, restore_pairs<FMT>()>::T;
+    // bytes of one G buffer
+    static size_t restore_g_bytes(const Geom &g) {
+        return sizeof(GT) * F::NA * (size_t)RestoreUnit<F, restore_pairs<FMT>()>::count(g);
+    }
+    template <bool UPDATE>
+    static cudaError_t restore(const Geom &g, const void *U, const void *Ein, void *Eout, const void *Gin, void *Gout,
+                               double gam, int it, double *partial, int max_blocks, const Finish &fin, cudaStream_t st) {
+        // max_blocks is 8 a multiprocessor.  FP64: 3 (a grid of 4 would hold every register for
+        // the whole launch, and the request loop's ticks wait for its blocks: 2.0 ms a tick
+        // beside a 128^3 preparation, against 0.24 ms alone)
+        const int need = grid_for(RestoreUnit<F, restore_pairs<FMT>()>::count(g), kThreadsRestore);
+        const int most = F::PAIRED ? max_blocks : max_blocks / 8 * 3;
+        k_restore<FMT, UPDATE><<<need < most ? need : most, kThreadsRestore, 0, st>>>(
+            g, U, Ein, Eout, static_cast<const GT *>(Gin), static_cast<GT *>(Gout), gam, it, partial, fin);
+        return cudaGetLastError();
+    }
+    static cudaError_t restore_deviation(const Geom &g, const void *U, const void *E, void *Gout, double *partial,
+                                         int max_blocks, const Finish &fin, cudaStream_t st) {
+        return restore<false>(g, U, E, nullptr, nullptr, Gout, 0.0, -1, partial, max_blocks, fin, st);
+    }
+    static cudaError_t restore_step(const Geom &g, const void *U, const void *Ein, void *Eout, const void *Gin, void *Gout,
+                                    double gam, int it, double *partial, int max_blocks, const Finish &fin,
+                                    cudaStream_t st) {
+        return restore<true>(g, U, Ein, Eout, Gin, Gout, gam, it, partial, max_blocks, fin, st);
+    }
+    // the restore iteration per site with its two kernels (FP32, odd nz)
     static cudaError_t gauss_compute_it(const Geom &g, const void *U, const void *E, double *G, double *partial,
                                         int max_blocks, const Finish &fin, cudaStream_t st) {
-        if constexpr (Fmt<FMT>::PAIRED) {
-            if (restore_paired(g)) {
-                const int need = grid_for(g.V >> 1, kRedThreads), blocks = need < max_blocks ? need : max_blocks;
-                k_gauss_compute_pair_it<FMT><<<blocks, kRedThreads, 0, st>>>(g, U, E, reinterpret_cast<f2 *>(G),
-                                                                             partial, fin);
-                return cudaGetLastError();
-            }
+        if constexpr (F::PAIRED) {
+            k_gauss_compute_it<FMT><<<reduce_grid(g, max_blocks), kRedThreads, 0, st>>>(g, U, E, G, partial, fin);
+            return cudaGetLastError();
         }
-        k_gauss_compute_it<FMT><<<reduce_grid(g, max_blocks), kRedThreads, 0, st>>>(g, U, E, G, partial, fin);
-        return cudaGetLastError();
+        return cudaErrorInvalidValue;
     }
     static cudaError_t gauss_update_it(const Geom &g, const void *U, void *E, const double *G, double gam,
                                        const double *ctl, int it, cudaStream_t st) {
-        if constexpr (Fmt<FMT>::PAIRED) {
-            if (restore_paired(g)) {
-                k_gauss_update_pair_it<FMT><<<grid_for(g.V >> 1, kThreadsPair), kThreadsPair, 0, st>>>(
-                    g, U, E, reinterpret_cast<const f2 *>(G), (float)gam, ctl, it);
-                return cudaGetLastError();
-            }
+        if constexpr (F::PAIRED) {
+            k_gauss_update_it<FMT><<<grid_for(g.V, TPB), TPB, 0, st>>>(g, U, E, G, gam, ctl, it);
+            return cudaGetLastError();
         }
-        k_gauss_update_it<FMT><<<grid_for(g.V, TPB), TPB, 0, st>>>(g, U, E, G, gam, ctl, it);
-        return cudaGetLastError();
+        return cudaErrorInvalidValue;
     }
     static cudaError_t set_zero(const Geom &g, void *U, void *E, cudaStream_t st) {
         k_set_zero<FMT><<<grid_for(g.V, 256), 256, 0, st>>>(g, U, E);

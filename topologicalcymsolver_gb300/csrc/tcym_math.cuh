@@ -294,6 +294,10 @@ template <class T> struct SU2 {
         out[1] = fma(q[2], c0, fma(-q[0], c2, fma(q[3], c1, e[1])));
         out[2] = fma(q[0], c1, fma(-q[1], c0, fma(q[3], c2, e[2])));
     }
+    // the other way: V (e^a t^a) V^dagger
+    static TCYM_HD void transport_back(const Mat &v, const T *e, T *out) {
+        transport(Mat{{-v.q[0], -v.q[1], -v.q[2], v.q[3]}}, e, out);
+    }
     static TCYM_HD T retr_one_minus(const Mat &v) { return T(2) * (T(1) - v.q[3]); }
     // exp(i c t^k e^k) = cos(d/2) + i sin(d/2) (c e / d).sigma, d = |c e|
     static TCYM_HD Mat iexp(T c, const T *e) {
@@ -544,6 +548,42 @@ template <class T> struct SU3 {
         out[2] = T(0.5) * (m00 - m11);
         out[3] = m20.re; out[4] = m20.im;
         out[5] = m21.re; out[6] = m21.im;
+        out[7] = T(0.86602540378443864676) * (m00 + m11);
+    }
+    // the other way, V (e^a t^a) V^dagger: rows 0 and 1 of V H, and of (V H) V^dagger the
+    // entries above the diagonal and the first two on it
+    static TCYM_HD void transport_back(const Mat &v, const T *e, T *out) {
+        const T is3 = T(0.57735026918962576450914878050196);
+        const T a7 = is3 * e[7];
+        const T a0 = a7 + e[2], a1 = a7 - e[2], a2 = T(-2) * a7;
+        const cx<T> h10{e[0], e[1]}, h20{e[3], e[4]}, h21{e[5], e[6]};
+        cx<T> w[2][3];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const cx<T> x = v.m[i][0], y = v.m[i][1], z = v.m[i][2];
+            w[i][0] = cfma(h10, y, cfma(h20, z, cx<T>{a0 * x.re, a0 * x.im}));
+            w[i][1] = cfma_cn(h10, x, cfma(h21, z, cx<T>{a1 * y.re, a1 * y.im}));
+            w[i][2] = cfma_cn(h20, x, cfma_cn(h21, y, cx<T>{a2 * z.re, a2 * z.im}));
+        }
+        auto entry = [&](int i, int j) {  // (W V^dagger)_ij
+            const cx<T> x = w[i][0], y = v.m[j][0];
+            cx<T> acc{x.re * y.re, x.im * y.re};
+            acc.re = fma(x.im, y.im, acc.re);
+            acc.im = fma(-x.re, y.im, acc.im);
+            return cfma_nc(w[i][2], v.m[j][2], cfma_nc(w[i][1], v.m[j][1], acc));
+        };
+        auto diagonal = [&](int i) {
+            T r = w[i][0].re * v.m[i][0].re;
+            r = fma(w[i][0].im, v.m[i][0].im, r);
+            r = fma(w[i][1].re, v.m[i][1].re, fma(w[i][1].im, v.m[i][1].im, r));
+            return fma(w[i][2].re, v.m[i][2].re, fma(w[i][2].im, v.m[i][2].im, r));
+        };
+        const cx<T> m01 = entry(0, 1), m02 = entry(0, 2), m12 = entry(1, 2);
+        const T m00 = diagonal(0), m11 = diagonal(1);
+        out[0] = m01.re; out[1] = -m01.im;
+        out[2] = T(0.5) * (m00 - m11);
+        out[3] = m02.re; out[4] = -m02.im;
+        out[5] = m12.re; out[6] = -m12.im;
         out[7] = T(0.86602540378443864676) * (m00 + m11);
     }
     static TCYM_HD T retr_one_minus(const Mat &v) { return T(3) - (v.m[0][0].re + v.m[1][1].re + v.m[2][2].re); }

@@ -6,8 +6,8 @@
 namespace tcym {
 
 __global__ void __launch_bounds__(kRedThreads) k_finalize(const double *partial, int blocks, Finish fin) {
-    __shared__ double t[P_WIDTH];
-    sum_records<kUsedAll, kRedThreads>(partial, blocks, t);
+    __shared__ double sh[used_count(kUsedAll) * kRedThreads], t[P_WIDTH];
+    sum_records<kUsedAll, kRedThreads, false>(partial, blocks, sh, t);
     finish_record(t, fin);
 }
 
@@ -24,9 +24,9 @@ cudaError_t finalize_obs(const double *partial, int blocks, int na, int64_t V, d
 
 // One block per member; out[2i] = E.B, out[2i+1] = N_CS of member i.
 __global__ void __launch_bounds__(kRedThreads) k_finalize_members(const MemberReduce *items, double *out) {
-    __shared__ double t[P_WIDTH];
+    __shared__ double sh[used_count(kUsedSample) * kRedThreads], t[P_WIDTH];
     const MemberReduce it = items[blockIdx.x];
-    sum_records<kUsedSample, kRedThreads>(it.partial + (int64_t)it.red_begin * P_WIDTH, it.red_blocks, t);
+    sum_records<kUsedSample, kRedThreads, false>(it.partial + (int64_t)it.red_begin * P_WIDTH, it.red_blocks, sh, t);
     const double v = (double)it.V;
     finish_record(t, Finish{it.result, nullptr, 1.0 / v, (double)it.na * v, 3.0 * v, it.ncs_dt, 0.0, 0, 0},
                   out ? out + 2 * blockIdx.x : nullptr, out ? out + 2 * blockIdx.x + 1 : nullptr);

@@ -739,6 +739,102 @@ TCYM_HD void site_gauss_update(const Geom &g, const void *U, void *E, const doub
     }
 }
 
+// ------------------------------------------------------------- restore, fused
+// A storage unit of the fused restore: a site pair of FP32 pair storage with even nz, in
+// packed FP32, or a site of an FP64 lattice.  G is held as planes G[a * count + i] of T.
+template <class F, bool PAIR> struct RestoreUnit;
+template <class F> struct RestoreUnit<F, true> {
+    using T = f2;
+    using C = float;
+    using G = typename F::G2;
+    using Mat = typename F::Mat2;
+    static TCYM_HD int64_t count(const Geom &g) { return g.V >> 1; }
+    PairNbhd nb;
+    int64_t n;
+    TCYM_HD RestoreUnit(const Geom &g, int64_t i) : nb(g, i), n(g.V >> 1) {}
+    TCYM_HD Mat link(const void *U, int mu, int a) const { return F::load2(U, n, mu, nb.at(mu, a), nb.swapped(mu, a)); }
+    TCYM_HD void load_e(const void *E, int mu, int a, T *e) const {
+        F::load_e2(E, n, mu, nb.at(mu, a), e);
+        if (nb.swapped(mu, a)) {
+#pragma unroll
+            for (int k = 0; k < F::NA; ++k) e[k] = swap_f2(e[k]);
+        }
+    }
+    TCYM_HD void store_e(void *E, int mu, const T *e) const { F::store_e2(E, n, mu, nb.p, e); }
+    TCYM_HD void load_g(const T *G, int mu, int a, T *v) const {
+        const int64_t i = nb.at(mu, a);
+        const bool sw = nb.swapped(mu, a);
+#pragma unroll
+        for (int k = 0; k < F::NA; ++k) v[k] = sw ? swap_f2(G[k * n + i]) : G[k * n + i];
+    }
+    TCYM_HD int64_t self() const { return nb.p; }
+};
+template <class F> struct RestoreUnit<F, false> {
+    using T = typename F::T;
+    using C = T;
+    using G = typename F::G;
+    using Mat = typename F::Mat;
+    static TCYM_HD int64_t count(const Geom &g) { return g.V; }
+    Nbhd nb;
+    int64_t n;
+    TCYM_HD RestoreUnit(const Geom &g, int64_t i) : nb(g, i), n(g.V) {}
+    TCYM_HD Mat link(const void *U, int mu, int a) const { return F::load(U, n, mu, nb.at(mu, a)); }
+    TCYM_HD void load_e(const void *E, int mu, int a, T *e) const { F::load_e(E, n, mu, nb.at(mu, a), e); }
+    TCYM_HD void store_e(void *E, int mu, const T *e) const { F::store_e(E, n, mu, nb.s, e); }
+    TCYM_HD void load_g(const T *G, int mu, int a, T *v) const {
+        const int64_t i = nb.at(mu, a);
+#pragma unroll
+        for (int k = 0; k < F::NA; ++k) v[k] = G[k * n + i];
+    }
+    TCYM_HD int64_t self() const { return nb.s; }
+};
+
+// One sub-step of the restore and the next deviation at once (UPDATE), or the deviation
+// alone.  With E'_mu(x) = E_mu(x) - gam (G(x) - U_mu(x) G(x+mu) U_mu^dag(x)), the new
+// deviation's term from below is
+//   U^dag(x-mu) E'(x-mu) U(x-mu) = U^dag(x-mu) [E(x-mu) - gam G(x-mu)] U(x-mu) + gam G(x),
+// so each unit forms its own new fields and its new G from the old ones of its neighbours
+// (the three gam G(x) taken off at the start).
+// gv receives the new G.
+template <class F, bool PAIR, bool UPDATE>
+TCYM_HD void unit_restore(const Geom &g, const void *U, const void *Ein, void *Eout,
+                          const typename RestoreUnit<F, PAIR>::T *Gin, typename RestoreUnit<F, PAIR>::C gam, int64_t i,
+                          typename RestoreUnit<F, PAIR>::T *gv) {
+    using RU = RestoreUnit<F, PAIR>;
+    using T = typename RU::T;
+    using G = typename RU::G;
+    constexpr int NA = F::NA;
+    const RU u(g, i);
+    const T mg(-gam);
+    T gx[NA];
+    if (UPDATE) u.load_g(Gin, 0, 0, gx);
+#pragma unroll
+    for (int a = 0; a < NA; ++a) gv[a] = UPDATE ? T(-3) * T(gam) * gx[a] : T(0);
+#pragma unroll 1
+    for (int mu = 0; mu < 3; ++mu) {
+        T e[NA], q[NA], t[NA];
+        u.load_e(Ein, mu, -1, e);
+        if (UPDATE) {
+            u.load_g(Gin, mu, -1, q);
+#pragma unroll
+            for (int a = 0; a < NA; ++a) e[a] = fma(mg, q[a], e[a]);
+        }
+        G::transport(u.link(U, mu, -1), e, t);
+#pragma unroll
+        for (int a = 0; a < NA; ++a) gv[a] = gv[a] - t[a];
+        u.load_e(Ein, mu, 0, e);
+        if (UPDATE) {
+            u.load_g(Gin, mu, 1, q);
+            G::transport_back(u.link(U, mu, 0), q, t);
+#pragma unroll
+            for (int a = 0; a < NA; ++a) e[a] = fma(mg, gx[a] - t[a], e[a]);
+            u.store_e(Eout, mu, e);
+        }
+#pragma unroll
+        for (int a = 0; a < NA; ++a) gv[a] = gv[a] + e[a];
+    }
+}
+
 // ------------------------------------------------------------ initial conditions
 template <class F> TCYM_HD void site_set_zero(const Geom &g, void *U, void *E, int64_t s) {
     using T = typename F::T;
