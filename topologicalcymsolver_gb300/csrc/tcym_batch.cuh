@@ -233,9 +233,22 @@ __global__ void __launch_bounds__(kThreadsPair, batch_min_blocks_for<FMT>())
 
 // The N_CS sample (mask OBS_EDOTB) of every member: one record per reduction work item
 // of kThreadsObs units, site pairs for members in FP32 pair storage with even nz (as
-// k_obs_pair), sites for the others.
+// k_obs_units), sites for the others.
 __host__ __device__ __forceinline__ int member_records(bool paired, int64_t V) {
     return (int)(((paired ? V >> 1 : V) + kThreadsObs - 1) / kThreadsObs);
+}
+template <class F, bool PAIR>
+__device__ __forceinline__ void sample_unit(const Geom &g, const void *u, const void *e, int64_t i, double *v) {
+#pragma unroll 1
+    for (int mu = 0; mu < 3; ++mu) {
+        typename Unit<F, PAIR>::T esq, bsq;
+        v[P_EDB] += lanes_sum(unit_clover<F, PAIR>(g, u, e, i, mu, esq, bsq));
+        const double es = lanes_sum(esq), bs = lanes_sum(bsq);
+        // fixed slots (a run-time index would put v in local memory)
+        if (mu == 0) { v[P_ESQ0] += es; v[P_BSQ0] += bs; }
+        else if (mu == 1) { v[P_ESQ0 + 1] += es; v[P_BSQ0 + 1] += bs; }
+        else { v[P_ESQ0 + 2] += es; v[P_BSQ0 + 2] += bs; }
+    }
 }
 template <int FMT>
 __global__ void __launch_bounds__(kThreadsObs, Fmt<FMT>::NA == 8 ? 2 : 4)
@@ -250,30 +263,19 @@ __global__ void __launch_bounds__(kThreadsObs, Fmt<FMT>::NA == 8 ? 2 : 4)
 #pragma unroll
         for (int q = 0; q < P_WIDTH; ++q) v[q] = 0.0;
         const int64_t i = (int64_t)(item - members[mi].red_begin) * blockDim.x + threadIdx.x;
-        bool paired = false;
         if constexpr (F::PAIRED) {
-            paired = members[mi].paired;
-            const int64_t Vh = g.V >> 1, plane = (int64_t)g.nx * g.ny;
-            if (paired && i < Vh) {
-                const bool seam = i < plane || i >= Vh - plane;
-#pragma unroll 1
-                for (int mu = 0; mu < 3; ++mu) {
-                    f2 esq, bsq;
-                    const f2 edb = seam ? pair_edotb_obs<F, true>(g, u, e, i, mu, esq, bsq)
-                                        : pair_edotb_obs<F, false>(g, u, e, i, mu, esq, bsq);
-                    const double es = (double)esq.v.x + (double)esq.v.y, bs = (double)bsq.v.x + (double)bsq.v.y;
-                    if (mu == 0) { v[P_ESQ0] += es; v[P_BSQ0] += bs; }
-                    else if (mu == 1) { v[P_ESQ0 + 1] += es; v[P_BSQ0 + 1] += bs; }
-                    else { v[P_ESQ0 + 2] += es; v[P_BSQ0 + 2] += bs; }
-                    v[P_EDB] += (double)edb.v.x + (double)edb.v.y;
+            if (!members[mi].paired) {
+                if (i < g.V) {
+                    SiteObs<F> o;
+                    site_observables<F>(g, u, e, OBS_EDOTB, i, o);
+                    for (int q = 0; q < 3; ++q) { v[P_ESQ0 + q] = o.esq[q]; v[P_BSQ0 + q] = o.bsq[q]; }
+                    v[P_EDB] = o.edotb;
                 }
+            } else if (i < (g.V >> 1)) {
+                sample_unit<F, true>(g, u, e, i, v);
             }
-        }
-        if (!paired && i < g.V) {
-            SiteObs<F> o;
-            site_observables<F>(g, u, e, OBS_EDOTB, i, o);
-            for (int q = 0; q < 3; ++q) { v[P_ESQ0 + q] = o.esq[q]; v[P_BSQ0 + q] = o.bsq[q]; }
-            v[P_EDB] = o.edotb;
+        } else if (i < g.V) {
+            sample_unit<F, false>(g, u, e, i, v);
         }
         block_record<kUsedSample, kThreadsObs, false>(v, sh, partial + (int64_t)item * P_WIDTH);
         __syncthreads();

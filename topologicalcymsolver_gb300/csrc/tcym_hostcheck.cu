@@ -149,11 +149,20 @@ template <int FMT> struct H {
                         if (nb.parity() == p) link_flow<F>(g, U, mu, fc, cn, uc, s);
                     }
     }
+    // E^2, plaquette B^2 and clover E.B of an FP64 site by the units' code, in place of site_observables'
+    static void unit_sample(const Geom &g, const void *U, const void *E, int64_t s, SiteObs<F> &o) {
+        if constexpr (!F::PAIRED) {
+            o.edotb = 0;
+            for (int mu = 0; mu < 3; ++mu) o.edotb += unit_clover<F, false>(g, U, E, s, mu, o.esq[mu], o.bsq[mu]);
+            unit_gauss<F, false>(g, U, E, s, o.g);
+        }
+    }
     static void observables(const Geom &g, const void *U, const void *E, int mask, double *out) {
         double esq[3] = {0, 0, 0}, bsq[3] = {0, 0, 0}, gsq = 0, usq = 0, edb = 0, gmax = 0, gabs = 0, umax = 0;
         for (int64_t s = 0; s < g.V; ++s) {
             SiteObs<F> o;
             site_observables<F>(g, U, E, mask, s, o);
+            if (mask == OBS_ALL) unit_sample(g, U, E, s, o);
             for (int m = 0; m < 3; ++m) { esq[m] += o.esq[m]; bsq[m] += o.bsq[m]; usq += o.un[m] * o.un[m]; umax = std::fmax(umax, o.un[m]); }
             for (int a = 0; a < F::NA; ++a) { gsq += o.g[a] * o.g[a]; gmax = std::fmax(gmax, o.g[a]); gabs = std::fmax(gabs, std::fabs(o.g[a])); }
             edb += o.edotb;
@@ -177,12 +186,11 @@ template <int FMT> struct H {
         if constexpr (F::PAIRED) {
             if (g.nz % 2) return false;
             double esq[3] = {0, 0, 0}, bsq[3] = {0, 0, 0}, edb = 0;
-            const int64_t Vh = g.V >> 1, plane = (int64_t)g.nx * g.ny;
+            const int64_t Vh = g.V >> 1;
             for (int64_t p = 0; p < Vh; ++p)
                 for (int mu = 0; mu < 3; ++mu) {
                     f2 e2, b2;
-                    const f2 d = (p < plane || p >= Vh - plane) ? pair_edotb_obs<F, true>(g, U, E, p, mu, e2, b2)
-                                                                : pair_edotb_obs<F, false>(g, U, E, p, mu, e2, b2);
+                    const f2 d = unit_clover<F, true>(g, U, E, p, mu, e2, b2);
                     esq[mu] += (double)e2.v.x + (double)e2.v.y;
                     bsq[mu] += (double)b2.v.x + (double)b2.v.y;
                     edb += (double)d.v.x + (double)d.v.y;
@@ -242,7 +250,7 @@ template <int FMT> struct H {
     }
     // the fused restore's schedule (tcym_gauss_restore) on the host
     template <bool PAIR> static int restore_fused(const Geom &g, const void *U, void *E, double tol, int maxit) {
-        using RU = RestoreUnit<F, PAIR>;
+        using RU = Unit<F, PAIR>;
         using RT = typename RU::T;
         const int64_t n = RU::count(g);
         const size_t ebytes = sizeof(typename RU::C) * 3 * (PAIR ? 2 * n : n) * F::NA;

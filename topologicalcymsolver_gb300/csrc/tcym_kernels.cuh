@@ -401,19 +401,20 @@ __device__ __forceinline__ void reduce_and_finish(const double *v, double *parti
     static_assert(NT >= 128, "finish_record spreads over four warps");
     __shared__ double sh[used_count(USED) * NT], total[P_WIDTH];
     __shared__ int last;
-    block_record<USED, NT, true>(v, sh, partial + (int64_t)blockIdx.x * used_count(USED));
+    const unsigned block = blockIdx.x + gridDim.x * blockIdx.y, blocks = gridDim.x * gridDim.y;
+    block_record<USED, NT, true>(v, sh, partial + (int64_t)block * used_count(USED));
     __threadfence();  // the record before the ticket
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned *ticket = reinterpret_cast<unsigned *>(f.result + R_TICKET);
-        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        last = atomicAdd(ticket, 1u) == blocks - 1;
         if (last) *ticket = 0;
     }
     __syncthreads();
     if (!last) return;
     __threadfence();
     if (f.ctl && (double)f.it >= f.ctl[0]) return;  // a deviation past the restore's stop: the result stays
-    sum_records<USED, NT, true>(partial, gridDim.x, sh, total);
+    sum_records<USED, NT, true>(partial, blocks, sh, total);
     finish_record(total, f);
 }
 // the record alone (callers that sum the records in a launch of their own)
@@ -449,59 +450,81 @@ __global__ void __launch_bounds__(kRedThreads) k_observables(Geom g, const void 
     reduce_and_finish<FULL ? kUsedAll : kUsedSample, kRedThreads>(v, partial, fin);
 }
 
-// The observables of FP32 pair storage with even nz, one thread per site pair in packed
-// FP32: the N_CS sample (mask OBS_EDOTB: E^2, plaquette B^2, clover E.B), and FULL
-// (OBS_ALL) the Gauss and unitarity violations too.  A pair's sums run in packed FP32
-// (the Gauss violation's, which cancel, exactly), everything across pairs in FP64.  Per
-// site, with FP64 sums and one lane of every pair vector used, all observables took
-// 2794 us for SU(3) and 638 us for SU(2) at 128^3 on GB300.
+// Storage units (Unit): pairs for the FP32 formats with even nz, sites for FP64.
+template <int FMT> constexpr bool unit_pairs() { return Fmt<FMT>::PAIRED; }
+
+// The observables of a lattice in storage units: the N_CS sample (mask OBS_EDOTB: E^2,
+// plaquette B^2, clover E.B) and, FULL (OBS_ALL), the Gauss and unitarity violations.  A
+// thread takes a unit and a direction (blockIdx.y; FULL: 3 is the violations), so a small
+// lattice has three or four times its units in threads; a unit's sums run in the storage's
+// precision (the Gauss violation's, which cancel, exactly), everything across units in
+// FP64.  SU(3) FP64 is bound by its multiply-adds (0.87 ms at 48^3), the others wait for L2.
+// All observables, with the call, on GB300, one thread a site or pair / by unit and direction:
+// SU(3) FP64 16^3 370 / 74 us, 48^3 1067 / 964; SU(2) FP64 16^3 87 / 37; SU(3) FP32 16^3
+// 40 / 30, 64^3 130 / 114, 128^3 790 / 702; SU(2) FP32 96^3 and 128^3 126 and 213 / 124 and 260
+// (there a thread that shares a pair's links between directions would be faster).  SU(3) by
+// two blocks of 255 registers: three of 168 spill (FP32 64^3 126 us, FP64 48^3 997).
 constexpr int kThreadsObs = 128;
+// a unit's contribution to its direction's sums
+template <class T> __device__ __forceinline__ double lanes_sum(T x) { return (double)x; }
+template <> __device__ __forceinline__ double lanes_sum<f2>(f2 x) { return (double)x.v.x + (double)x.v.y; }
+__device__ __forceinline__ void lanes_max(double x, double &gmax, double &gabs) {
+    gmax = fmax(gmax, x);
+    gabs = fmax(gabs, fabs(x));
+}
+__device__ __forceinline__ void lanes_max(f2 x, float &gmax, float &gabs) {
+    gmax = fmaxf(gmax, fmaxf(x.v.x, x.v.y));
+    gabs = fmaxf(gabs, fmaxf(fabsf(x.v.x), fabsf(x.v.y)));
+}
 template <int FMT, bool FULL>
 __global__ void __launch_bounds__(kThreadsObs, Fmt<FMT>::NA == 8 ? 2 : 4)
-    k_obs_pair(Geom g, const void *U, const void *E, double *partial, Finish fin) {
+    k_obs_units(Geom g, const void *U, const void *E, double *partial, Finish fin) {
     using F = Fmt<FMT>;
-    double v[P_WIDTH];
-#pragma unroll
-    for (int k = 0; k < P_WIDTH; ++k) v[k] = 0.0;
-    float gmax = 0.f, gabs = 0.f, umax = 0.f;
-    const int64_t Vh = g.V >> 1, plane = (int64_t)g.nx * g.ny;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < Vh; p += (int64_t)gridDim.x * blockDim.x) {
-        const bool seam = p < plane || p >= Vh - plane;
-#pragma unroll 1
-        for (int mu = 0; mu < 3; ++mu) {
-            f2 esq, bsq;
-            const f2 edb = seam ? pair_edotb_obs<F, true>(g, U, E, p, mu, esq, bsq)
-                                : pair_edotb_obs<F, false>(g, U, E, p, mu, esq, bsq);
-            const double es = (double)esq.v.x + (double)esq.v.y, bs = (double)bsq.v.x + (double)bsq.v.y;
-            // fixed slots (a run-time index would put v in local memory)
-            if (mu == 0) { v[P_ESQ0] += es; v[P_BSQ0] += bs; }
-            else if (mu == 1) { v[P_ESQ0 + 1] += es; v[P_BSQ0 + 1] += bs; }
-            else { v[P_ESQ0 + 2] += es; v[P_BSQ0 + 2] += bs; }
-            v[P_EDB] += (double)edb.v.x + (double)edb.v.y;
+    using UN = Unit<F, unit_pairs<FMT>()>;
+    using T = typename UN::T;
+    const int mu = blockIdx.y;
+    const int64_t n = UN::count(g), step = (int64_t)gridDim.x * blockDim.x;
+    double es = 0.0, bs = 0.0, edb = 0.0, gsq = 0.0, usq = 0.0;
+    typename UN::C gmax = 0, gabs = 0, umax = 0, unused = 0;
+    if (!FULL || mu < 3) {
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
+            T esq, bsq;
+            edb += lanes_sum(unit_clover<F, unit_pairs<FMT>()>(g, U, E, i, mu, esq, bsq));
+            es += lanes_sum(esq);
+            bs += lanes_sum(bsq);
         }
-        if constexpr (FULL) {
-            f2 gv[F::NA], gsq(0.0), usq(0.0);
-            pair_gauss<F, true>(g, U, E, p, gv);
+    } else {
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
+            T gv[F::NA], q(0), w(0);
+            unit_gauss<F, unit_pairs<FMT>()>(g, U, E, i, gv);
 #pragma unroll
             for (int a = 0; a < F::NA; ++a) {
-                const float x = gv[a].v.x, y = gv[a].v.y;
-                gsq = fma(gv[a], gv[a], gsq);
-                gmax = fmaxf(gmax, fmaxf(x, y));
-                gabs = fmaxf(gabs, fmaxf(fabsf(x), fabsf(y)));
+                q = fma(gv[a], gv[a], q);
+                lanes_max(gv[a], gmax, gabs);
             }
+            const UN u(g, i);
 #pragma unroll 1
-            for (int mu = 0; mu < 3; ++mu) {
-                const f2 n = F::G2::unitarity_square(F::load2(U, Vh, mu, p, false));
-                usq = usq + n;
-                umax = fmaxf(umax, fmaxf(n.v.x, n.v.y));
+            for (int d = 0; d < 3; ++d) {
+                const T un = UN::G::unitarity_square(u.link(U, d, 0));
+                w = w + un;
+                lanes_max(un, umax, unused);
             }
-            v[P_GSQ] += (double)gsq.v.x + (double)gsq.v.y;
-            v[P_USQ] += (double)usq.v.x + (double)usq.v.y;
+            gsq += lanes_sum(q);
+            usq += lanes_sum(w);
         }
     }
+    double v[P_WIDTH];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        v[P_ESQ0 + k] = k == mu ? es : 0.0;
+        v[P_BSQ0 + k] = k == mu ? bs : 0.0;
+    }
+    v[P_EDB] = edb;
+    v[P_GSQ] = gsq;
+    v[P_USQ] = usq;
     v[P_GMAX] = gmax;
     v[P_GABS] = gabs;
-    v[P_UMAX] = sqrtf(umax);
+    v[P_UMAX] = sqrt((double)umax);
     reduce_and_finish<FULL ? kUsedAll : kUsedSample, kThreadsObs>(v, partial, fin);
 }
 
@@ -569,16 +592,15 @@ __global__ void __launch_bounds__(threads_for<FMT>()) k_gauss_update_it(Geom g, 
 // iteration past the stop returns at once, and a deviation past it leaves the result of
 // the last one.
 constexpr int kThreadsRestore = 128;
-template <int FMT> constexpr bool restore_pairs() { return Fmt<FMT>::PAIRED; }
 template <int FMT, bool UPDATE>
 __global__ void __launch_bounds__(kThreadsRestore, 4)
     k_restore(Geom g, const void *U, const void *Ein, void *Eout,
-              const typename RestoreUnit<Fmt<FMT>, restore_pairs<FMT>()>::T *Gin,
-              typename RestoreUnit<Fmt<FMT>, restore_pairs<FMT>()>::T *Gout, double gam, int it, double *partial,
+              const typename Unit<Fmt<FMT>, unit_pairs<FMT>()>::T *Gin,
+              typename Unit<Fmt<FMT>, unit_pairs<FMT>()>::T *Gout, double gam, int it, double *partial,
               Finish fin) {
     using F = Fmt<FMT>;
-    constexpr bool PAIR = restore_pairs<FMT>();
-    using RU = RestoreUnit<F, PAIR>;
+    constexpr bool PAIR = unit_pairs<FMT>();
+    using RU = Unit<F, PAIR>;
     if (UPDATE && (double)it >= fin.ctl[0]) return;  // the same value for every thread of the grid
     const int64_t n = RU::count(g);
     typename RU::C gsq = 0, gmax = 0, gabs = 0;
@@ -777,13 +799,16 @@ template <int FMT> struct Launch {
     // the observables `mask` into fin's result block; max_blocks: records in `partial`
     static cudaError_t observables(const Geom &g, const void *U, const void *E, int mask, double *partial,
                                    int max_blocks, const Finish &fin, cudaStream_t st) {
-        if constexpr (Fmt<FMT>::PAIRED) {
-            if ((mask == OBS_EDOTB || mask == OBS_ALL) && g.nz % 2 == 0) {
-                const int need = grid_for(g.V >> 1, kThreadsObs), blocks = need < max_blocks ? need : max_blocks;
-                if (mask == OBS_ALL) k_obs_pair<FMT, true><<<blocks, kThreadsObs, 0, st>>>(g, U, E, partial, fin);
-                else k_obs_pair<FMT, false><<<blocks, kThreadsObs, 0, st>>>(g, U, E, partial, fin);
-                return cudaGetLastError();
+        if ((mask == OBS_EDOTB || mask == OBS_ALL) && (!F::PAIRED || g.nz % 2 == 0)) {
+            const int need = grid_for(Unit<F, unit_pairs<FMT>()>::count(g), kThreadsObs);
+            if (mask == OBS_ALL) {  // at most max_blocks records
+                const int x = need < max_blocks / 4 ? need : max_blocks / 4;
+                k_obs_units<FMT, true><<<dim3((unsigned)x, 4), kThreadsObs, 0, st>>>(g, U, E, partial, fin);
+            } else {
+                const int x = need < max_blocks / 3 ? need : max_blocks / 3;
+                k_obs_units<FMT, false><<<dim3((unsigned)x, 3), kThreadsObs, 0, st>>>(g, U, E, partial, fin);
             }
+            return cudaGetLastError();
         }
         const int blocks = reduce_grid(g, max_blocks);
         if (mask & (OBS_GAUSS | OBS_UNIT))
@@ -794,10 +819,10 @@ template <int FMT> struct Launch {
     }
     // The fused restore's launches: E and G alternate between two buffers each.
     static bool restore_fused(const Geom &g) { return !F::PAIRED || g.nz % 2 == 0; }
-    using GT = typename RestoreUnit<F, restore_pairs<FMT>()>::T;
+    using GT = typename Unit<F, unit_pairs<FMT>()>::T;
     // bytes of one G buffer
     static size_t restore_g_bytes(const Geom &g) {
-        return sizeof(GT) * F::NA * (size_t)RestoreUnit<F, restore_pairs<FMT>()>::count(g);
+        return sizeof(GT) * F::NA * (size_t)Unit<F, unit_pairs<FMT>()>::count(g);
     }
     template <bool UPDATE>
     static cudaError_t restore(const Geom &g, const void *U, const void *Ein, void *Eout, const void *Gin, void *Gout,
@@ -805,7 +830,7 @@ template <int FMT> struct Launch {
         // max_blocks is 8 a multiprocessor.  FP64: 3 (a grid of 4 would hold every register for
         // the whole launch, and the request loop's ticks wait for its blocks: 2.0 ms a tick
         // beside a 128^3 preparation, against 0.24 ms alone)
-        const int need = grid_for(RestoreUnit<F, restore_pairs<FMT>()>::count(g), kThreadsRestore);
+        const int need = grid_for(Unit<F, unit_pairs<FMT>()>::count(g), kThreadsRestore);
         const int most = F::PAIRED ? max_blocks : max_blocks / 8 * 3;
         k_restore<FMT, UPDATE><<<need < most ? need : most, kThreadsRestore, 0, st>>>(
             g, U, Ein, Eout, static_cast<const GT *>(Gin), static_cast<GT *>(Gout), gam, it, partial, fin);

@@ -235,6 +235,9 @@ template <class T> struct SU2 {
     static TCYM_HD Mat add(const Mat &a, const Mat &b) {
         return Mat{{a.q[0] + b.q[0], a.q[1] + b.q[1], a.q[2] + b.q[2], a.q[3] + b.q[3]}};
     }
+    static TCYM_HD Mat sub(const Mat &a, const Mat &b) {
+        return Mat{{a.q[0] - b.q[0], a.q[1] - b.q[1], a.q[2] - b.q[2], a.q[3] - b.q[3]}};
+    }
     static TCYM_HD Mat scale(T s, const Mat &a) { return Mat{{s * a.q[0], s * a.q[1], s * a.q[2], s * a.q[3]}}; }
     // quaternion product (u3 + i u.s)(v3 + i v.s) = u3 v3 - u.v + i (u3 v + v3 u - u x v).s
     // with optional conjugation of either factor
@@ -276,6 +279,10 @@ template <class T> struct SU2 {
         const Mat w = mulx<false, true>(a, b);
         proj(w, out);
     }
+    // Re tr(1 - a b^dag)
+    static TCYM_HD T retr_one_minus_dag(const Mat &a, const Mat &b) {
+        return T(2) * (T(1) - fma(a.q[0], b.q[0], fma(a.q[1], b.q[1], fma(a.q[2], b.q[2], a.q[3] * b.q[3]))));
+    }
     // p = proj(a b^dag) / kLoopScale for group elements a, b (a plaquette's two halves):
     // the vector part of the product, its sign left to the scale
     static constexpr double kLoopScale = -1.0;
@@ -313,6 +320,7 @@ template <class T> struct SU2 {
         Mat w = mulx<false, true>(mulx<false, false>(v, q), v);
         out[0] = w.q[0]; out[1] = w.q[1]; out[2] = w.q[2];
     }
+    static TCYM_HD void transport_any(const Mat &v, const T *e, T *out) { inverse_adjoint(v, e, out); }
     static TCYM_HD void inverse_adjoint(const Mat &v, const T *e, T *out) {
         Mat q{{e[0], e[1], e[2], T(0)}};
         Mat w = mulx<false, false>(mulx<true, false>(v, q), v);
@@ -371,6 +379,12 @@ template <class T> struct SU3 {
         Mat r;
         for (int i = 0; i < 3; ++i)
             for (int j = 0; j < 3; ++j) r.m[i][j] = a.m[i][j] + b.m[i][j];
+        return r;
+    }
+    static TCYM_HD Mat sub(const Mat &a, const Mat &b) {
+        Mat r;
+        for (int i = 0; i < 3; ++i)
+            for (int j = 0; j < 3; ++j) r.m[i][j] = a.m[i][j] - b.m[i][j];
         return r;
     }
     static TCYM_HD Mat scale(T s, const Mat &a) {
@@ -483,6 +497,18 @@ template <class T> struct SU3 {
             }
         proj(w, p);
     }
+    // Re tr(1 - a b^dag)
+    static TCYM_HD T retr_one_minus_dag(const Mat &a, const Mat &b) {
+        T r[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            r[i] = T(1);
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                r[i] = fma(-a.m[i][k].re, b.m[i][k].re, fma(-a.m[i][k].im, b.m[i][k].im, r[i]));
+        }
+        return r[0] + r[1] + r[2];
+    }
     // p = proj(a b^dag) / kLoopScale for group elements a (rows 0 and 1 are read) and b:
     // rows 0 and 1 of the product are formed, and of its row 2 = conj(row0 x row1) the
     // parts that proj reads
@@ -516,14 +542,17 @@ template <class T> struct SU3 {
     // only columns 0 and 1 of H V are formed: the entries below the diagonal and the
     // first two diagonal ones of V^dagger (H V) need no more, and the third follows
     // from the trace (108 operations; inverse_adjoint's two full products take 216).
-    static TCYM_HD void transport(const Mat &v, const T *e, T *out) {
+    static TCYM_HD void transport(const Mat &v, const T *e, T *out) { transport_columns<2>(v, e, out); }
+    // the same for any matrix V, whose third diagonal entry the trace does not give (144)
+    static TCYM_HD void transport_any(const Mat &v, const T *e, T *out) { transport_columns<3>(v, e, out); }
+    template <int NC> static TCYM_HD void transport_columns(const Mat &v, const T *e, T *out) {
         const T is3 = T(0.57735026918962576450914878050196);
         const T a7 = is3 * e[7];
         const T a0 = a7 + e[2], a1 = a7 - e[2], a2 = T(-2) * a7;
         const cx<T> h10{e[0], e[1]}, h20{e[3], e[4]}, h21{e[5], e[6]};
-        cx<T> w[3][2];
+        cx<T> w[3][NC];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
+        for (int j = 0; j < NC; ++j) {
             const cx<T> x = v.m[0][j], y = v.m[1][j], z = v.m[2][j];
             w[0][j] = cfma_cn(h10, y, cfma_cn(h20, z, cx<T>{a0 * x.re, a0 * x.im}));
             w[1][j] = cfma(h10, x, cfma_cn(h21, z, cx<T>{a1 * y.re, a1 * y.im}));
@@ -548,7 +577,8 @@ template <class T> struct SU3 {
         out[2] = T(0.5) * (m00 - m11);
         out[3] = m20.re; out[4] = m20.im;
         out[5] = m21.re; out[6] = m21.im;
-        out[7] = T(0.86602540378443864676) * (m00 + m11);
+        if constexpr (NC == 3) out[7] = T(0.5) * is3 * fma(T(-2), diagonal(2), m00 + m11);
+        else out[7] = T(0.86602540378443864676) * (m00 + m11);
     }
     // the other way, V (e^a t^a) V^dagger: rows 0 and 1 of V H, and of (V H) V^dagger the
     // entries above the diagonal and the first two on it

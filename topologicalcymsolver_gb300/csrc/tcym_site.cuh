@@ -571,81 +571,117 @@ TCYM_HD void site_observables(const Geom &g, const void *U, const void *E, int m
     }
 }
 
-// The N_CS sample's observables (mask OBS_EDOTB) of direction mu for both sites of
-// pair p of FP32 pair storage (even nz), in packed FP32 (lane 0: site p, lane 1:
-// its partner p + Vh): E_mu^2 into esq, the plaquette term of B_mu^2 into bsq, and
-// the clover E_mu . B_mu returned, as site_observables forms them.  SEAM: the pair
-// may step across the z seam, where a neighbour's lanes come swapped.  The clover
-// average's projection is the average of the leaves' projections (proj is linear),
-// so each leaf is a left-to-right chain of products whose last one is projected
-// at once (proj_mul, proj_mul_dag) and no 3x3 sum is held; E.B accumulates in FP32.
-template <class F, bool SEAM>
-TCYM_HD f2 pair_edotb_obs(const Geom &g, const void *U, const void *E, int64_t p, int mu, f2 &esq, f2 &bsq) {
-    using G2 = typename F::G2;
-    using M2 = typename F::Mat2;
+// A storage unit: a site pair of FP32 pair storage with even nz, in packed FP32, or a
+// site of an FP64 lattice, with its links and fields and its neighbours'; the restore's G as
+// planes G[a * count + i] of T.
+template <class F, bool PAIR> struct Unit;
+template <class F> struct Unit<F, true> {
+    using T = f2;
+    using C = float;
+    using G = typename F::G2;
+    using Mat = typename F::Mat2;
+    static TCYM_HD int64_t count(const Geom &g) { return g.V >> 1; }
+    PairNbhd nb;
+    int64_t n;
+    TCYM_HD Unit(const Geom &g, int64_t i) : nb(g, i), n(g.V >> 1) {}
+    TCYM_HD Mat link(const void *U, int mu, int a) const { return F::load2(U, n, mu, nb.at(mu, a), nb.swapped(mu, a)); }
+    // the link along d at a steps along j and b along k
+    TCYM_HD Mat link(const void *U, int d, int j, int a, int k, int b) const {
+        return F::load2(U, n, d, nb.at(j, a, k, b), nb.swapped(j, a, k, b));
+    }
+    TCYM_HD void load_e(const void *E, int mu, int a, T *e) const {
+        F::load_e2(E, n, mu, nb.at(mu, a), e);
+        if (nb.swapped(mu, a)) {
+#pragma unroll
+            for (int k = 0; k < F::NA; ++k) e[k] = swap_f2(e[k]);
+        }
+    }
+    TCYM_HD void store_e(void *E, int mu, const T *e) const { F::store_e2(E, n, mu, nb.p, e); }
+    TCYM_HD void load_g(const T *G, int mu, int a, T *v) const {
+        const int64_t i = nb.at(mu, a);
+        const bool sw = nb.swapped(mu, a);
+#pragma unroll
+        for (int k = 0; k < F::NA; ++k) v[k] = sw ? swap_f2(G[k * n + i]) : G[k * n + i];
+    }
+    TCYM_HD int64_t self() const { return nb.p; }
+    // a measurement's products: group elements
+    template <bool DA, bool DB> static TCYM_HD Mat times(const Mat &a, const Mat &b) { return G::template mulu<DA, DB>(a, b); }
+    static TCYM_HD void transport(const Mat &v, const T *e, T *out) { G::transport(v, e, out); }
+};
+template <class F> struct Unit<F, false> {
+    using T = typename F::T;
+    using C = T;
+    using G = typename F::G;
+    using Mat = typename F::Mat;
+    static TCYM_HD int64_t count(const Geom &g) { return g.V; }
+    Nbhd nb;
+    int64_t n;
+    TCYM_HD Unit(const Geom &g, int64_t i) : nb(g, i), n(g.V) {}
+    TCYM_HD Mat link(const void *U, int mu, int a) const { return F::load(U, n, mu, nb.at(mu, a)); }
+    TCYM_HD Mat link(const void *U, int d, int j, int a, int k, int b) const {
+        return F::load(U, n, d, nb.at(j, a, k, b));
+    }
+    TCYM_HD void load_e(const void *E, int mu, int a, T *e) const { F::load_e(E, n, mu, nb.at(mu, a), e); }
+    TCYM_HD void store_e(void *E, int mu, const T *e) const { F::store_e(E, n, mu, nb.s, e); }
+    TCYM_HD void load_g(const T *G, int mu, int a, T *v) const {
+        const int64_t i = nb.at(mu, a);
+#pragma unroll
+        for (int k = 0; k < F::NA; ++k) v[k] = G[k * n + i];
+    }
+    TCYM_HD int64_t self() const { return nb.s; }
+    // a measurement's products: any matrices
+    template <bool DA, bool DB> static TCYM_HD Mat times(const Mat &a, const Mat &b) { return G::template mulx<DA, DB>(a, b); }
+    static TCYM_HD void transport(const Mat &v, const T *e, T *out) { G::transport_any(v, e, out); }
+};
+
+// The N_CS sample's observables (mask OBS_EDOTB) of direction mu for unit i: E_mu^2 into
+// esq, the plaquette term of B_mu^2 into bsq, and the clover E_mu . B_mu returned, as
+// site_observables forms them.  The clover average's projection is the average of the
+// leaves' projections (proj is linear), and proj(Q^dag) = -proj(Q): leaves that end in the
+// same link, one of them daggered, are summed before they are multiplied by it (ten
+// products for the four leaves instead of twelve).  An FP64 site's links may be off the
+// group (a pair's third rows are not stored), so there whole products are formed.  Both
+// sums of a unit run in the storage's precision.
+template <class F, bool PAIR>
+TCYM_HD typename Unit<F, PAIR>::T unit_clover(const Geom &g, const void *U, const void *E, int64_t i, int mu,
+                                              typename Unit<F, PAIR>::T &esq, typename Unit<F, PAIR>::T &bsq) {
+    using UN = Unit<F, PAIR>;
+    using T = typename UN::T;
+    using G = typename UN::G;
+    using M = typename UN::Mat;
     constexpr int NA = F::NA;
-    const int64_t Vh = g.V >> 1;
-    const PairNbhd nb(g, p);
+    const UN u(g, i);
     // clover of plane (j, k) = (mu+1, mu+2): the leaves of clover_leaves(j, k)
     const int j = mu == 2 ? 0 : mu + 1, k = mu == 0 ? 2 : mu - 1;
-    auto L = [&](int d, int a, int b) {
-        return F::load2(U, Vh, d, nb.at(j, a, k, b), SEAM && nb.swapped(j, a, k, b));
-    };
-    f2 b[NA], pr[NA];
-    {
-        // Q0 = U_j(x) U_k(x+j) U_j^dag(x+k) U_k^dag(x), whole: its trace is the plaquette term
-        M2 t = G2::mul(L(j, 0, 0), L(k, 1, 0));
-        t = G2::template mulx<false, true>(t, L(j, 0, 1));
-        const M2 q0 = G2::template mulx<false, true>(t, L(k, 0, 0));
-        bsq = f2(4.0) * G2::retr_one_minus(q0);
-        G2::proj(q0, b);
+    auto L = [&](int d, int a, int b) { return u.link(U, d, j, a, k, b); };
+    T b[NA], pr[NA];
+    {   // Q2 - Q0^dag = (U_k^dag(x-k) U_j(x-k) U_k(x-k+j) - U_k(x) U_j(x+k) U_k^dag(x+j)) U_j^dag(x)
+        const M end = L(j, 0, 0);
+        const M q0 = UN::template times<false, true>(UN::template times<false, false>(L(k, 0, 0), L(j, 0, 1)), L(k, 1, 0));
+        bsq = T(4) * G::retr_one_minus_dag(q0, end);
+        const M q2 = UN::template times<false, false>(UN::template times<true, false>(L(k, 0, -1), L(j, 0, -1)), L(k, 1, -1));
+        G::proj_mul_dag(G::sub(q2, q0), end, b);
     }
-    {
-        // Q1 = U_k(x) U_j^dag(x+k-j) U_k^dag(x-j) U_j(x-j)
-        M2 t = G2::template mulx<false, true>(L(k, 0, 0), L(j, -1, 1));
-        t = G2::template mulx<false, true>(t, L(k, -1, 0));
-        G2::proj_mul(t, L(j, -1, 0), pr);
+    {   // Q1 - Q3^dag = (U_k(x) U_j^dag(x+k-j) U_k^dag(x-j) - U_k^dag(x-k) U_j^dag(x-j-k) U_k(x-j-k)) U_j(x-j)
+        const M q1 = UN::template times<false, true>(UN::template times<false, true>(L(k, 0, 0), L(j, -1, 1)), L(k, -1, 0));
+        const M q3 = UN::template times<false, false>(UN::template times<true, true>(L(k, 0, -1), L(j, -1, -1)), L(k, -1, -1));
+        G::proj_mul(G::sub(q1, q3), L(j, -1, 0), pr);
 #pragma unroll
         for (int a = 0; a < NA; ++a) b[a] = b[a] + pr[a];
-    }
-    {
-        // Q2 = U_k^dag(x-k) U_j(x-k) U_k(x-k+j) U_j^dag(x)
-        M2 t = G2::template mulx<true, false>(L(k, 0, -1), L(j, 0, -1));
-        t = G2::mul(t, L(k, 1, -1));
-        G2::proj_mul_dag(t, L(j, 0, 0), pr);
-#pragma unroll
-        for (int a = 0; a < NA; ++a) b[a] = b[a] + pr[a];
-    }
-    {
-        // Q3 = U_j^dag(x-j) U_k^dag(x-j-k) U_j(x-j-k) U_k(x-k)
-        M2 t = G2::template mulx<true, true>(L(j, -1, 0), L(k, -1, -1));
-        t = G2::mul(t, L(j, -1, -1));
-        G2::proj_mul(t, L(k, 0, -1), pr);
-#pragma unroll
-        for (int a = 0; a < NA; ++a) b[a] = f2(0.25) * (b[a] + pr[a]);
     }
     // E_mu(x) and U_mu^dag(x-mu) E_mu(x-mu) U_mu(x-mu)
-    f2 e[NA], et[NA];
-    {
-        f2 em[NA];
-        const int64_t pm = nb.at(mu, -1);
-        const bool sw = SEAM && nb.swapped(mu, -1);
-        F::load_e2(E, Vh, mu, pm, em);
-        if (sw) {
-#pragma unroll
-            for (int a = 0; a < NA; ++a) em[a] = swap_f2(em[a]);
-        }
-        G2::inverse_adjoint(F::load2(U, Vh, mu, pm, sw), em, et);
-    }
-    F::load_e2(E, Vh, mu, p, e);
-    f2 sq(0.0), dot(0.0);
+    T e[NA], et[NA];
+    u.load_e(E, mu, -1, e);
+    UN::transport(u.link(U, mu, -1), e, et);
+    u.load_e(E, mu, 0, e);
+    T sq(0), dot(0);
 #pragma unroll
     for (int a = 0; a < NA; ++a) {
         sq = fma(e[a], e[a], sq);
         dot = fma(e[a] + et[a], b[a], dot);
     }
     esq = sq;
-    return dot;
+    return T(0.25) * dot;
 }
 
 // A sum of FP32 products and terms with its rounding errors carried beside it: each
@@ -667,33 +703,32 @@ template <class T> struct ExactSum {
     }
     TCYM_HD T value() const { return s + e; }
 };
-// The Gauss violation G(x) = sum_mu E_mu(x) - U_mu^dag(x-mu) E_mu(x-mu) U_mu(x-mu) of both
-// sites of pair p of FP32 pair storage (even nz).  G of a restored field is a sum that
-// cancels, so its six terms are summed with their rounding errors (ExactSum).
-template <class F, bool SEAM> TCYM_HD void pair_gauss(const Geom &g, const void *U, const void *E, int64_t p, f2 *gv) {
-    using G2 = typename F::G2;
+// The Gauss violation G(x) = sum_mu E_mu(x) - U_mu^dag(x-mu) E_mu(x-mu) U_mu(x-mu) of unit
+// i.  G of a restored field is a sum that cancels, so pairs sum their six FP32 terms with
+// the rounding errors (ExactSum).
+template <class F, bool PAIR>
+TCYM_HD void unit_gauss(const Geom &g, const void *U, const void *E, int64_t i, typename Unit<F, PAIR>::T *gv) {
+    using UN = Unit<F, PAIR>;
+    using T = typename UN::T;
     constexpr int NA = F::NA;
-    const int64_t Vh = g.V >> 1;
-    const PairNbhd nb(g, p);
-    ExactSum<f2> s[NA];
+    const UN u(g, i);
+    ExactSum<T> s[NA];
 #pragma unroll
-    for (int a = 0; a < NA; ++a) s[a] = ExactSum<f2>(f2(0.0));
+    for (int a = 0; a < NA; ++a) s[a] = ExactSum<T>(T(0));
 #pragma unroll 1
     for (int mu = 0; mu < 3; ++mu) {
-        const int64_t pm = nb.at(mu, -1);
-        const bool sw = SEAM && nb.swapped(mu, -1);
-        f2 e[NA], t[NA];
-        F::load_e2(E, Vh, mu, pm, e);
-        if (sw) {
-#pragma unroll
-            for (int a = 0; a < NA; ++a) e[a] = swap_f2(e[a]);
-        }
-        G2::transport(F::load2(U, Vh, mu, pm, sw), e, t);
-        F::load_e2(E, Vh, mu, p, e);
+        T e[NA], t[NA];
+        u.load_e(E, mu, -1, e);
+        UN::transport(u.link(U, mu, -1), e, t);
+        u.load_e(E, mu, 0, e);
 #pragma unroll
         for (int a = 0; a < NA; ++a) {
-            s[a].add(e[a]);
-            s[a].add(-t[a]);
+            if constexpr (PAIR) {
+                s[a].add(e[a]);
+                s[a].add(-t[a]);
+            } else {
+                s[a].s = s[a].s + (e[a] - t[a]);
+            }
         }
     }
 #pragma unroll
@@ -740,55 +775,6 @@ TCYM_HD void site_gauss_update(const Geom &g, const void *U, void *E, const doub
 }
 
 // ------------------------------------------------------------- restore, fused
-// A storage unit of the fused restore: a site pair of FP32 pair storage with even nz, in
-// packed FP32, or a site of an FP64 lattice.  G is held as planes G[a * count + i] of T.
-template <class F, bool PAIR> struct RestoreUnit;
-template <class F> struct RestoreUnit<F, true> {
-    using T = f2;
-    using C = float;
-    using G = typename F::G2;
-    using Mat = typename F::Mat2;
-    static TCYM_HD int64_t count(const Geom &g) { return g.V >> 1; }
-    PairNbhd nb;
-    int64_t n;
-    TCYM_HD RestoreUnit(const Geom &g, int64_t i) : nb(g, i), n(g.V >> 1) {}
-    TCYM_HD Mat link(const void *U, int mu, int a) const { return F::load2(U, n, mu, nb.at(mu, a), nb.swapped(mu, a)); }
-    TCYM_HD void load_e(const void *E, int mu, int a, T *e) const {
-        F::load_e2(E, n, mu, nb.at(mu, a), e);
-        if (nb.swapped(mu, a)) {
-#pragma unroll
-            for (int k = 0; k < F::NA; ++k) e[k] = swap_f2(e[k]);
-        }
-    }
-    TCYM_HD void store_e(void *E, int mu, const T *e) const { F::store_e2(E, n, mu, nb.p, e); }
-    TCYM_HD void load_g(const T *G, int mu, int a, T *v) const {
-        const int64_t i = nb.at(mu, a);
-        const bool sw = nb.swapped(mu, a);
-#pragma unroll
-        for (int k = 0; k < F::NA; ++k) v[k] = sw ? swap_f2(G[k * n + i]) : G[k * n + i];
-    }
-    TCYM_HD int64_t self() const { return nb.p; }
-};
-template <class F> struct RestoreUnit<F, false> {
-    using T = typename F::T;
-    using C = T;
-    using G = typename F::G;
-    using Mat = typename F::Mat;
-    static TCYM_HD int64_t count(const Geom &g) { return g.V; }
-    Nbhd nb;
-    int64_t n;
-    TCYM_HD RestoreUnit(const Geom &g, int64_t i) : nb(g, i), n(g.V) {}
-    TCYM_HD Mat link(const void *U, int mu, int a) const { return F::load(U, n, mu, nb.at(mu, a)); }
-    TCYM_HD void load_e(const void *E, int mu, int a, T *e) const { F::load_e(E, n, mu, nb.at(mu, a), e); }
-    TCYM_HD void store_e(void *E, int mu, const T *e) const { F::store_e(E, n, mu, nb.s, e); }
-    TCYM_HD void load_g(const T *G, int mu, int a, T *v) const {
-        const int64_t i = nb.at(mu, a);
-#pragma unroll
-        for (int k = 0; k < F::NA; ++k) v[k] = G[k * n + i];
-    }
-    TCYM_HD int64_t self() const { return nb.s; }
-};
-
 // One sub-step of the restore and the next deviation at once (UPDATE), or the deviation
 // alone.  With E'_mu(x) = E_mu(x) - gam (G(x) - U_mu(x) G(x+mu) U_mu^dag(x)), the new
 // deviation's term from below is
@@ -798,9 +784,9 @@ template <class F> struct RestoreUnit<F, false> {
 // gv receives the new G.
 template <class F, bool PAIR, bool UPDATE>
 TCYM_HD void unit_restore(const Geom &g, const void *U, const void *Ein, void *Eout,
-                          const typename RestoreUnit<F, PAIR>::T *Gin, typename RestoreUnit<F, PAIR>::C gam, int64_t i,
-                          typename RestoreUnit<F, PAIR>::T *gv) {
-    using RU = RestoreUnit<F, PAIR>;
+                          const typename Unit<F, PAIR>::T *Gin, typename Unit<F, PAIR>::C gam, int64_t i,
+                          typename Unit<F, PAIR>::T *gv) {
+    using RU = Unit<F, PAIR>;
     using T = typename RU::T;
     using G = typename RU::G;
     constexpr int NA = F::NA;
