@@ -299,7 +299,7 @@ def run_ours(a):
         f1.synchronize()
         t64 = f0.elapsed_time(f1) * 1e-3 / a.steps
         fp64 = {"value": links / t64, "unit": UNIT, "ms_per_step": t64 * 1e3, "steps": a.steps,
-                "kernel": "k_step<SU3 FP64> (one site per thread, full 3x3 complex links, FP64 arithmetic)",
+                "kernel": "k_march<SU3 FP64> (blocks that share their plaquettes, full 3x3 complex links, FP64 arithmetic)",
                 "bytes_per_link_update": 416,
                 "hbm_frac": round(416 * links / t64 / 1e9 / measured_peak()[0], 4),
                 "fp32_over_fp64": round((total / a.steps) ** -1 / t64 ** -1, 2),

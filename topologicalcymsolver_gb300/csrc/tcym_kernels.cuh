@@ -587,7 +587,8 @@ __global__ void __launch_bounds__(threads_for<FMT>()) k_gauss_update_it(Geom g, 
 // sub-step's update and the next deviation (unit_restore), from the fields Ein and G Gin
 // into Eout and Gout, so a sub-step reads the links once and is one launch.  Bound by
 // memory (SU(3) FP32 128^3: 838 MB, 123 us at the measured copy rate); an iteration of
-// three (deviation, update) pairs of launches took 785 us there and 128 us at 64^3.
+// three (deviation, update) pairs of launches took 785 us there and 128 us at 64^3, this one
+// 502 and 99.
 // UPDATE: the update belongs to iteration `it`, the deviation to fin.it; a launch of an
 // iteration past the stop returns at once, and a deviation past it leaves the result of
 // the last one.

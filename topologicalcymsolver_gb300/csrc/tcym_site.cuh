@@ -903,7 +903,8 @@ template <class F> TCYM_HD void site_reunitarize(const Geom &g, void *U, int64_t
 // the entry with one rounding.  A pair with an entry whose sum lies within 1e-13 of the
 // middle of two FP32 numbers (about one warp in 200), or further off the group, or not
 // finite, takes the FP64 projection.  That one ran at the FP64 rate, 1184 us for SU(3) and
-// 336 us for SU(2) at 128^3 on GB300; this one is bound by memory and FP32 arithmetic.
+// 336 us for SU(2) at 128^3 on GB300; this one takes 245 and 53 us, bound by FP32
+// arithmetic (SU(3)) and memory (SU(2); reading and writing the links: 89 and 30 us).
 constexpr float kProjDeviation = 3e-5f, kProjTie = 1e-13f;
 TCYM_HD bool beyond(f2 d, float t) { return !(fabsf(d.v.x) <= t && fabsf(d.v.y) <= t); }
 // a value and its error
