@@ -160,7 +160,7 @@ template <class F> struct March {
             int step;
             if (j < pro) {
                 T t[NA];
-                G::transport(F::load(U, V, 2, (int64_t)zp * plane + u.idx), pr, t);
+                G::rotate(F::load(U, V, 2, (int64_t)zp * plane + u.idx), pr, t);
                 dst = below + (k - 1) * NA * sites + e;
                 step = sites;
 #pragma unroll
@@ -211,7 +211,7 @@ template <class F> struct March {
                 T q[NA], t[NA];
 #pragma unroll
                 for (int a = 0; a < NA; ++a) q[a] = own[a * slots + from];
-                G::transport(F::load(U, V, nu, src), q, t);
+                G::rotate(F::load(U, V, nu, src), q, t);
                 if (nu == 2) {
                     T *b = below + (k - 1) * NA * sites + e;  // no other task's
 #pragma unroll

@@ -292,7 +292,7 @@ template <class T> struct SU2 {
     }
     // components of V^dagger (e^a t^a) V for a group element V: the rotation
     // e + 2 (v3 q x e + q x (q x e)) of its vector part q
-    static TCYM_HD void transport(const Mat &v, const T *e, T *out) {
+    static TCYM_HD void rotate(const Mat &v, const T *e, T *out) {
         const T *q = v.q;
         const T c0 = T(2) * fma(q[1], e[2], -(q[2] * e[1]));
         const T c1 = T(2) * fma(q[2], e[0], -(q[0] * e[2]));
@@ -301,10 +301,9 @@ template <class T> struct SU2 {
         out[1] = fma(q[2], c0, fma(-q[0], c2, fma(q[3], c1, e[1])));
         out[2] = fma(q[0], c1, fma(-q[1], c0, fma(q[3], c2, e[2])));
     }
-    // the other way: V (e^a t^a) V^dagger
-    static TCYM_HD void transport_back(const Mat &v, const T *e, T *out) {
-        transport(Mat{{-v.q[0], -v.q[1], -v.q[2], v.q[3]}}, e, out);
-    }
+    // V^dagger (e^a t^a) V and V (e^a t^a) V^dagger for any V
+    static TCYM_HD void transport(const Mat &v, const T *e, T *out) { inverse_adjoint(v, e, out); }
+    static TCYM_HD void transport_back(const Mat &v, const T *e, T *out) { adjoint(v, e, out); }
     static TCYM_HD T retr_one_minus(const Mat &v) { return T(2) * (T(1) - v.q[3]); }
     // exp(i c t^k e^k) = cos(d/2) + i sin(d/2) (c e / d).sigma, d = |c e|
     static TCYM_HD Mat iexp(T c, const T *e) {
@@ -320,7 +319,6 @@ template <class T> struct SU2 {
         Mat w = mulx<false, true>(mulx<false, false>(v, q), v);
         out[0] = w.q[0]; out[1] = w.q[1]; out[2] = w.q[2];
     }
-    static TCYM_HD void transport_any(const Mat &v, const T *e, T *out) { inverse_adjoint(v, e, out); }
     static TCYM_HD void inverse_adjoint(const Mat &v, const T *e, T *out) {
         Mat q{{e[0], e[1], e[2], T(0)}};
         Mat w = mulx<false, false>(mulx<true, false>(v, q), v);
@@ -542,9 +540,10 @@ template <class T> struct SU3 {
     // only columns 0 and 1 of H V are formed: the entries below the diagonal and the
     // first two diagonal ones of V^dagger (H V) need no more, and the third follows
     // from the trace (108 operations; inverse_adjoint's two full products take 216).
-    static TCYM_HD void transport(const Mat &v, const T *e, T *out) { transport_columns<2>(v, e, out); }
-    // the same for any matrix V, whose third diagonal entry the trace does not give (144)
-    static TCYM_HD void transport_any(const Mat &v, const T *e, T *out) { transport_columns<3>(v, e, out); }
+    static TCYM_HD void rotate(const Mat &v, const T *e, T *out) { transport_columns<2>(v, e, out); }
+    // the same for any matrix V (links drift off the group, and callers load what they
+    // like), whose third diagonal entry the trace does not give (144)
+    static TCYM_HD void transport(const Mat &v, const T *e, T *out) { transport_columns<3>(v, e, out); }
     template <int NC> static TCYM_HD void transport_columns(const Mat &v, const T *e, T *out) {
         const T is3 = T(0.57735026918962576450914878050196);
         const T a7 = is3 * e[7];
@@ -580,16 +579,16 @@ template <class T> struct SU3 {
         if constexpr (NC == 3) out[7] = T(0.5) * is3 * fma(T(-2), diagonal(2), m00 + m11);
         else out[7] = T(0.86602540378443864676) * (m00 + m11);
     }
-    // the other way, V (e^a t^a) V^dagger: rows 0 and 1 of V H, and of (V H) V^dagger the
-    // entries above the diagonal and the first two on it
+    // the other way, V (e^a t^a) V^dagger for any V: V H, and of (V H) V^dagger the entries
+    // above the diagonal and those on it
     static TCYM_HD void transport_back(const Mat &v, const T *e, T *out) {
         const T is3 = T(0.57735026918962576450914878050196);
         const T a7 = is3 * e[7];
         const T a0 = a7 + e[2], a1 = a7 - e[2], a2 = T(-2) * a7;
         const cx<T> h10{e[0], e[1]}, h20{e[3], e[4]}, h21{e[5], e[6]};
-        cx<T> w[2][3];
+        cx<T> w[3][3];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < 3; ++i) {
             const cx<T> x = v.m[i][0], y = v.m[i][1], z = v.m[i][2];
             w[i][0] = cfma(h10, y, cfma(h20, z, cx<T>{a0 * x.re, a0 * x.im}));
             w[i][1] = cfma_cn(h10, x, cfma(h21, z, cx<T>{a1 * y.re, a1 * y.im}));
@@ -614,7 +613,7 @@ template <class T> struct SU3 {
         out[2] = T(0.5) * (m00 - m11);
         out[3] = m02.re; out[4] = -m02.im;
         out[5] = m12.re; out[6] = -m12.im;
-        out[7] = T(0.86602540378443864676) * (m00 + m11);
+        out[7] = T(0.5) * is3 * fma(T(-2), diagonal(2), m00 + m11);
     }
     static TCYM_HD T retr_one_minus(const Mat &v) { return T(3) - (v.m[0][0].re + v.m[1][1].re + v.m[2][2].re); }
 

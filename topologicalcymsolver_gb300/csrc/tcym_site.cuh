@@ -606,7 +606,10 @@ template <class F> struct Unit<F, true> {
     TCYM_HD int64_t self() const { return nb.p; }
     // a measurement's products: group elements
     template <bool DA, bool DB> static TCYM_HD Mat times(const Mat &a, const Mat &b) { return G::template mulu<DA, DB>(a, b); }
-    static TCYM_HD void transport(const Mat &v, const T *e, T *out) { G::transport(v, e, out); }
+    static TCYM_HD void transport(const Mat &v, const T *e, T *out) { G::rotate(v, e, out); }
+    // V^dagger e V for any V.  Whole products: their components are means of two entries with
+    // roundings of their own (a restored SU(3) field's violation 6.0e-8 rms, 6.2e-8 by G::transport)
+    static TCYM_HD void transport_any(const Mat &v, const T *e, T *out) { G::inverse_adjoint(v, e, out); }
 };
 template <class F> struct Unit<F, false> {
     using T = typename F::T;
@@ -631,7 +634,8 @@ template <class F> struct Unit<F, false> {
     TCYM_HD int64_t self() const { return nb.s; }
     // a measurement's products: any matrices
     template <bool DA, bool DB> static TCYM_HD Mat times(const Mat &a, const Mat &b) { return G::template mulx<DA, DB>(a, b); }
-    static TCYM_HD void transport(const Mat &v, const T *e, T *out) { G::transport_any(v, e, out); }
+    static TCYM_HD void transport(const Mat &v, const T *e, T *out) { G::transport(v, e, out); }
+    static TCYM_HD void transport_any(const Mat &v, const T *e, T *out) { G::transport(v, e, out); }
 };
 
 // The N_CS sample's observables (mask OBS_EDOTB) of direction mu for unit i: E_mu^2 into
@@ -776,11 +780,13 @@ TCYM_HD void site_gauss_update(const Geom &g, const void *U, void *E, const doub
 
 // ------------------------------------------------------------- restore, fused
 // One sub-step of the restore and the next deviation at once (UPDATE), or the deviation
-// alone.  With E'_mu(x) = E_mu(x) - gam (G(x) - U_mu(x) G(x+mu) U_mu^dag(x)), the new
-// deviation's term from below is
-//   U^dag(x-mu) E'(x-mu) U(x-mu) = U^dag(x-mu) [E(x-mu) - gam G(x-mu)] U(x-mu) + gam G(x),
-// so each unit forms its own new fields and its new G from the old ones of its neighbours
-// (the three gam G(x) taken off at the start).
+// alone.  The new deviation is that of the new fields, whatever the links: each unit forms
+// its own three,
+//   E'_mu(x) = E_mu(x) - gam (G(x) - U_mu(x) G(x+mu) U_mu^dag(x)),
+// and its lower neighbours' E'_mu(x-mu) again, from the old fields and G and by the same
+// arithmetic.  (On the group U^dag(x-mu) E'(x-mu) U(x-mu) holds gam G(x) itself, which would
+// spare the neighbour's transport of G(x); links a few 1e-7 off it, as FP32 ones between
+// reunitarisations, would leave a violation of that size.)
 // gv receives the new G.
 template <class F, bool PAIR, bool UPDATE>
 TCYM_HD void unit_restore(const Geom &g, const void *U, const void *Ein, void *Eout,
@@ -789,35 +795,37 @@ TCYM_HD void unit_restore(const Geom &g, const void *U, const void *Ein, void *E
     using RU = Unit<F, PAIR>;
     using T = typename RU::T;
     using G = typename RU::G;
+    using M = typename RU::Mat;
     constexpr int NA = F::NA;
     const RU u(g, i);
     const T mg(-gam);
     T gx[NA];
     if (UPDATE) u.load_g(Gin, 0, 0, gx);
 #pragma unroll
-    for (int a = 0; a < NA; ++a) gv[a] = UPDATE ? T(-3) * T(gam) * gx[a] : T(0);
+    for (int a = 0; a < NA; ++a) gv[a] = T(0);
 #pragma unroll 1
     for (int mu = 0; mu < 3; ++mu) {
         T e[NA], q[NA], t[NA];
+        const M below = u.link(U, mu, -1);
         u.load_e(Ein, mu, -1, e);
         if (UPDATE) {
+            G::transport_back(below, gx, t);
             u.load_g(Gin, mu, -1, q);
 #pragma unroll
-            for (int a = 0; a < NA; ++a) e[a] = fma(mg, q[a], e[a]);
+            for (int a = 0; a < NA; ++a) e[a] = fma(mg, q[a] - t[a], e[a]);
         }
-        G::transport(u.link(U, mu, -1), e, t);
-#pragma unroll
-        for (int a = 0; a < NA; ++a) gv[a] = gv[a] - t[a];
+        RU::transport_any(below, e, t);
         u.load_e(Ein, mu, 0, e);
         if (UPDATE) {
+            T s[NA];
             u.load_g(Gin, mu, 1, q);
-            G::transport_back(u.link(U, mu, 0), q, t);
+            G::transport_back(u.link(U, mu, 0), q, s);
 #pragma unroll
-            for (int a = 0; a < NA; ++a) e[a] = fma(mg, gx[a] - t[a], e[a]);
+            for (int a = 0; a < NA; ++a) e[a] = fma(mg, gx[a] - s[a], e[a]);
             u.store_e(Eout, mu, e);
         }
 #pragma unroll
-        for (int a = 0; a < NA; ++a) gv[a] = gv[a] + e[a];
+        for (int a = 0; a < NA; ++a) gv[a] = gv[a] + (e[a] - t[a]);
     }
 }
 
