@@ -124,10 +124,10 @@ template <class F> struct March {
         // P = [U_k(x) U_nu(x+k)] [U_nu(x) U_k(x+nu)]^dag
         const Mat a = F::load(U, V, k, at);
         const Mat b = F::load(U, V, nu, k == 0 ? ax : (k == 1 ? ay : az));
-        const Mat t1 = G::template mulu<false, false>(a, b);
+        const Mat t1 = G::template mulx<false, false>(a, b);
         const Mat c = F::load(U, V, nu, at);
         const Mat d = F::load(U, V, k, nu == 0 ? ax : (nu == 1 ? ay : az));
-        const Mat t2 = G::template mulu<false, false>(c, d);
+        const Mat t2 = G::template mulx<false, false>(c, d);
         G::loop_proj(t1, t2, pr);
     }
 
@@ -160,7 +160,7 @@ template <class F> struct March {
             int step;
             if (j < pro) {
                 T t[NA];
-                G::rotate(F::load(U, V, 2, (int64_t)zp * plane + u.idx), pr, t);
+                G::carry(F::load(U, V, 2, (int64_t)zp * plane + u.idx), pr, t);
                 dst = below + (k - 1) * NA * sites + e;
                 step = sites;
 #pragma unroll
@@ -211,7 +211,7 @@ template <class F> struct March {
                 T q[NA], t[NA];
 #pragma unroll
                 for (int a = 0; a < NA; ++a) q[a] = own[a * slots + from];
-                G::rotate(F::load(U, V, nu, src), q, t);
+                G::carry(F::load(U, V, nu, src), q, t);
                 if (nu == 2) {
                     T *b = below + (k - 1) * NA * sites + e;  // no other task's
 #pragma unroll

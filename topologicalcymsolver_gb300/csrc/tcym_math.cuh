@@ -283,15 +283,32 @@ template <class T> struct SU2 {
     static TCYM_HD T retr_one_minus_dag(const Mat &a, const Mat &b) {
         return T(2) * (T(1) - fma(a.q[0], b.q[0], fma(a.q[1], b.q[1], fma(a.q[2], b.q[2], a.q[3] * b.q[3]))));
     }
-    // p = proj(a b^dag) / kLoopScale for group elements a, b (a plaquette's two halves):
-    // the vector part of the product, its sign left to the scale
+    // p = proj(a b^dag) / kLoopScale (a, b: a plaquette's two halves): the vector part of the
+    // product, its sign left to the scale
     static constexpr double kLoopScale = -1.0;
     static TCYM_HD void loop_proj(const Mat &a, const Mat &b, T *p) {
         const Mat w = mulx<false, true>(a, b);
         p[0] = w.q[0]; p[1] = w.q[1]; p[2] = w.q[2];
     }
-    // components of V^dagger (e^a t^a) V for a group element V: the rotation
-    // e + 2 (v3 q x e + q x (q x e)) of its vector part q
+    // components of V^-1 (e^a t^a) V for any quaternion V but zero: the rotation
+    // e + (2 / |V|^2) (v3 q x e + q x (q x e)) by its vector part q.  A link's |V|^2 = 1 + d is
+    // near 1: three terms in d for |d| <= 1e-4 (the first omitted one d^4), else a division.
+    static TCYM_HD void carry(const Mat &v, const T *e, T *out) {
+        const T *q = v.q;
+        const T d = fma(q[3], q[3], fma(q[0], q[0], fma(q[1], q[1], fma(q[2], q[2], T(-1)))));
+        T s = fma(T(-2) * d, fma(-d, T(1) - d, T(1)), T(2));
+        if (!(fabs(d) <= T(1e-4))) {
+            const T n = fma(q[3], q[3], fma(q[0], q[0], fma(q[1], q[1], q[2] * q[2])));
+            s = n > T(0) ? quot(T(2), n) : T(0);  // a zero link's loop is zero
+        }
+        const T c0 = s * fma(q[1], e[2], -(q[2] * e[1]));
+        const T c1 = s * fma(q[2], e[0], -(q[0] * e[2]));
+        const T c2 = s * fma(q[0], e[1], -(q[1] * e[0]));
+        out[0] = fma(q[1], c2, fma(-q[2], c1, fma(q[3], c0, e[0])));
+        out[1] = fma(q[2], c0, fma(-q[0], c2, fma(q[3], c1, e[1])));
+        out[2] = fma(q[0], c1, fma(-q[1], c0, fma(q[3], c2, e[2])));
+    }
+    // the same for a group element, whose |V|^2 is 1
     static TCYM_HD void rotate(const Mat &v, const T *e, T *out) {
         const T *q = v.q;
         const T c0 = T(2) * fma(q[1], e[2], -(q[2] * e[1]));
@@ -507,40 +524,40 @@ template <class T> struct SU3 {
         }
         return r[0] + r[1] + r[2];
     }
-    // p = proj(a b^dag) / kLoopScale for group elements a (rows 0 and 1 are read) and b:
-    // rows 0 and 1 of the product are formed, and of its row 2 = conj(row0 x row1) the
-    // parts that proj reads
+    // p = proj(a b^dag) / kLoopScale: the sums of two entries that proj reads
     static constexpr double kLoopScale = -0.5;
     static TCYM_HD void loop_proj(const Mat &a, const Mat &b, T *p) {
-        cx<T> w[2][3];
+        auto im = [&](int i, int j, T acc) {  // acc + Im (a b^dag)_ij
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+            for (int k = 0; k < 3; ++k)
+                acc = fma(a.m[i][k].im, b.m[j][k].re, fma(-a.m[i][k].re, b.m[j][k].im, acc));
+            return acc;
+        };
+        auto re = [&](int i, int j) {
+            T acc = T(0);
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                cx<T> acc{a.m[i][0].re * b.m[j][0].re, a.m[i][0].im * b.m[j][0].re};
-                acc.re = fma(a.m[i][0].im, b.m[j][0].im, acc.re);
-                acc.im = fma(-a.m[i][0].re, b.m[j][0].im, acc.im);
-                acc = cfma_nc(a.m[i][1], b.m[j][1], acc);
-                w[i][j] = cfma_nc(a.m[i][2], b.m[j][2], acc);
-            }
-        const cx<T> w20 = conj_cross(w[0][1], w[1][2], w[0][2], w[1][1]);
-        const cx<T> w21 = conj_cross(w[0][2], w[1][0], w[0][0], w[1][2]);
-        const T w22 = conj_cross(w[0][0], w[1][1], w[0][1], w[1][0]).im;
+            for (int k = 0; k < 3; ++k)
+                acc = fma(a.m[i][k].re, b.m[j][k].re, fma(a.m[i][k].im, b.m[j][k].im, acc));
+            return acc;
+        };
         const T is3 = T(0.57735026918962576450914878050196);
-        p[0] = w[0][1].im + w[1][0].im;
-        p[1] = w[0][1].re - w[1][0].re;
-        p[2] = w[0][0].im - w[1][1].im;
-        p[3] = w[0][2].im + w20.im;
-        p[4] = w[0][2].re - w20.re;
-        p[5] = w[1][2].im + w21.im;
-        p[6] = w[1][2].re - w21.re;
-        p[7] = is3 * fma(T(-2), w22, w[0][0].im + w[1][1].im);
+        const T w00 = im(0, 0, T(0)), w11 = im(1, 1, T(0)), w22 = im(2, 2, T(0));
+        p[0] = im(0, 1, im(1, 0, T(0)));
+        p[1] = re(0, 1) - re(1, 0);
+        p[2] = w00 - w11;
+        p[3] = im(0, 2, im(2, 0, T(0)));
+        p[4] = re(0, 2) - re(2, 0);
+        p[5] = im(1, 2, im(2, 1, T(0)));
+        p[6] = re(1, 2) - re(2, 1);
+        p[7] = is3 * fma(T(-2), w22, w00 + w11);
     }
     // components of V^dagger (e^a t^a) V for a group element V.  With H = 2 e^a t^a,
     // only columns 0 and 1 of H V are formed: the entries below the diagonal and the
     // first two diagonal ones of V^dagger (H V) need no more, and the third follows
     // from the trace (108 operations; inverse_adjoint's two full products take 216).
     static TCYM_HD void rotate(const Mat &v, const T *e, T *out) { transport_columns<2>(v, e, out); }
+    // a plaquette's projection carried along a link (V^-1 e V on the group)
+    static TCYM_HD void carry(const Mat &v, const T *e, T *out) { transport(v, e, out); }
     // the same for any matrix V (links drift off the group, and callers load what they
     // like), whose third diagonal entry the trace does not give (144)
     static TCYM_HD void transport(const Mat &v, const T *e, T *out) { transport_columns<3>(v, e, out); }
