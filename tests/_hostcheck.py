@@ -33,6 +33,7 @@ def load():
         L.hc_flow_cb.argtypes = [ctypes.c_int, ip, _vp, ctypes.c_double, ctypes.c_int]
         L.hc_observables.argtypes = [ctypes.c_int, ip, _vp, _vp, ctypes.c_int, _vp]
         L.hc_edotb_pair.argtypes = [ctypes.c_int, ip, _vp, _vp, _vp]
+        L.hc_gauss.argtypes = [ctypes.c_int, ip, _vp, _vp, ctypes.c_int, _vp]
         L.hc_gauss_restore.argtypes = [ctypes.c_int, ip, _vp, _vp, ctypes.c_double, ctypes.c_int]
         L.hc_reunitarize.argtypes = [ctypes.c_int, ip, _vp]
         L.hc_reunitarize_fp64.argtypes = [ctypes.c_int, ip, _vp]
@@ -123,6 +124,13 @@ class HostLattice:
         """The N_CS sample through the paired code, or None where the storage is not paired."""
         out = np.zeros(16)
         ok = self.L.hc_edotb_pair(self.fmt, self.n, _p(self.U[self.cur]), _p(self.E), _p(out))
+        return out if ok else None
+
+    def gauss(self, pairs):
+        """The Gauss violation of every site through the paired (None where the storage is not paired) or the
+        per-site code."""
+        out = np.zeros((int(np.prod(self.shape)), NA[self.nc]))
+        ok = self.L.hc_gauss(self.fmt, self.n, _p(self.U[self.cur]), _p(self.E), int(pairs), _p(out))
         return out if ok else None
 
     def gauss_restore(self, tol=1e-14, maxit=10000):

@@ -233,6 +233,31 @@ template <int FMT> struct H {
         F::G::ilog((T)c, m, o);
         for (int a = 0; a < F::NA; ++a) out[a] = (double)o[a];
     }
+    // the Gauss violation of every site by the pairs' code, out[s * NA + a]
+    static bool gauss_pair(const Geom &g, const void *U, const void *E, double *out) {
+        if constexpr (F::PAIRED) {
+            if (g.nz % 2) return false;
+            const int64_t Vh = g.V >> 1;
+            for (int64_t p = 0; p < Vh; ++p) {
+                f2 gv[F::NA];
+                unit_gauss<F, true>(g, U, E, p, gv);
+                for (int a = 0; a < F::NA; ++a) {
+                    out[p * F::NA + a] = gv[a].v.x;
+                    out[(p + Vh) * F::NA + a] = gv[a].v.y;
+                }
+            }
+            return true;
+        }
+        return false;
+    }
+    // the same site by site, as the other formats measure it
+    static void gauss_sites(const Geom &g, const void *U, const void *E, double *out) {
+        for (int64_t s = 0; s < g.V; ++s) {
+            SiteObs<F> o;
+            site_observables<F>(g, U, E, OBS_GAUSS, s, o);
+            for (int a = 0; a < F::NA; ++a) out[s * F::NA + a] = o.g[a];
+        }
+    }
     static void geodesic(const Geom &g, const void *Uold, const void *Unew, double c, void *Umid, void *Emid) {
         for (int64_t s = 0; s < g.V; ++s) site_geodesic<F>(g, Uold, Unew, c, Umid, Emid, s);
     }
@@ -388,6 +413,16 @@ int hc_edotb_pair(int fmt, const int *n, const void *U, const void *E, double *o
     Geom g = geom(n);
     int ok = 0;
     HC_DISPATCH(fmt, ok = HH::edotb_pair(g, U, E, out));
+    return ok;
+}
+// the Gauss violation of every site, by pairs (0: the storage holds none) or site by site
+int hc_gauss(int fmt, const int *n, const void *U, const void *E, int pairs, double *out) {
+    Geom g = geom(n);
+    int ok = 1;
+    HC_DISPATCH(fmt, {
+        if (pairs) ok = HH::gauss_pair(g, U, E, out);
+        else HH::gauss_sites(g, U, E, out);
+    });
     return ok;
 }
 int hc_gauss_restore(int fmt, const int *n, const void *U, void *E, double tol, int maxit) {

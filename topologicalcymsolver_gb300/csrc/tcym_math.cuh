@@ -308,16 +308,6 @@ template <class T> struct SU2 {
         out[1] = fma(q[2], c0, fma(-q[0], c2, fma(q[3], c1, e[1])));
         out[2] = fma(q[0], c1, fma(-q[1], c0, fma(q[3], c2, e[2])));
     }
-    // the same for a group element, whose |V|^2 is 1
-    static TCYM_HD void rotate(const Mat &v, const T *e, T *out) {
-        const T *q = v.q;
-        const T c0 = T(2) * fma(q[1], e[2], -(q[2] * e[1]));
-        const T c1 = T(2) * fma(q[2], e[0], -(q[0] * e[2]));
-        const T c2 = T(2) * fma(q[0], e[1], -(q[1] * e[0]));
-        out[0] = fma(q[1], c2, fma(-q[2], c1, fma(q[3], c0, e[0])));
-        out[1] = fma(q[2], c0, fma(-q[0], c2, fma(q[3], c1, e[1])));
-        out[2] = fma(q[0], c1, fma(-q[1], c0, fma(q[3], c2, e[2])));
-    }
     // V^dagger (e^a t^a) V and V (e^a t^a) V^dagger for any V
     static TCYM_HD void transport(const Mat &v, const T *e, T *out) { inverse_adjoint(v, e, out); }
     static TCYM_HD void transport_back(const Mat &v, const T *e, T *out) { adjoint(v, e, out); }
@@ -551,24 +541,18 @@ template <class T> struct SU3 {
         p[6] = re(1, 2) - re(2, 1);
         p[7] = is3 * fma(T(-2), w22, w00 + w11);
     }
-    // components of V^dagger (e^a t^a) V for a group element V.  With H = 2 e^a t^a,
-    // only columns 0 and 1 of H V are formed: the entries below the diagonal and the
-    // first two diagonal ones of V^dagger (H V) need no more, and the third follows
-    // from the trace (108 operations; inverse_adjoint's two full products take 216).
-    static TCYM_HD void rotate(const Mat &v, const T *e, T *out) { transport_columns<2>(v, e, out); }
-    // a plaquette's projection carried along a link (V^-1 e V on the group)
-    static TCYM_HD void carry(const Mat &v, const T *e, T *out) { transport(v, e, out); }
-    // the same for any matrix V (links drift off the group, and callers load what they
-    // like), whose third diagonal entry the trace does not give (144)
-    static TCYM_HD void transport(const Mat &v, const T *e, T *out) { transport_columns<3>(v, e, out); }
-    template <int NC> static TCYM_HD void transport_columns(const Mat &v, const T *e, T *out) {
+    // components of V^dagger (e^a t^a) V for any matrix V (links drift off the group, and
+    // callers load what they like).  With H = 2 e^a t^a: H V, and of V^dagger (H V) the entries
+    // below the diagonal and those on it (144 operations; inverse_adjoint's two full products
+    // take 216)
+    static TCYM_HD void transport(const Mat &v, const T *e, T *out) {
         const T is3 = T(0.57735026918962576450914878050196);
         const T a7 = is3 * e[7];
         const T a0 = a7 + e[2], a1 = a7 - e[2], a2 = T(-2) * a7;
         const cx<T> h10{e[0], e[1]}, h20{e[3], e[4]}, h21{e[5], e[6]};
-        cx<T> w[3][NC];
+        cx<T> w[3][3];
 #pragma unroll
-        for (int j = 0; j < NC; ++j) {
+        for (int j = 0; j < 3; ++j) {
             const cx<T> x = v.m[0][j], y = v.m[1][j], z = v.m[2][j];
             w[0][j] = cfma_cn(h10, y, cfma_cn(h20, z, cx<T>{a0 * x.re, a0 * x.im}));
             w[1][j] = cfma(h10, x, cfma_cn(h21, z, cx<T>{a1 * y.re, a1 * y.im}));
@@ -593,9 +577,10 @@ template <class T> struct SU3 {
         out[2] = T(0.5) * (m00 - m11);
         out[3] = m20.re; out[4] = m20.im;
         out[5] = m21.re; out[6] = m21.im;
-        if constexpr (NC == 3) out[7] = T(0.5) * is3 * fma(T(-2), diagonal(2), m00 + m11);
-        else out[7] = T(0.86602540378443864676) * (m00 + m11);
+        out[7] = T(0.5) * is3 * fma(T(-2), diagonal(2), m00 + m11);
     }
+    // a plaquette's projection carried along a link (V^-1 e V on the group)
+    static TCYM_HD void carry(const Mat &v, const T *e, T *out) { transport(v, e, out); }
     // the other way, V (e^a t^a) V^dagger for any V: V H, and of (V H) V^dagger the entries
     // above the diagonal and those on it
     static TCYM_HD void transport_back(const Mat &v, const T *e, T *out) {

@@ -604,12 +604,9 @@ template <class F> struct Unit<F, true> {
         for (int k = 0; k < F::NA; ++k) v[k] = sw ? swap_f2(G[k * n + i]) : G[k * n + i];
     }
     TCYM_HD int64_t self() const { return nb.p; }
-    // a measurement's products: group elements
-    template <bool DA, bool DB> static TCYM_HD Mat times(const Mat &a, const Mat &b) { return G::template mulu<DA, DB>(a, b); }
-    static TCYM_HD void transport(const Mat &v, const T *e, T *out) { G::rotate(v, e, out); }
     // V^dagger e V for any V.  Whole products: their components are means of two entries with
     // roundings of their own (a restored SU(3) field's violation 6.0e-8 rms, 6.2e-8 by G::transport)
-    static TCYM_HD void transport_any(const Mat &v, const T *e, T *out) { G::inverse_adjoint(v, e, out); }
+    static TCYM_HD void transport(const Mat &v, const T *e, T *out) { G::inverse_adjoint(v, e, out); }
 };
 template <class F> struct Unit<F, false> {
     using T = typename F::T;
@@ -632,10 +629,7 @@ template <class F> struct Unit<F, false> {
         for (int k = 0; k < F::NA; ++k) v[k] = G[k * n + i];
     }
     TCYM_HD int64_t self() const { return nb.s; }
-    // a measurement's products: any matrices
-    template <bool DA, bool DB> static TCYM_HD Mat times(const Mat &a, const Mat &b) { return G::template mulx<DA, DB>(a, b); }
     static TCYM_HD void transport(const Mat &v, const T *e, T *out) { G::transport(v, e, out); }
-    static TCYM_HD void transport_any(const Mat &v, const T *e, T *out) { G::transport(v, e, out); }
 };
 
 // The N_CS sample's observables (mask OBS_EDOTB) of direction mu for unit i: E_mu^2 into
@@ -643,9 +637,9 @@ template <class F> struct Unit<F, false> {
 // site_observables forms them.  The clover average's projection is the average of the
 // leaves' projections (proj is linear), and proj(Q^dag) = -proj(Q): leaves that end in the
 // same link, one of them daggered, are summed before they are multiplied by it (ten
-// products for the four leaves instead of twelve).  An FP64 site's links may be off the
-// group (a pair's third rows are not stored), so there whole products are formed.  Both
-// sums of a unit run in the storage's precision.
+// products for the four leaves instead of twelve).  Links may be off the group (FP32 ones
+// drift between reunitarisations), so whole products are formed.  Both sums of a unit run in
+// the storage's precision.
 template <class F, bool PAIR>
 TCYM_HD typename Unit<F, PAIR>::T unit_clover(const Geom &g, const void *U, const void *E, int64_t i, int mu,
                                               typename Unit<F, PAIR>::T &esq, typename Unit<F, PAIR>::T &bsq) {
@@ -661,14 +655,14 @@ TCYM_HD typename Unit<F, PAIR>::T unit_clover(const Geom &g, const void *U, cons
     T b[NA], pr[NA];
     {   // Q2 - Q0^dag = (U_k^dag(x-k) U_j(x-k) U_k(x-k+j) - U_k(x) U_j(x+k) U_k^dag(x+j)) U_j^dag(x)
         const M end = L(j, 0, 0);
-        const M q0 = UN::template times<false, true>(UN::template times<false, false>(L(k, 0, 0), L(j, 0, 1)), L(k, 1, 0));
+        const M q0 = G::template mulx<false, true>(G::template mulx<false, false>(L(k, 0, 0), L(j, 0, 1)), L(k, 1, 0));
         bsq = T(4) * G::retr_one_minus_dag(q0, end);
-        const M q2 = UN::template times<false, false>(UN::template times<true, false>(L(k, 0, -1), L(j, 0, -1)), L(k, 1, -1));
+        const M q2 = G::template mulx<false, false>(G::template mulx<true, false>(L(k, 0, -1), L(j, 0, -1)), L(k, 1, -1));
         G::proj_mul_dag(G::sub(q2, q0), end, b);
     }
     {   // Q1 - Q3^dag = (U_k(x) U_j^dag(x+k-j) U_k^dag(x-j) - U_k^dag(x-k) U_j^dag(x-j-k) U_k(x-j-k)) U_j(x-j)
-        const M q1 = UN::template times<false, true>(UN::template times<false, true>(L(k, 0, 0), L(j, -1, 1)), L(k, -1, 0));
-        const M q3 = UN::template times<false, false>(UN::template times<true, true>(L(k, 0, -1), L(j, -1, -1)), L(k, -1, -1));
+        const M q1 = G::template mulx<false, true>(G::template mulx<false, true>(L(k, 0, 0), L(j, -1, 1)), L(k, -1, 0));
+        const M q3 = G::template mulx<false, false>(G::template mulx<true, true>(L(k, 0, -1), L(j, -1, -1)), L(k, -1, -1));
         G::proj_mul(G::sub(q1, q3), L(j, -1, 0), pr);
 #pragma unroll
         for (int a = 0; a < NA; ++a) b[a] = b[a] + pr[a];
@@ -814,7 +808,7 @@ TCYM_HD void unit_restore(const Geom &g, const void *U, const void *Ein, void *E
 #pragma unroll
             for (int a = 0; a < NA; ++a) e[a] = fma(mg, q[a] - t[a], e[a]);
         }
-        RU::transport_any(below, e, t);
+        RU::transport(below, e, t);
         u.load_e(Ein, mu, 0, e);
         if (UPDATE) {
             T s[NA];
