@@ -538,23 +538,21 @@ extern "C" int tcym_gauss_restore(tcym_lattice lat, double tol, int maxit, int *
     const double init[4] = {(double)maxit, 0.0, 0.0, 0.0};
     CK(cudaMemcpyAsync(ctl, init, sizeof(init), cudaMemcpyHostToDevice, lat->stream));
     auto finish = [&](int it, bool check) { return make_finish(lat->result, na, lat->g.V, 0.0, ctl, tol, it, check); };
-    // the fused restore keeps the fields and G in two buffers each: the second E in the link
-    // buffer that the next step overwrites, the second G behind it (FP64) or in the second
-    // half of the violation array, which holds doubles (FP32 pairs)
+    // the fused restore (FP32 pairs) keeps the fields and G in two buffers each: the second E in
+    // the link buffer that the next step overwrites, the second G in the second half of the
+    // violation array, which holds doubles
     bool fused = false;
     size_t gbytes = 0;
     DISPATCH(lat->fmt, { fused = L::restore_fused(lat->g); gbytes = L::restore_g_bytes(lat->g); });
     const size_t ebytes = 3 * tcym_field_bytes(lat->fmt) * tcym_stored_sites(lat->fmt, lat->g.V);
-    char *const spare = static_cast<char *>(lat->U[1 - lat->cur]);
+    void *const spare = lat->U[1 - lat->cur];
     void *const Ebuf[2] = {lat->E, spare};
-    void *const Gbuf[2] = {lat->gauss, lat->precision == TCYM_FP64 ? spare + ebytes : reinterpret_cast<char *>(lat->gauss) + gbytes};
+    void *const Gbuf[2] = {lat->gauss, reinterpret_cast<char *>(lat->gauss) + gbytes};
     const void *U = lat->U[lat->cur];
     auto deviation = [&](int it, bool check) -> int {
         const Finish fin = finish(it, check);
-        DISPATCH(lat->fmt, CK(fused ? L::restore_deviation(lat->g, U, lat->E, Gbuf[0], lat->partial, lat->max_blocks, fin,
-                                                           lat->stream)
-                                    : L::gauss_compute_it(lat->g, U, lat->E, lat->gauss, lat->partial, lat->max_blocks,
-                                                          fin, lat->stream)));
+        DISPATCH(lat->fmt,
+                 CK(L::restore_deviation(lat->g, U, lat->E, lat->gauss, lat->partial, lat->max_blocks, fin, lat->stream)));
         return TCYM_OK;
     };
     // sub-step k of iteration it
@@ -567,7 +565,7 @@ extern "C" int tcym_gauss_restore(tcym_lattice lat, double tol, int maxit, int *
                                                   lat->partial, lat->max_blocks, fin, lat->stream)));
         } else {
             if ((r = deviation(it, k == 2))) return r;
-            DISPATCH(lat->fmt, CK(L::gauss_update_it(lat->g, U, lat->E, lat->gauss, gam[k], ctl, it, lat->stream)));
+            DISPATCH(lat->fmt, CK(L::restore_update(lat->g, U, lat->E, lat->gauss, gam[k], ctl, it, lat->stream)));
         }
         return r;
     };

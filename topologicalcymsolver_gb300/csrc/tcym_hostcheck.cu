@@ -273,40 +273,53 @@ template <int FMT> struct H {
     static void reunitarize_fp64(const Geom &g, void *U) {
         for (int64_t s = 0; s < g.V; ++s) site_reunitarize<F>(g, U, s);
     }
-    // the fused restore's schedule (tcym_gauss_restore) on the host
-    template <bool PAIR> static int restore_fused(const Geom &g, const void *U, void *E, double tol, int maxit) {
+    // the restore by units as tcym_gauss_restore runs it: one pass a sub-step for pairs, two for FP64
+    template <bool PAIR> static int restore_units(const Geom &g, const void *U, void *E, double tol, int maxit) {
         using RU = Unit<F, PAIR>;
         using RT = typename RU::T;
+        using C = typename RU::C;
         const int64_t n = RU::count(g);
-        const size_t ebytes = sizeof(typename RU::C) * 3 * (PAIR ? 2 * n : n) * F::NA;
+        const size_t ebytes = sizeof(C) * 3 * (PAIR ? 2 * n : n) * F::NA;
         std::vector<RT> G0(F::NA * n), G1(F::NA * n);
         std::vector<char> E1(ebytes);
         RT *G[2] = {G0.data(), G1.data()};
         void *Eb[2] = {E, E1.data()};
         const double gam[3] = {7.0 / 24.0, 7.0 / 48.0, 7.0 / 72.0};
         double gmax = 0;
-        auto take = [&](const RT *gv, int64_t i, RT *out) {
+        RT gv[F::NA];
+        auto take = [&](int64_t i, RT *out) {
             for (int a = 0; a < F::NA; ++a) {
                 out[a * n + i] = gv[a];
                 if constexpr (PAIR) gmax = std::fmax(gmax, std::fmax((double)gv[a].v.x, (double)gv[a].v.y));
                 else gmax = std::fmax(gmax, (double)gv[a]);
             }
         };
-        RT gv[F::NA];
-        for (int64_t i = 0; i < n; ++i) {
-            unit_restore<F, PAIR, false>(g, U, E, nullptr, nullptr, 0, i, gv);
-            take(gv, i, G[0]);
-        }
+        auto deviation = [&]() {
+            gmax = 0;
+            for (int64_t i = 0; i < n; ++i) {
+                unit_deviation<F, PAIR>(g, U, E, i, gv);
+                take(i, G[0]);
+            }
+        };
+        deviation();
         int it = 0, sub = 0;
         double last = gmax;
         while (it < maxit && last > tol) {
-            for (int k = 0; k < 3; ++k, sub ^= 1) {
-                gmax = 0;
-                for (int64_t i = 0; i < n; ++i) {
-                    unit_restore<F, PAIR, true>(g, U, Eb[sub], Eb[1 - sub], G[sub], (typename RU::C)gam[k], i, gv);
-                    take(gv, i, G[1 - sub]);
+            for (int k = 0; k < 3; ++k) {
+                if constexpr (PAIR) {
+                    gmax = 0;
+                    for (int64_t i = 0; i < n; ++i) {
+                        unit_restore_next<F, PAIR>(g, U, Eb[sub], Eb[1 - sub], G[sub], (C)gam[k], i, gv);
+                        take(i, G[1 - sub]);
+                    }
+                    sub ^= 1;
+                    if (k == 1) last = gmax;  // the third deviation
+                } else {
+                    deviation();
+                    if (k == 2) last = gmax;
+                    for (int mu = 0; mu < 3; ++mu)
+                        for (int64_t i = 0; i < n; ++i) unit_restore<F, PAIR>(g, U, E, G[0], (C)gam[k], i, mu);
                 }
-                if (k == 1) last = gmax;  // the third deviation
             }
             ++it;
         }
@@ -314,9 +327,9 @@ template <int FMT> struct H {
         return it;
     }
     static int gauss_restore(const Geom &g, const void *U, void *E, double tol, int maxit) {
-        if constexpr (!F::PAIRED) return restore_fused<false>(g, U, E, tol, maxit);
+        if constexpr (!F::PAIRED) return restore_units<false>(g, U, E, tol, maxit);
         if constexpr (F::PAIRED)
-            if (g.nz % 2 == 0) return restore_fused<true>(g, U, E, tol, maxit);
+            if (g.nz % 2 == 0) return restore_units<true>(g, U, E, tol, maxit);
         std::vector<double> G((size_t)F::NA * g.V);
         const double gam[3] = {7.0 / 24.0, 7.0 / 48.0, 7.0 / 72.0};
         auto dev = [&]() {

@@ -583,46 +583,36 @@ __global__ void __launch_bounds__(threads_for<FMT>()) k_gauss_update_it(Geom g, 
     site_gauss_update<Fmt<FMT>>(g, U, E, G, gam, s);
 }
 
-// The fused restore (FP32 with even nz in site pairs, FP64): a thread per unit does a
-// sub-step's update and the next deviation (unit_restore), from the fields Ein and G Gin
-// into Eout and Gout, so a sub-step reads the links once and is one launch.  Bound by
-// memory (SU(3) FP32 128^3: 838 MB, 123 us at the measured copy rate); an iteration of
-// three (deviation, update) pairs of launches took 785 us there and 128 us at 64^3, this one
-// 502 and 99.
-// UPDATE: the update belongs to iteration `it`, the deviation to fin.it; a launch of an
-// iteration past the stop returns at once, and a deviation past it leaves the result of
-// the last one.
+// The restore by units (FP32 with even nz in site pairs, FP64): a thread a unit forms the
+// deviation (k_deviation); FP32 pairs then do a sub-step's update and the next deviation in
+// one pass over the links, from the fields Ein and G Gin into Eout and Gout (k_restore_next),
+// FP64 updates with a thread a unit and direction (k_restore, blockIdx.y).  FP32 is bound by
+// memory and launches, FP64 by its multiply-adds, of which one pass does half as many again
+// (each neighbour's update a second time).  An iteration of three sub-steps on GB300, one pass
+// / two: SU(3) FP32 32^3 46 / 58 us, 64^3 133 / 120, 128^3 702 / 786; SU(2) FP32 32^3 36 / 46, 128^3
+// 275 / 355; FP64 48^3 SU(3) 960 / 669, SU(2) 234 / 185.
 constexpr int kThreadsRestore = 128;
-template <int FMT, bool UPDATE>
-__global__ void __launch_bounds__(kThreadsRestore, 4)
-    k_restore(Geom g, const void *U, const void *Ein, void *Eout,
-              const typename Unit<Fmt<FMT>, unit_pairs<FMT>()>::T *Gin,
-              typename Unit<Fmt<FMT>, unit_pairs<FMT>()>::T *Gout, double gam, int it, double *partial,
-              Finish fin) {
-    using F = Fmt<FMT>;
-    constexpr bool PAIR = unit_pairs<FMT>();
-    using RU = Unit<F, PAIR>;
-    if (UPDATE && (double)it >= fin.ctl[0]) return;  // the same value for every thread of the grid
-    const int64_t n = RU::count(g);
-    typename RU::C gsq = 0, gmax = 0, gabs = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        typename RU::T gv[F::NA];
-        unit_restore<F, PAIR, UPDATE>(g, U, Ein, Eout, Gin, (typename RU::C)gam, i, gv);
+template <int FMT> using UnitG = typename Unit<Fmt<FMT>, unit_pairs<FMT>()>::T;
+// a unit's violation into G and its thread's sums v
+template <int FMT, class C>
+__device__ __forceinline__ void take_deviation(const UnitG<FMT> *gv, UnitG<FMT> *G, int64_t n, int64_t i, C &gsq, C &gmax,
+                                               C &gabs) {
 #pragma unroll
-        for (int a = 0; a < F::NA; ++a) {
-            Gout[a * n + i] = gv[a];
-            if constexpr (PAIR) {
-                const float x = gv[a].v.x, y = gv[a].v.y;
-                gsq = fmaf(x, x, fmaf(y, y, gsq));
-                gmax = fmaxf(gmax, fmaxf(x, y));
-                gabs = fmaxf(gabs, fmaxf(fabsf(x), fabsf(y)));
-            } else {
-                gsq = fma(gv[a], gv[a], gsq);
-                gmax = fmax(gmax, gv[a]);
-                gabs = fmax(gabs, fabs(gv[a]));
-            }
+    for (int a = 0; a < Fmt<FMT>::NA; ++a) {
+        G[a * n + i] = gv[a];
+        if constexpr (unit_pairs<FMT>()) {
+            const float x = gv[a].v.x, y = gv[a].v.y;
+            gsq = fmaf(x, x, fmaf(y, y, gsq));
+            gmax = fmaxf(gmax, fmaxf(x, y));
+            gabs = fmaxf(gabs, fmaxf(fabsf(x), fabsf(y)));
+        } else {
+            gsq = fma(gv[a], gv[a], gsq);
+            gmax = fmax(gmax, gv[a]);
+            gabs = fmax(gabs, fabs(gv[a]));
         }
     }
+}
+__device__ __forceinline__ void finish_deviation(double gsq, double gmax, double gabs, double *partial, const Finish &fin) {
     double v[P_WIDTH];
 #pragma unroll
     for (int k = 0; k < P_WIDTH; ++k) v[k] = 0.0;
@@ -630,6 +620,48 @@ __global__ void __launch_bounds__(kThreadsRestore, 4)
     v[P_GMAX] = gmax;
     v[P_GABS] = gabs;
     reduce_and_finish<kUsedGauss, kThreadsRestore>(v, partial, fin);
+}
+// the deviation in iteration fin.it: a launch of an iteration past the stop returns at once
+template <int FMT>
+__global__ void __launch_bounds__(kThreadsRestore, 4)
+    k_deviation(Geom g, const void *U, const void *E, UnitG<FMT> *G, double *partial, Finish fin) {
+    using F = Fmt<FMT>;
+    using RU = Unit<F, unit_pairs<FMT>()>;
+    if ((double)fin.it >= fin.ctl[0]) return;  // the same value for every thread of the grid
+    const int64_t n = RU::count(g);
+    typename RU::C gsq = 0, gmax = 0, gabs = 0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        UnitG<FMT> gv[F::NA];
+        unit_deviation<F, unit_pairs<FMT>()>(g, U, E, i, gv);
+        take_deviation<FMT>(gv, G, n, i, gsq, gmax, gabs);
+    }
+    finish_deviation(gsq, gmax, gabs, partial, fin);
+}
+template <int FMT>
+__global__ void __launch_bounds__(kThreadsRestore, 4)
+    k_restore(Geom g, const void *U, void *E, const UnitG<FMT> *G, double gam, const double *ctl, int it) {
+    using RU = Unit<Fmt<FMT>, unit_pairs<FMT>()>;
+    if ((double)it >= ctl[0]) return;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < RU::count(g)) unit_restore<Fmt<FMT>, unit_pairs<FMT>()>(g, U, E, G, (typename RU::C)gam, i, blockIdx.y);
+}
+// The update belongs to iteration `it`, the deviation to fin.it; a deviation past the stop
+// leaves the result of the last one.  (SU(3): three blocks of 168 registers; four spill, 809 us
+// at 128^3.)
+template <int FMT>
+__global__ void __launch_bounds__(kThreadsRestore, Fmt<FMT>::NA == 8 ? 3 : 4)
+    k_restore_next(Geom g, const void *U, const void *Ein, void *Eout, const UnitG<FMT> *Gin, UnitG<FMT> *Gout, float gam,
+                   int it, double *partial, Finish fin) {
+    using F = Fmt<FMT>;
+    if ((double)it >= fin.ctl[0]) return;
+    const int64_t n = Unit<F, true>::count(g);
+    float gsq = 0, gmax = 0, gabs = 0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        UnitG<FMT> gv[F::NA];
+        unit_restore_next<F, true>(g, U, Ein, Eout, Gin, gam, i, gv);
+        take_deviation<FMT>(gv, Gout, n, i, gsq, gmax, gabs);
+    }
+    finish_deviation(gsq, gmax, gabs, partial, fin);
 }
 
 template <int FMT> __global__ void k_set_zero(Geom g, void *U, void *E) {
@@ -818,47 +850,49 @@ template <int FMT> struct Launch {
             k_observables<FMT, false><<<blocks, kRedThreads, 0, st>>>(g, U, E, mask, partial, fin);
         return cudaGetLastError();
     }
-    // The fused restore's launches: E and G alternate between two buffers each.
-    static bool restore_fused(const Geom &g) { return !F::PAIRED || g.nz % 2 == 0; }
-    using GT = typename Unit<F, unit_pairs<FMT>()>::T;
-    // bytes of one G buffer
-    static size_t restore_g_bytes(const Geom &g) {
-        return sizeof(GT) * F::NA * (size_t)Unit<F, unit_pairs<FMT>()>::count(g);
-    }
-    template <bool UPDATE>
-    static cudaError_t restore(const Geom &g, const void *U, const void *Ein, void *Eout, const void *Gin, void *Gout,
-                               double gam, int it, double *partial, int max_blocks, const Finish &fin, cudaStream_t st) {
+    // The restore.  Does a sub-step update and form the next deviation in one launch?
+    static bool restore_fused(const Geom &g) { return F::PAIRED && g.nz % 2 == 0; }
+    // bytes of one G buffer of the fused restore
+    static size_t restore_g_bytes(const Geom &g) { return sizeof(f2) * F::NA * (size_t)(g.V >> 1); }
+    // the deviation G of E, in iteration fin.it: by units, or per site (FP32, odd nz; G: na V doubles)
+    static cudaError_t restore_deviation(const Geom &g, const void *U, const void *E, void *G, double *partial,
+                                         int max_blocks, const Finish &fin, cudaStream_t st) {
+        if constexpr (F::PAIRED) {
+            if (g.nz % 2) {
+                k_gauss_compute_it<FMT><<<reduce_grid(g, max_blocks), kRedThreads, 0, st>>>(
+                    g, U, E, static_cast<double *>(G), partial, fin);
+                return cudaGetLastError();
+            }
+        }
         // max_blocks is 8 a multiprocessor.  FP64: 3 (a grid of 4 would hold every register for
         // the whole launch, and the request loop's ticks wait for its blocks: 2.0 ms a tick
         // beside a 128^3 preparation, against 0.24 ms alone)
         const int need = grid_for(Unit<F, unit_pairs<FMT>()>::count(g), kThreadsRestore);
         const int most = F::PAIRED ? max_blocks : max_blocks / 8 * 3;
-        k_restore<FMT, UPDATE><<<need < most ? need : most, kThreadsRestore, 0, st>>>(
-            g, U, Ein, Eout, static_cast<const GT *>(Gin), static_cast<GT *>(Gout), gam, it, partial, fin);
+        k_deviation<FMT><<<need < most ? need : most, kThreadsRestore, 0, st>>>(g, U, E, static_cast<UnitG<FMT> *>(G),
+                                                                                partial, fin);
         return cudaGetLastError();
     }
-    static cudaError_t restore_deviation(const Geom &g, const void *U, const void *E, void *Gout, double *partial,
-                                         int max_blocks, const Finish &fin, cudaStream_t st) {
-        return restore<false>(g, U, E, nullptr, nullptr, Gout, 0.0, -1, partial, max_blocks, fin, st);
+    // the update by it in iteration `it` (not fused)
+    static cudaError_t restore_update(const Geom &g, const void *U, void *E, const void *G, double gam, const double *ctl,
+                                      int it, cudaStream_t st) {
+        if constexpr (F::PAIRED) {
+            k_gauss_update_it<FMT><<<grid_for(g.V, TPB), TPB, 0, st>>>(g, U, E, static_cast<const double *>(G), gam, ctl, it);
+        } else {
+            k_restore<FMT><<<dim3((unsigned)grid_for(g.V, kThreadsRestore), 3), kThreadsRestore, 0, st>>>(
+                g, U, E, static_cast<const UnitG<FMT> *>(G), gam, ctl, it);
+        }
+        return cudaGetLastError();
     }
+    // both (fused)
     static cudaError_t restore_step(const Geom &g, const void *U, const void *Ein, void *Eout, const void *Gin, void *Gout,
                                     double gam, int it, double *partial, int max_blocks, const Finish &fin,
                                     cudaStream_t st) {
-        return restore<true>(g, U, Ein, Eout, Gin, Gout, gam, it, partial, max_blocks, fin, st);
-    }
-    // the restore iteration per site with its two kernels (FP32, odd nz)
-    static cudaError_t gauss_compute_it(const Geom &g, const void *U, const void *E, double *G, double *partial,
-                                        int max_blocks, const Finish &fin, cudaStream_t st) {
         if constexpr (F::PAIRED) {
-            k_gauss_compute_it<FMT><<<reduce_grid(g, max_blocks), kRedThreads, 0, st>>>(g, U, E, G, partial, fin);
-            return cudaGetLastError();
-        }
-        return cudaErrorInvalidValue;
-    }
-    static cudaError_t gauss_update_it(const Geom &g, const void *U, void *E, const double *G, double gam,
-                                       const double *ctl, int it, cudaStream_t st) {
-        if constexpr (F::PAIRED) {
-            k_gauss_update_it<FMT><<<grid_for(g.V, TPB), TPB, 0, st>>>(g, U, E, G, gam, ctl, it);
+            const int need = grid_for(g.V >> 1, kThreadsRestore);
+            k_restore_next<FMT><<<need < max_blocks ? need : max_blocks, kThreadsRestore, 0, st>>>(
+                g, U, Ein, Eout, static_cast<const UnitG<FMT> *>(Gin), static_cast<UnitG<FMT> *>(Gout), (float)gam, it,
+                partial, fin);
             return cudaGetLastError();
         }
         return cudaErrorInvalidValue;

@@ -772,52 +772,84 @@ TCYM_HD void site_gauss_update(const Geom &g, const void *U, void *E, const doub
     }
 }
 
-// ------------------------------------------------------------- restore, fused
-// One sub-step of the restore and the next deviation at once (UPDATE), or the deviation
-// alone.  The new deviation is that of the new fields, whatever the links: each unit forms
-// its own three,
-//   E'_mu(x) = E_mu(x) - gam (G(x) - U_mu(x) G(x+mu) U_mu^dag(x)),
-// and its lower neighbours' E'_mu(x-mu) again, from the old fields and G and by the same
-// arithmetic.  (On the group U^dag(x-mu) E'(x-mu) U(x-mu) holds gam G(x) itself, which would
-// spare the neighbour's transport of G(x); links a few 1e-7 off it, as FP32 ones between
-// reunitarisations, would leave a violation of that size.)
-// gv receives the new G.
-template <class F, bool PAIR, bool UPDATE>
-TCYM_HD void unit_restore(const Geom &g, const void *U, const void *Ein, void *Eout,
-                          const typename Unit<F, PAIR>::T *Gin, typename Unit<F, PAIR>::C gam, int64_t i,
-                          typename Unit<F, PAIR>::T *gv) {
+// ------------------------------------------------------------- restore, by units
+// The deviation G(x) = sum_mu E_mu(x) - U_mu^dag(x-mu) E_mu(x-mu) U_mu(x-mu) of unit i, in
+// the storage's precision, for any links.
+template <class F, bool PAIR>
+TCYM_HD void unit_deviation(const Geom &g, const void *U, const void *E, int64_t i, typename Unit<F, PAIR>::T *gv) {
     using RU = Unit<F, PAIR>;
     using T = typename RU::T;
-    using G = typename RU::G;
-    using M = typename RU::Mat;
     constexpr int NA = F::NA;
     const RU u(g, i);
-    const T mg(-gam);
-    T gx[NA];
-    if (UPDATE) u.load_g(Gin, 0, 0, gx);
 #pragma unroll
     for (int a = 0; a < NA; ++a) gv[a] = T(0);
 #pragma unroll 1
     for (int mu = 0; mu < 3; ++mu) {
-        T e[NA], q[NA], t[NA];
-        const M below = u.link(U, mu, -1);
-        u.load_e(Ein, mu, -1, e);
-        if (UPDATE) {
+        T e[NA], t[NA];
+        u.load_e(E, mu, -1, e);
+        RU::transport(u.link(U, mu, -1), e, t);
+        u.load_e(E, mu, 0, e);
+#pragma unroll
+        for (int a = 0; a < NA; ++a) gv[a] = gv[a] + (e[a] - t[a]);
+    }
+}
+// A sub-step's update of field mu of unit i,
+//   E'_mu(x) = E_mu(x) - gam (G(x) - U_mu(x) G(x+mu) U_mu^dag(x)).
+template <class F, bool PAIR>
+TCYM_HD void unit_restore(const Geom &g, const void *U, void *E, const typename Unit<F, PAIR>::T *G,
+                          typename Unit<F, PAIR>::C gam, int64_t i, int mu) {
+    using RU = Unit<F, PAIR>;
+    using T = typename RU::T;
+    constexpr int NA = F::NA;
+    const RU u(g, i);
+    const T mg(-gam);
+    T q[NA], t[NA], e[NA];
+    u.load_g(G, mu, 1, q);
+    RU::G::transport_back(u.link(U, mu, 0), q, t);
+    u.load_g(G, 0, 0, q);
+    u.load_e(E, mu, 0, e);
+#pragma unroll
+    for (int a = 0; a < NA; ++a) e[a] = fma(mg, q[a] - t[a], e[a]);
+    u.store_e(E, mu, e);
+}
+// The update of all of unit i's fields, from Ein and Gin into Eout, and the next deviation gv
+// at once: that of the new fields, whatever the links.  The unit forms its lower neighbours'
+// E'_mu(x-mu) again, by the arithmetic that stores them.  (On the group
+// U^dag(x-mu) E'(x-mu) U(x-mu) holds gam G(x) itself, which would spare the neighbour's
+// transport of G(x); links a few 1e-7 off it, as FP32 ones between reunitarisations, would
+// leave a violation of that size.)
+template <class F, bool PAIR>
+TCYM_HD void unit_restore_next(const Geom &g, const void *U, const void *Ein, void *Eout,
+                               const typename Unit<F, PAIR>::T *Gin, typename Unit<F, PAIR>::C gam, int64_t i,
+                               typename Unit<F, PAIR>::T *gv) {
+    using RU = Unit<F, PAIR>;
+    using T = typename RU::T;
+    using G = typename RU::G;
+    constexpr int NA = F::NA;
+    const RU u(g, i);
+    const T mg(-gam);
+    T gx[NA];
+    u.load_g(Gin, 0, 0, gx);
+#pragma unroll
+    for (int a = 0; a < NA; ++a) gv[a] = T(0);
+#pragma unroll 1
+    for (int mu = 0; mu < 3; ++mu) {
+        T e[NA], q[NA], t[NA], s[NA];
+        {
+            const typename RU::Mat below = u.link(U, mu, -1);
             G::transport_back(below, gx, t);
+            u.load_e(Ein, mu, -1, e);
             u.load_g(Gin, mu, -1, q);
 #pragma unroll
             for (int a = 0; a < NA; ++a) e[a] = fma(mg, q[a] - t[a], e[a]);
+            RU::transport(below, e, t);
         }
-        RU::transport(below, e, t);
         u.load_e(Ein, mu, 0, e);
-        if (UPDATE) {
-            T s[NA];
-            u.load_g(Gin, mu, 1, q);
-            G::transport_back(u.link(U, mu, 0), q, s);
+        u.load_g(Gin, mu, 1, q);
+        G::transport_back(u.link(U, mu, 0), q, s);
 #pragma unroll
-            for (int a = 0; a < NA; ++a) e[a] = fma(mg, gx[a] - s[a], e[a]);
-            u.store_e(Eout, mu, e);
-        }
+        for (int a = 0; a < NA; ++a) e[a] = fma(mg, gx[a] - s[a], e[a]);
+        u.store_e(Eout, mu, e);
 #pragma unroll
         for (int a = 0; a < NA; ++a) gv[a] = gv[a] + (e[a] - t[a]);
     }
