@@ -33,6 +33,8 @@ def load():
         L.hc_flow_cb.argtypes = [ctypes.c_int, ip, _vp, ctypes.c_double, ctypes.c_int]
         L.hc_observables.argtypes = [ctypes.c_int, ip, _vp, _vp, ctypes.c_int, _vp]
         L.hc_edotb_pair.argtypes = [ctypes.c_int, ip, _vp, _vp, _vp]
+        L.hc_pair_sums.argtypes = [ctypes.c_int, ctypes.c_int64, ctypes.c_int64, _vp, _vp, _vp, _vp]
+        L.hc_violation_sums.argtypes = [ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_int, _vp, _vp]
         L.hc_gauss.argtypes = [ctypes.c_int, ip, _vp, _vp, ctypes.c_int, _vp]
         L.hc_gauss_restore.argtypes = [ctypes.c_int, ip, _vp, _vp, ctypes.c_double, ctypes.c_int]
         L.hc_reunitarize.argtypes = [ctypes.c_int, ip, _vp]
@@ -169,6 +171,23 @@ class HostLattice:
         """UMid, EMid (into this lattice) of the geodesic from old's links to new's."""
         self.L.hc_geodesic(self.fmt, self.n, _p(old.U[old.cur]), _p(new.U[new.cur]), c, _p(self.U[self.cur]),
                            _p(self.E))
+
+
+def pair_sums(e, et, b, count=1):
+    """(pairs / count, 2): E.E and (E + E').B / 4 summed over `count` pairs' float32 components (pairs, NA, 2 lanes)."""
+    out = np.zeros((e.shape[0] // count, 2))
+    load().hc_pair_sums(e.shape[1], e.shape[0], count, *(_p(np.ascontiguousarray(x, np.float32)) for x in (e, et, b)),
+                        _p(out))
+    return out
+
+
+def violation_sums(t, count=1):
+    """(pairs / count, 3): sum of squares, largest component and largest magnitude (from 0 on) of `count` pairs'
+    violations, each the sum of float32 terms t (pairs, NA, terms, 2 lanes)."""
+    t = np.ascontiguousarray(t, np.float32)
+    out = np.zeros((t.shape[0] // count, 3))
+    load().hc_violation_sums(t.shape[1], t.shape[0], count, t.shape[2], _p(t), _p(out))
+    return out
 
 
 def iexp(nc, prec, c, alpha):

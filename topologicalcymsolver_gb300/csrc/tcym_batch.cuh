@@ -242,7 +242,7 @@ __device__ __forceinline__ void sample_unit(const Geom &g, const void *u, const 
 #pragma unroll 1
     for (int mu = 0; mu < 3; ++mu) {
         typename Unit<F, PAIR>::T esq, bsq;
-        v[P_EDB] += lanes_sum(unit_clover<F, PAIR>(g, u, e, i, mu, esq, bsq));
+        v[P_EDB] += lanes_sum(unit_sample<F, PAIR>(g, u, e, i, mu, esq, bsq));
         const double es = lanes_sum(esq), bs = lanes_sum(bsq);
         // fixed slots (a run-time index would put v in local memory)
         if (mu == 0) { v[P_ESQ0] += es; v[P_BSQ0] += bs; }

@@ -150,11 +150,13 @@ template <int FMT> struct H {
                     }
     }
     // E^2, plaquette B^2 and clover E.B of an FP64 site by the units' code, in place of site_observables'
-    static void unit_sample(const Geom &g, const void *U, const void *E, int64_t s, SiteObs<F> &o) {
+    static void sample_units(const Geom &g, const void *U, const void *E, int64_t s, SiteObs<F> &o) {
         if constexpr (!F::PAIRED) {
             o.edotb = 0;
-            for (int mu = 0; mu < 3; ++mu) o.edotb += unit_clover<F, false>(g, U, E, s, mu, o.esq[mu], o.bsq[mu]);
-            unit_gauss<F, false>(g, U, E, s, o.g);
+            for (int mu = 0; mu < 3; ++mu) o.edotb += unit_sample<F, false>(g, U, E, s, mu, o.esq[mu], o.bsq[mu]);
+            WideSum<double> gv[F::NA];
+            unit_gauss<F, false>(g, U, E, s, gv);
+            for (int a = 0; a < F::NA; ++a) o.g[a] = lane64(gv[a], 0);
         }
     }
     static void observables(const Geom &g, const void *U, const void *E, int mask, double *out) {
@@ -162,7 +164,7 @@ template <int FMT> struct H {
         for (int64_t s = 0; s < g.V; ++s) {
             SiteObs<F> o;
             site_observables<F>(g, U, E, mask, s, o);
-            if (mask == OBS_ALL) unit_sample(g, U, E, s, o);
+            if (mask == OBS_ALL) sample_units(g, U, E, s, o);
             for (int m = 0; m < 3; ++m) { esq[m] += o.esq[m]; bsq[m] += o.bsq[m]; usq += o.un[m] * o.un[m]; umax = std::fmax(umax, o.un[m]); }
             for (int a = 0; a < F::NA; ++a) { gsq += o.g[a] * o.g[a]; gmax = std::fmax(gmax, o.g[a]); gabs = std::fmax(gabs, std::fabs(o.g[a])); }
             edb += o.edotb;
@@ -190,7 +192,7 @@ template <int FMT> struct H {
             for (int64_t p = 0; p < Vh; ++p)
                 for (int mu = 0; mu < 3; ++mu) {
                     f2 e2, b2;
-                    const f2 d = unit_clover<F, true>(g, U, E, p, mu, e2, b2);
+                    const f2 d = unit_sample<F, true>(g, U, E, p, mu, e2, b2);
                     esq[mu] += (double)e2.v.x + (double)e2.v.y;
                     bsq[mu] += (double)b2.v.x + (double)b2.v.y;
                     edb += (double)d.v.x + (double)d.v.y;
@@ -239,11 +241,11 @@ template <int FMT> struct H {
             if (g.nz % 2) return false;
             const int64_t Vh = g.V >> 1;
             for (int64_t p = 0; p < Vh; ++p) {
-                f2 gv[F::NA];
+                WideSum<f2> gv[F::NA];
                 unit_gauss<F, true>(g, U, E, p, gv);
                 for (int a = 0; a < F::NA; ++a) {
-                    out[p * F::NA + a] = gv[a].v.x;
-                    out[(p + Vh) * F::NA + a] = gv[a].v.y;
+                    out[p * F::NA + a] = lane64(gv[a], 0);
+                    out[(p + Vh) * F::NA + a] = lane64(gv[a], 1);
                 }
             }
             return true;
@@ -427,6 +429,63 @@ int hc_edotb_pair(int fmt, const int *n, const void *U, const void *E, double *o
     int ok = 0;
     HC_DISPATCH(fmt, ok = HH::edotb_pair(g, U, E, out));
     return ok;
+}
+// E.E and (E + E').B / 4, summed over `count` pairs at a time as a thread of the device sums
+// them, of n pairs' components e[pair][component][lane]
+}  // extern "C"
+template <int NA> static void pair_sums(int64_t n, int64_t count, const float *e, const float *et, const float *b, double *out) {
+    for (int64_t i0 = 0; i0 < n; i0 += count) {
+        FieldSums<f2, NA> sums;
+        for (int again = 0; again < 2; ++again) {
+            for (int64_t i = i0; i < i0 + count && i < n; ++i) {
+                f2 x[NA], y[NA], z[NA];
+                for (int a = 0; a < NA; ++a) {
+                    const int64_t j = 2 * (i * NA + a);
+                    x[a] = f2(e[j], e[j + 1]); y[a] = f2(et[j], et[j + 1]); z[a] = f2(b[j], b[j + 1]);
+                }
+                if (again) sums.add64(x, y, z);
+                else sums.add(x, y, z);
+            }
+            if (again || sums.exact()) break;
+        }
+        out[2 * (i0 / count)] = sums.sq;
+        out[2 * (i0 / count) + 1] = sums.dot;
+    }
+}
+// sum of squares, largest component and largest magnitude (from 0 on) of n pairs' violations,
+// each the sum of k FP32 terms t[pair][component][term][lane]
+template <int NA> static void violation_sums(int64_t n, int64_t count, int k, const float *t, double *out) {
+    for (int64_t i0 = 0; i0 < n; i0 += count) {
+        ViolationSums<f2, NA> sums;
+        for (int again = 0; again < 2; ++again) {
+            for (int64_t i = i0; i < i0 + count && i < n; ++i) {
+                WideSum<f2> s[NA];
+                for (int a = 0; a < NA; ++a) {
+                    s[a] = WideSum<f2>(f2(0.0));
+                    for (int j = 0; j < k; ++j) {
+                        const float *x = t + 2 * ((i * NA + a) * k + j);
+                        s[a].add(f2(x[0], x[1]));
+                    }
+                }
+                if (again) sums.add64(s);
+                else sums.add(s);
+            }
+            if (again || sums.exact()) break;
+        }
+        double *o = out + 3 * (i0 / count);
+        o[0] = sums.sq; o[1] = sums.most; o[2] = sums.mag;
+    }
+}
+extern "C" {
+int hc_pair_sums(int na, int64_t n, int64_t count, const float *e, const float *et, const float *b, double *out) {
+    if (na == 3) pair_sums<3>(n, count, e, et, b, out);
+    else pair_sums<8>(n, count, e, et, b, out);
+    return 0;
+}
+int hc_violation_sums(int na, int64_t n, int64_t count, int k, const float *t, double *out) {
+    if (na == 3) violation_sums<3>(n, count, k, t, out);
+    else violation_sums<8>(n, count, k, t, out);
+    return 0;
 }
 // the Gauss violation of every site, by pairs (0: the storage holds none) or site by site
 int hc_gauss(int fmt, const int *n, const void *U, const void *E, int pairs, double *out) {

@@ -456,9 +456,9 @@ template <int FMT> constexpr bool unit_pairs() { return Fmt<FMT>::PAIRED; }
 // The observables of a lattice in storage units: the N_CS sample (mask OBS_EDOTB: E^2,
 // plaquette B^2, clover E.B) and, FULL (OBS_ALL), the Gauss and unitarity violations.  A
 // thread takes a unit and a direction (blockIdx.y; FULL: 3 is the violations), so a small
-// lattice has three or four times its units in threads; a unit's sums run in the storage's
-// precision (the Gauss violation's, which cancel, exactly), everything across units in
-// FP64.  SU(3) FP64 is bound by its multiply-adds (0.87 ms at 48^3), the others wait for L2.
+// lattice has three or four times its units in threads.  The sample's sums over components
+// run in the storage's precision, those of all observables in FP64 (FieldSums, ViolationSums), and
+// everything across units in FP64.  SU(3) FP64 is bound by its multiply-adds (0.87 ms at 48^3), the others wait for L2.
 // All observables, with the call, on GB300, one thread a site or pair / by unit and direction:
 // SU(3) FP64 16^3 370 / 74 us, 48^3 1067 / 964; SU(2) FP64 16^3 87 / 37; SU(3) FP32 16^3
 // 40 / 30, 64^3 130 / 114, 128^3 790 / 702; SU(2) FP32 96^3 and 128^3 126 and 213 / 124 and 260
@@ -468,14 +468,8 @@ constexpr int kThreadsObs = 128;
 // a unit's contribution to its direction's sums
 template <class T> __device__ __forceinline__ double lanes_sum(T x) { return (double)x; }
 template <> __device__ __forceinline__ double lanes_sum<f2>(f2 x) { return (double)x.v.x + (double)x.v.y; }
-__device__ __forceinline__ void lanes_max(double x, double &gmax, double &gabs) {
-    gmax = fmax(gmax, x);
-    gabs = fmax(gabs, fabs(x));
-}
-__device__ __forceinline__ void lanes_max(f2 x, float &gmax, float &gabs) {
-    gmax = fmaxf(gmax, fmaxf(x.v.x, x.v.y));
-    gabs = fmaxf(gabs, fmaxf(fabsf(x.v.x), fabsf(x.v.y)));
-}
+__device__ __forceinline__ double lanes_max(double x, double m) { return fmax(m, x); }
+__device__ __forceinline__ float lanes_max(f2 x, float m) { return fmaxf(m, fmaxf(x.v.x, x.v.y)); }
 template <int FMT, bool FULL>
 __global__ void __launch_bounds__(kThreadsObs, Fmt<FMT>::NA == 8 ? 2 : 4)
     k_obs_units(Geom g, const void *U, const void *E, double *partial, Finish fin) {
@@ -484,33 +478,54 @@ __global__ void __launch_bounds__(kThreadsObs, Fmt<FMT>::NA == 8 ? 2 : 4)
     using T = typename UN::T;
     const int mu = blockIdx.y;
     const int64_t n = UN::count(g), step = (int64_t)gridDim.x * blockDim.x;
-    double es = 0.0, bs = 0.0, edb = 0.0, gsq = 0.0, usq = 0.0;
-    typename UN::C gmax = 0, gabs = 0, umax = 0, unused = 0;
-    if (!FULL || mu < 3) {
-        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
-            T esq, bsq;
-            edb += lanes_sum(unit_clover<F, unit_pairs<FMT>()>(g, U, E, i, mu, esq, bsq));
-            es += lanes_sum(esq);
-            bs += lanes_sum(bsq);
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    double es = 0.0, bs = 0.0, edb = 0.0, gsq = 0.0, usq = 0.0, gmax = 0.0, gabs = 0.0;
+    typename UN::C umax = 0;
+    if constexpr (FULL) {
+        if (mu < 3) {
+            FieldSums<T, F::NA> sums;
+            for (int again = 0; again < 2; ++again) {
+                bs = 0.0;
+                for (int64_t i = i0; i < n; i += step) {
+                    T e[F::NA], et[F::NA], b[F::NA], bsq;
+                    unit_clover<F, unit_pairs<FMT>()>(g, U, E, i, mu, e, et, b, bsq);
+                    if (again) sums.add64(e, et, b);
+                    else sums.add(e, et, b);
+                    bs += lanes_sum(bsq);
+                }
+                if (again || sums.exact()) break;
+            }
+            es = sums.sq;
+            edb = sums.dot;
+        } else {
+            ViolationSums<T, F::NA> sums;
+            for (int again = 0; again < 2; ++again) {
+                usq = 0.0;
+                for (int64_t i = i0; i < n; i += step) {
+                    WideSum<T> s[F::NA];
+                    unit_gauss<F, unit_pairs<FMT>()>(g, U, E, i, s);
+                    if (again) sums.add64(s);
+                    else sums.add(s);
+                    const UN u(g, i);
+#pragma unroll 1
+                    for (int d = 0; d < 3; ++d) {
+                        const T un = UN::G::unitarity_square(u.link(U, d, 0));
+                        usq += lanes_sum(un);
+                        umax = lanes_max(un, umax);
+                    }
+                }
+                if (again || sums.exact()) break;
+            }
+            gsq = sums.sq;
+            gmax = sums.most;
+            gabs = sums.mag;
         }
     } else {
-        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
-            T gv[F::NA], q(0), w(0);
-            unit_gauss<F, unit_pairs<FMT>()>(g, U, E, i, gv);
-#pragma unroll
-            for (int a = 0; a < F::NA; ++a) {
-                q = fma(gv[a], gv[a], q);
-                lanes_max(gv[a], gmax, gabs);
-            }
-            const UN u(g, i);
-#pragma unroll 1
-            for (int d = 0; d < 3; ++d) {
-                const T un = UN::G::unitarity_square(u.link(U, d, 0));
-                w = w + un;
-                lanes_max(un, umax, unused);
-            }
-            gsq += lanes_sum(q);
-            usq += lanes_sum(w);
+        for (int64_t i = i0; i < n; i += step) {
+            T esq, bsq;
+            edb += lanes_sum(unit_sample<F, unit_pairs<FMT>()>(g, U, E, i, mu, esq, bsq));
+            es += lanes_sum(esq);
+            bs += lanes_sum(bsq);
         }
     }
     double v[P_WIDTH];

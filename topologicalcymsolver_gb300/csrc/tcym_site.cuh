@@ -632,56 +632,6 @@ template <class F> struct Unit<F, false> {
     static TCYM_HD void transport(const Mat &v, const T *e, T *out) { G::transport(v, e, out); }
 };
 
-// The N_CS sample's observables (mask OBS_EDOTB) of direction mu for unit i: E_mu^2 into
-// esq, the plaquette term of B_mu^2 into bsq, and the clover E_mu . B_mu returned, as
-// site_observables forms them.  The clover average's projection is the average of the
-// leaves' projections (proj is linear), and proj(Q^dag) = -proj(Q): leaves that end in the
-// same link, one of them daggered, are summed before they are multiplied by it (ten
-// products for the four leaves instead of twelve).  Links may be off the group (FP32 ones
-// drift between reunitarisations), so whole products are formed.  Both sums of a unit run in
-// the storage's precision.
-template <class F, bool PAIR>
-TCYM_HD typename Unit<F, PAIR>::T unit_clover(const Geom &g, const void *U, const void *E, int64_t i, int mu,
-                                              typename Unit<F, PAIR>::T &esq, typename Unit<F, PAIR>::T &bsq) {
-    using UN = Unit<F, PAIR>;
-    using T = typename UN::T;
-    using G = typename UN::G;
-    using M = typename UN::Mat;
-    constexpr int NA = F::NA;
-    const UN u(g, i);
-    // clover of plane (j, k) = (mu+1, mu+2): the leaves of clover_leaves(j, k)
-    const int j = mu == 2 ? 0 : mu + 1, k = mu == 0 ? 2 : mu - 1;
-    auto L = [&](int d, int a, int b) { return u.link(U, d, j, a, k, b); };
-    T b[NA], pr[NA];
-    {   // Q2 - Q0^dag = (U_k^dag(x-k) U_j(x-k) U_k(x-k+j) - U_k(x) U_j(x+k) U_k^dag(x+j)) U_j^dag(x)
-        const M end = L(j, 0, 0);
-        const M q0 = G::template mulx<false, true>(G::template mulx<false, false>(L(k, 0, 0), L(j, 0, 1)), L(k, 1, 0));
-        bsq = T(4) * G::retr_one_minus_dag(q0, end);
-        const M q2 = G::template mulx<false, false>(G::template mulx<true, false>(L(k, 0, -1), L(j, 0, -1)), L(k, 1, -1));
-        G::proj_mul_dag(G::sub(q2, q0), end, b);
-    }
-    {   // Q1 - Q3^dag = (U_k(x) U_j^dag(x+k-j) U_k^dag(x-j) - U_k^dag(x-k) U_j^dag(x-j-k) U_k(x-j-k)) U_j(x-j)
-        const M q1 = G::template mulx<false, true>(G::template mulx<false, true>(L(k, 0, 0), L(j, -1, 1)), L(k, -1, 0));
-        const M q3 = G::template mulx<false, false>(G::template mulx<true, true>(L(k, 0, -1), L(j, -1, -1)), L(k, -1, -1));
-        G::proj_mul(G::sub(q1, q3), L(j, -1, 0), pr);
-#pragma unroll
-        for (int a = 0; a < NA; ++a) b[a] = b[a] + pr[a];
-    }
-    // E_mu(x) and U_mu^dag(x-mu) E_mu(x-mu) U_mu(x-mu)
-    T e[NA], et[NA];
-    u.load_e(E, mu, -1, e);
-    UN::transport(u.link(U, mu, -1), e, et);
-    u.load_e(E, mu, 0, e);
-    T sq(0), dot(0);
-#pragma unroll
-    for (int a = 0; a < NA; ++a) {
-        sq = fma(e[a], e[a], sq);
-        dot = fma(e[a] + et[a], b[a], dot);
-    }
-    esq = sq;
-    return T(0.25) * dot;
-}
-
 // A sum of FP32 products and terms with its rounding errors carried beside it: each
 // product split exactly by a fused multiply-add, each sum by Knuth's two-sum, so that
 // value() is good to about 2^-47 of the largest term.
@@ -699,20 +649,151 @@ template <class T> struct ExactSum {
         e = e + fma(a, b, -x);
         add(x);
     }
-    TCYM_HD T value() const { return s + e; }
 };
+// The same with the errors' own errors, good to FP64's last bit and more (22 packed
+// instructions a product of both lanes).
+template <class T> struct WideSum {
+    T s, e, c;
+    WideSum() = default;
+    TCYM_HD explicit WideSum(T start) : s(start), e(T(0)), c(T(0)) {}
+    static TCYM_HD T two_sum(T &s, T x) {
+        const T t = s + x, b = t - s, r = (s - (t - b)) + (x - b);
+        s = t;
+        return r;
+    }
+    TCYM_HD void add_error(T x) { c = c + two_sum(e, x); }
+    TCYM_HD void add(T x) { add_error(two_sum(s, x)); }
+    TCYM_HD void mul(T a, T b) {
+        const T x = a * b;
+        add(x);
+        add_error(fma(a, b, -x));
+    }
+};
+// the sum of lane l in FP64 (of a sum that is infinite or NaN, the plain one: its errors are NaN)
+TCYM_HD double lane64(const WideSum<f2> &x, int l) {
+    const float e = lane(x.e, l);
+    return (double)lane(x.s, l) + (e == e ? (double)e + (double)lane(x.c, l) : 0.0);
+}
+TCYM_HD double lane64(const WideSum<double> &x, int) { return x.s; }
+
+// Unit i's fields of direction mu for its measurement: E_mu(x) into e, the field carried
+// from below, U_mu^dag(x-mu) E_mu(x-mu) U_mu(x-mu), into et, four times the projection of the
+// clover average of B_mu into b and the plaquette term of B_mu^2 into bsq, as
+// site_observables forms them.  The clover average's projection is the average of the
+// leaves' projections (proj is linear), and proj(Q^dag) = -proj(Q): leaves that end in the
+// same link, one of them daggered, are summed before they are multiplied by it (ten
+// products for the four leaves instead of twelve).  Links may be off the group (FP32 ones
+// drift between reunitarisations), so whole products are formed.
+template <class F, bool PAIR, class T = typename Unit<F, PAIR>::T>
+TCYM_HD void unit_clover(const Geom &g, const void *U, const void *E, int64_t i, int mu, T *e, T *et, T *b, T &bsq) {
+    using UN = Unit<F, PAIR>;
+    using G = typename UN::G;
+    using M = typename UN::Mat;
+    constexpr int NA = F::NA;
+    const UN u(g, i);
+    // clover of plane (j, k) = (mu+1, mu+2): the leaves of clover_leaves(j, k)
+    const int j = mu == 2 ? 0 : mu + 1, k = mu == 0 ? 2 : mu - 1;
+    auto L = [&](int d, int a, int b) { return u.link(U, d, j, a, k, b); };
+    T pr[NA];
+    {   // Q2 - Q0^dag = (U_k^dag(x-k) U_j(x-k) U_k(x-k+j) - U_k(x) U_j(x+k) U_k^dag(x+j)) U_j^dag(x)
+        const M end = L(j, 0, 0);
+        const M q0 = G::template mulx<false, true>(G::template mulx<false, false>(L(k, 0, 0), L(j, 0, 1)), L(k, 1, 0));
+        bsq = T(4) * G::retr_one_minus_dag(q0, end);
+        const M q2 = G::template mulx<false, false>(G::template mulx<true, false>(L(k, 0, -1), L(j, 0, -1)), L(k, 1, -1));
+        G::proj_mul_dag(G::sub(q2, q0), end, b);
+    }
+    {   // Q1 - Q3^dag = (U_k(x) U_j^dag(x+k-j) U_k^dag(x-j) - U_k^dag(x-k) U_j^dag(x-j-k) U_k(x-j-k)) U_j(x-j)
+        const M q1 = G::template mulx<false, true>(G::template mulx<false, true>(L(k, 0, 0), L(j, -1, 1)), L(k, -1, 0));
+        const M q3 = G::template mulx<false, false>(G::template mulx<true, true>(L(k, 0, -1), L(j, -1, -1)), L(k, -1, -1));
+        G::proj_mul(G::sub(q1, q3), L(j, -1, 0), pr);
+#pragma unroll
+        for (int a = 0; a < NA; ++a) b[a] = b[a] + pr[a];
+    }
+    u.load_e(E, mu, -1, e);
+    UN::transport(u.link(U, mu, -1), e, et);
+    u.load_e(E, mu, 0, e);
+}
+// The N_CS sample (mask OBS_EDOTB) of unit i: E_mu^2 into esq, the plaquette term into bsq, and
+// the clover E_mu . B_mu returned; sums over components in the storage's precision.
+template <class F, bool PAIR, class T = typename Unit<F, PAIR>::T>
+TCYM_HD T unit_sample(const Geom &g, const void *U, const void *E, int64_t i, int mu, T &esq, T &bsq) {
+    constexpr int NA = F::NA;
+    T e[NA], et[NA], b[NA], dot(0);
+    unit_clover<F, PAIR>(g, U, E, i, mu, e, et, b, bsq);
+    esq = T(0);
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        esq = fma(e[a], e[a], esq);
+        dot = fma(e[a] + et[a], b[a], dot);
+    }
+    return T(0.25) * dot;
+}
+// The sums of all observables over a thread's units, in FP64 (FieldSums, ViolationSums).
+// Pairs sum in FP32 with the errors kept (WideSum): GB300 converts to FP64 and adds there at
+// 1/64 of the FP32 rate.  That is exact while products neither overflow nor lose their errors, to
+// 1e-45 each, below FP32's range: where the result says otherwise (exact()), or is zero, the
+// thread sums again in FP64 (add64).
+TCYM_HD bool exact_range(double squares) { return squares >= 1e-28 && squares <= 1e30; }
+// sums of E_mu^2 and of E_mu.B_mu, from unit_clover's fields
+template <class T, int NA> struct FieldSums;
+template <int NA> struct FieldSums<double, NA> {
+    double sq = 0, dot = 0;
+    TCYM_HD void add(const double *e, const double *et, const double *b) { add64(e, et, b); }
+    TCYM_HD void add64(const double *e, const double *et, const double *b) {
+        double s = 0, d = 0;
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            s = fma(e[a], e[a], s);
+            d = fma(e[a] + et[a], b[a], d);
+        }
+        sq += s;
+        dot += 0.25 * d;
+    }
+    TCYM_HD bool exact() { return true; }
+};
+template <int NA> struct FieldSums<f2, NA> {
+    WideSum<f2> s{f2(0.0)}, d{f2(0.0)};
+    double sq = 0, dot = 0;  // the results, of exact() or add64
+    TCYM_HD void add(const f2 *e, const f2 *et, const f2 *b) {
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            s.mul(e[a], e[a]);
+            d.mul(e[a], b[a]);
+            d.mul(et[a], b[a]);
+        }
+    }
+    TCYM_HD bool exact() {
+        const double x = lane64(s, 0), y = lane64(s, 1), u = lane64(d, 0), v = lane64(d, 1);
+        if (!(exact_range(x) && exact_range(y) && fabs(u) <= 1e30 && fabs(v) <= 1e30)) return false;
+        sq = x + y;
+        dot = 0.25 * (u + v);
+        return true;
+    }
+    TCYM_HD void add64(const f2 *e, const f2 *et, const f2 *b) {
+        for (int l = 0; l < 2; ++l) {
+            FieldSums<double, NA> o;
+            double x[NA], y[NA], z[NA];
+#pragma unroll
+            for (int a = 0; a < NA; ++a) { x[a] = lane(e[a], l); y[a] = lane(et[a], l); z[a] = lane(b[a], l); }
+            o.add64(x, y, z);
+            sq += o.sq;
+            dot += o.dot;
+        }
+    }
+};
+
 // The Gauss violation G(x) = sum_mu E_mu(x) - U_mu^dag(x-mu) E_mu(x-mu) U_mu(x-mu) of unit
 // i.  G of a restored field is a sum that cancels, so pairs sum their six FP32 terms with
-// the rounding errors (ExactSum).
+// the rounding errors (WideSum).
 template <class F, bool PAIR>
-TCYM_HD void unit_gauss(const Geom &g, const void *U, const void *E, int64_t i, typename Unit<F, PAIR>::T *gv) {
+TCYM_HD void unit_gauss(const Geom &g, const void *U, const void *E, int64_t i,
+                        WideSum<typename Unit<F, PAIR>::T> *s) {
     using UN = Unit<F, PAIR>;
     using T = typename UN::T;
     constexpr int NA = F::NA;
     const UN u(g, i);
-    ExactSum<T> s[NA];
 #pragma unroll
-    for (int a = 0; a < NA; ++a) s[a] = ExactSum<T>(T(0));
+    for (int a = 0; a < NA; ++a) s[a] = WideSum<T>(T(0));
 #pragma unroll 1
     for (int mu = 0; mu < 3; ++mu) {
         T e[NA], t[NA];
@@ -729,9 +810,74 @@ TCYM_HD void unit_gauss(const Geom &g, const void *U, const void *E, int64_t i, 
             }
         }
     }
-#pragma unroll
-    for (int a = 0; a < NA; ++a) gv[a] = s[a].value();
 }
+
+// Sum of squares, largest component and largest magnitude (from 0 on) of units' violations.
+template <class T, int NA> struct ViolationSums;
+template <int NA> struct ViolationSums<double, NA> {
+    double sq = 0, most = 0, mag = 0;
+    TCYM_HD void add(const WideSum<double> *g) { add64(g); }
+    TCYM_HD void add64(const WideSum<double> *g) {
+        double q = 0;
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            q = fma(g[a].s, g[a].s, q);
+            most = fmax(most, g[a].s);
+            mag = fmax(mag, fabs(g[a].s));
+        }
+        sq += q;
+    }
+    TCYM_HD bool exact() { return true; }
+};
+template <int NA> struct ViolationSums<f2, NA> {
+    // nearest FP32 number, rest and its rest: the largest component and the largest negative of one
+    struct Wide {
+        float h, l, c;
+    };
+    WideSum<f2> s{f2(0.0)};
+    Wide up{0, 0, 0}, down{0, 0, 0};
+    double sq = 0, most = 0, mag = 0;
+    static TCYM_HD void larger(Wide x, Wide &m) {
+        if (x.h > m.h || (x.h == m.h && x.l > m.l)) m = x;
+    }
+    static TCYM_HD double whole(const Wide &x) { return (double)x.h + ((double)x.l + (double)x.c); }
+    TCYM_HD void add(const WideSum<f2> *g) {
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            f2 h = g[a].s;
+            const f2 l = WideSum<f2>::two_sum(h, g[a].e);
+            s.mul(h, h);
+            s.mul(h + h, l);
+            s.c = fma(l, l, s.c);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const Wide x{lane(h, k), lane(l, k), lane(g[a].c, k)};
+                larger(x, up);
+                larger(Wide{-x.h, -x.l, -x.c}, down);
+            }
+        }
+    }
+    TCYM_HD bool exact() {
+        const double x = lane64(s, 0), y = lane64(s, 1);
+        if (!(exact_range(x) && exact_range(y))) return false;
+        sq = x + y;
+        most = whole(up);
+        mag = fmax(most, whole(down));
+        return true;
+    }
+    TCYM_HD void add64(const WideSum<f2> *g) {
+        ViolationSums<double, NA> o;
+        for (int l = 0; l < 2; ++l) {
+            WideSum<double> x[NA];
+#pragma unroll
+            for (int a = 0; a < NA; ++a) x[a].s = lane64(g[a], l);
+            o.add64(x);
+        }
+        sq += o.sq;
+        most = fmax(most, o.most);
+        mag = fmax(mag, o.mag);
+    }
+};
 
 // Gauss violation G(x) in working precision T, for the restore iteration.
 template <class F>
