@@ -30,6 +30,7 @@ def load():
                               ctypes.c_double, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int, ctypes.c_int,
                               ctypes.c_int]
         L.hc_march.argtypes = [ctypes.c_int, ip, _vp, _vp, _vp, ctypes.c_double] + [ctypes.c_int] * 4
+        L.hc_by_sites.argtypes = [ip, ctypes.c_int]
         L.hc_flow_cb.argtypes = [ctypes.c_int, ip, _vp, ctypes.c_double, ctypes.c_int]
         L.hc_observables.argtypes = [ctypes.c_int, ip, _vp, _vp, ctypes.c_int, _vp]
         L.hc_edotb_pair.argtypes = [ctypes.c_int, ip, _vp, _vp, _vp]
@@ -171,6 +172,11 @@ class HostLattice:
         """UMid, EMid (into this lattice) of the geodesic from old's links to new's."""
         self.L.hc_geodesic(self.fmt, self.n, _p(old.U[old.cur]), _p(new.U[new.cur]), c, _p(self.U[self.cur]),
                            _p(self.E))
+
+
+def by_sites(shape, sms=152):
+    """Does the FP64 step of a lattice alone on `sms` multiprocessors go by sites (and not by tiles)?"""
+    return bool(load().hc_by_sites((ctypes.c_int * 3)(*shape), sms))
 
 
 def pair_sums(e, et, b, count=1):

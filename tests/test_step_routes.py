@@ -1,0 +1,62 @@
+"""The FP64 step by tiles or by sites, whichever the lattice's extents fit: the rule, and both
+routes against the oracle."""
+import numpy as np
+import pytest
+
+from tests import _hostcheck as hc
+
+# by sites: a nearly full first wave of blocks and extents the tiles fit badly; tiles: small, just
+# past the wave, large
+SITES = [(26, 26, 26), (33, 20, 27)]
+TILES = [(8, 8, 8), (24, 24, 24), (28, 28, 28), (48, 48, 48)]
+
+
+def test_rule():
+    assert all(hc.by_sites(n) for n in SITES) and not any(hc.by_sites(n) for n in TILES)
+
+
+def state(P, nc, shape):
+    V = int(np.prod(shape))
+    U, E = np.zeros((V, 3, hc.NM[nc])), np.zeros((V, 3, hc.NA[nc]))
+    P.random_links(shape, U, 0.5, 3)
+    P.gaussian_efield(shape, E, 0.7, 4)
+    return U, E
+
+
+@pytest.mark.parametrize("nc", [2, 3])
+@pytest.mark.parametrize("shape", [SITES[0]])
+def test_host_by_sites(oracle_port, nc, shape):
+    """Two steps: rounding, 1e-14 of fields of order 1 each."""
+    P = oracle_port[nc]
+    U, E = state(P, nc, shape)
+    H = hc.HostLattice(nc, "f64", shape)
+    H.upload(U, E)
+    H.leapfrog(0.05, 2)
+    P.leapfrog(shape, U, E, 0.05, 2)
+    assert max(np.abs(x - y).max() for x, y in zip(H.download(), (U, E))) < 1e-13
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nc", [2, 3])
+@pytest.mark.parametrize("shape", [*SITES, TILES[1]])
+def test_gpu_routes(ctx, oracle_port, nc, shape):
+    """Leapfrog, Langevin, the flow and the two half updates on each route, 1e-12 after ten steps."""
+    import topologicalcymsolver_gb300 as tcym
+
+    P = oracle_port[nc]
+    U, E = state(P, nc, shape)
+    lat = tcym.Lattice(ctx, nc, shape, tcym.FP64)
+    lat.upload(U, E)
+    lat.leapfrog(0.05, 4)
+    P.leapfrog(shape, U, E, 0.05, 4)
+    lat.langevin(0.02, 1.0, 0.6, 7, 5, 4)
+    P.langevin(shape, U, E, 0.02, 1.0, 0.6, 7, 5, 4)
+    lat.update_e(0.03)
+    P.update_e(shape, U, E, 0.03)
+    lat.update_u(0.03)
+    P.update_u(shape, U, E, 0.03)
+    assert max(np.abs(x - y).max() for x, y in zip(lat.download(), (U, E))) < 1e-12
+    lat.flow(0.02, 2)
+    P.flow(shape, U, E, 0.02, 2)
+    assert np.abs(lat.download()[0] - U).max() < 1e-12
+    lat.close()

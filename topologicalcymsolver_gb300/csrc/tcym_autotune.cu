@@ -132,7 +132,7 @@ const Tile &tcym_lattice_tile_of(tcym_lattice lat) {
 
 const MarchTile &tcym_lattice_march_of(tcym_lattice lat, bool batched) {
     MarchTile &t = lat->march[batched];
-    if (t.tx == 0) t = march_tile(lat->g, batched ? 0 : lat->ctx->sm_count);
+    if (t.threads == 0) t = batched ? march_tile(lat->g, 0) : step_tile(lat->g, lat->ctx->sm_count);
     return t;
 }
 

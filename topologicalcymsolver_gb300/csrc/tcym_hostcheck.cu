@@ -77,14 +77,15 @@ template <int FMT> struct H {
     // the per-site step as Launch::step_sites runs it
     static void sites(const Geom &g, const void *Uin, void *Uout, void *E, const StepCoef<T> &c, bool doU,
                       const SiteRange &r) {
-        if constexpr (F::PAIRED) {
-            T sm[3 * F::NA];
-            for (int64_t s = r.s0; s < r.s1; ++s) {
-                if (doU) site_step<F, true>(g, Uin, Uout, E, c, s, 0, sm, 1);
-                else site_step<F, false>(g, Uin, Uout, E, c, s, 0, sm, 1);
-            }
-        } else {
-            march(g, Uin, Uout, E, c, doU, r, march_tile(g, 152));
+        const MarchTile t = step_tile(g, 152);
+        if (!F::PAIRED && t.tx != 0) {
+            march(g, Uin, Uout, E, c, doU, r, t);
+            return;
+        }
+        T sm[3 * F::NA];
+        for (int64_t s = r.s0; s < r.s1; ++s) {
+            if (doU) site_step<F, true>(g, Uin, Uout, E, c, s, 0, sm, 1);
+            else site_step<F, false>(g, Uin, Uout, E, c, s, 0, sm, 1);
         }
     }
     // the device's FP64 step, block by block, phase by phase and thread by thread
@@ -414,6 +415,8 @@ int hc_march(int fmt, const int *n, const void *Uin, void *Uout, void *E, double
     HC_DISPATCH(fmt, HH::march(g, Uin, Uout, E, cast<HH::T>(c), true, SiteRange{0, g.nz, 0, g.V}, t));
     return 0;
 }
+// does the FP64 step of a lattice alone on `sms` multiprocessors go by sites?
+int hc_by_sites(const int *n, int sms) { return step_tile(geom(n), sms).tx == 0; }
 int hc_flow_cb(int fmt, const int *n, void *U, double dtau, int nsweeps) {
     Geom g = geom(n);
     HC_DISPATCH(fmt, HH::flow_cb(g, U, dtau, nsweeps));

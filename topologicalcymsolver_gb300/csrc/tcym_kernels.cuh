@@ -32,7 +32,7 @@ enum : int {
 constexpr int kThreadsSU2 = TCYM_SU2_THREADS;
 constexpr int kThreadsSU3 = 128;
 constexpr int kRedThreads = 256;
-// Resident blocks per SM requested for the per-site FP32 step and the checkerboard flow
+// Resident blocks per SM requested for the per-site step and the checkerboard flow
 // (register cap = 65536 / (blocks * threads)).
 template <int FMT> constexpr int min_blocks_for() {
     return Fmt<FMT>::NA == 8 ? 4 : (FMT == FMT_SU2_F32 ? 8 : 1);
@@ -126,12 +126,12 @@ template <class T> StepCoef<T> coef_cast(const StepCoef<double> &c) {
 // shared-memory slots of the plaquette projections (site_step, site_step_pair)
 template <int FMT> constexpr int plaq_slots() { return 3 * Fmt<FMT>::NA; }
 
-// the per-site FP32 step (odd nz; DO_U false: the E update alone), sites [s0, s1)
+// the per-site step (FP32 with odd nz, FP64 by step_tile; DO_U false: the E update alone),
+// sites [s0, s1)
 template <int FMT, bool DO_U>
 __global__ void __launch_bounds__(threads_for<FMT>(), min_blocks_for<FMT>()) k_step(Geom g, const void *Uin, void *Uout, void *E,
-                                                             StepCoef<float> c, int64_t s0, int64_t s1) {
-    static_assert(Fmt<FMT>::PAIRED, "the FP64 formats step through k_march");
-    __shared__ float sm[plaq_slots<FMT>() * threads_for<FMT>()];
+                                                             StepCoef<typename Fmt<FMT>::T> c, int64_t s0, int64_t s1) {
+    __shared__ typename Fmt<FMT>::T sm[plaq_slots<FMT>() * threads_for<FMT>()];
     const int64_t s = s0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= s1) return;
     site_step<Fmt<FMT>, DO_U>(g, Uin, Uout, E, c, s, 0, sm + threadIdx.x, threads_for<FMT>());
@@ -792,12 +792,14 @@ template <int FMT> struct Launch {
     static cudaError_t step_sites(const Geom &g, const void *Uin, void *Uout, void *E, const StepCoef<double> &cd,
                                   const MarchTile &m, const SiteRange &r, cudaStream_t st) {
         const StepCoef<T> c = coef_cast<T>(cd);
-        if constexpr (F::PAIRED) {
-            k_step<FMT, DO_U><<<grid_for(r.s1 - r.s0, TPB), TPB, 0, st>>>(g, Uin, Uout, E, c, r.s0, r.s1);
-        } else {
-            const unsigned blocks = (unsigned)march_blocks(m, r.z1 - r.z0);
-            k_march<FMT, DO_U><<<blocks, m.threads, march_smem<F>(m), st>>>(g, Uin, Uout, E, c, m, r);
+        if constexpr (!F::PAIRED) {
+            if (m.tx != 0) {
+                const unsigned blocks = (unsigned)march_blocks(m, r.z1 - r.z0);
+                k_march<FMT, DO_U><<<blocks, m.threads, march_smem<F>(m), st>>>(g, Uin, Uout, E, c, m, r);
+                return cudaGetLastError();
+            }
         }
+        k_step<FMT, DO_U><<<grid_for(r.s1 - r.s0, TPB), TPB, 0, st>>>(g, Uin, Uout, E, c, r.s0, r.s1);
         return cudaGetLastError();
     }
     // Lattices whose paired step spreads a pair over three threads (k_step_split): up to

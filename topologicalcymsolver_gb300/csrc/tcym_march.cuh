@@ -30,7 +30,8 @@
 
 namespace tcym {
 
-// How the blocks cover the sites: tx x ty tiles of a plane, zl planes a block.
+// How the blocks cover the sites: tx x ty tiles of a plane, zl planes a block (tx 0: a
+// lattice that steps faster by sites, site_step).
 struct MarchTile {
     int tx, ty, tiles_x, tiles_y, zl, threads;
 };
@@ -249,15 +250,15 @@ template <class F> struct March {
 
 // The tiling of a lattice stepped alone (sms: the device's multiprocessors) or among
 // others (sms = 0).  Its cost model is the multiply-adds of the busiest multiprocessor, in
-// whole warps: a block's tasks are phase 1's plaquettes (268 for SU(3) in FP64), phase 2's links (500)
-// and the first plane's extra 2 S plaquettes with their rotations (400); alone, the
+// whole warps: a block's tasks are phase 1's plaquettes (310 for SU(3) in FP64), phase 2's links (572)
+// and the first plane's extra 2 S plaquettes with their rotations (454); alone, the
 // multiprocessor with the most blocks decides, fewer than six warps on it leave its FP64
 // unit idle in proportion, and every plane adds the latency of its two phases (as 6000
 // multiply-adds).  Among others the blocks fill the device whatever their number, so
 // larger blocks, which repeat less, are better, up to 8 planes (the launch's tail).
 // Measured on GB300, FP64 per step, the rule's choice / 16 x 8 tiles of 8 planes: SU(3)
 // 16^3 37 / 678 us, 48^3 516 / 714 us; SU(2) 16^3 10 / 140 us.
-inline MarchTile march_tile(const Geom &g, int sms) {
+inline MarchTile march_tile(const Geom &g, int sms, double *least = nullptr) {
     MarchTile best{};
     double cost = 0;
     for (int kx = (g.nx + 15) / 16; kx <= g.nx; ++kx) {
@@ -269,7 +270,7 @@ inline MarchTile march_tile(const Geom &g, int sms) {
             if (tx * ty < 16 && best.tx) break;
             const double S = (double)tx * ty, halo = (tx == g.nx ? 0 : ty) + (ty == g.ny ? 0 : tx);
             auto warps_of = [](double n) { return 32.0 * (int)((n + 31) / 32); };
-            const double plane = 268 * warps_of(3 * S + 2 * halo) + 500 * warps_of(3 * S), first = 400 * warps_of(2 * S);
+            const double plane = 310 * warps_of(3 * S + 2 * halo) + 572 * warps_of(3 * S), first = 454 * warps_of(2 * S);
             const double tiles = (double)((g.nx + tx - 1) / tx) * ((g.ny + ty - 1) / ty);
             for (int zl = 1; zl <= g.nz && zl <= (sms ? 16 : 8); ++zl) {
                 const double blocks = tiles * ((g.nz + zl - 1) / zl);
@@ -286,7 +287,20 @@ inline MarchTile march_tile(const Geom &g, int sms) {
             }
         }
     }
+    if (least) *least = cost;
     return best;
+}
+// The same, or by sites (site_step in blocks of 128: 3400 a site by the same measure) where
+// that costs the busiest multiprocessor less: lattices that fill the device's first wave of
+// such blocks and whose extents the tiles fit badly.  By sites / by tiles, us a step on GB300, SU(3): 26^3
+// 119 / 150, 33 x 20 x 27 119 / 148, 18 x 28 x 34 119 / 119; 24^3 119 / 105, 28^3 228 / 158, 48^3
+// 676 / 588; SU(2) 26^3 29 / 33, 28^3 49 / 33.
+inline MarchTile step_tile(const Geom &g, int sms) {
+    double least;
+    MarchTile t = march_tile(g, sms, &least);
+    const int64_t blocks = (g.V + 127) / 128;
+    if (3400.0 * 128 * (double)((blocks + sms - 1) / sms) < least) t.tx = 0;
+    return t;
 }
 
 }  // namespace tcym

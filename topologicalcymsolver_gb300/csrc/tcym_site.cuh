@@ -121,8 +121,7 @@ TCYM_HD void add_plaquette_force(const T *sm, int stride, int mu, const C (&cnu)
     for (int a = 0; a < NA; ++a) f[a] = fma(cp, sm[(mu * NA + a) * stride], fma(-cm, sm[(n2 * NA + a) * stride], f[a]));
 }
 
-// One site of the FP32 formats' per-site step (odd nz; DO_U false: the E update alone,
-// Uout unused).  sm: 3 * NA slots of T for this site, stride apart.
+// One site of the per-site step (DO_U false: the E update alone, Uout unused).  sm: 3 * NA slots of T for this site, stride apart.
 template <class F, bool DO_U>
 TCYM_HD void site_step(const Geom &g, const void *Uin, void *Uout, void *E, const StepCoef<typename F::T> &c,
                        int64_t s, uint64_t step_add, typename F::T *sm, int stride) {
