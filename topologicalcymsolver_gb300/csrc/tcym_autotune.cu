@@ -130,9 +130,9 @@ const Tile &tcym_lattice_tile_of(tcym_lattice lat) {
     return lat->tile;
 }
 
-const MarchTile &tcym_lattice_march_of(tcym_lattice lat, bool batched) {
-    MarchTile &t = lat->march[batched];
-    if (t.threads == 0) t = batched ? march_tile(lat->g, 0) : step_tile(lat->g, lat->ctx->sm_count);
+const MarchTile &tcym_lattice_march_of(tcym_lattice lat) {
+    MarchTile &t = lat->march;
+    if (t.threads == 0) t = step_tile(lat->g, lat->ctx->sm_count);
     return t;
 }
 

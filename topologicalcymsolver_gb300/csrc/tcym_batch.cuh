@@ -40,6 +40,7 @@ template <class T> struct Member {
 #define TCYM_SU3_BATCH_MINBLOCKS 3
 #endif
 template <int FMT> constexpr int batch_min_blocks_for() {
+    if (!Fmt<FMT>::PAIRED) return min_blocks_for<FMT>();
     return Fmt<FMT>::NA == 3 ? TCYM_SU2_BATCH_MINBLOCKS : TCYM_SU3_BATCH_MINBLOCKS;
 }
 
@@ -78,14 +79,14 @@ __global__ void __launch_bounds__(kThreadsPair, batch_min_blocks_for<FMT>())
     else
         site_step_pair<Fmt<FMT>, false>(g, m.U[in], m.U[in ^ 1], m.E, m.c, p, (uint64_t)k, sm + threadIdx.x, kThreadsPair);
 }
-// The same for the members stepped per site, whose work items follow from item0 on: FP32
-// with odd nz, and FP64.
+// The same for the members stepped per site, whose work items follow from item0 on (FP32
+// with odd nz, FP64), and for FP64 members stepped by tiles.
 template <int FMT>
 __global__ void __launch_bounds__(threads_for<FMT>(), batch_min_blocks_for<FMT>())
-    k_sites_batch(const Member<float> *__restrict__ members, int nmembers, int item0, int k) {
-    __shared__ float sm[plaq_slots<FMT>() * threads_for<FMT>()];
+    k_sites_batch(const Member<typename Fmt<FMT>::T> *__restrict__ members, int nmembers, int item0, int k) {
+    __shared__ typename Fmt<FMT>::T sm[plaq_slots<FMT>() * threads_for<FMT>()];
     const int item = item0 + blockIdx.x;
-    const Member<float> &m = members[find_member(members, nmembers, item, false)];
+    const Member<typename Fmt<FMT>::T> &m = members[find_member(members, nmembers, item, false)];
     const Geom g = m.g;
     const int64_t s = (int64_t)(item - m.block_begin) * blockDim.x + threadIdx.x;
     if (s >= g.V) return;
@@ -293,17 +294,20 @@ template <int FMT> struct LaunchBatch {
         }
         return cudaErrorInvalidValue;
     }
-    // work items of a member stepped per site
+    // work items of a member stepped per site, or by the tiles m
     static int site_items(const Geom &g, const MarchTile &m) {
-        return Fmt<FMT>::PAIRED ? grid_for(g.V, threads_for<FMT>()) : (int)march_blocks(m, g.nz);
+        return m.tx == 0 ? grid_for(g.V, threads_for<FMT>()) : (int)march_blocks(m, g.nz);
     }
-    // the members [m0, m0 + n) stepped per site, work items [item0, item1)
-    static cudaError_t sites(const Member<T> *members, int m0, int n, int item0, int item1, int k, size_t smem,
+    // the members [m0, m0 + n) stepped per site, or (threads > 0) by tiles, work items [item0, item1)
+    static cudaError_t sites(const Member<T> *members, int m0, int n, int item0, int item1, int k, int threads, size_t smem,
                              cudaStream_t st) {
-        if constexpr (Fmt<FMT>::PAIRED)
-            k_sites_batch<FMT><<<item1 - item0, threads_for<FMT>(), 0, st>>>(members + m0, n, item0, k);
-        else
-            k_march_batch<FMT><<<item1 - item0, kMarchThreads, smem, st>>>(members + m0, n, item0, k);
+        if constexpr (!Fmt<FMT>::PAIRED) {
+            if (threads > 0) {
+                k_march_batch<FMT><<<item1 - item0, threads, smem, st>>>(members + m0, n, item0, k);
+                return cudaGetLastError();
+            }
+        }
+        k_sites_batch<FMT><<<item1 - item0, threads_for<FMT>(), 0, st>>>(members + m0, n, item0, k);
         return cudaGetLastError();
     }
     // the members [m0, m0 + n) of one coefficient class, work items [item0, item1),

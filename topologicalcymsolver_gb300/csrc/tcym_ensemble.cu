@@ -12,7 +12,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cstring>
+#include <map>
 #include <new>
 #include <tuple>
 #include <vector>
@@ -40,7 +42,17 @@ struct FmtGroup {
     // step work items: those of the paired members first (idx is ordered so), then from
     // pair_blocks on those of the members stepped per site, the first of them npaired
     int total_blocks = 0, pair_blocks = 0, npaired = 0;
-    size_t march_smem = 0;       // shared memory of the FP64 step's blocks (the largest)
+    int march_threads = 0;       // threads and shared memory of the FP64 step's blocks (the largest)
+    size_t march_smem = 0;
+    // FP64: the members' tilings and their costs by extents, for a number of sites in all; the
+    // members step by tiles, or all by sites
+    struct Tiling {
+        MarchTile tile;
+        double cost = 0;
+    };
+    int64_t sites = 0;
+    std::map<std::array<int, 3>, Tiling> march;
+    bool by_sites = false;
     int red_total = 0, red_grid = 0, red_offset = 0;
     bool tiled = false;          // some paired member is tiled: the kernel that reads every member's tiling
     // runs of members (idx is ordered by coefficients) that share the mode, force, staple
@@ -94,12 +106,40 @@ struct tcym_ensemble_s {
         if (e_ != cudaSuccess) return fail(ens->ctx, e_, #call);  \
     } while (0)
 
+// The tiling of an FP64 member: its share of the device is its share of the group's sites.
+static const FmtGroup::Tiling &member_march(FmtGroup &G, tcym_lattice lat) {
+    FmtGroup::Tiling &t = G.march[{lat->g.nx, lat->g.ny, lat->g.nz}];
+    if (t.tile.threads == 0)
+        t.tile = march_tile(lat->g, (double)lat->ctx->sm_count * (double)lat->g.V / (double)G.sites, lat->g.V == G.sites, &t.cost);
+    return t;
+}
+// How FP64 members step: by tiles, or all by sites (one launch) unless tiles cost 5% less by
+// the rule's measure, which among others is off by a few per cent.  By sites before / the rule's
+// choice / blocks as large as if the members always filled the device, us a step on GB300, SU(3): one 8^3
+// 119 / 42 / 327, 24 of 13^3 344 / 311 / 525, 8 of 26^3 904 / 812 / 873, 24 of 32^3 4591 / 4116 / 4230,
+// 16 of 16^3 to 48^3 3807 / 3386 / 3380; SU(2): one 8^3 28 / 11 / 70, 24 of 32^3 926 / 775 / 802.
+static void choose_march(tcym_ensemble ens, FmtGroup &G) {
+    int64_t sites = 0;
+    for (int i : G.idx) sites += ens->members[i].lat->g.V;
+    if (sites != G.sites) G.march.clear();
+    G.sites = sites;
+    double tiles = 0, by_sites = 0;  // each member's estimate of the group's time, by its sites
+    for (int i : G.idx) {
+        const tcym_lattice L = ens->members[i].lat;
+        const double share = (double)L->g.V / (double)sites;
+        tiles += share * member_march(G, L).cost;
+        by_sites += share * sites_cost(L->g.V, ens->ctx->sm_count * share);
+    }
+    G.by_sites = by_sites * (G.idx.size() > 1 ? 0.95 : 1) < tiles;
+}
+
 template <int FMT> static void fill_group(tcym_ensemble ens, FmtGroup &G, int sm_count) {
     using T = typename Fmt<FMT>::T;
     std::vector<Member<T>> tab(G.idx.size());
     int blk = 0, red = 0;
     G.tiled = false;
     G.pair_blocks = G.npaired = 0;
+    G.march_threads = 0;
     G.march_smem = 0;
     G.classes.clear();
     G.member_block.assign(G.idx.size(), 0);
@@ -133,8 +173,9 @@ template <int FMT> static void fill_group(tcym_ensemble ens, FmtGroup &G, int sm
             G.npaired = (int)i + 1;
             G.pair_blocks = blk;
         } else {
-            if (!Fmt<FMT>::PAIRED) {
-                m.march = tcym_lattice_march_of(L, true);
+            if (!Fmt<FMT>::PAIRED && !G.by_sites) {
+                m.march = member_march(G, L).tile;
+                G.march_threads = std::max(G.march_threads, m.march.threads);
                 G.march_smem = std::max(G.march_smem, march_smem<Fmt<FMT>>(m.march));
             }
             blk += LaunchBatch<FMT>::site_items(L->g, m.march);
@@ -163,6 +204,7 @@ static void fill_all(tcym_ensemble ens) {
                    std::make_tuple(b.lat->g.nz % 2, b.mode, b.dt, b.lat->a[0], b.lat->a[1], b.lat->a[2]);
         });
     const int sm = ens->ctx->sm_count;
+    for (int f : {FMT_SU2_F64, FMT_SU3_F64}) choose_march(ens, ens->groups[f]);
     fill_group<FMT_SU2_F32>(ens, ens->groups[FMT_SU2_F32], sm);
     fill_group<FMT_SU2_F64>(ens, ens->groups[FMT_SU2_F64], sm);
     fill_group<FMT_SU3_F32>(ens, ens->groups[FMT_SU3_F32], sm);
@@ -256,9 +298,9 @@ template <int FMT> static cudaError_t launch_group_step(tcym_ensemble ens, int f
                     e = LaunchBatch<FMT>::step_uniform(table, c.m0, c.m1 - c.m0, c.item0, c.item1, k, c.coef, s);
         }
     }
-    const int n = (int)G.idx.size();
-    if (e == cudaSuccess && n > G.npaired)
-        e = LaunchBatch<FMT>::sites(table, G.npaired, n - G.npaired, G.pair_blocks, G.total_blocks, k, G.march_smem, s);
+    const int n = (int)G.idx.size() - G.npaired;
+    if (e == cudaSuccess && n > 0)
+        e = LaunchBatch<FMT>::sites(table, G.npaired, n, G.pair_blocks, G.total_blocks, k, G.march_threads, G.march_smem, s);
     return e;
 }
 

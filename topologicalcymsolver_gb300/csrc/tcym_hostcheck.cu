@@ -411,7 +411,7 @@ int hc_march(int fmt, const int *n, const void *Uin, void *Uout, void *E, double
              int threads) {
     Geom g = geom(n);
     StepCoef<double> c = coef(MODE_LEAPFROG, dt, 0, 0, 0, 0);
-    const MarchTile t = tx ? MarchTile{tx, ty, (g.nx + tx - 1) / tx, (g.ny + ty - 1) / ty, zl, threads} : march_tile(g, threads);
+    const MarchTile t = tx ? MarchTile{tx, ty, (g.nx + tx - 1) / tx, (g.ny + ty - 1) / ty, zl, threads} : march_tile(g, threads > 0 ? threads : 0.5, threads > 0);
     HC_DISPATCH(fmt, HH::march(g, Uin, Uout, E, cast<HH::T>(c), true, SiteRange{0, g.nz, 0, g.V}, t));
     return 0;
 }

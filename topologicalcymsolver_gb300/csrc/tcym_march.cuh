@@ -248,17 +248,21 @@ template <class F> struct March {
     }
 };
 
-// The tiling of a lattice stepped alone (sms: the device's multiprocessors) or among
-// others (sms = 0).  Its cost model is the multiply-adds of the busiest multiprocessor, in
-// whole warps: a block's tasks are phase 1's plaquettes (310 for SU(3) in FP64), phase 2's links (572)
-// and the first plane's extra 2 S plaquettes with their rotations (454); alone, the
-// multiprocessor with the most blocks decides, fewer than six warps on it leave its FP64
-// unit idle in proportion, and every plane adds the latency of its two phases (as 6000
-// multiply-adds).  Among others the blocks fill the device whatever their number, so
-// larger blocks, which repeat less, are better, up to 8 planes (the launch's tail).
+// The blocks' cost, in multiply-adds of whole warps: phase 1's plaquettes (310 for SU(3) in
+// FP64) and phase 2's links (572) of each plane, and the first plane's extra 2 S plaquettes with
+// their rotations (454).
+inline double march_warps(double n) { return 32.0 * (int)((n + 31) / 32); }
+inline double march_plane(int S, int halo) { return 310 * march_warps(3 * S + 2 * halo) + 572 * march_warps(3 * S); }
+inline double march_first(int S) { return 454 * march_warps(2 * S); }
+// The tiling of a lattice that has the share `sms` of a device's multiprocessors, alone or among
+// others (an ensemble's members).  Its cost model is the work of the busiest multiprocessor, that
+// with the most blocks: alone these are full ones, among others two of them, the rest the
+// average block.  Fewer than six warps on it leave its FP64 unit idle in proportion, and every plane adds
+// the latency of its two phases (as 6000 multiply-adds).  Blocks walk up to 16 planes, among
+// others 8 (the launch's tail).
 // Measured on GB300, FP64 per step, the rule's choice / 16 x 8 tiles of 8 planes: SU(3)
-// 16^3 37 / 678 us, 48^3 516 / 714 us; SU(2) 16^3 10 / 140 us.
-inline MarchTile march_tile(const Geom &g, int sms, double *least = nullptr) {
+// 16^3 43 / 678 us, 48^3 587 / 714 us; SU(2) 16^3 12 / 140 us.
+inline MarchTile march_tile(const Geom &g, double sms, bool alone, double *least = nullptr) {
     MarchTile best{};
     double cost = 0;
     for (int kx = (g.nx + 15) / 16; kx <= g.nx; ++kx) {
@@ -268,21 +272,29 @@ inline MarchTile march_tile(const Geom &g, int sms, double *least = nullptr) {
             const int ty = (g.ny + ky - 1) / ky;
             if (tx * ty > kMarchSites) continue;
             if (tx * ty < 16 && best.tx) break;
-            const double S = (double)tx * ty, halo = (tx == g.nx ? 0 : ty) + (ty == g.ny ? 0 : tx);
-            auto warps_of = [](double n) { return 32.0 * (int)((n + 31) / 32); };
-            const double plane = 310 * warps_of(3 * S + 2 * halo) + 572 * warps_of(3 * S), first = 454 * warps_of(2 * S);
-            const double tiles = (double)((g.nx + tx - 1) / tx) * ((g.ny + ty - 1) / ty);
-            for (int zl = 1; zl <= g.nz && zl <= (sms ? 16 : 8); ++zl) {
-                const double blocks = tiles * ((g.nz + zl - 1) / zl);
-                const double per_sm = sms ? (double)(((int64_t)blocks + sms - 1) / sms) : blocks;
-                const int tasks = (int)(3 * S + 2 * halo + (zl == 1 ? 2 * S : 0));
+            const int nx = (g.nx + tx - 1) / tx, ny = (g.ny + ty - 1) / ty;
+            const int halo = (tx == g.nx ? 0 : ty) + (ty == g.ny ? 0 : tx), S = tx * ty;
+            const double plane = march_plane(S, halo), first = march_first(S);
+            double planes = 0, firsts = 0;  // of all tiles, ragged ones as they are
+            for (int i = 0; i < 2; ++i)
+                for (int j = 0; j < 2; ++j) {
+                    const int w = i ? g.nx - tx * (nx - 1) : tx, h = j ? g.ny - ty * (ny - 1) : ty;
+                    const double n = (double)(i ? 1 : nx - 1) * (j ? 1 : ny - 1);
+                    planes += n * march_plane(w * h, (w == g.nx ? 0 : h) + (h == g.ny ? 0 : w));
+                    firsts += n * march_first(w * h);
+                }
+            for (int zl = 1; zl <= g.nz && zl <= (alone ? 16 : 8); ++zl) {
+                const int chunks = (g.nz + zl - 1) / zl;
+                const double blocks = (double)nx * ny * chunks, per_sm = ceil(blocks / sms);
+                const int tasks = 3 * S + 2 * halo + (zl == 1 ? 2 * S : 0);
                 const int threads = tasks > kMarchThreads ? kMarchThreads : (tasks + 31) / 32 * 32;
-                const double warps = per_sm * threads / 32;
-                double c = per_sm * (zl * plane + first);
-                if (sms) c = c * (warps < 6 ? 6 / warps : 1) + 6000.0 * zl;
+                const double warps = per_sm * threads / 32, block = zl * plane + first;
+                double c = per_sm * block;
+                if (!alone && per_sm > 2) c = 2 * block + (per_sm - 2) * (g.nz * planes + chunks * firsts) / blocks;
+                c = c * (warps < 6 ? 6 / warps : 1) + 6000.0 * zl;
                 if (!best.tx || c < cost) {
                     cost = c;
-                    best = MarchTile{tx, ty, (g.nx + tx - 1) / tx, (g.ny + ty - 1) / ty, zl, sms ? threads : kMarchThreads};
+                    best = MarchTile{tx, ty, nx, ny, zl, threads};
                 }
             }
         }
@@ -290,16 +302,16 @@ inline MarchTile march_tile(const Geom &g, int sms, double *least = nullptr) {
     if (least) *least = cost;
     return best;
 }
-// The same, or by sites (site_step in blocks of 128: 3400 a site by the same measure) where
-// that costs the busiest multiprocessor less: lattices that fill the device's first wave of
-// such blocks and whose extents the tiles fit badly.  By sites / by tiles, us a step on GB300, SU(3): 26^3
-// 119 / 150, 33 x 20 x 27 119 / 148, 18 x 28 x 34 119 / 119; 24^3 119 / 105, 28^3 228 / 158, 48^3
-// 676 / 588; SU(2) 26^3 29 / 33, 28^3 49 / 33.
-inline MarchTile step_tile(const Geom &g, int sms) {
+// The cost of a step by sites (site_step in blocks of 128), by the same measure.
+inline double sites_cost(int64_t V, double sms) { return 3150.0 * 128 * ceil((double)((V + 127) / 128) / sms); }
+// The step of a lattice alone: by tiles, or by sites (tx 0) where that costs less: extents that
+// the tiles fit badly, in waves of blocks that are nearly full.  By sites / by tiles, us a step
+// on GB300, SU(3) 18 x 28 x 34 109 / 119, 26^3 109 / 150, 33 x 20 x 27 109 / 148, 24^3 109 / 105,
+// 28^3 209 / 158, 48^3 619 / 587; SU(2) 26^3 25 / 33, 28^3 43 / 33.
+inline MarchTile step_tile(const Geom &g, double sms) {
     double least;
-    MarchTile t = march_tile(g, sms, &least);
-    const int64_t blocks = (g.V + 127) / 128;
-    if (3400.0 * 128 * (double)((blocks + sms - 1) / sms) < least) t.tx = 0;
+    MarchTile t = march_tile(g, sms, true, &least);
+    if (sites_cost(g.V, sms) < least) t.tx = 0;
     return t;
 }
 
