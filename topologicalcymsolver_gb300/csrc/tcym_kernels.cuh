@@ -295,18 +295,23 @@ __device__ __forceinline__ double warp_op(int k, double v) {
 }
 
 // The block's record from its threads' values, the used slots only, one after the other
-// (COMPACT) or each in its place; sh: used_count(USED) * NT doubles.
+// (COMPACT) or each in its place; own: of these the ones that the block fills (the others of
+// its record are not written); sh: used_count(USED) * NT doubles.
 template <unsigned USED, int NT, bool COMPACT>
-__device__ __forceinline__ void block_record(const double *v, double *sh, double *record) {
+__device__ __forceinline__ void block_record(const double *v, double *sh, double *record, unsigned own = USED) {
     constexpr int NQ = used_count(USED);
     const int lane = threadIdx.x & 31;
     int q = 0;
 #pragma unroll
     for (int k = 0; k < P_WIDTH; ++k)
-        if (USED >> k & 1) sh[(q++) * NT + threadIdx.x] = v[k];
+        if (USED >> k & 1) {
+            if (own >> k & 1) sh[q * NT + threadIdx.x] = v[k];
+            ++q;
+        }
     __syncthreads();
     for (q = threadIdx.x >> 5; q < NQ; q += NT / 32) {
         const int k = used_slot(USED, q);
+        if (!(own >> k & 1)) continue;
         double r = sh[q * NT + lane];
 #pragma unroll
         for (int i = 1; i < NT / 32; ++i) r = slot_op(k, r, sh[q * NT + lane + 32 * i]);
@@ -372,20 +377,25 @@ __device__ __forceinline__ void finish_record(const double *t, const Finish &f, 
 // The totals of `blocks` records into t[0..P_WIDTH): thread i takes the records i, i + NT,
 // ..., all slots' loads in flight together (a warp a slot, one load after the other, waited
 // 10 us for the 1024 records of a 64^3 lattice), then the block's columns are summed as any
-// block's.  sh: used_count(USED) * NT doubles.
-template <unsigned USED, int NT, bool COMPACT>
-__device__ __forceinline__ void sum_records(const double *partial, int blocks, double *sh, double *t) {
+// block's.  own(b): the slots that record b holds; sh: used_count(USED) * NT doubles.
+template <unsigned USED> struct AllSlots {
+    __device__ unsigned operator()(unsigned) const { return USED; }
+};
+template <unsigned USED, int NT, bool COMPACT, class OWN = AllSlots<USED>>
+__device__ __forceinline__ void sum_records(const double *partial, int blocks, double *sh, double *t,
+                                            const OWN &own = OWN()) {
     constexpr int NQ = used_count(USED);
     double v[P_WIDTH];
 #pragma unroll
     for (int k = 0; k < P_WIDTH; ++k) v[k] = 0.0;  // every slot's sum or maximum starts at 0
 #pragma unroll 4
     for (int b = threadIdx.x; b < blocks; b += NT) {
+        const unsigned filled = own(b);
         int q = 0;
 #pragma unroll
         for (int k = 0; k < P_WIDTH; ++k)
             if (USED >> k & 1) {
-                v[k] = slot_op(k, v[k], __ldcg(&partial[COMPACT ? (int64_t)b * NQ + q : (int64_t)b * P_WIDTH + k]));
+                if (filled >> k & 1) v[k] = slot_op(k, v[k], __ldcg(&partial[COMPACT ? (int64_t)b * NQ + q : (int64_t)b * P_WIDTH + k]));
                 ++q;
             }
     }
@@ -396,13 +406,14 @@ __device__ __forceinline__ void sum_records(const double *partial, int blocks, d
 
 // The end of a reduction kernel of NT >= 128 threads a block: this block's record, and
 // in the last block the result.
-template <unsigned USED, int NT>
-__device__ __forceinline__ void reduce_and_finish(const double *v, double *partial, const Finish &f) {
+template <unsigned USED, int NT, class OWN = AllSlots<USED>>
+__device__ __forceinline__ void reduce_and_finish(const double *v, double *partial, const Finish &f,
+                                                  const OWN &own = OWN()) {
     static_assert(NT >= 128, "finish_record spreads over four warps");
     __shared__ double sh[used_count(USED) * NT], total[P_WIDTH];
     __shared__ int last;
     const unsigned block = blockIdx.x + gridDim.x * blockIdx.y, blocks = gridDim.x * gridDim.y;
-    block_record<USED, NT, true>(v, sh, partial + (int64_t)block * used_count(USED));
+    block_record<USED, NT, true>(v, sh, partial + (int64_t)block * used_count(USED), own(block));
     __threadfence();  // the record before the ticket
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -414,7 +425,7 @@ __device__ __forceinline__ void reduce_and_finish(const double *v, double *parti
     if (!last) return;
     __threadfence();
     if (f.ctl && (double)f.it >= f.ctl[0]) return;  // a deviation past the restore's stop: the result stays
-    sum_records<USED, NT, true>(partial, blocks, sh, total);
+    sum_records<USED, NT, true>(partial, blocks, sh, total, own);
     finish_record(total, f);
 }
 // the record alone (callers that sum the records in a launch of their own)
@@ -470,6 +481,16 @@ template <class T> __device__ __forceinline__ double lanes_sum(T x) { return (do
 template <> __device__ __forceinline__ double lanes_sum<f2>(f2 x) { return (double)x.v.x + (double)x.v.y; }
 __device__ __forceinline__ double lanes_max(double x, double m) { return fmax(m, x); }
 __device__ __forceinline__ float lanes_max(f2 x, float m) { return fmaxf(m, fmaxf(x.v.x, x.v.y)); }
+// the slots of a block's record: those of its direction, or the violations' (a block of 128
+// sites that summed all 12 spent a tenth of a small FP64 lattice's time on zeros)
+struct UnitSlots {
+    unsigned blocks;  // of a direction
+    __device__ unsigned operator()(unsigned b) const {
+        const unsigned mu = b / blocks;
+        return mu < 3 ? (1u << P_ESQ0 | 1u << P_BSQ0) << mu | 1u << P_EDB
+                      : 1u << P_GSQ | 1u << P_USQ | 1u << P_GMAX | 1u << P_GABS | 1u << P_UMAX;
+    }
+};
 template <int FMT, bool FULL>
 __global__ void __launch_bounds__(kThreadsObs, Fmt<FMT>::NA == 8 ? 2 : 4)
     k_obs_units(Geom g, const void *U, const void *E, double *partial, Finish fin) {
@@ -540,7 +561,7 @@ __global__ void __launch_bounds__(kThreadsObs, Fmt<FMT>::NA == 8 ? 2 : 4)
     v[P_GMAX] = gmax;
     v[P_GABS] = gabs;
     v[P_UMAX] = sqrt((double)umax);
-    reduce_and_finish<FULL ? kUsedAll : kUsedSample, kThreadsObs>(v, partial, fin);
+    reduce_and_finish<FULL ? kUsedAll : kUsedSample, kThreadsObs>(v, partial, fin, UnitSlots{gridDim.x});
 }
 
 // Gauss violation into the FP64 scratch G[a*V + s]; partial maxima as for observables.
