@@ -83,8 +83,11 @@ struct tcym_ensemble_s {
     tcym_ctx ctx = nullptr;
     std::vector<EnsMember> members;
     FmtGroup groups[4];
-    cudaStream_t st[4] = {nullptr, nullptr, nullptr, nullptr};
-    cudaEvent_t fork = nullptr, join[4] = {nullptr, nullptr, nullptr, nullptr};
+    // chains of a chunk's steps: one a format, and one for the FP32 members of each group
+    // stepped per site beside paired ones (chain_of)
+    static constexpr int kChains = 6;
+    cudaStream_t st[kChains] = {};
+    cudaEvent_t fork = nullptr, join[kChains] = {};
     double *partial = nullptr;
     size_t partial_records = 0;
     MemberReduce *d_reduce = nullptr;
@@ -284,10 +287,20 @@ static int upload_tables(tcym_ensemble ens) {
     return TCYM_OK;
 }
 
-template <int FMT> static cudaError_t launch_group_step(tcym_ensemble ens, int f, int k, cudaStream_t s) {
+// The members of a group step in two parts that do not wait for each other: the paired ones
+// (part 0), those stepped per site or by tiles (part 1).  One after the other on one chain,
+// a launch each, they took longer than one launch of a kernel for both kinds; us a step on GB300, one
+// launch / one chain / a chain each: an 8^3 and a 13^3 FP32 member SU(3) 13 / 25 / 13, SU(2) 8 / 15 / 9;
+// 4 each of 8^3, 13^3, 20^3, 33^3 SU(3) 66 / 69 / 63, SU(2) 24 / 30 / 23.
+static bool has_part(const FmtGroup &G, int part) { return part ? G.npaired < (int)G.idx.size() : G.npaired > 0; }
+static int chain_of(const FmtGroup &G, int f, int part) { return part == 1 && has_part(G, 0) ? 4 + f / 2 : f; }
+template <int FMT> static cudaError_t launch_group_step(tcym_ensemble ens, int f, int part, int k, cudaStream_t s) {
     using T = typename Fmt<FMT>::T;
     const FmtGroup &G = ens->groups[f];
     const Member<T> *table = static_cast<const Member<T> *>(G.d_members);
+    if (part == 1)
+        return LaunchBatch<FMT>::sites(table, G.npaired, (int)G.idx.size() - G.npaired, G.pair_blocks, G.total_blocks, k,
+                                       G.march_threads, G.march_smem, s);
     cudaError_t e = cudaSuccess;
     if constexpr (Fmt<FMT>::PAIRED) {
         if (G.tiled) {
@@ -298,9 +311,6 @@ template <int FMT> static cudaError_t launch_group_step(tcym_ensemble ens, int f
                     e = LaunchBatch<FMT>::step_uniform(table, c.m0, c.m1 - c.m0, c.item0, c.item1, k, c.coef, s);
         }
     }
-    const int n = (int)G.idx.size() - G.npaired;
-    if (e == cudaSuccess && n > 0)
-        e = LaunchBatch<FMT>::sites(table, G.npaired, n, G.pair_blocks, G.total_blocks, k, G.march_threads, G.march_smem, s);
     return e;
 }
 
@@ -368,16 +378,16 @@ static cudaError_t group_persistent(tcym_ensemble ens, int f, int nsteps, cudaSt
     return launch_group_persistent<FMT_SU3_F32>(ens, f, nsteps, s);
 }
 
-static cudaError_t group_step(tcym_ensemble ens, int f, int k, cudaStream_t s) {
+static cudaError_t group_step(tcym_ensemble ens, int f, int part, int k, cudaStream_t s) {
     switch (f) {
-        case FMT_SU2_F32: return launch_group_step<FMT_SU2_F32>(ens, f, k, s);
-        case FMT_SU2_F64: return launch_group_step<FMT_SU2_F64>(ens, f, k, s);
-        case FMT_SU3_F32: return launch_group_step<FMT_SU3_F32>(ens, f, k, s);
-        default: return launch_group_step<FMT_SU3_F64>(ens, f, k, s);
+        case FMT_SU2_F32: return launch_group_step<FMT_SU2_F32>(ens, f, part, k, s);
+        case FMT_SU2_F64: return launch_group_step<FMT_SU2_F64>(ens, f, part, k, s);
+        case FMT_SU3_F32: return launch_group_step<FMT_SU3_F32>(ens, f, part, k, s);
+        default: return launch_group_step<FMT_SU3_F64>(ens, f, part, k, s);
     }
 }
 
-// Captures nsteps steps of every format chain into one graph.
+// Captures nsteps steps of every chain into one graph.
 static int capture(tcym_ensemble ens, int nsteps) {
     if (ens->exec) {
         cudaGraphExecDestroy(ens->exec);
@@ -388,20 +398,22 @@ static int capture(tcym_ensemble ens, int nsteps) {
     if (r) return r;
     CKE(cudaStreamBeginCapture(ens->st[0], cudaStreamCaptureModeThreadLocal));
     cudaError_t err = cudaEventRecord(ens->fork, ens->st[0]);
-    for (int f = 0; f < 4 && err == cudaSuccess; ++f) {
-        if (ens->groups[f].idx.empty()) continue;
-        cudaStream_t s = ens->st[f];
-        if (f != 0) err = cudaStreamWaitEvent(s, ens->fork, 0);
-        if (persistent_format(ens, f)) {
-            if (err == cudaSuccess) err = group_persistent(ens, f, nsteps, s);
-        } else {
-            for (int k = 0; k < nsteps && err == cudaSuccess; ++k) err = group_step(ens, f, k, s);
+    for (int f = 0; f < 4; ++f)
+        for (int part = 0; part < 2 && err == cudaSuccess; ++part) {
+            if (!has_part(ens->groups[f], part)) continue;
+            const int c = chain_of(ens->groups[f], f, part);
+            cudaStream_t s = ens->st[c];
+            if (c != 0) err = cudaStreamWaitEvent(s, ens->fork, 0);
+            if (persistent_format(ens, f)) {
+                if (err == cudaSuccess) err = group_persistent(ens, f, nsteps, s);
+            } else {
+                for (int k = 0; k < nsteps && err == cudaSuccess; ++k) err = group_step(ens, f, part, k, s);
+            }
+            if (c != 0 && err == cudaSuccess) {
+                err = cudaEventRecord(ens->join[c], s);
+                if (err == cudaSuccess) err = cudaStreamWaitEvent(ens->st[0], ens->join[c], 0);
+            }
         }
-        if (f != 0 && err == cudaSuccess) {
-            err = cudaEventRecord(ens->join[f], s);
-            if (err == cudaSuccess) err = cudaStreamWaitEvent(ens->st[0], ens->join[f], 0);
-        }
-    }
     cudaError_t e2 = cudaStreamEndCapture(ens->st[0], &graph);
     if (err != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
@@ -427,10 +439,11 @@ extern "C" int tcym_ensemble_create(tcym_ctx ctx, tcym_ensemble *out) {
     // them (a request being prepared in the request loop) fills the SMs they leave
     int lo = 0, hi = 0;
     cudaError_t e = cudaDeviceGetStreamPriorityRange(&lo, &hi);
-    for (int i = 0; i < 4 && e == cudaSuccess; ++i)
+    for (int i = 0; i < tcym_ensemble_s::kChains && e == cudaSuccess; ++i)
         e = cudaStreamCreateWithPriority(&ens->st[i], cudaStreamNonBlocking, hi);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ens->fork, cudaEventDisableTiming);
-    for (int i = 0; i < 4 && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&ens->join[i], cudaEventDisableTiming);
+    for (int i = 0; i < tcym_ensemble_s::kChains && e == cudaSuccess; ++i)
+        e = cudaEventCreateWithFlags(&ens->join[i], cudaEventDisableTiming);
     if (e != cudaSuccess) {
         int r = fail(ctx, e, "tcym_ensemble_create");
         tcym_ensemble_destroy(ens);
@@ -443,7 +456,7 @@ extern "C" int tcym_ensemble_create(tcym_ctx ctx, tcym_ensemble *out) {
 extern "C" int tcym_ensemble_destroy(tcym_ensemble ens) {
     if (!ens) return TCYM_ERR_ARG;
     cudaSetDevice(ens->ctx->device);
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < tcym_ensemble_s::kChains; ++i)
         if (ens->st[i]) cudaStreamSynchronize(ens->st[i]);
     if (ens->exec) cudaGraphExecDestroy(ens->exec);
     for (int f = 0; f < 4; ++f) {
@@ -455,7 +468,7 @@ extern "C" int tcym_ensemble_destroy(tcym_ensemble ens) {
     cudaFree(ens->d_reduce);
     cudaFree(ens->d_out);
     if (ens->h_out) cudaFreeHost(ens->h_out);
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < tcym_ensemble_s::kChains; ++i) {
         if (ens->join[i]) cudaEventDestroy(ens->join[i]);
         if (ens->st[i]) cudaStreamDestroy(ens->st[i]);
     }
