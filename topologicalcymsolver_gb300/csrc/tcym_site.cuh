@@ -1077,15 +1077,18 @@ template <class F> TCYM_HD void site_reunitarize(const Geom &g, void *U, int64_t
 // projection moves it by increments of that size: with d0 = |r0|^2 - 1 and D = <r0, r1>,
 //   r0' = r0 (1 + d0)^(-1/2),  r1' = (r1 - D r0 / (1 + d0)) (1 + d1)^(-1/2),
 //   d1 = |r1|^2 - 1 - |D|^2 / (1 + d0)
-// (SU(2): the first line).  The deviations and the increments are formed as sums of a
-// value and its error (ExactSum), good to 3e-14 for deviations up to 3e-5, and added to
-// the entry with one rounding.  A pair with an entry whose sum lies within 1e-13 of the
-// middle of two FP32 numbers (about one warp in 200), or further off the group, or not
-// finite, takes the FP64 projection.  That one ran at the FP64 rate, 1184 us for SU(3) and
-// 336 us for SU(2) at 128^3 on GB300; this one takes 245 and 53 us, bound by FP32
-// arithmetic (SU(3)) and memory (SU(2); reading and writing the links: 89 and 30 us).
-constexpr float kProjDeviation = 3e-5f, kProjTie = 1e-13f;
-TCYM_HD bool beyond(f2 d, float t) { return !(fabsf(d.v.x) <= t && fabsf(d.v.y) <= t); }
+// (SU(2): the first line), D a deviation against sum_k |r0_k| |r1_k|.  The deviations and the
+// increments are formed as sums of a value and its error (ExactSum), for deviations up to
+// 3e-5 good to 3e-14 of the numbers summed (the entry; in row 1 the entry of r0 times that
+// sum too), and added to the entry with one rounding.  A pair with an entry whose sum lies
+// within 1e-13 of them from the middle of two FP32 numbers (about one warp in 100; the small
+// entries of links near the identity no more often than others), or further off the group, or
+// not finite, takes the FP64 projection.  That one ran at the FP64 rate, 1184 us for SU(3) and
+// 336 us for SU(2) at 128^3 on GB300; this one takes 207 and 52 us, bound by FP32 arithmetic
+// (SU(3)) and memory (SU(2); reading and writing the links: 89 and 30 us).  (A bound of 1e-13
+// whatever the entry sent fields of width 1e-2 and less there: 778 to 1200 and 69 to 339 us.)
+constexpr float kProjDeviation = 3e-5f, kProjTie = 1e-13f, kProjLeast = 1e-28f;
+TCYM_HD bool beyond(f2 d, f2 t) { return !(fabsf(d.v.x) <= t.v.x && fabsf(d.v.y) <= t.v.y); }
 // a value and its error
 struct F2E {
     f2 s, e;
@@ -1100,22 +1103,25 @@ TCYM_HD F2E split(const ExactSum<f2> &x) {
 TCYM_HD F2E inv_root_m1(F2E d) {
     return F2E{f2(-0.5) * d.s, fma(d.s * d.s, fma(f2(-0.3125), d.s, f2(0.375)), f2(-0.5) * d.e)};
 }
-// x + (i.s + i.e) rounded once; tie: the exact sum lies within kProjTie of a rounding
-// boundary of some lane (half the distance from the result to its neighbour on that side)
-TCYM_HD f2 add_once(f2 x, F2E i, bool &tie) {
+// x + (i.s + i.e) rounded once; tie: the exact sum may lie on the other side of a rounding
+// boundary in some lane, being within kProjTie * scale of one (half the distance from the
+// result to its neighbour on that side).  scale: the size of the numbers that the increment's
+// error is relative to; 0 where it is exactly zero.  (Below kProjLeast products underflow.)
+TCYM_HD f2 add_once(f2 x, F2E i, f2 scale, bool &tie) {
     const f2 t = x + i.s, b = t - x;
     const f2 err = ((x - (t - b)) + (i.s - b)) + i.e;  // the exact sum is t + err
     const f2 r = t + err;
     const f2 left = err - (r - t);  // the exact sum is r + left
-    auto near_tie = [](float r, float left) {
-        if (left == 0.0f) return false;
+    auto near_tie = [](float r, float left, float scale) {
+        if (scale == 0.0f) return false;
         // the neighbour of r on the side of the remainder, and half the way there
         const float n = nextafterf(r, left > 0.0f ? INFINITY : -INFINITY);
-        return !(fabsf(fabsf(0.5f * (n - r)) - fabsf(left)) > kProjTie);
+        return !(scale >= kProjLeast && fabsf(fabsf(0.5f * (n - r)) - fabsf(left)) > kProjTie * scale);
     };
-    tie |= near_tie(r.v.x, left.v.x) || near_tie(r.v.y, left.v.y);
+    tie |= near_tie(r.v.x, left.v.x, scale.v.x) || near_tie(r.v.y, left.v.y, scale.v.y);
     return r;
 }
+TCYM_HD f2 abs_f2(f2 x) { return f2(fabsf(x.v.x), fabsf(x.v.y)); }
 template <class F> TCYM_HD void pair_reunitarize_fp64(void *U, int64_t V, int mu, int64_t p) {
     using G64 = Group64<F>;
     const int64_t Vh = pair_sites(V);
@@ -1139,18 +1145,21 @@ template <class F> TCYM_HD void pair_reunitarize(void *U, int64_t V, int mu, int
 #pragma unroll
         for (int k = 0; k < 4; ++k) n.mul(u.q[k], u.q[k]);
         const F2E d = split(n);
-        slow = beyond(d.s, kProjDeviation);
+        slow = beyond(d.s, f2(kProjDeviation));
         const F2E h = inv_root_m1(d);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const ExactSum<f2> i = scaled(h, u.q[k]);
-            u.q[k] = add_once(u.q[k], F2E{i.s, i.e}, slow);
+            u.q[k] = add_once(u.q[k], F2E{i.s, i.e}, abs_f2(u.q[k]), slow);
         }
     } else {
         ExactSum<f2> n0(f2(-1.0)), n1(f2(-1.0)), dr(f2(0.0)), di(f2(0.0));
+        auto size = [](const cx<f2> &z) { return abs_f2(z.re) + abs_f2(z.im); };
+        f2 S(0.0);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const cx<f2> a = u.m[0][k], b = u.m[1][k];
+            S = fma(size(a), size(b), S);
             n0.mul(a.re, a.re); n0.mul(a.im, a.im);
             n1.mul(b.re, b.re); n1.mul(b.im, b.im);
             dr.mul(a.re, b.re); dr.mul(a.im, b.im);
@@ -1159,8 +1168,8 @@ template <class F> TCYM_HD void pair_reunitarize(void *U, int64_t V, int mu, int
         const F2E d0 = split(n0), Dr = split(dr), Di = split(di);
         n1.add(-fma(Dr.s, Dr.s, Di.s * Di.s));  // |D|^2, at most 2e-9, to 2e-16
         const F2E d1 = split(n1);
-        slow = beyond(d0.s, kProjDeviation) || beyond(d1.s, kProjDeviation) || beyond(Dr.s, kProjDeviation) ||
-               beyond(Di.s, kProjDeviation);
+        const f2 t(kProjDeviation);
+        slow = beyond(d0.s, t) || beyond(d1.s, t) || beyond(Dr.s, t * S) || beyond(Di.s, t * S);
         const F2E h0 = inv_root_m1(d0), h1 = inv_root_m1(d1);
         // c = D (1 + h1) / (1 + d0)
         const f2 w = h1.s - d0.s;
@@ -1173,9 +1182,12 @@ template <class F> TCYM_HD void pair_reunitarize(void *U, int64_t V, int mu, int
             ii.mul(-cr.s, a.im); ii.mul(-ci.s, a.re);
             ir.e = fma(-cr.e, a.re, fma(ci.e, a.im, ir.e));
             ii.e = fma(-cr.e, a.im, fma(-ci.e, a.re, ii.e));
-            u.m[1][k] = cx<f2>{add_once(b.re, F2E{ir.s, ir.e}, slow), add_once(b.im, F2E{ii.s, ii.e}, slow)};
+            const f2 z = size(a) * S;
+            u.m[1][k] = cx<f2>{add_once(b.re, F2E{ir.s, ir.e}, abs_f2(b.re) + z, slow),
+                               add_once(b.im, F2E{ii.s, ii.e}, abs_f2(b.im) + z, slow)};
             const ExactSum<f2> jr = scaled(h0, a.re), ji = scaled(h0, a.im);
-            u.m[0][k] = cx<f2>{add_once(a.re, F2E{jr.s, jr.e}, slow), add_once(a.im, F2E{ji.s, ji.e}, slow)};
+            u.m[0][k] = cx<f2>{add_once(a.re, F2E{jr.s, jr.e}, abs_f2(a.re), slow),
+                               add_once(a.im, F2E{ji.s, ji.e}, abs_f2(a.im), slow)};
         }
     }
     if (slow) pair_reunitarize_fp64<F>(U, V, mu, p);
