@@ -265,14 +265,15 @@ inline double march_first(int S) { return 454 * march_warps(2 * S); }
 inline MarchTile march_tile(const Geom &g, double sms, bool alone, double *least = nullptr) {
     MarchTile best{};
     double cost = 0;
-    for (int kx = (g.nx + 15) / 16; kx <= g.nx; ++kx) {
-        const int tx = (g.nx + kx - 1) / kx;
+    for (int tx = g.nx < 16 ? g.nx : 16; tx > 0; --tx) {
+        const int nx = (g.nx + tx - 1) / tx;
+        if ((g.nx + nx - 1) / nx != tx) continue;  // as many smaller tiles do
         if (tx < 4 && best.tx) break;
-        for (int ky = 1; ky <= g.ny; ++ky) {
-            const int ty = (g.ny + ky - 1) / ky;
-            if (tx * ty > kMarchSites) continue;
+        const int most = kMarchSites / tx;
+        for (int ty = g.ny < most ? g.ny : most; ty > 0; --ty) {
+            const int ny = (g.ny + ty - 1) / ty;
+            if ((g.ny + ny - 1) / ny != ty) continue;
             if (tx * ty < 16 && best.tx) break;
-            const int nx = (g.nx + tx - 1) / tx, ny = (g.ny + ty - 1) / ty;
             const int halo = (tx == g.nx ? 0 : ty) + (ty == g.ny ? 0 : tx), S = tx * ty;
             const double plane = march_plane(S, halo), first = march_first(S);
             double planes = 0, firsts = 0;  // of all tiles, ragged ones as they are
