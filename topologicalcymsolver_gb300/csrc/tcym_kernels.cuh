@@ -853,9 +853,9 @@ template <int FMT> struct Launch {
         FlowCoefT<T> c;
         for (int i = 0; i < 3; ++i) { c.fc[i] = (T)fc[i]; c.cn[i] = (T)cn[i]; c.uc[i] = (T)uc[i]; }
         if constexpr (F::PAIRED) {
-            if (g.nz % 4 == 0) {
-                const dim3 grid((unsigned)grid_for(g.nx / 2, kCbX), (unsigned)grid_for(g.ny, kCbY),
-                                (unsigned)grid_for(g.nz / 2, kCbZ));
+            const dim3 grid((unsigned)grid_for(g.nx / 2, kCbX), (unsigned)grid_for(g.ny, kCbY),
+                            (unsigned)grid_for(g.nz / 2, kCbZ));
+            if (g.nz % 4 == 0 && grid.y <= 65535 && grid.z <= 65535) {  // the most of a launch; beyond, per site
                 k_flow_cb_pair<FMT><<<grid, kThreadsPair, 0, st>>>(g, U, parity, mu, c);
                 return cudaGetLastError();
             }
