@@ -53,6 +53,14 @@ def test_violation_as_in_fp64(na, width, cancel):
     assert (np.abs(o[:, 2] - np.abs(g).max((1, 2))) <= eps).all()
 
 
+def test_zero_fields_of_broken_links():
+    """0 * infinity in E.B is NaN, as in FP64; zeros alone are zero."""
+    z, b = np.zeros((2, 8, 2), np.float32), np.ones((2, 8, 2), np.float32)
+    b[1, 4, 0] = np.inf
+    o = hc.pair_sums(z, -z, b)
+    assert o[0].tolist() == [0, 0] and o[1, 0] == 0 and np.isnan(o[1, 1])
+
+
 def test_infinite_and_nan_violation():
     """As FP64: maxima drop NaN, squares keep it."""
     t = np.ones((4, 8, 1, 2), np.float32)

@@ -5,6 +5,8 @@
 // arithmetic of the device path.
 #pragma once
 
+#include <string.h>
+
 #include <type_traits>
 
 #include "tcym_layout.cuh"
@@ -730,9 +732,21 @@ TCYM_HD T unit_sample(const Geom &g, const void *U, const void *E, int64_t i, in
 // The sums of all observables over a thread's units, in FP64 (FieldSums, ViolationSums).
 // Pairs sum in FP32 with the errors kept (WideSum): GB300 converts to FP64 and adds there at
 // 1/64 of the FP32 rate.  That is exact while products neither overflow nor lose their errors, to
-// 1e-45 each, below FP32's range: where the result says otherwise (exact()), or is zero, the
-// thread sums again in FP64 (add64).
+// 1e-45 each, below FP32's range: where the result says otherwise (exact()) the thread sums
+// again in FP64 (add64).
 TCYM_HD bool exact_range(double squares) { return squares >= 1e-28 && squares <= 1e30; }
+// the bits of both lanes but their signs: 0 for zeros alone
+TCYM_HD unsigned nonzero_bits(f2 x) {
+    unsigned a, b;
+#ifdef __CUDA_ARCH__
+    a = __float_as_uint(x.v.x);
+    b = __float_as_uint(x.v.y);
+#else
+    memcpy(&a, &x.v.x, sizeof a);
+    memcpy(&b, &x.v.y, sizeof b);
+#endif
+    return (a | b) & 0x7fffffffu;
+}
 // sums of E_mu^2 and of E_mu.B_mu, from unit_clover's fields
 template <class T, int NA> struct FieldSums;
 template <int NA> struct FieldSums<double, NA> {
@@ -752,16 +766,19 @@ template <int NA> struct FieldSums<double, NA> {
 };
 template <int NA> struct FieldSums<f2, NA> {
     WideSum<f2> s{f2(0.0)}, d{f2(0.0)};
+    unsigned bits = 0;       // of the fields: a lattice of zeros is summed once
     double sq = 0, dot = 0;  // the results, of exact() or add64
     TCYM_HD void add(const f2 *e, const f2 *et, const f2 *b) {
 #pragma unroll
         for (int a = 0; a < NA; ++a) {
+            bits |= nonzero_bits(e[a]) | nonzero_bits(et[a]);
             s.mul(e[a], e[a]);
             d.mul(e[a], b[a]);
             d.mul(et[a], b[a]);
         }
     }
     TCYM_HD bool exact() {
+        if (bits == 0) return d.s.v.x == 0.0f && d.s.v.y == 0.0f;  // (an infinite or NaN b shows)
         const double x = lane64(s, 0), y = lane64(s, 1), u = lane64(d, 0), v = lane64(d, 1);
         if (!(exact_range(x) && exact_range(y) && fabs(u) <= 1e30 && fabs(v) <= 1e30)) return false;
         sq = x + y;
@@ -834,6 +851,7 @@ template <int NA> struct ViolationSums<f2, NA> {
         float h, l, c;
     };
     WideSum<f2> s{f2(0.0)};
+    unsigned bits = 0;
     Wide up{0, 0, 0}, down{0, 0, 0};
     double sq = 0, most = 0, mag = 0;
     static TCYM_HD void larger(Wide x, Wide &m) {
@@ -845,6 +863,7 @@ template <int NA> struct ViolationSums<f2, NA> {
         for (int a = 0; a < NA; ++a) {
             f2 h = g[a].s;
             const f2 l = WideSum<f2>::two_sum(h, g[a].e);
+            bits |= nonzero_bits(h) | nonzero_bits(l) | nonzero_bits(g[a].c);
             s.mul(h, h);
             s.mul(h + h, l);
             s.c = fma(l, l, s.c);
@@ -857,6 +876,7 @@ template <int NA> struct ViolationSums<f2, NA> {
         }
     }
     TCYM_HD bool exact() {
+        if (bits == 0) return true;
         const double x = lane64(s, 0), y = lane64(s, 1);
         if (!(exact_range(x) && exact_range(y))) return false;
         sq = x + y;
