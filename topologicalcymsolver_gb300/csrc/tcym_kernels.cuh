@@ -1,10 +1,10 @@
 // CUDA kernels and their launchers, one instantiation per storage format
 // (tcym_kern_su{2,3}_f{32,64}*.cu).
 //
-// Every kernel is one thread per site (or per link for the checkerboard
-// flow), grid-strided over the lattice.  Reductions are deterministic: each
-// block writes one partial record (FP64) and a single-block finaliser sums the
-// partials in block order, so a result never depends on scheduling.
+// A thread takes a site, a site pair (FP32 formats with even nz), one of its directions or
+// one of its links (the FP64 step: tasks of a tile, tcym_march.cuh).  Reductions are
+// deterministic: each block writes a partial record (FP64) and the last block to finish sums
+// the records in block order, so a result never depends on scheduling.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -18,7 +18,7 @@ namespace tcym {
 enum : int {
     P_ESQ0 = 0, P_BSQ0 = 3, P_GSQ = 6, P_USQ = 7, P_EDB = 8, P_GMAX = 9, P_GABS = 10, P_UMAX = 11, P_WIDTH = 12
 };
-// device result block (doubles), written by finalize_obs
+// device result block (doubles), written by finish_record
 enum : int {
     R_ESQ0 = 0, R_BSQ0 = 3, R_GMAX = 6, R_GRMS = 7, R_GABS = 8, R_UMAX = 9, R_URMS = 10, R_EDB = 11,
     R_NCS = 12, R_NCS_COMP = 13, R_NONFINITE = 14,
@@ -258,18 +258,6 @@ __global__ void __launch_bounds__(kThreadsPair, Fmt<FMT>::NA == 8 ? 4 : 8)
     else pair_link_flow<Fmt<FMT>, false>(g, U, mu, c.fc, c.cn, c.uc, p);
 }
 
-// block reduction helpers (FP64)
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-__device__ __forceinline__ double warp_max(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
 // Reductions.  On GB300 a warp's FP64 add takes 16 cycles of its SM's one FP64 unit, so
 // a block's record (up to 12 values) is summed with as few as the tree allows: every
 // thread's values go to shared memory, a warp takes a value, adds its 256/32 columns and
@@ -469,12 +457,11 @@ template <int FMT> constexpr bool unit_pairs() { return Fmt<FMT>::PAIRED; }
 // thread takes a unit and a direction (blockIdx.y; FULL: 3 is the violations), so a small
 // lattice has three or four times its units in threads.  The sample's sums over components
 // run in the storage's precision, those of all observables in FP64 (FieldSums, ViolationSums), and
-// everything across units in FP64.  SU(3) FP64 is bound by its multiply-adds (0.87 ms at 48^3), the others wait for L2.
-// All observables, with the call, on GB300, one thread a site or pair / by unit and direction:
-// SU(3) FP64 16^3 370 / 74 us, 48^3 1067 / 964; SU(2) FP64 16^3 87 / 37; SU(3) FP32 16^3
-// 40 / 30, 64^3 130 / 114, 128^3 790 / 702; SU(2) FP32 96^3 and 128^3 126 and 213 / 124 and 260
-// (there a thread that shares a pair's links between directions would be faster).  SU(3) by
-// two blocks of 255 registers: three of 168 spill (FP32 64^3 126 us, FP64 48^3 997).
+// everything across units in FP64.  SU(3) FP64 is bound by its multiply-adds (0.87 ms at 48^3),
+// the others wait for L2.  All observables, with the call, on GB300, one thread a site / by unit
+// and direction: SU(3) FP64 16^3 375 / 75 us, 48^3 1074 / 949; SU(2) FP64 16^3 91 / 38, 48^3 224 /
+// 199; SU(3) FP32 16^3 86 / 30, 64^3 412 / 145, 128^3 2792 / 973; SU(2) FP32 64^3 147 / 74, 128^3
+// 640 / 309.  SU(3) by two blocks of 255 registers: three of 168 spill (FP64 48^3 997 us).
 constexpr int kThreadsObs = 128;
 // a unit's contribution to its direction's sums
 template <class T> __device__ __forceinline__ double lanes_sum(T x) { return (double)x; }
@@ -824,7 +811,8 @@ template <int FMT> struct Launch {
         return cudaGetLastError();
     }
     // Lattices whose paired step spreads a pair over three threads (k_step_split): up to
-    // about a wave of its blocks.  Per step by k_step_pair / k_step_split on GB300: SU(3)
+    // about a wave of its blocks on GB300's 152 multiprocessors (5 of 32 SU(3) pairs each, 8 of
+    // SU(2)'s).  Per step by k_step_pair / k_step_split on GB300: SU(3)
     // 16^3 13.4 / 8.2 us, 24^3 13.4 / 8.3, 32^3 14.4 / 12.3, 48^3 23.7 / 26.6; SU(2) 16^3 to
     // 32^3 8.2 / 6.2 us, 48^3 10.3 / 10.3.
     static bool split_step(const Geom &g) { return (g.V >> 1) <= (F::NA == 8 ? 25000 : 33000); }

@@ -6,14 +6,18 @@
 // The force on U_mu(x) sums, over nu != mu, the plaquette above the link (corner x)
 // minus the one below it (corner x - nu) carried to x.  With P_{mu nu}(y) the
 // plaquette that starts and ends at y, the loop below the link, run from x, is
-// U_nu^dag(x-nu) P_{mu nu}(x-nu) U_nu(x-nu), and proj(V^dag P V) = Ad(V^dag) proj(P)
+// U_nu^-1(x-nu) P_{mu nu}(x-nu) U_nu(x-nu), and proj(V^-1 P V) = Ad(V^-1) proj(P)
 // for a group element V.  So with p_{mu nu}(y) = proj(P_{mu nu}(y)) the reference's
 // bracket (Dynamics.cpp:184-188) is
-//   f_mu(x) = sum_nu c_nu [ p_{mu nu}(x) - Ad(U_nu^dag(x-nu)) p_{mu nu}(x-nu) ],
+//   f_mu(x) = sum_nu c_nu [ p_{mu nu}(x) - Ad(U_nu^-1(x-nu)) p_{mu nu}(x-nu) ],
 // and a step needs three plaquettes a site, each projected once and used by four links,
 // and six rotations of an algebra vector, where the staple form takes three plaquettes,
 // six lower staples and three more projections a site.  FP64 is bound by its
-// multiply-adds (1.2 TFLOP/s on GB300): SU(3) about 2300 a site against 3200.
+// multiply-adds (1.2 TFLOP/s on GB300): SU(3) about 2650 a site against 3230.
+// Links may be a little off the group (copied from FP32 storage, loaded with few digits).  For
+// SU(2) the identity holds for any quaternion V.  For SU(3) it is off by V's deviation eps (E
+// by 0.6 eps of a dt = 0.05 step, where staples whose third rows follow from the first two are
+// off by 1.2 eps), so plaquettes are whole products and Ad(V^-1) is taken as V^dagger p V.
 //
 // A block owns a tx x ty tile of a z-plane and walks zl planes up in z.  Per plane, phase
 // 1 forms the projections of the tile and of the row and column just below it in x and
