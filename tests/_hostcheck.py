@@ -30,6 +30,7 @@ def load():
                               ctypes.c_double, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int, ctypes.c_int,
                               ctypes.c_int]
         L.hc_march.argtypes = [ctypes.c_int, ip, _vp, _vp, _vp, ctypes.c_double] + [ctypes.c_int] * 4
+        L.hc_cb_tile.argtypes = [ip, ctypes.c_int, ip]
         L.hc_by_sites.argtypes = [ip, ctypes.c_int]
         L.hc_flow_cb.argtypes = [ctypes.c_int, ip, _vp, ctypes.c_double, ctypes.c_int]
         L.hc_observables.argtypes = [ctypes.c_int, ip, _vp, _vp, ctypes.c_int, _vp]
@@ -177,6 +178,12 @@ class HostLattice:
 def by_sites(shape, sms=152):
     """Does the FP64 step of a lattice alone on `sms` multiprocessors go by sites (and not by tiles)?"""
     return bool(load().hc_by_sites((ctypes.c_int * 3)(*shape), sms))
+
+
+def cb_tile(shape, nc):
+    """The checkerboard tiles' shape in pairs of a parity, rows and planes, or None where FP32 goes per site."""
+    out = (ctypes.c_int * 3)()
+    return tuple(out) if load().hc_cb_tile((ctypes.c_int * 3)(*shape), nc == 3, out) else None
 
 
 def pair_sums(e, et, b, count=1):

@@ -130,7 +130,7 @@ template <int FMT> struct H {
     static void flow_cb(const Geom &g, void *U, double dtau, int nsweeps) {
         const T fc[3] = {T(-2), T(-2), T(-2)}, cn[3] = {T(1), T(1), T(1)}, uc[3] = {T(-dtau), T(-dtau), T(-dtau)};
         if constexpr (F::PAIRED) {
-            if (g.nz % 4 == 0) {  // pairs of one parity, as the device takes them
+            if (g.nz % 4 == 0) {  // pairs of one parity, as the device takes them (small SU(2) lattices apart)
                 const int64_t plane = (int64_t)g.nx * g.ny, Vh = g.V >> 1;
                 for (int k = 0; k < 6 * nsweeps; ++k)
                     for (int64_t p = 0; p < Vh; ++p) {
@@ -417,6 +417,14 @@ int hc_march(int fmt, const int *n, const void *Uin, void *Uout, void *E, double
 }
 // does the FP64 step of a lattice alone on `sms` multiprocessors go by sites?
 int hc_by_sites(const int *n, int sms) { return step_tile(geom(n), sms).tx == 0; }
+// the checkerboard tiles of a lattice, their shape in out[3]; returns whether an FP32 lattice
+// goes by pairs
+int hc_cb_tile(const int *n, int su3, int *out) {
+    Geom g = geom(n);
+    const CbTile t = cb_tile(g);
+    out[0] = 1 << t.lx; out[1] = 1 << t.ly; out[2] = 1 << t.lz;
+    return cb_pairs(g, su3 != 0);
+}
 int hc_flow_cb(int fmt, const int *n, void *U, double dtau, int nsweeps) {
     Geom g = geom(n);
     HC_DISPATCH(fmt, HH::flow_cb(g, U, dtau, nsweeps));

@@ -238,23 +238,23 @@ __global__ void __launch_bounds__(threads_for<FMT>(), min_blocks_for<FMT>()) k_f
     link_flow<Fmt<FMT>>(g, U, mu, c.fc, c.cn, c.uc, s);
 }
 // FP32 pair storage with nz / 2 even (a pair's sites have one parity): a thread per pair,
-// a block a tile of 8 pairs of the parity x 4 rows x 4 planes.  It waits for links from
+// a block a tile of 8 pairs of the parity x 4 rows x 4 planes, or of other powers of two where
+// that leaves fewer threads idle (cb_tile).  It waits for links from
 // L2 (13 of them a thread), of which the tile finds its neighbours' in L1.  A sweep (six
 // sub-sweeps) on GB300: SU(2) 96^3 149 us per site (one lane of every pair vector, twice the
 // sectors), 92 us by pairs in index order, 76 us by tiles; SU(3) 96^3 522 / 258 / 256 us.
 // (16 x 4 x 2: 75 and 250 us, but half idle at nx = 16.)
-constexpr int kCbX = 8, kCbY = 4, kCbZ = 4;
-static_assert(kCbX * kCbY * kCbZ == kThreadsPair, "a block is a tile");
 template <int FMT>
 __global__ void __launch_bounds__(kThreadsPair, Fmt<FMT>::NA == 8 ? 4 : 8)
-    k_flow_cb_pair(Geom g, void *U, int parity, int mu, FlowCoefT<float> c) {
+    k_flow_cb_pair(Geom g, void *U, int parity, int mu, FlowCoefT<float> c, CbTile t) {
     const int i = threadIdx.x, nzh = g.nz >> 1;
-    const int xh = blockIdx.x * kCbX + i % kCbX, y = blockIdx.y * kCbY + i / kCbX % kCbY;
-    const int z0 = blockIdx.z * kCbZ, z = z0 + i / (kCbX * kCbY);
+    const int xh = (blockIdx.x << t.lx) + (i & ((1 << t.lx) - 1));
+    const int y = (blockIdx.y << t.ly) + (i >> t.lx & ((1 << t.ly) - 1));
+    const int z0 = blockIdx.z << t.lz, z = z0 + (i >> (t.lx + t.ly));
     if (2 * xh >= g.nx || y >= g.ny || z >= nzh) return;
     const int64_t p = 2 * xh + ((y + z + parity) & 1) + (int64_t)g.nx * (y + (int64_t)g.ny * z);
     // block-uniform: does the block hold a plane next to the seam?
-    if (z0 == 0 || z0 + kCbZ >= nzh) pair_link_flow<Fmt<FMT>, true>(g, U, mu, c.fc, c.cn, c.uc, p);
+    if (z0 == 0 || z0 + (1 << t.lz) >= nzh) pair_link_flow<Fmt<FMT>, true>(g, U, mu, c.fc, c.cn, c.uc, p);
     else pair_link_flow<Fmt<FMT>, false>(g, U, mu, c.fc, c.cn, c.uc, p);
 }
 
@@ -841,10 +841,11 @@ template <int FMT> struct Launch {
         FlowCoefT<T> c;
         for (int i = 0; i < 3; ++i) { c.fc[i] = (T)fc[i]; c.cn[i] = (T)cn[i]; c.uc[i] = (T)uc[i]; }
         if constexpr (F::PAIRED) {
-            const dim3 grid((unsigned)grid_for(g.nx / 2, kCbX), (unsigned)grid_for(g.ny, kCbY),
-                            (unsigned)grid_for(g.nz / 2, kCbZ));
-            if (g.nz % 4 == 0 && grid.y <= 65535 && grid.z <= 65535) {  // the most of a launch; beyond, per site
-                k_flow_cb_pair<FMT><<<grid, kThreadsPair, 0, st>>>(g, U, parity, mu, c);
+            if (cb_pairs(g, F::NA == 8)) {
+                const CbTile t = cb_tile(g);
+                const dim3 grid((unsigned)grid_for(g.nx / 2, 1 << t.lx), (unsigned)grid_for(g.ny, 1 << t.ly),
+                                (unsigned)grid_for(g.nz / 2, 1 << t.lz));
+                k_flow_cb_pair<FMT><<<grid, kThreadsPair, 0, st>>>(g, U, parity, mu, c, t);
                 return cudaGetLastError();
             }
         }

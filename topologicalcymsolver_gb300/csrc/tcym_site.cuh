@@ -5,6 +5,7 @@
 // arithmetic of the device path.
 #pragma once
 
+#include <stdlib.h>
 #include <string.h>
 
 #include <type_traits>
@@ -380,6 +381,47 @@ TCYM_HD void pair_link_flow(const Geom &g, void *U, int mu, const float (&fc)[3]
 #pragma unroll
     for (int a = 0; a < F::NA; ++a) f[a] = f[a] * fm;
     F::store2(U, Vh, mu, p, G2::iexp_mul(f2(sel3(uc, mu)), f, u));
+}
+
+// How the blocks of 128 threads cover the pairs of one parity in a checkerboard sub-sweep of
+// pairs: 2^lx of them along x, 2^ly rows, 2^lz planes; lx + ly + lz = 7.
+struct CbTile {
+    int lx, ly, lz;
+};
+inline int64_t cb_blocks(const Geom &g, const CbTile &t) {
+    auto n = [](int64_t sites, int l) { return (sites + (1 << l) - 1) >> l; };
+    return n(g.nx / 2, t.lx) * n(g.ny, t.ly) * n(g.nz / 2, t.lz);
+}
+// 8 x 4 x 4, unless a shape no narrower than the lattice's rows or 8 needs a third fewer blocks
+// (thin lattices: 2 x 256 x 256 took 209 us a sweep of SU(3) by 8 x 4 x 4, an eighth of whose
+// threads had a pair, 108 per site); of these the fewest blocks, then the nearest to it.
+inline CbTile cb_tile(const Geom &g) {
+    CbTile best{3, 2, 2};
+    const int64_t usual = cb_blocks(g, best);
+    int64_t blocks = usual;
+    int far = 0;
+    for (int lx = 0; lx <= 7; ++lx) {
+        if (lx < 3 && (1 << lx) < g.nx / 2) continue;
+        for (int ly = 0; lx + ly <= 7; ++ly) {
+            const CbTile t{lx, ly, 7 - lx - ly};
+            const int64_t n = cb_blocks(g, t);
+            const int d = abs(lx - 3) + abs(ly - 2) + abs(t.lz - 2);
+            if (3 * n > 2 * usual || n > blocks || (n == blocks && d >= far)) continue;
+            best = t;
+            blocks = n;
+            far = d;
+        }
+    }
+    return best;
+}
+// Does the checkerboard flow of an FP32 lattice go by pairs?  Where they have one parity (nz / 2
+// even) and a launch's grid holds the tiles (65535 along y and z); of SU(2) from 4096 sites
+// on: below, a sub-sweep is one thread's latency, and a pair's sines take their lanes one after the
+// other (12^3 31 us a sweep per site, 37 by pairs; 20^3 37 and 37).
+inline bool cb_pairs(const Geom &g, bool su3) {
+    if (g.nz % 4 != 0 || (!su3 && g.V <= 4096)) return false;
+    const CbTile t = cb_tile(g);
+    return (g.ny >> t.ly) < 65535 && (g.nz / 2 >> t.lz) < 65535;
 }
 
 // ----------------------------------------------------------------- observables
