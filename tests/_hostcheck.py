@@ -31,7 +31,7 @@ def load():
                               ctypes.c_int]
         L.hc_march.argtypes = [ctypes.c_int, ip, _vp, _vp, _vp, ctypes.c_double] + [ctypes.c_int] * 4
         L.hc_cb_tile.argtypes = [ip, ctypes.c_int, ip]
-        L.hc_by_sites.argtypes = [ip, ctypes.c_int]
+        L.hc_by_sites.argtypes = [ip, ctypes.c_int, ctypes.c_int, ctypes.c_int]
         L.hc_flow_cb.argtypes = [ctypes.c_int, ip, _vp, ctypes.c_double, ctypes.c_int]
         L.hc_observables.argtypes = [ctypes.c_int, ip, _vp, _vp, ctypes.c_int, _vp]
         L.hc_edotb_pair.argtypes = [ctypes.c_int, ip, _vp, _vp, _vp]
@@ -175,9 +175,10 @@ class HostLattice:
                            _p(self.E))
 
 
-def by_sites(shape, sms=152):
-    """Does the FP64 step of a lattice alone on `sms` multiprocessors go by sites (and not by tiles)?"""
-    return bool(load().hc_by_sites((ctypes.c_int * 3)(*shape), sms))
+def by_sites(shape, sms=152, links=True, nc=3):
+    """Does the FP64 step (or the E update alone) of a lattice alone on `sms` multiprocessors go by sites (and not by
+    tiles)?"""
+    return bool(load().hc_by_sites((ctypes.c_int * 3)(*shape), sms, nc == 3, links))
 
 
 def cb_tile(shape, nc):

@@ -15,6 +15,13 @@ def test_rule():
     assert all(hc.by_sites(n) for n in SITES) and not any(hc.by_sites(n) for n in TILES)
 
 
+def test_rule_of_the_field_update():
+    """Without the exponential sites win a little more."""
+    assert all(hc.by_sites(n, links=False) for n in [*SITES, (32, 32, 32)])
+    assert not any(hc.by_sites(n, links=False) for n in [(8, 8, 8), (28, 28, 28), (48, 48, 48)])
+    assert hc.by_sites((36, 36, 36), links=False, nc=2) and not hc.by_sites((36, 36, 36), links=False, nc=3)
+
+
 def state(P, nc, shape):
     V = int(np.prod(shape))
     U, E = np.zeros((V, 3, hc.NM[nc])), np.zeros((V, 3, hc.NA[nc]))
@@ -38,7 +45,7 @@ def test_host_by_sites(oracle_port, nc, shape):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("nc", [2, 3])
-@pytest.mark.parametrize("shape", [*SITES, TILES[1]])
+@pytest.mark.parametrize("shape", [*SITES, TILES[1], (32, 32, 32)])  # the last: E alone by sites
 def test_gpu_routes(ctx, oracle_port, nc, shape):
     """Leapfrog, Langevin, the flow and the two half updates on each route, 1e-12 after ten steps."""
     import topologicalcymsolver_gb300 as tcym

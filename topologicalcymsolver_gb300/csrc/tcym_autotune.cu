@@ -130,9 +130,9 @@ const Tile &tcym_lattice_tile_of(tcym_lattice lat) {
     return lat->tile;
 }
 
-const MarchTile &tcym_lattice_march_of(tcym_lattice lat) {
-    MarchTile &t = lat->march;
-    if (t.threads == 0) t = step_tile(lat->g, lat->ctx->sm_count);
+const MarchTile &tcym_lattice_march_of(tcym_lattice lat, bool links) {
+    MarchTile &t = lat->march[links];
+    if (t.threads == 0) t = step_tile(lat->g, lat->ctx->sm_count, lat->nc == 3, links);
     return t;
 }
 

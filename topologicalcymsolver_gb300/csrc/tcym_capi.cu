@@ -673,7 +673,7 @@ int tcym_run_steps(tcym_lattice lat, int mode, double dt, double gamma, double T
     for (int i = 0; i < nsteps; ++i) {
         StepCoef<double> c = tcym_coef(lat->a, mode, dt, gamma, T, seed, step0 + (uint64_t)i);
         const Tile &t = tcym_lattice_tile_of(lat);
-        const MarchTile &m = tcym_lattice_march_of(lat);
+        const MarchTile &m = tcym_lattice_march_of(lat, true);
         DISPATCH(lat->fmt, CK(L::step(lat->g, lat->U[lat->cur], lat->U[1 - lat->cur], lat->E, c, t, m, lat->stream)));
         lat->cur ^= 1;
         ++lat->steps_done;
@@ -739,7 +739,7 @@ static cudaError_t host_step_pipeline(tcym_lattice lat, const StepCoef<double> &
         if (err == cudaSuccess) err = cudaEventRecord(e, from);
         if (err == cudaSuccess) err = cudaStreamWaitEvent(to, e, 0);
     };
-    const MarchTile &mt = tcym_lattice_march_of(lat);
+    const MarchTile &mt = tcym_lattice_march_of(lat, true);
     const std::vector<int64_t> bounds = pipeline_bounds(N, P, C);
     pipeline_schedule(bounds, P, [&](int op, int64_t j) {
         if (err != cudaSuccess) return;
@@ -892,7 +892,7 @@ extern "C" int tcym_update_e(tcym_lattice lat, double dt) {
     tcym_ctx ctx = lat->ctx;
     cudaSetDevice(ctx->device);
     StepCoef<double> c = tcym_coef(lat->a, MODE_LEAPFROG, dt, 0, 0, 0, 0);
-    DISPATCH(lat->fmt, CK(L::update_e(lat->g, lat->U[lat->cur], lat->E, c, tcym_lattice_march_of(lat),
+    DISPATCH(lat->fmt, CK(L::update_e(lat->g, lat->U[lat->cur], lat->E, c, tcym_lattice_march_of(lat, false),
                                       lat->stream)));
     return TCYM_OK;
 }
@@ -934,13 +934,13 @@ extern "C" int tcym_flow(tcym_lattice lat, double dtau, int nsteps, int mode, in
         if (mode == TCYM_FLOW_SIMULTANEOUS) {
             // F into E and U' = exp(-i dtau F) U into the other buffer; U stays intact
             const Tile &t = tcym_lattice_tile_of(lat);
-            const MarchTile &m = tcym_lattice_march_of(lat);
+            const MarchTile &m = tcym_lattice_march_of(lat, true);
             DISPATCH(lat->fmt, CK(L::step(lat->g, lat->U[lat->cur], lat->U[1 - lat->cur], lat->E, c, t, m,
                                           lat->stream)));
         } else {
             if (calibrate)  // the force of the state before the sweep, for the trapezoid rule
                 DISPATCH(lat->fmt, CK(L::update_e(lat->g, lat->U[lat->cur], lat->E, c,
-                                                  tcym_lattice_march_of(lat), lat->stream)));
+                                                  tcym_lattice_march_of(lat, false), lat->stream)));
         }
         if (calibrate) {
             if ((r = tcym_reduce(lat, op, 0.0))) return r;

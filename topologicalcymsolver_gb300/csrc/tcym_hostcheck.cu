@@ -77,7 +77,7 @@ template <int FMT> struct H {
     // the per-site step as Launch::step_sites runs it
     static void sites(const Geom &g, const void *Uin, void *Uout, void *E, const StepCoef<T> &c, bool doU,
                       const SiteRange &r) {
-        const MarchTile t = step_tile(g, 152);
+        const MarchTile t = step_tile(g, 152, F::NA == 8, doU);
         if (!F::PAIRED && t.tx != 0) {
             march(g, Uin, Uout, E, c, doU, r, t);
             return;
@@ -415,8 +415,8 @@ int hc_march(int fmt, const int *n, const void *Uin, void *Uout, void *E, double
     HC_DISPATCH(fmt, HH::march(g, Uin, Uout, E, cast<HH::T>(c), true, SiteRange{0, g.nz, 0, g.V}, t));
     return 0;
 }
-// does the FP64 step of a lattice alone on `sms` multiprocessors go by sites?
-int hc_by_sites(const int *n, int sms) { return step_tile(geom(n), sms).tx == 0; }
+// does the FP64 step (links) or E update of a lattice alone on `sms` multiprocessors go by sites?
+int hc_by_sites(const int *n, int sms, int su3, int links) { return step_tile(geom(n), sms, su3 != 0, links != 0).tx == 0; }
 // the checkerboard tiles of a lattice, their shape in out[3]; returns whether an FP32 lattice
 // goes by pairs
 int hc_cb_tile(const int *n, int su3, int *out) {

@@ -63,7 +63,7 @@ struct tcym_lattice_s {
     cudaMemPool_t pool = nullptr;
     tcym::Tile tile{};   // block tiling of the paired step
     bool tile_chosen = false;
-    tcym::MarchTile march{};  // tiling of the FP64 step, alone (threads 0: not chosen yet)
+    tcym::MarchTile march[2]{};  // tiling of the FP64 E update, of the whole step (threads 0: not chosen yet)
     cudaStream_t side[2] = {nullptr, nullptr};  // pipelined host transfers (created with the staging)
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     // tcym_leapfrog_host's pipeline: streams for the host-to-device copies, their
@@ -102,7 +102,7 @@ cudaError_t tcym_lattice_alloc(tcym_lattice lat, void **p, size_t bytes);
 void tcym_lattice_free_mem(tcym_lattice lat, void *p);
 // the block tiling of lat's paired step, autotuned on first use (tcym_autotune.cu)
 const tcym::Tile &tcym_lattice_tile_of(tcym_lattice lat);
-// the tiling of lat's FP64 step, alone, by the rule of step_tile on first use
-const tcym::MarchTile &tcym_lattice_march_of(tcym_lattice lat);
+// the tiling of lat's FP64 step (links) or E update, by the rule of step_tile on first use
+const tcym::MarchTile &tcym_lattice_march_of(tcym_lattice lat, bool links);
 int tcym_run_steps(tcym_lattice lat, int mode, double dt, double gamma, double T, uint64_t seed, uint64_t step0,
                    int nsteps);

@@ -253,10 +253,12 @@ template <class F> struct March {
 };
 
 // The blocks' cost, in multiply-adds of whole warps: phase 1's plaquettes (310 for SU(3) in
-// FP64) and phase 2's links (572) of each plane, and the first plane's extra 2 S plaquettes with
-// their rotations (454).
+// FP64) and phase 2's links (572, of which E alone 350) of each plane, and the first plane's
+// extra 2 S plaquettes with their rotations (454).
 inline double march_warps(double n) { return 32.0 * (int)((n + 31) / 32); }
-inline double march_plane(int S, int halo) { return 310 * march_warps(3 * S + 2 * halo) + 572 * march_warps(3 * S); }
+inline double march_plane(int S, int halo, bool links) {
+    return 310 * march_warps(3 * S + 2 * halo) + (links ? 572 : 350) * march_warps(3 * S);
+}
 inline double march_first(int S) { return 454 * march_warps(2 * S); }
 // The tiling of a lattice that has the share `sms` of a device's multiprocessors, alone or among
 // others (an ensemble's members).  Its cost model is the work of the busiest multiprocessor, that
@@ -266,7 +268,7 @@ inline double march_first(int S) { return 454 * march_warps(2 * S); }
 // others 8 (the launch's tail).
 // Measured on GB300, FP64 per step, the rule's choice / 16 x 8 tiles of 8 planes: SU(3)
 // 16^3 43 / 678 us, 48^3 587 / 714 us; SU(2) 16^3 12 / 140 us.
-inline MarchTile march_tile(const Geom &g, double sms, bool alone, double *least = nullptr) {
+inline MarchTile march_tile(const Geom &g, double sms, bool alone, double *least = nullptr, bool links = true) {
     MarchTile best{};
     double cost = 0;
     for (int tx = g.nx < 16 ? g.nx : 16; tx > 0; --tx) {
@@ -279,13 +281,13 @@ inline MarchTile march_tile(const Geom &g, double sms, bool alone, double *least
             if ((g.ny + ny - 1) / ny != ty) continue;
             if (tx * ty < 16 && best.tx) break;
             const int halo = (tx == g.nx ? 0 : ty) + (ty == g.ny ? 0 : tx), S = tx * ty;
-            const double plane = march_plane(S, halo), first = march_first(S);
+            const double plane = march_plane(S, halo, links), first = march_first(S);
             double planes = 0, firsts = 0;  // of all tiles, ragged ones as they are
             for (int i = 0; i < 2; ++i)
                 for (int j = 0; j < 2; ++j) {
                     const int w = i ? g.nx - tx * (nx - 1) : tx, h = j ? g.ny - ty * (ny - 1) : ty;
                     const double n = (double)(i ? 1 : nx - 1) * (j ? 1 : ny - 1);
-                    planes += n * march_plane(w * h, (w == g.nx ? 0 : h) + (h == g.ny ? 0 : w));
+                    planes += n * march_plane(w * h, (w == g.nx ? 0 : h) + (h == g.ny ? 0 : w), links);
                     firsts += n * march_first(w * h);
                 }
             for (int zl = 1; zl <= g.nz && zl <= (alone ? 16 : 8); ++zl) {
@@ -307,16 +309,21 @@ inline MarchTile march_tile(const Geom &g, double sms, bool alone, double *least
     if (least) *least = cost;
     return best;
 }
-// The cost of a step by sites (site_step in blocks of 128), by the same measure.
-inline double sites_cost(int64_t V, double sms) { return 3150.0 * 128 * ceil((double)((V + 127) / 128) / sms); }
+// The cost of a step (links) or of the E update alone by sites (site_step in blocks of 128), by
+// the same measure.
+inline double sites_cost(int64_t V, double sms, bool links = true) {
+    return (links ? 3150.0 : 2400.0) * 128 * ceil((double)((V + 127) / 128) / sms);
+}
 // The step of a lattice alone: by tiles, or by sites (tx 0) where that costs less: extents that
 // the tiles fit badly, in waves of blocks that are nearly full.  By sites / by tiles, us a step
 // on GB300, SU(3) 18 x 28 x 34 109 / 119, 26^3 109 / 150, 33 x 20 x 27 109 / 148, 24^3 109 / 105,
-// 28^3 209 / 158, 48^3 619 / 587; SU(2) 26^3 25 / 33, 28^3 43 / 33.
-inline MarchTile step_tile(const Geom &g, double sms) {
+// 28^3 209 / 158, 48^3 619 / 587; SU(2) 26^3 25 / 33, 28^3 43 / 33.  E alone: SU(3) 32^3 162 / 165, 48^3
+// 476 / 450; of SU(2), where tiles must cost a tenth less (its few operations weigh their
+// barriers more), 32^3 33 / 36, 36^3 46 / 52, 40^3 60 / 58.
+inline MarchTile step_tile(const Geom &g, double sms, bool su3, bool links) {
     double least;
-    MarchTile t = march_tile(g, sms, true, &least);
-    if (sites_cost(g.V, sms) < least) t.tx = 0;
+    MarchTile t = march_tile(g, sms, true, &least, links);
+    if (sites_cost(g.V, sms, links) * (su3 || links ? 1 : 0.9) < least) t.tx = 0;
     return t;
 }
 
