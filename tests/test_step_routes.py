@@ -72,28 +72,36 @@ def test_gpu_routes(ctx, oracle_port, nc, shape):
 @pytest.mark.gpu
 @pytest.mark.parametrize("nc", [2, 3])
 # the same share by sites and by tiles in one ensemble, ragged ones, and one member alone
-@pytest.mark.parametrize("shapes", [[(8, 8, 8), (13, 13, 13), (16, 16, 16), (11, 5, 7), (32, 32, 32)], [(13, 13, 13)] * 12,
+@pytest.mark.parametrize("shapes", [[(8, 8, 8), (13, 13, 13), (16, 16, 16), (11, 5, 7), (32, 32, 32)], [(13, 13, 13)] * 12, [(17, 17, 17)] * 20,
                                     [(26, 26, 26)], [(24, 24, 24)]])
 def test_gpu_ensemble_routes(ctx, oracle_port, nc, shapes):
-    """FP64 members, whatever their routes, against the oracle: 1e-12 after six steps."""
+    """FP64 members, whatever their routes, bit for bit as the lattice alone, and against the oracle: 1e-12
+    after six steps."""
     import topologicalcymsolver_gb300 as tcym
 
     P = oracle_port[nc]
     ens, members = tcym.Ensemble(ctx), []
     for i, shape in enumerate(shapes):
         U, E = state(P, nc, shape)
-        lat = tcym.Lattice(ctx, nc, shape, tcym.FP64)
-        lat.upload(U, E)
+        lat, alone = (tcym.Lattice(ctx, nc, shape, tcym.FP64) for _ in range(2))
+        for x in (lat, alone):
+            x.upload(U, E)
+        if i % 2:
+            alone.langevin(0.02, 1.0, 0.6, 9, 3, 6)
+        else:
+            alone.leapfrog(0.05, 6)
         if i % 2:
             ens.add(lat, 0.02, tcym.DYN_LANGEVIN, 1.0, 0.6, 9, 3)
             P.langevin(shape, U, E, 0.02, 1.0, 0.6, 9, 3, 6)
         else:
             ens.add(lat, 0.05)
             P.leapfrog(shape, U, E, 0.05, 6)
-        members.append((lat, U, E))
+        members.append((lat, alone, U, E))
     ens.step(4)
     ens.step(2)
     ens.close()
-    for lat, U, E in members:
+    for lat, alone, U, E in members:
         assert max(np.abs(x - y).max() for x, y in zip(lat.download(), (U, E))) < 1e-12
+        assert all(np.array_equal(x, y) for x, y in zip(lat.download(), alone.download()))
         lat.close()
+        alone.close()

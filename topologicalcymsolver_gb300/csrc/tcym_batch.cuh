@@ -298,17 +298,19 @@ template <int FMT> struct LaunchBatch {
     static int site_items(const Geom &g, const MarchTile &m) {
         return m.tx == 0 ? grid_for(g.V, threads_for<FMT>()) : (int)march_blocks(m, g.nz);
     }
-    // the members [m0, m0 + n) stepped per site, or (threads > 0) by tiles, work items [item0, item1)
-    static cudaError_t sites(const Member<T> *members, int m0, int n, int item0, int item1, int k, int threads, size_t smem,
-                             cudaStream_t st) {
-        if constexpr (!Fmt<FMT>::PAIRED) {
-            if (threads > 0) {
-                k_march_batch<FMT><<<item1 - item0, threads, smem, st>>>(members + m0, n, item0, k);
-                return cudaGetLastError();
-            }
-        }
+    // the members [m0, m0 + n) stepped per site, work items [item0, item1)
+    static cudaError_t sites(const Member<T> *members, int m0, int n, int item0, int item1, int k, cudaStream_t st) {
         k_sites_batch<FMT><<<item1 - item0, threads_for<FMT>(), 0, st>>>(members + m0, n, item0, k);
         return cudaGetLastError();
+    }
+    // those stepped by tiles (FP64)
+    static cudaError_t march(const Member<T> *members, int m0, int n, int item0, int item1, int k, int threads,
+                             size_t smem, cudaStream_t st) {
+        if constexpr (!Fmt<FMT>::PAIRED) {
+            k_march_batch<FMT><<<item1 - item0, threads, smem, st>>>(members + m0, n, item0, k);
+            return cudaGetLastError();
+        }
+        return cudaErrorInvalidValue;
     }
     // the members [m0, m0 + n) of one coefficient class, work items [item0, item1),
     // stepped with their shared coefficients cu (k_step_batch_uniform)

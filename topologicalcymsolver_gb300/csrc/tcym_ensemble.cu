@@ -39,20 +39,14 @@ struct FmtGroup {
     void *d_members = nullptr;   // device Member<T> table
     size_t d_bytes = 0;
     std::vector<char> h_members; // host copy of the table
-    // step work items: those of the paired members first (idx is ordered so), then from
-    // pair_blocks on those of the members stepped per site, the first of them npaired
-    int total_blocks = 0, pair_blocks = 0, npaired = 0;
+    // step work items in two parts (idx is ordered so): FP32 members in pairs, then per site;
+    // FP64 members per site, then by tiles.  The second part begins at member nfirst and
+    // work item first_blocks.
+    int total_blocks = 0, first_blocks = 0, nfirst = 0;
     int march_threads = 0;       // threads and shared memory of the FP64 step's blocks (the largest)
     size_t march_smem = 0;
-    // FP64: the members' tilings and their costs by extents, for a number of sites in all; the
-    // members step by tiles, or all by sites
-    struct Tiling {
-        MarchTile tile;
-        double cost = 0;
-    };
-    int64_t sites = 0;
-    std::map<std::array<int, 3>, Tiling> march;
-    bool by_sites = false;
+    int64_t sites = 0;           // of all members
+    std::map<std::array<int, 3>, MarchTile> march;  // FP64: the tilings by extents, for that many sites
     int red_total = 0, red_grid = 0, red_offset = 0;
     bool tiled = false;          // some paired member is tiled: the kernel that reads every member's tiling
     // runs of members (idx is ordered by coefficients) that share the mode, force, staple
@@ -83,9 +77,8 @@ struct tcym_ensemble_s {
     tcym_ctx ctx = nullptr;
     std::vector<EnsMember> members;
     FmtGroup groups[4];
-    // chains of a chunk's steps: one a format, and one for the FP32 members of each group
-    // stepped per site beside paired ones (chain_of)
-    static constexpr int kChains = 6;
+    // chains of a chunk's steps: one a format and part of its members (chain_of)
+    static constexpr int kChains = 8;
     cudaStream_t st[kChains] = {};
     cudaEvent_t fork = nullptr, join[kChains] = {};
     double *partial = nullptr;
@@ -109,31 +102,24 @@ struct tcym_ensemble_s {
         if (e_ != cudaSuccess) return fail(ens->ctx, e_, #call);  \
     } while (0)
 
-// The tiling of an FP64 member: its share of the device is its share of the group's sites.
-static const FmtGroup::Tiling &member_march(FmtGroup &G, tcym_lattice lat) {
-    FmtGroup::Tiling &t = G.march[{lat->g.nx, lat->g.ny, lat->g.nz}];
-    if (t.tile.threads == 0)
-        t.tile = march_tile(lat->g, (double)lat->ctx->sm_count * (double)lat->g.V / (double)G.sites, lat->g.V == G.sites, &t.cost);
+// How an FP64 member steps: by sites where the lattice alone does (a member's arithmetic does not
+// depend on the others), else by tiles, of which any gives the same bits, for its share of the
+// device: its share of the group's sites.  All by sites / by the rule / by tiles as large as
+// if the members always filled the device, us a step on GB300, SU(3): one 8^3 119 / 42 / 327, 24 of
+// 8^3 120 / 110 / 328, 8 of 26^3 904 / 813 / 873, 24 of 32^3 4591 / 4067 / 4230, 16 of 16^3 to 48^3 3807 / 3388 /
+// 3380; SU(2): one 8^3 28 / 11 / 70, 24 of 32^3 926 / 792 / 802.  Some small odd lattices, of which
+// the device holds one or two waves of tiles, would be faster by sites: 24 of 13^3 344 / 463 / 525, of
+// 19^3 1018 / 1108 / 947 (alone: 119 / 44 and 119 / 64).
+static const MarchTile &member_march(FmtGroup &G, tcym_lattice lat) {
+    const MarchTile &alone = tcym_lattice_march_of(lat, true);
+    if (alone.tx == 0 || lat->g.V == G.sites) return alone;
+    MarchTile &t = G.march[{lat->g.nx, lat->g.ny, lat->g.nz}];
+    if (t.threads == 0) t = march_tile(lat->g, (double)lat->ctx->sm_count * (double)lat->g.V / (double)G.sites, false);
     return t;
 }
-// How FP64 members step: by tiles, or all by sites (one launch) unless tiles cost 5% less by
-// the rule's measure, which among others is off by a few per cent.  By sites before / the rule's
-// choice / blocks as large as if the members always filled the device, us a step on GB300, SU(3): one 8^3
-// 119 / 42 / 327, 24 of 13^3 344 / 311 / 525, 8 of 26^3 904 / 812 / 873, 24 of 32^3 4591 / 4116 / 4230,
-// 16 of 16^3 to 48^3 3807 / 3386 / 3380; SU(2): one 8^3 28 / 11 / 70, 24 of 32^3 926 / 775 / 802.
-static void choose_march(tcym_ensemble ens, FmtGroup &G) {
-    int64_t sites = 0;
-    for (int i : G.idx) sites += ens->members[i].lat->g.V;
-    if (sites != G.sites) G.march.clear();
-    G.sites = sites;
-    double tiles = 0, by_sites = 0;  // each member's estimate of the group's time, by its sites
-    for (int i : G.idx) {
-        const tcym_lattice L = ens->members[i].lat;
-        const double share = (double)L->g.V / (double)sites;
-        tiles += share * member_march(G, L).cost;
-        by_sites += share * sites_cost(L->g.V, ens->ctx->sm_count * share);
-    }
-    G.by_sites = by_sites * (G.idx.size() > 1 ? 0.95 : 1) < tiles;
+// Is a member stepped in its format's second part (FmtGroup)?
+static bool second_part(tcym_lattice lat) {
+    return lat->precision == TCYM_FP32 ? lat->g.nz % 2 != 0 : tcym_lattice_march_of(lat, true).tx != 0;
 }
 
 template <int FMT> static void fill_group(tcym_ensemble ens, FmtGroup &G, int sm_count) {
@@ -141,7 +127,7 @@ template <int FMT> static void fill_group(tcym_ensemble ens, FmtGroup &G, int sm
     std::vector<Member<T>> tab(G.idx.size());
     int blk = 0, red = 0;
     G.tiled = false;
-    G.pair_blocks = G.npaired = 0;
+    G.first_blocks = G.nfirst = 0;
     G.march_threads = 0;
     G.march_smem = 0;
     G.classes.clear();
@@ -173,15 +159,19 @@ template <int FMT> static void fill_group(tcym_ensemble ens, FmtGroup &G, int sm
             blk += (int)tile_blocks(L->g, m.tile);
             G.classes.back().m1 = (int)i + 1;
             G.classes.back().item1 = blk;
-            G.npaired = (int)i + 1;
-            G.pair_blocks = blk;
         } else {
-            if (!Fmt<FMT>::PAIRED && !G.by_sites) {
-                m.march = member_march(G, L).tile;
-                G.march_threads = std::max(G.march_threads, m.march.threads);
-                G.march_smem = std::max(G.march_smem, march_smem<Fmt<FMT>>(m.march));
+            if (!Fmt<FMT>::PAIRED) {
+                m.march = member_march(G, L);
+                if (m.march.tx != 0) {
+                    G.march_threads = std::max(G.march_threads, m.march.threads);
+                    G.march_smem = std::max(G.march_smem, march_smem<Fmt<FMT>>(m.march));
+                }
             }
             blk += LaunchBatch<FMT>::site_items(L->g, m.march);
+        }
+        if (!second_part(L)) {
+            G.nfirst = (int)i + 1;
+            G.first_blocks = blk;
         }
         m.red_begin = red;
         m.red_blocks = member_records(m.paired, L->g.V);
@@ -198,16 +188,20 @@ template <int FMT> static void fill_group(tcym_ensemble ens, FmtGroup &G, int sm
 static void fill_all(tcym_ensemble ens) {
     for (int f = 0; f < 4; ++f) ens->groups[f].idx.clear();
     for (size_t i = 0; i < ens->members.size(); ++i) ens->groups[ens->members[i].lat->fmt].idx.push_back((int)i);
-    // paired members first, and members with the same step coefficients next to each other
-    // (mode, dt, spacings decide them)
-    for (auto &G : ens->groups)
+    // by parts, and members with the same step coefficients next to each other (mode, dt,
+    // spacings decide them)
+    for (FmtGroup &G : ens->groups) {
+        int64_t sites = 0;
+        for (int i : G.idx) sites += ens->members[i].lat->g.V;
+        if (sites != G.sites) G.march.clear();
+        G.sites = sites;
         std::stable_sort(G.idx.begin(), G.idx.end(), [&](int x, int y) {
             const EnsMember &a = ens->members[x], &b = ens->members[y];
-            return std::make_tuple(a.lat->g.nz % 2, a.mode, a.dt, a.lat->a[0], a.lat->a[1], a.lat->a[2]) <
-                   std::make_tuple(b.lat->g.nz % 2, b.mode, b.dt, b.lat->a[0], b.lat->a[1], b.lat->a[2]);
+            return std::make_tuple(second_part(a.lat), a.mode, a.dt, a.lat->a[0], a.lat->a[1], a.lat->a[2]) <
+                   std::make_tuple(second_part(b.lat), b.mode, b.dt, b.lat->a[0], b.lat->a[1], b.lat->a[2]);
         });
+    }
     const int sm = ens->ctx->sm_count;
-    for (int f : {FMT_SU2_F64, FMT_SU3_F64}) choose_march(ens, ens->groups[f]);
     fill_group<FMT_SU2_F32>(ens, ens->groups[FMT_SU2_F32], sm);
     fill_group<FMT_SU2_F64>(ens, ens->groups[FMT_SU2_F64], sm);
     fill_group<FMT_SU3_F32>(ens, ens->groups[FMT_SU3_F32], sm);
@@ -287,38 +281,37 @@ static int upload_tables(tcym_ensemble ens) {
     return TCYM_OK;
 }
 
-// The members of a group step in two parts that do not wait for each other: the paired ones
-// (part 0), those stepped per site or by tiles (part 1).  One after the other on one chain,
-// a launch each, they took longer than one launch of a kernel for both kinds; us a step on GB300, one
-// launch / one chain / a chain each: an 8^3 and a 13^3 FP32 member SU(3) 13 / 25 / 13, SU(2) 8 / 15 / 9;
-// 4 each of 8^3, 13^3, 20^3, 33^3 SU(3) 66 / 69 / 63, SU(2) 24 / 30 / 23.
-static bool has_part(const FmtGroup &G, int part) { return part ? G.npaired < (int)G.idx.size() : G.npaired > 0; }
-static int chain_of(const FmtGroup &G, int f, int part) { return part == 1 && has_part(G, 0) ? 4 + f / 2 : f; }
+// The two parts of a group do not wait for each other.  One after the other on one chain,
+// a launch each, FP32 members in pairs and per site took longer than one launch of a kernel for
+// both kinds; us a step on GB300, one launch / one chain / a chain each: an 8^3 and a 13^3 member SU(3)
+// 13 / 25 / 13, SU(2) 8 / 15 / 9; 4 each of 8^3, 13^3, 20^3, 33^3 SU(3) 66 / 69 / 63, SU(2) 24 / 30 / 23.
+static bool has_part(const FmtGroup &G, int part) { return part ? G.nfirst < (int)G.idx.size() : G.nfirst > 0; }
+static int chain_of(const FmtGroup &G, int f, int part) { return part == 1 && has_part(G, 0) ? 4 + f : f; }
 template <int FMT> static cudaError_t launch_group_step(tcym_ensemble ens, int f, int part, int k, cudaStream_t s) {
     using T = typename Fmt<FMT>::T;
     const FmtGroup &G = ens->groups[f];
     const Member<T> *table = static_cast<const Member<T> *>(G.d_members);
-    if (part == 1)
-        return LaunchBatch<FMT>::sites(table, G.npaired, (int)G.idx.size() - G.npaired, G.pair_blocks, G.total_blocks, k,
-                                       G.march_threads, G.march_smem, s);
-    cudaError_t e = cudaSuccess;
+    const int n = (int)G.idx.size() - G.nfirst;
     if constexpr (Fmt<FMT>::PAIRED) {
-        if (G.tiled) {
-            e = LaunchBatch<FMT>::step(table, G.npaired, G.pair_blocks, k, s);
-        } else {
-            for (const FmtGroup::Class &c : G.classes)
-                if (e == cudaSuccess)
-                    e = LaunchBatch<FMT>::step_uniform(table, c.m0, c.m1 - c.m0, c.item0, c.item1, k, c.coef, s);
-        }
+        if (part == 1) return LaunchBatch<FMT>::sites(table, G.nfirst, n, G.first_blocks, G.total_blocks, k, s);
+        if (G.tiled) return LaunchBatch<FMT>::step(table, G.nfirst, G.first_blocks, k, s);
+        cudaError_t e = cudaSuccess;
+        for (const FmtGroup::Class &c : G.classes)
+            if (e == cudaSuccess)
+                e = LaunchBatch<FMT>::step_uniform(table, c.m0, c.m1 - c.m0, c.item0, c.item1, k, c.coef, s);
+        return e;
+    } else {
+        if (part == 0) return LaunchBatch<FMT>::sites(table, 0, G.nfirst, 0, G.first_blocks, k, s);
+        return LaunchBatch<FMT>::march(table, G.nfirst, n, G.first_blocks, G.total_blocks, k, G.march_threads,
+                                       G.march_smem, s);
     }
-    return e;
 }
 
 // Does format f step by persistent K-step launches?
 static bool persistent_format(tcym_ensemble ens, int f) {
     const FmtGroup &G = ens->groups[f];
     return ens->persistent && (f == FMT_SU2_F32 || f == FMT_SU3_F32) && !G.tiled && !G.idx.empty() &&
-           G.npaired == (int)G.idx.size();
+           G.nfirst == (int)G.idx.size();
 }
 
 // Schedules and control words of the persistent launches for chunks of nsteps
