@@ -154,7 +154,7 @@ __device__ __forceinline__ void march_block(const Geom &g, const void *Uin, void
         __syncthreads();
     }
 }
-// Resident blocks of kMarchThreads per SM: two at 128 registers for SU(3) (FP64 keeps 72
+// Resident blocks of kMarchThreads per SM: two at 128 registers for SU(3) (FP64 keeps 24
 // bytes of spills; at one block, 255 registers, the FP64 unit is not kept busy), three for SU(2).
 template <int FMT> constexpr int march_min_blocks() { return Fmt<FMT>::NA == 8 ? 2 : 3; }
 // DO_U: the whole step, the new links into Uout; else the E update alone
