@@ -368,6 +368,52 @@ Geom geom(const int *n) { return Geom{n[0], n[1], n[2], (int64_t)n[0] * n[1] * n
         default: return -1;                                     \
     }
 
+// E.E and (E + E').B / 4, summed over `count` pairs at a time as a thread of the device sums
+// them, of n pairs' components e[pair][component][lane]
+template <int NA> void pair_sums(int64_t n, int64_t count, const float *e, const float *et, const float *b, double *out) {
+    for (int64_t i0 = 0; i0 < n; i0 += count) {
+        FieldSums<f2, NA> sums;
+        for (int again = 0; again < 2; ++again) {
+            for (int64_t i = i0; i < i0 + count && i < n; ++i) {
+                f2 x[NA], y[NA], z[NA];
+                for (int a = 0; a < NA; ++a) {
+                    const int64_t j = 2 * (i * NA + a);
+                    x[a] = f2(e[j], e[j + 1]); y[a] = f2(et[j], et[j + 1]); z[a] = f2(b[j], b[j + 1]);
+                }
+                if (again) sums.add64(x, y, z);
+                else sums.add(x, y, z);
+            }
+            if (again || sums.exact()) break;
+        }
+        out[2 * (i0 / count)] = sums.sq;
+        out[2 * (i0 / count) + 1] = sums.dot;
+    }
+}
+// sum of squares, largest component and largest magnitude (from 0 on) of n pairs' violations,
+// each the sum of k FP32 terms t[pair][component][term][lane]
+template <int NA> void violation_sums(int64_t n, int64_t count, int k, const float *t, double *out) {
+    for (int64_t i0 = 0; i0 < n; i0 += count) {
+        ViolationSums<f2, NA> sums;
+        for (int again = 0; again < 2; ++again) {
+            for (int64_t i = i0; i < i0 + count && i < n; ++i) {
+                WideSum<f2> s[NA];
+                for (int a = 0; a < NA; ++a) {
+                    s[a] = WideSum<f2>(f2(0.0));
+                    for (int j = 0; j < k; ++j) {
+                        const float *x = t + 2 * ((i * NA + a) * k + j);
+                        s[a].add(f2(x[0], x[1]));
+                    }
+                }
+                if (again) sums.add64(s);
+                else sums.add(s);
+            }
+            if (again || sums.exact()) break;
+        }
+        double *o = out + 3 * (i0 / count);
+        o[0] = sums.sq; o[1] = sums.most; o[2] = sums.mag;
+    }
+}
+
 }  // namespace
 
 extern "C" {
@@ -441,53 +487,7 @@ int hc_edotb_pair(int fmt, const int *n, const void *U, const void *E, double *o
     HC_DISPATCH(fmt, ok = HH::edotb_pair(g, U, E, out));
     return ok;
 }
-// E.E and (E + E').B / 4, summed over `count` pairs at a time as a thread of the device sums
-// them, of n pairs' components e[pair][component][lane]
-}  // extern "C"
-template <int NA> static void pair_sums(int64_t n, int64_t count, const float *e, const float *et, const float *b, double *out) {
-    for (int64_t i0 = 0; i0 < n; i0 += count) {
-        FieldSums<f2, NA> sums;
-        for (int again = 0; again < 2; ++again) {
-            for (int64_t i = i0; i < i0 + count && i < n; ++i) {
-                f2 x[NA], y[NA], z[NA];
-                for (int a = 0; a < NA; ++a) {
-                    const int64_t j = 2 * (i * NA + a);
-                    x[a] = f2(e[j], e[j + 1]); y[a] = f2(et[j], et[j + 1]); z[a] = f2(b[j], b[j + 1]);
-                }
-                if (again) sums.add64(x, y, z);
-                else sums.add(x, y, z);
-            }
-            if (again || sums.exact()) break;
-        }
-        out[2 * (i0 / count)] = sums.sq;
-        out[2 * (i0 / count) + 1] = sums.dot;
-    }
-}
-// sum of squares, largest component and largest magnitude (from 0 on) of n pairs' violations,
-// each the sum of k FP32 terms t[pair][component][term][lane]
-template <int NA> static void violation_sums(int64_t n, int64_t count, int k, const float *t, double *out) {
-    for (int64_t i0 = 0; i0 < n; i0 += count) {
-        ViolationSums<f2, NA> sums;
-        for (int again = 0; again < 2; ++again) {
-            for (int64_t i = i0; i < i0 + count && i < n; ++i) {
-                WideSum<f2> s[NA];
-                for (int a = 0; a < NA; ++a) {
-                    s[a] = WideSum<f2>(f2(0.0));
-                    for (int j = 0; j < k; ++j) {
-                        const float *x = t + 2 * ((i * NA + a) * k + j);
-                        s[a].add(f2(x[0], x[1]));
-                    }
-                }
-                if (again) sums.add64(s);
-                else sums.add(s);
-            }
-            if (again || sums.exact()) break;
-        }
-        double *o = out + 3 * (i0 / count);
-        o[0] = sums.sq; o[1] = sums.most; o[2] = sums.mag;
-    }
-}
-extern "C" {
+// n pairs in groups of `count` (pair_sums, violation_sums)
 int hc_pair_sums(int na, int64_t n, int64_t count, const float *e, const float *et, const float *b, double *out) {
     if (na == 3) pair_sums<3>(n, count, e, et, b, out);
     else pair_sums<8>(n, count, e, et, b, out);
