@@ -281,7 +281,8 @@ template <class T> struct SU2 {
     }
     // Re tr(1 - a b^dag)
     static TCYM_HD T retr_one_minus_dag(const Mat &a, const Mat &b) {
-        return T(2) * (T(1) - fma(a.q[0], b.q[0], fma(a.q[1], b.q[1], fma(a.q[2], b.q[2], a.q[3] * b.q[3]))));
+        // from 1 down: near the identity what is left after the first product is small
+        return T(2) * fma(-a.q[0], b.q[0], fma(-a.q[1], b.q[1], fma(-a.q[2], b.q[2], fma(-a.q[3], b.q[3], T(1)))));
     }
     // p = proj(a b^dag) / kLoopScale (a, b: a plaquette's two halves): the vector part of the
     // product, its sign left to the scale
